@@ -11,13 +11,24 @@
 // Every touched unpeeled item moves to bucket max(count, k).  Buckets are 64-bit (the
 // reference's are 32-bit, ligra/bucket.h:15-16, exact only below 2^32 - 1).
 //
-// Device design: one cooperative persistent kernel runs all rounds.  Phases are separated by
-// a grid barrier whose wait is bounded in time (on expiry the kernel records PB_ETIMEOUT and
-// returns; the context stays usable).  Buckets are kept as a near/far split: the near list
-// holds the unpeeled items whose bucket lies below a window bound; each round scans only the
-// near list (frontier extraction fused with the next minimum), and the window advances (one
-// pass over the alive list, a log2 histogram of distances to the minimum) when the near list
-// runs dry.  Frontier items with little work run one per warp; heavy ones one per CTA.
+// Device design: one cooperative persistent kernel runs all rounds.  A round has two phases, each
+// closed by one grid barrier whose wait is bounded in time (on expiry the kernel records
+// PB_ETIMEOUT and returns; the context stays usable):
+//   F: the near list (the unpeeled items whose bucket lies below a window bound) is scanned; the
+//      items of bucket k form the frontier, the least other bucket seeds the next minimum;
+//   P: the frontier is processed.  The decrement that lowers an item's count also feeds the next
+//      minimum and, when it is the one that crosses the window bound, adds the item to the near
+//      list, so no pass over touched items follows.
+// An item's bucket is max(count, k) (k: the last round's bucket), so it needs no storage.  The
+// window advances (one pass over the alive list, a log2 histogram of distances to the minimum)
+// when the near list runs dry.
+//
+// What bounds it: most rounds are light (a few items, 2^12 .. 2^17 probes), so a round's time is
+// its chain of dependent L2 round trips (about 0.35 us each) plus the barriers, not its probes.
+// The phases are therefore cut to short chains: probes that hit go to a queue of the warp and are
+// charged 32 at a time (one chain per 32 hits instead of one per probe step with a hit), a
+// barrier is one release add and one acquire poll, and per-round statistics stay in shared
+// memory.
 #include <algorithm>
 #include <functional>
 #include <memory>
@@ -33,45 +44,58 @@ namespace pb {
 namespace {
 
 constexpr int kPT = 512;
-constexpr int kWarpSlots = 512;    // per-warp table slots (keys, values, hit counters: 6 KiB)
-constexpr int kBlockSlots = 8192;  // per-CTA table slots (96 KiB), shares memory with warp tables
+constexpr int kPW = kPT / 32;
+// Shared-memory table area of a CTA, in 32-bit words (84 KiB; with the fixed part two CTAs fit an
+// SM).  Wing: keys, values and hit counters (three equal parts, per CTA or per warp); tip: keys
+// and values (power-of-two parts).
+constexpr uint32_t kPoolWords = 21504;
+constexpr uint32_t kWingSlots = kPoolWords / 3;            // 7168 slots, probe sets up to kWingSet
+constexpr uint32_t kWingSet = 4096;
+constexpr uint32_t kWingWarpSlots = kPoolWords / 3 / kPW;  // 448 slots, probe sets up to kWingWarpSet
+constexpr uint32_t kWingWarpSet = 256;
+constexpr uint32_t kTipSlots = 8192;      // two-hop lists of up to 4096 wedges
+constexpr uint32_t kTipWarpSlots = 512;   // two-hop lists of up to 256 wedges
 constexpr uint32_t kEmpty = 0xFFFFFFFFu;
 constexpr unsigned long long kInf = ~0ull;
-constexpr uint8_t ALIVE = 0, ACTIVE = 1, PEELED = 2;
+// Item states.  The frontier of round r is marked 1 + (r & 1); the next round turns the marks
+// into PEELED, so a mark never outlives the round after its own.
+constexpr uint8_t ALIVE = 0, PEELED = 3;
 constexpr unsigned ERR_TIMEOUT = 1u;
 constexpr unsigned long long kBarrierTimeoutNs = 60ull * 1000000000ull;  // 60 s per wait
+constexpr unsigned long long kBarErr = 1ull << 63;  // barrier word: some wait or invariant failed
 
 struct Ctl {
   unsigned long long nm[2];       // next minimum per round parity
   unsigned long long k_lo, win_hi;
   unsigned long long rounds, work;
-  unsigned flen_small[2], flen_big[2], flen_huge[2];
-  unsigned tlen[2];
+  // Frontier lists per round parity: items in the high word, their work units in the low word, so
+  // that one add gives an item its position and its first unit (units ascend with positions).
+  unsigned long long fsmall[2], fbig[2], fhuge[2];
   unsigned cur_small[2], cur_big[2];
-  unsigned units;  // work units (chunks of CTA-level items) of the current round
-  unsigned long long round_cost[2];  // summed cost estimate of the round's CTA-level items
-  unsigned near_len;
-  unsigned alive;                 // unpeeled items
+  unsigned long long round_est[2];   // summed cost estimate of the round (range mode, tracing)
+  unsigned long long near_len;
+  unsigned near_done;             // range mode: near items already taken (kept across launches)
+  unsigned alive;                 // unpeeled items (written when the kernel ends or pauses)
   unsigned alen[2];               // alive list lengths
   unsigned hist[66];
-  unsigned bar_count, bar_gen, err;
+  unsigned err;
+  unsigned long long bar;       // arrivals at grid barriers since the control block was made
+  unsigned long long bar_base;  // bar when the current launch began
   unsigned long long round;   // next round to run (kept across launches)
   unsigned alist_cur;         // current alive list (kept across launches)
   unsigned started;           // alive list initialised
   unsigned alive_at_compact;  // unpeeled items when the lists were last compacted
   unsigned min_gain;          // pause for compaction once this many more items are peeled
   // Instrumentation (CTA 0): device time per phase and work counters.
-  unsigned long long t_last, phase_ns[4];  // advance, F, P, U
+  unsigned trace;                          // phase times are kept
+  unsigned long long phase_ns[3];          // advance, F, P
   unsigned long long barrier_timeout_ns;   // bound of every grid-barrier wait
   unsigned test_skip_arrival;              // test hook: CTA 0 never arrives at grid barriers
-  unsigned long long scanned, touched_total, n_small, n_big, n_huge, advances;
+  unsigned long long scanned, n_small, n_big, n_huge, advances;
   // Phase-P time of the rounds binned by log2 of their estimated work (frontier cost sum).
-  unsigned long long round_est[2];
   unsigned long long pbin_ns[42], pbin_rounds[42], pbin_est[42];
   // Near-window size: at least near_min items, or alive / near_div.
   unsigned near_min, near_div;
-  // Barriers of CTA groups that process heavy tip items concurrently.
-  unsigned gbar_count[32], gbar_gen[32];
   // Range mode (the coarse pass of the two-phase peel): each window is one partition, its
   // frontier every unpeeled item whose count is below the window bound, repeated until no
   // unpeeled item is below it.  The bound is chosen so that the window holds about
@@ -84,15 +108,15 @@ struct Ctl {
   unsigned long long part_done, part_used, part_ratio_q;
   unsigned long long whist[66];    // estimated work per log2 distance bin
   unsigned long long wsub[256];    // estimated work per linear sub-bin of the chosen octave
-  // Wing items per probe structure (warp table, CTA table, dense markers, grid) and their probes;
+  // Wing items per probe structure (warp table, CTA table, dense markers) and their probes;
   // probes that walked the probe set against a binary search (the reverse direction).
-  unsigned long long mode_items[4], mode_work[4], rev_work;
-  unsigned prev_items;  // frontier items of the previous round
-  unsigned wunits;      // warp units of the current round (global prefix only)
+  unsigned long long mode_items[3], mode_work[3], rev_work;
 };
 constexpr unsigned kMaxGroups = 32;
+// Pairs per CTA below which tip_items_flat uses fewer CTAs.
+constexpr unsigned long long kFlatPairs = 1024;
 // Device memory for grid-shared dense counters (one n-sized slice per concurrent heavy tip
-// item group or per fine-pass instance with a CTA range of its own).
+// item or per fine-pass instance with a CTA range of its own).
 constexpr int64_t kGsharedBudget = int64_t(2) << 30;
 
 
@@ -110,27 +134,25 @@ struct Lists {
   const uint32_t* u_of;       // output edge index -> count-side vertex (wing only)
   const int64_t* S;      // per count-side vertex then per centre vertex: sum of neighbour degrees (wing)
   const int64_t* wk;     // per count-side vertex: two-hop wedges sum(deg(v) - 1) (tip)
+  const uint32_t* info;  // per edge (wing): how its item is peeled (wing_info_kernel)
   int64_t nK, nC;
 };
+// Lists::info: work units of the item, whether it runs on warps, whether it walks from the centre.
+constexpr uint32_t kInfoUnits = 0x1FFFu, kInfoSmall = 1u << 13, kInfoFromV = 1u << 31;
 
 struct Work {
-  int64_t* D;        // buckets (final: tip / wing numbers)
+  int64_t* D;        // final tip / wing numbers (range mode: the counts when the partition opened)
   int64_t* cnt;      // butterfly counts
   uint8_t* state;
-  uint8_t* in_near;
-  uint32_t* touched;
   uint32_t* alist[2];
   uint32_t* near;
-  uint32_t* fsmall[2];
-  uint32_t* fbig[2];
-  uint32_t* fchunks[2];  // work units of each CTA-level item (parallel to fbig)
-  uint32_t* uprefix;     // exclusive prefix of fchunks for the current round (N + 1)
-  uint32_t* fwchunks[2]; // warp units of each warp-level wing item (parallel to fsmall)
-  uint32_t* wprefix;     // exclusive prefix of fwchunks (N + 1)
-  uint32_t* fhuge[2];
-  uint32_t* tlist[2];
-  uint32_t* gshared;   // grid-shared dense counters / probe markers for huge items (zeroed);
-                       // tip: ngroups slices of gshared_stride counters, one per CTA group
+  // Frontier of a round, per parity: warp-level items from the front, CTA-level items from the
+  // back (an item is in one of them).  What phase P needs of an item is written once by phase F:
+  // wing: {edge, probe vertex a | from_v << 31, first-level vertex b, first unit}; tip: {vertex,
+  // its list start, its degree, two-hop list length (saturated)}.
+  uint4* front[2];
+  uint4* fhuge[2];       // tip only
+  uint32_t* gshared;     // tip: ngroups slices of gshared_stride grid-shared dense counters (zeroed)
   int64_t gshared_stride;
   unsigned ngroups;
   uint32_t* gscratch;  // per-CTA dense scratch (dense counters / probe markers)
@@ -158,6 +180,24 @@ __shared__ unsigned s_vb, s_vg;
 __device__ __forceinline__ unsigned vblock() { return s_vb; }
 __device__ __forceinline__ unsigned vgrid() { return s_vg; }
 
+// Per-CTA copies of the round's parameters (set at the start of every round) and of the
+// instance's barrier state.
+__shared__ unsigned long long s_win_hi;
+__shared__ long long s_k;
+__shared__ unsigned s_act;  // state mark of this round's frontier
+__shared__ unsigned long long s_bar_target, s_bar_timeout;
+__shared__ unsigned s_err, s_skip_arrival;
+
+// Statistics of CTA 0 (phase times, round counts) and of every CTA (wing probes), written to the
+// control block when the instance ends or pauses.
+struct Stats {
+  unsigned long long t_last, phase_ns[3];
+  unsigned long long pbin_ns[42], pbin_rounds[42], pbin_est[42];
+  unsigned long long rounds, scanned, n_small, n_big, n_huge, advances, part_done;
+  unsigned long long mode_items[3], mode_work[3], rev_work;
+};
+__shared__ Stats s_st;
+
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -166,187 +206,205 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
 
 // CTA 0 charges the time since its previous mark to phase `ph` (called right after barriers).
 // Phase P is also binned by log2 of the round's estimated work (est).
-__device__ __forceinline__ void phase_mark(Ctl* ctl, int ph, unsigned long long est = 0) {
-  if (vblock() == 0 && threadIdx.x == 0) {
+__device__ __forceinline__ void phase_mark(bool trace, int ph, unsigned long long est = 0) {
+  if (trace && threadIdx.x == 0) {
     const unsigned long long now = globaltimer_ns();
-    if (ctl->t_last) {
-      ctl->phase_ns[ph] += now - ctl->t_last;
+    if (s_st.t_last) {
+      s_st.phase_ns[ph] += now - s_st.t_last;
       if (ph == 2) {
         const int b = est ? min(41, 64 - __clzll(est)) : 0;
-        ctl->pbin_ns[b] += now - ctl->t_last;
-        ctl->pbin_rounds[b] += 1;
-        ctl->pbin_est[b] += est;
+        s_st.pbin_ns[b] += now - s_st.t_last;
+        s_st.pbin_rounds[b] += 1;
+        s_st.pbin_est[b] += est;
       }
     }
-    ctl->t_last = now;
+    s_st.t_last = now;
   }
 }
+
+// Records an error and makes every barrier of the instance fail from here on.
+__device__ __noinline__ void raise_err(Ctl* ctl, unsigned code) {
+  atomicOr(&ctl->err, code);
+  atomicOr(&ctl->bar, kBarErr);
+  *(volatile unsigned*)&s_err = 1u;
+}
+
+// Control-block words every thread needs after a barrier: read by one warp per CTA (thousands of
+// warps reading one address queue up at its L2 slice) and handed on through shared memory.
+__shared__ unsigned long long s_words[3];
 
 // Barrier over the CTAs of one peel instance (a cooperative launch keeps every CTA co-resident).
-// Bounded: a wait longer than the control block's timeout sets ERR_TIMEOUT and returns false.
-__device__ bool grid_barrier(Ctl* ctl) {
-  __shared__ int ok;
-  if (vgrid() == 1) {  // one CTA: a block barrier orders its global memory accesses too
-    __syncthreads();
-    return *(volatile unsigned*)&ctl->err == 0;
-  }
+// Arrivals are counted in one 64-bit word that is never reset: a barrier is complete when the
+// word reaches the CTA count times the number of barriers so far, so it costs one release add and
+// the acquire polls of the word (1.4 us on 148 CTAs).  Bounded: a wait longer than the control block's
+// timeout sets ERR_TIMEOUT and returns false.
+// w0 .. w2: control-block words that land in s_words (null: none).
+__device__ __forceinline__ bool grid_barrier(Ctl* ctl, const unsigned long long* w0 = nullptr,
+                                             const unsigned long long* w1 = nullptr,
+                                             const unsigned long long* w2 = nullptr) {
+  int bad = 0;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    volatile unsigned* vgen = &ctl->bar_gen;
-    const unsigned gen = *vgen;
-    __threadfence();
-    // (test hook) without CTA 0's arrival no CTA is last, so every wait runs out.
-    const unsigned arrived =
-        (vblock() == 0 && *(volatile unsigned*)&ctl->test_skip_arrival) ? 0xFFFFFFFFu : atomicAdd(&ctl->bar_count, 1u);
-    ok = 1;
-    if (arrived == vgrid() - 1) {
-      atomicExch(&ctl->bar_count, 0u);
-      __threadfence();
-      atomicAdd(&ctl->bar_gen, 1u);
-    } else {
-      const unsigned long long t0 = globaltimer_ns();
-      while (*vgen == gen) {
-        if (*(volatile unsigned*)&ctl->err) { ok = 0; break; }
-        if (globaltimer_ns() - t0 > ctl->barrier_timeout_ns) {
-          atomicOr(&ctl->err, ERR_TIMEOUT);
-          ok = 0;
-          break;
+  if (threadIdx.x < 32) {
+    if (vgrid() == 1) {  // one CTA: a block barrier orders its global memory accesses too
+      bad = (int)*(volatile unsigned*)&s_err;
+    } else if (threadIdx.x == 0) {
+      const unsigned long long target = s_bar_target + vgrid();
+      s_bar_target = target;
+      // (test hook) without CTA 0's arrivals no barrier completes, so every wait runs out.
+      if (!s_skip_arrival)
+        asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&ctl->bar), "l"(1ull) : "memory");
+      unsigned long long t0 = 0, seen;
+      unsigned polls = 0;
+      while (true) {
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(seen) : "l"(&ctl->bar) : "memory");
+        if (seen >= target) break;  // the error bit is above every count
+        if ((++polls & 63u) == 0) {
+          const unsigned long long now = globaltimer_ns();
+          if (!t0) t0 = now;
+          else if (now - t0 > s_bar_timeout) raise_err(ctl, ERR_TIMEOUT);
         }
       }
+      bad = (seen & kBarErr) != 0;
     }
-    __threadfence();
-    if (*(volatile unsigned*)&ctl->err) ok = 0;
-  }
-  __syncthreads();
-  return ok != 0;
-}
-
-// Barrier over `size` CTAs of a group (slot: the group's counters).  Bounded like grid_barrier.
-__device__ bool group_barrier(Ctl* ctl, unsigned slot, unsigned size) {
-  __shared__ int gok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    volatile unsigned* vgen = &ctl->gbar_gen[slot];
-    const unsigned gen = *vgen;
-    __threadfence();
-    const unsigned arrived = atomicAdd(&ctl->gbar_count[slot], 1u);
-    gok = 1;
-    if (arrived == size - 1) {
-      atomicExch(&ctl->gbar_count[slot], 0u);
-      __threadfence();
-      atomicAdd(&ctl->gbar_gen[slot], 1u);
-    } else {
-      const unsigned long long t0 = globaltimer_ns();
-      while (*vgen == gen) {
-        if (*(volatile unsigned*)&ctl->err) { gok = 0; break; }
-        if (globaltimer_ns() - t0 > ctl->barrier_timeout_ns) {
-          atomicOr(&ctl->err, ERR_TIMEOUT);
-          gok = 0;
-          break;
-        }
-      }
+    if (w0) {
+      __syncwarp();
+      const unsigned long long* w = threadIdx.x == 0 ? w0 : (threadIdx.x == 1 ? w1 : w2);
+      if (threadIdx.x < 3 && w) s_words[threadIdx.x] = *(const volatile unsigned long long*)w;
     }
-    __threadfence();
-    if (*(volatile unsigned*)&ctl->err) gok = 0;
   }
-  __syncthreads();
-  return gok != 0;
+  return __syncthreads_or(bad) == 0;
 }
 
-// Fibonacci hashing: the high bits of key * 2^32/phi, folded into the table size.
-__device__ __forceinline__ uint32_t hslot(uint32_t key, uint32_t mask) {
-  return __umulhi(key * 0x9E3779B1u, mask + 1u) & mask;
-}
+// Fibonacci hashing: the high bits of key * 2^32/phi, folded into the table size (any size).
+__device__ __forceinline__ uint32_t hslot(uint32_t key, uint32_t size) { return __umulhi(key * 0x9E3779B1u, size); }
 
-// Tables are sized to at least twice their key count, so probe sequences stay shorter than
-// the table; the bounds turn a broken invariant into a recorded error, not an endless loop.
+// Tables hold at most 4/7 of their slots, so probe sequences stay shorter than the table; the
+// bounds turn a broken invariant into a recorded error, not an endless loop.
 constexpr unsigned ERR_TABLE = 2u;
 
-__device__ __forceinline__ void t_add(uint32_t* keys, uint32_t* vals, uint32_t mask, uint32_t key, Ctl* ctl) {
-  uint32_t h = hslot(key, mask);
-  for (uint32_t probes = 0; probes <= mask; ++probes) {
+__device__ __forceinline__ void t_add(uint32_t* keys, uint32_t* vals, uint32_t size, uint32_t key, Ctl* ctl) {
+  uint32_t h = hslot(key, size);
+  for (uint32_t probes = 0; probes < size; ++probes) {
     uint32_t k = keys[h];
     if (k == key) { atomicAdd(&vals[h], 1u); return; }
     if (k == kEmpty) {
       uint32_t prev = atomicCAS(&keys[h], kEmpty, key);
       if (prev == kEmpty || prev == key) { atomicAdd(&vals[h], 1u); return; }
     }
-    h = (h + 1) & mask;
+    h = h + 1 == size ? 0u : h + 1;
   }
-  atomicOr(&ctl->err, ERR_TABLE);
+  raise_err(ctl, ERR_TABLE);
 }
 
 // Unique-key insert of (key, val).
-__device__ __forceinline__ void t_put(uint32_t* keys, uint32_t* vals, uint32_t mask, uint32_t key, uint32_t val,
+__device__ __forceinline__ void t_put(uint32_t* keys, uint32_t* vals, uint32_t size, uint32_t key, uint32_t val,
                                       Ctl* ctl) {
-  uint32_t h = hslot(key, mask);
-  for (uint32_t probes = 0; probes <= mask; ++probes) {
+  uint32_t h = hslot(key, size);
+  for (uint32_t probes = 0; probes < size; ++probes) {
     uint32_t prev = atomicCAS(&keys[h], kEmpty, key);
     if (prev == kEmpty) { vals[h] = val; return; }
-    h = (h + 1) & mask;
+    h = h + 1 == size ? 0u : h + 1;
   }
-  atomicOr(&ctl->err, ERR_TABLE);
+  raise_err(ctl, ERR_TABLE);
 }
 
 // Slot of key, or kEmpty when absent.
-__device__ __forceinline__ uint32_t t_slot(const uint32_t* keys, uint32_t mask, uint32_t key) {
-  uint32_t h = hslot(key, mask);
-  for (uint32_t probes = 0; probes <= mask; ++probes) {
+__device__ __forceinline__ uint32_t t_slot(const uint32_t* keys, uint32_t size, uint32_t key) {
+  uint32_t h = hslot(key, size);
+  for (uint32_t probes = 0; probes < size; ++probes) {
     const uint32_t k = keys[h];
     if (k == key) return h;
     if (k == kEmpty) return kEmpty;
-    h = (h + 1) & mask;
+    h = h + 1 == size ? 0u : h + 1;
   }
   return kEmpty;
 }
 
 __device__ __forceinline__ uint32_t np2(uint32_t x) { return x <= 1 ? 1u : 1u << (32 - __clz(x - 1)); }
 
-constexpr uint32_t kLocalUnits = 2048;  // rounds with at most this many CTA-level items lay
-                                        // out their work units in every CTA's shared memory
+constexpr uint32_t kQueue = 64;         // entries of a warp's queue (31 left over + 32 pushed)
 struct Shared {
+  unsigned long long red[32];
+  unsigned long long queue[kPW][kQueue];
   uint32_t incl[kPT];
   uint32_t sb[kPT];
   uint32_t len[kPT];
-  uint32_t cursor;
+  uint32_t acc[kPT];  // butterflies found through each first-level position of the chunk
+  uint4 flat[32];     // tip_items_flat: the items of the wave
   uint32_t scan[32];
-  unsigned long long red[32];
   uint32_t item;
   unsigned hist[66];
-  uint32_t uprefix[kLocalUnits + 1];
 };
 
 // A second-level position with this bit set walks the probe set instead (the reverse direction of
 // a wing intersection); list positions stay below 2^31 (2m <= 2^32).
 constexpr uint32_t kRevFlag = 0x80000000u;
 
+// A queue of 64-bit entries private to one warp.  push() is called by all lanes; once 32 entries
+// are waiting the warp handles them with all lanes at work: f(entry) per lane.  n is the same in
+// every lane.
+struct WarpQueue {
+  unsigned long long* buf;
+  unsigned n;
+  template <class F>
+  __device__ __forceinline__ void push(bool have, unsigned long long x, F&& f) {
+    const unsigned bal = __ballot_sync(0xffffffffu, have);
+    if (!bal) return;
+    if (have) buf[n + __popc(bal & ((1u << lane_id()) - 1u))] = x;
+    n += __popc(bal);
+    __syncwarp();
+    if (n >= 32) {
+      n -= 32;
+      f(buf[n + lane_id()]);
+      __syncwarp();
+    }
+  }
+  template <class F>
+  __device__ __forceinline__ void flush(F&& f) {
+    __syncwarp();
+    if (lane_id() < n) f(buf[lane_id()]);
+    n = 0;
+    __syncwarp();
+  }
+};
+
 // Flattened two-level iteration by one warp: first(j, L, sb) gives the second-level range
-// [sb, sb + L) of first-level position j in [b, e); f(j, q) is called once per pair.
-template <class First, class F>
-__device__ __forceinline__ void warp_iter(uint32_t b, uint32_t e, First&& first, F&& f, const uint32_t* __restrict__ arr) {
+// [sb, sb + L) of first-level position j in [b, e) (all lanes call it; valid: j < e); f(valid, lo,
+// q, x) gets the pairs of position j0 + lo, four steps of 32 loads at a time, and done() runs
+// after the last pair of each chunk of 32 positions (all lanes call both).
+template <class First, class F, class Done>
+__device__ __forceinline__ void warp_iter(uint32_t b, uint32_t e, const uint32_t* __restrict__ arr, First&& first, F&& f,
+                                          Done&& done) {
   const unsigned lane = lane_id();
   for (uint32_t j0 = b; j0 < e; j0 += 32) {
     const uint32_t j = j0 + lane;
     uint32_t L = 0, sb = 0;
-    if (j < e) first(j, L, sb);
+    first(j, j < e, L, sb);
     const uint32_t incl = warp_inclusive_scan(L);
     const uint32_t excl = incl - L;
     const uint32_t T = __shfl_sync(0xffffffffu, incl, 31);
-    for (uint32_t t0 = 0; t0 < T; t0 += 32) {
-      const uint32_t t = t0 + lane;
-      uint32_t lo = 0;
+    for (uint32_t t0 = 0; t0 < T; t0 += 128) {
+      uint32_t q[4], x[4], at[4];
 #pragma unroll
-      for (uint32_t step = 16; step > 0; step >>= 1) {
-        uint32_t x = __shfl_sync(0xffffffffu, incl, lo + step - 1);
-        if (x <= t) lo += step;
+      for (int r = 0; r < 4; ++r) {
+        const uint32_t t = t0 + 32 * r + lane;
+        uint32_t lo = 0;
+#pragma unroll
+        for (uint32_t step = 16; step > 0; step >>= 1) {
+          uint32_t y = __shfl_sync(0xffffffffu, incl, lo + step - 1);
+          if (y <= t) lo += step;
+        }
+        const uint32_t ex = __shfl_sync(0xffffffffu, excl, lo);
+        const uint32_t s = __shfl_sync(0xffffffffu, sb, lo);
+        at[r] = lo;
+        q[r] = s + (t - ex);
+        x[r] = t < T ? arr[q[r] & ~kRevFlag] : 0u;
       }
-      const uint32_t ex = __shfl_sync(0xffffffffu, excl, lo);
-      const uint32_t s = __shfl_sync(0xffffffffu, sb, lo);
-      if (t < T) {
-        const uint32_t q = s + (t - ex);
-        f(j0 + lo, q, arr[q & ~kRevFlag]);
-      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        if (t0 + 32 * r < T) f(t0 + 32 * r + lane < T, at[r], q[r], x[r]);
     }
+    done();
   }
 }
 
@@ -367,33 +425,28 @@ __device__ __forceinline__ uint32_t block_incl_scan(uint32_t x, uint32_t* smem, 
   return incl;
 }
 
-// Same iteration by the whole CTA.  Each chunk of kPT first-level positions has its second-level
-// ranges cut into pieces of at most kPiece entries; warps claim pieces from a shared-memory
-// counter, locate a piece's position once (binary search over the chunk's inclusive piece
-// counts) and walk it with 32 lanes, so consecutive lanes read consecutive entries and no
-// per-entry search is needed.
+// The same iteration by the whole CTA.  Each chunk of kPT first-level positions has its
+// second-level ranges cut into pieces of at most kPiece entries; pieces go to the warps in turn
+// (they are of one size, so no counter is needed), a warp locates a piece's position once (binary
+// search over the chunk's inclusive piece counts) and walks it with 32 lanes, so consecutive lanes
+// read consecutive entries.
 constexpr uint32_t kPiece = 128;
 
-template <class First, class F>
-__device__ __forceinline__ void block_iter(uint32_t b, uint32_t e, Shared& S, First&& first, F&& f,
-                                           const uint32_t* __restrict__ arr) {
+template <class First, class F, class Done>
+__device__ __forceinline__ void block_iter(uint32_t b, uint32_t e, Shared& S, const uint32_t* __restrict__ arr,
+                                           First&& first, F&& f, Done&& done) {
   const uint32_t tid = threadIdx.x, lane = tid & 31u;
   for (uint32_t j0 = b; j0 < e; j0 += kPT) {
     const uint32_t j = j0 + tid;
     uint32_t L = 0, sb = 0;
-    if (j < e) first(j, L, sb);
+    first(j, j < e, L, sb);
     uint32_t T;
     const uint32_t incl = block_incl_scan((L + kPiece - 1) / kPiece, S.scan, T);
     S.incl[tid] = incl;
     S.sb[tid] = sb;
     S.len[tid] = L;
-    if (tid == 0) S.cursor = 0;
     __syncthreads();
-    while (true) {
-      uint32_t p = 0;
-      if (lane == 0) p = atomicAdd(&S.cursor, 1u);
-      p = __shfl_sync(0xffffffffu, p, 0);
-      if (p >= T) break;
+    for (uint32_t p = tid >> 5; p < T; p += kPW) {
       uint32_t lo = 0;
 #pragma unroll
       for (uint32_t step = kPT / 2; step > 0; step >>= 1)
@@ -409,26 +462,25 @@ __device__ __forceinline__ void block_iter(uint32_t b, uint32_t e, Shared& S, Fi
         x[r] = k < kend ? arr[base + k] : 0u;
       }
 #pragma unroll
-      for (uint32_t r = 0; r < kPiece / 32; ++r) {
-        const uint32_t k = k0 + lane + 32 * r;
-        if (k < kend) f(j0 + lo, sbj + k, x[r]);
-      }
+      for (uint32_t r = 0; r < kPiece / 32; ++r)
+        if (k0 + 32 * r < kend) f(k0 + lane + 32 * r < kend, lo, sbj + k0 + lane + 32 * r, x[r]);
     }
-    __syncthreads();
+    done();
   }
 }
 
 // The same iteration restricted to flattened pair indices [lo, hi) (counted from the first
-// pair of [b, e)); every CTA of the grid takes one slice of a huge item.
+// pair of [b, e)); every CTA takes one slice of a heavy item.  Four pairs per thread are loaded
+// before any of them is used.
 template <class First, class F>
-__device__ __forceinline__ void block_iter_range(uint32_t b, uint32_t e, Shared& S, First&& first, F&& f,
-                                                 uint64_t lo, uint64_t hi, const uint32_t* __restrict__ arr) {
+__device__ __forceinline__ void block_iter_range(uint32_t b, uint32_t e, Shared& S, const uint32_t* __restrict__ arr,
+                                                 uint64_t lo, uint64_t hi, First&& first, F&& f) {
   const uint32_t tid = threadIdx.x;
   uint64_t base = 0;
   for (uint32_t j0 = b; j0 < e && base < hi; j0 += kPT) {
     const uint32_t j = j0 + tid;
     uint32_t L = 0, sb = 0;
-    if (j < e) first(j, L, sb);
+    first(j, j < e, L, sb);
     uint32_t T;
     const uint32_t incl = block_incl_scan(L, S.scan, T);
     S.incl[tid] = incl;
@@ -436,426 +488,383 @@ __device__ __forceinline__ void block_iter_range(uint32_t b, uint32_t e, Shared&
     __syncthreads();
     const uint64_t tb = lo > base ? lo - base : 0;
     const uint64_t te = (hi - base) < (uint64_t)T ? (hi - base) : (uint64_t)T;
-    for (uint64_t t0 = tb; t0 < te; t0 += kPT) {
-      const uint64_t tt = t0 + tid;
-      if (tt < te) {
-        const uint32_t t = (uint32_t)tt;
-        uint32_t lo2 = 0;
+    for (uint64_t t0 = tb; t0 < te; t0 += 4 * kPT) {
+      uint32_t x[4];
 #pragma unroll
-        for (uint32_t step = kPT / 2; step > 0; step >>= 1)
-          if (S.incl[lo2 + step - 1] <= t) lo2 += step;
-        const uint32_t ex = lo2 ? S.incl[lo2 - 1] : 0u;
-        const uint32_t q = S.sb[lo2] + (t - ex);
-        f(j0 + lo2, q, arr[q & ~kRevFlag]);
+      for (int r = 0; r < 4; ++r) {
+        const uint64_t tt = t0 + (uint64_t)r * kPT + tid;
+        x[r] = kEmpty;
+        if (tt < te) {
+          const uint32_t t = (uint32_t)tt;
+          uint32_t lo2 = 0;
+#pragma unroll
+          for (uint32_t step = kPT / 2; step > 0; step >>= 1)
+            if (S.incl[lo2 + step - 1] <= t) lo2 += step;
+          x[r] = arr[S.sb[lo2] + (t - (lo2 ? S.incl[lo2 - 1] : 0u))];
+        }
       }
+      f(x);
     }
     __syncthreads();
     base += T;
   }
 }
 
-// Sum of the second-level lengths of [b, e) (valid in every thread).
-template <class First>
-__device__ __forceinline__ uint64_t block_total(uint32_t b, uint32_t e, Shared& S, First&& first) {
-  unsigned long long sum = 0;
-  for (uint32_t j = b + threadIdx.x; j < e; j += kPT) {
-    uint32_t L = 0, sb = 0;
-    first(j, L, sb);
-    sum += L;
-  }
-  sum = warp_sum(sum);
-  if ((threadIdx.x & 31) == 0) S.red[threadIdx.x >> 5] = sum;
-  __syncthreads();
-  unsigned long long t = 0;
-  for (int w = 0; w < kPT / 32; ++w) t += S.red[w];
-  __syncthreads();
-  return t;
-}
-
-__device__ __forceinline__ void touch(const Work& W, Ctl* ctl, unsigned par, uint32_t x) {
-  if (W.touched[x] == 0 && atomicExch(&W.touched[x], 1u) == 0u) W.tlist[par][atomicAdd(&ctl->tlen[par], 1u)] = x;
-}
-
-// Window bound of the current round, per CTA (set at the start of every round).
-__shared__ unsigned long long s_win_hi;
-
-// Removes `amount` butterflies from an unpeeled item.  Only an item whose count falls below
-// the window bound can reach the frontier before the next window advance, so only those are
-// queued for re-bucketing; items that stay above it keep bucket == count implicitly (the
-// advance resynchronises buckets from counts, when no unpeeled item is in the near list).
-__device__ __forceinline__ bool mine(const Work& W, uint32_t x) { return !W.part || W.part[x] == W.my_part; }
-
-__device__ __forceinline__ void dec(const Work& W, Ctl* ctl, unsigned par, uint32_t x, int64_t amount) {
-  if (mine(W, x) && W.state[x] == ALIVE) {
-    const long long old = (long long)atomicAdd(reinterpret_cast<unsigned long long*>(&W.cnt[x]),
-                                               (unsigned long long)(-amount));
-    if ((unsigned long long)(old - amount) < s_win_hi) touch(W, ctl, par, x);
-  }
-}
-
-// Per-thread accumulator keyed by the first-level position.
-struct PosAcc {
-  uint32_t j = kEmpty;
-  int64_t acc = 0;
+// What a thread gathers during a phase P: the least bucket it moved an item to, and the wedges
+// or probes it processed.
+struct Acc {
+  unsigned long long mn;
+  unsigned long long work;
 };
 
-// ---- tip: process one frontier vertex -------------------------------------------------------
-__device__ void tip_item_warp(const Lists& G, const Work& W, Ctl* ctl, unsigned par, uint32_t u, uint32_t* keys,
-                              uint32_t* vals, unsigned long long& work) {
-  const unsigned lane = lane_id();
-  const int64_t wk = G.wk[u];
-  const uint32_t tsize = max(64u, np2(2u * (uint32_t)wk));
-  const uint32_t mask = tsize - 1;
-  for (uint32_t s = lane; s < tsize; s += 32) { keys[s] = kEmpty; vals[s] = 0; }
-  __syncwarp();
-  warp_iter(G.offK[u], G.offK[u + 1],
-            [&](uint32_t j, uint32_t& L, uint32_t& sb) {
-              const uint32_t v = G.edgK[j];
-              sb = G.offC[v];
-              L = G.offC[v + 1] - sb;
-            },
-            [&](uint32_t, uint32_t, uint32_t u2) {
-              if (u2 != u) t_add(keys, vals, mask, u2, ctl);
-            },
-            G.edgC);
-  __syncwarp();
-  for (uint32_t s = lane; s < tsize; s += 32) {
-    const uint32_t k = keys[s];
-    if (k == kEmpty) continue;
-    const int64_t w = vals[s];
-    if (w >= 2) dec(W, ctl, par, k, w * (w - 1) / 2);
+__device__ __forceinline__ bool mine(const Work& W, uint32_t x) { return !W.part || W.part[x] == W.my_part; }
+
+// Removes `amount` butterflies from item x, which is unpeeled and of this instance.  The decrement
+// whose result first lies below the window bound adds the item to the near list (counts only
+// fall, so exactly one decrement crosses); items above the bound cannot reach the frontier before
+// the next window advance, which reads their counts.
+__device__ __forceinline__ void dec_known(const Work& W, Ctl* ctl, Acc& A, uint32_t x, int64_t amount) {
+  const long long old = (long long)atomicAdd(reinterpret_cast<unsigned long long*>(&W.cnt[x]),
+                                             (unsigned long long)(-amount));
+  const unsigned long long nb = (unsigned long long)max(old - amount, s_k);
+  if (nb < s_win_hi) {
+    A.mn = min(A.mn, nb);
+    if ((unsigned long long)max(old, s_k) >= s_win_hi) W.near[atomicAdd(&ctl->near_len, 1ull)] = x;
   }
-  if (lane == 0) work += (unsigned long long)wk;
-  __syncwarp();
 }
 
-__device__ void tip_item_block(const Lists& G, const Work& W, Ctl* ctl, unsigned par, uint32_t u, uint32_t* table,
-                               Shared& S, unsigned long long& work) {
-  const int64_t wk = G.wk[u];
-  const bool hash = (uint64_t)2 * (uint64_t)wk <= (uint64_t)kBlockSlots;
-  uint32_t* keys = table;
-  uint32_t* vals = table + kBlockSlots;
-  uint32_t* gcnt = W.gscratch + (size_t)blockIdx.x * (size_t)W.gscratch_len;
-  const uint32_t tsize = hash ? max(64u, np2(2u * (uint32_t)wk)) : 0u;
-  const uint32_t mask = tsize - 1;
-  if (hash)
-    for (uint32_t s = threadIdx.x; s < tsize; s += kPT) { keys[s] = kEmpty; vals[s] = 0; }
-  __syncthreads();
-  auto first = [&](uint32_t j, uint32_t& L, uint32_t& sb) {
+__device__ __forceinline__ void dec(const Work& W, Ctl* ctl, Acc& A, uint32_t x, int64_t amount) {
+  if (W.state[x] == ALIVE && mine(W, x)) dec_known(W, ctl, A, x, amount);
+}
+
+// ---- tip: process one frontier vertex -------------------------------------------------------
+struct TipFirst {
+  const Lists& G;
+  __device__ __forceinline__ void operator()(uint32_t j, bool valid, uint32_t& L, uint32_t& sb) const {
+    if (!valid) return;
     const uint32_t v = G.edgK[j];
     sb = G.offC[v];
     L = G.offC[v + 1] - sb;
-  };
-  block_iter(G.offK[u], G.offK[u + 1], S, first, [&](uint32_t, uint32_t, uint32_t u2) {
-    if (u2 == u) return;
-    if (hash) t_add(keys, vals, mask, u2, ctl);
+  }
+};
+
+// Queue entries of tip items: (u2, w) with w wedges to u2.
+__device__ __forceinline__ void tip_charge(const Work& W, Ctl* ctl, Acc& A, unsigned long long x) {
+  const int64_t w = (int64_t)(x >> 32);
+  dec(W, ctl, A, (uint32_t)x, w * (w - 1) / 2);
+}
+
+__device__ void tip_item_warp(const Lists& G, const Work& W, Ctl* ctl, uint32_t u, uint32_t* keys, uint32_t* vals,
+                              WarpQueue& Q, Acc& A) {
+  const unsigned lane = lane_id();
+  const int64_t wk = G.wk[u];
+  const uint32_t tsize = max(64u, np2(2u * (uint32_t)wk));
+  for (uint32_t s = lane; s < tsize; s += 32) { keys[s] = kEmpty; vals[s] = 0; }
+  __syncwarp();
+  warp_iter(G.offK[u], G.offK[u + 1], G.edgC, TipFirst{G},
+            [&](bool valid, uint32_t, uint32_t, uint32_t u2) {
+              if (valid && u2 != u) t_add(keys, vals, tsize, u2, ctl);
+            },
+            [] {});
+  __syncwarp();
+  auto charge = [&](unsigned long long x) { tip_charge(W, ctl, A, x); };
+  for (uint32_t s = lane; s < tsize; s += 32) {
+    const uint32_t w = vals[s];
+    Q.push(w >= 2, ((unsigned long long)w << 32) | keys[s], charge);
+  }
+  Q.flush(charge);
+  if (lane == 0) A.work += (unsigned long long)wk;
+}
+
+__device__ void tip_item_block(const Lists& G, const Work& W, Ctl* ctl, uint32_t u, uint32_t* table, Shared& S,
+                               WarpQueue& Q, Acc& A) {
+  const int64_t wk = G.wk[u];
+  const bool hash = (uint64_t)2 * (uint64_t)wk <= (uint64_t)kTipSlots;
+  uint32_t* keys = table;
+  uint32_t* vals = table + kTipSlots;
+  uint32_t* gcnt = W.gscratch + (size_t)blockIdx.x * (size_t)W.gscratch_len;
+  const uint32_t tsize = hash ? max(64u, np2(2u * (uint32_t)wk)) : 0u;
+  if (hash)
+    for (uint32_t s = threadIdx.x; s < tsize; s += kPT) { keys[s] = kEmpty; vals[s] = 0; }
+  __syncthreads();
+  auto charge = [&](unsigned long long x) { tip_charge(W, ctl, A, x); };
+  const auto done = [] { __syncthreads(); };
+  block_iter(G.offK[u], G.offK[u + 1], S, G.edgC, TipFirst{G}, [&](bool valid, uint32_t, uint32_t, uint32_t u2) {
+    if (!valid || u2 == u) return;
+    if (hash) t_add(keys, vals, tsize, u2, ctl);
     else atomicAdd(&gcnt[u2], 1u);
-  }, G.edgC);
+  }, done);
   __syncthreads();
   if (hash) {
-    for (uint32_t s = threadIdx.x; s < tsize; s += kPT) {
-      const uint32_t k = keys[s];
-      if (k == kEmpty) continue;
-      const int64_t w = vals[s];
-      if (w >= 2) dec(W, ctl, par, k, w * (w - 1) / 2);
+    for (uint32_t s0 = 0; s0 < tsize; s0 += kPT) {
+      const uint32_t s = s0 + threadIdx.x;
+      const uint32_t w = s < tsize ? vals[s] : 0u;
+      Q.push(w >= 2, ((unsigned long long)w << 32) | (s < tsize ? keys[s] : 0u), charge);
     }
   } else {
-    block_iter(G.offK[u], G.offK[u + 1], S, first, [&](uint32_t, uint32_t, uint32_t u2) {
-      if (u2 == u) return;
-      const int64_t w = atomicExch(&gcnt[u2], 0u);
-      if (w >= 2) dec(W, ctl, par, u2, w * (w - 1) / 2);
-    }, G.edgC);
+    block_iter(G.offK[u], G.offK[u + 1], S, G.edgC, TipFirst{G}, [&](bool valid, uint32_t, uint32_t, uint32_t u2) {
+      uint32_t w = 0;
+      if (valid && u2 != u) w = atomicExch(&gcnt[u2], 0u);
+      Q.push(w >= 2, ((unsigned long long)w << 32) | u2, charge);
+    }, done);
   }
-  if (threadIdx.x == 0) work += (unsigned long long)wk;
+  Q.flush(charge);
+  if (threadIdx.x == 0) A.work += (unsigned long long)wk;
   __syncthreads();
+}
+
+// Heavy tip items of a round (at most W.ngroups of them, items i < nh from `huge`, the others
+// CTA-level ones read back from `big`): their flattened two-hop lists are cut into equal slices
+// over the instance's CTAs.  Every wedge adds one to the item's grid-shared dense counter of u2;
+// the add that returns j removes j butterflies from u2 at once (0 + 1 + ... + (w - 1) = C(w, 2)),
+// so one pass and no barrier is needed.  clear: the same walk resets the counters (after a
+// barrier), on the CTAs from the other end of the grid: those at this end scan the near list.
+__device__ void tip_items_flat(const Lists& G, const Work& W, Ctl* ctl, const uint4* huge, unsigned nh, const uint4* big,
+                               unsigned n, bool clear, Shared& S, Acc& A) {
+  if (threadIdx.x < 32) {
+    unsigned long long t = 0;
+    uint4 d = make_uint4(0, 0, 0, 0);
+    if (threadIdx.x < n) {
+      d = threadIdx.x < nh ? huge[threadIdx.x] : big[-(int)(threadIdx.x - nh)];
+      t = d.w == 0xFFFFFFFFu ? (unsigned long long)G.wk[d.x] + d.z : d.w;
+    }
+    S.flat[threadIdx.x] = d;
+    S.red[threadIdx.x] = warp_inclusive_scan(t);
+  }
+  __syncthreads();
+  const unsigned long long T = S.red[31];
+  const unsigned nuse = (unsigned)min((unsigned long long)vgrid(), T / kFlatPairs + 1ull);
+  const unsigned vb = clear ? vgrid() - 1u - vblock() : vblock();
+  if (T && vb < nuse) {
+    const unsigned long long lo = T * vb / nuse, hi = T * (vb + 1) / nuse;
+    for (unsigned i = 0; i < n; ++i) {
+      const unsigned long long tb = i ? S.red[i - 1] : 0ull, te = S.red[i];
+      if (te <= lo || tb >= hi) continue;  // uniform across the CTA
+      const uint32_t u = S.flat[i].x, b = S.flat[i].y;
+      uint32_t* cnt = W.gshared + (size_t)i * (size_t)W.gshared_stride;
+      block_iter_range(b, b + S.flat[i].z, S, G.edgC, lo > tb ? lo - tb : 0ull, min(hi, te) - tb, TipFirst{G},
+                       [&](const uint32_t* x) {
+                         if (clear) {
+#pragma unroll
+                           for (int r = 0; r < 4; ++r)
+                             if (x[r] != kEmpty) cnt[x[r]] = 0u;
+                           return;
+                         }
+                         uint32_t j[4];
+                         uint8_t st[4];
+#pragma unroll
+                         for (int r = 0; r < 4; ++r) {
+                           j[r] = 0;
+                           st[r] = PEELED;
+                           if (x[r] != kEmpty && x[r] != u) {
+                             j[r] = atomicAdd(&cnt[x[r]], 1u);
+                             st[r] = W.state[x[r]];
+                           }
+                         }
+#pragma unroll
+                         for (int r = 0; r < 4; ++r)
+                           if (j[r] && st[r] == ALIVE && mine(W, x[r])) dec_known(W, ctl, A, x[r], (int64_t)j[r]);
+                       });
+    }
+  }
+  if (!clear && vblock() == 0 && threadIdx.x == 0) A.work += T;
+  __syncthreads();  // S.red is reused
 }
 
 // ---- wing: process one frontier edge --------------------------------------------------------
 // Orientation A (walk from the centre v): probe set N(u) (centre -> edge), first level N(v)
 // (u2, edge e2), second level N(u2) (v2, edge e3), probe v2 -> e4.
 // Orientation B (walk from u): probe set N(v) (count-side vertex -> edge), first level N(u)
-// (v2, e4), second level N(v2) (u2, e3), probe u2 -> e2.  Both find the same butterflies.
+// (v2, e4), second level N(v2) (u2, e3), probe u2 -> e2.  Both find the same butterflies, and
+// run the same code with the two sides' lists exchanged.
 
 // Binary-searching a list of length dbig for each of dsmall keys beats scanning it.
 __device__ __forceinline__ bool reverse_cheaper(uint32_t dsmall, uint32_t dbig) {
   return (uint64_t)dsmall * (uint64_t)(33u - __clz(dbig | 1u)) < (uint64_t)dbig;
 }
 
-struct WingEdge {
-  uint32_t e1, u, v;
-  bool from_v;
-};
-
-// An edge of a lower partition is gone; one of a higher partition is present and unpeeled.
-__device__ __forceinline__ bool skip_edge(const Work& W, uint32_t e, uint32_t e1) {
-  if (W.part) {
-    const uint32_t p = W.part[e];
-    if (p != W.my_part) return p < W.my_part;
-  }
+// How edge e stands towards frontier edge e1: ES_GONE (peeled earlier, or in this round's
+// frontier with a smaller index: the tie rule), ES_CHARGE (unpeeled, loses the butterfly) or
+// ES_KEEP (in this round's frontier with a larger index, or of a higher partition: the butterfly
+// exists but the edge is not charged).  Edges of lower partitions are gone.
+enum EdgeStatus : uint32_t { ES_GONE = 0, ES_CHARGE = 1, ES_KEEP = 2 };
+__device__ __forceinline__ uint32_t edge_status(const Work& W, uint32_t e, uint32_t e1) {
   const uint8_t s = W.state[e];
-  return s == PEELED || (s == ACTIVE && e < e1);
-}
-
-__device__ __forceinline__ bool edge_gone(const Work& W, uint32_t e) {
   if (W.part) {
     const uint32_t p = W.part[e];
-    if (p != W.my_part) return p < W.my_part;
+    if (p != W.my_part) return p < W.my_part ? ES_GONE : ES_KEEP;
   }
-  return W.state[e] == PEELED;
+  return s == ALIVE ? ES_CHARGE : (s == s_act && e >= e1 ? ES_KEEP : ES_GONE);
 }
 
-// In this round's frontier with a smaller index than e1 (the tie rule).
-__device__ __forceinline__ bool active_before(const Work& W, uint32_t e, uint32_t e1) {
-  return e < e1 && mine(W, e) && W.state[e] == ACTIVE;
-}
+enum Level { LV_WARP = 0, LV_BLOCK = 1 };
+constexpr uint32_t kKeepBit = 0x80000000u;   // probe-set edges that are not charged (m < 2^31)
+constexpr uint32_t kNoSlot = 0x3FFFu;        // queue entries found through the dense markers
 
-// Item granularity: one warp, one CTA, or the whole grid (huge items; all CTAs call it).
-enum Level { LV_WARP = 0, LV_BLOCK = 1, LV_GRID = 2 };
-
+// The units [chunk, chunk_end) of nchunks (slices of the first level) of one frontier edge, by one
+// warp or one CTA.
 template <int kLevel>
-__device__ bool wing_item(const Lists& G, const Work& W, Ctl* ctl, unsigned par, const WingEdge& E, uint32_t* keys,
-                          uint32_t* vals, uint32_t slots, Shared* S, unsigned long long& work, uint32_t chunk = 0,
-                          uint32_t nchunks = 1, uint32_t chunk_end = 0) {
-  // First-level slice: units [chunk, chunk_end) of nchunks (chunk_end 0: chunk + 1).
-  if (chunk_end == 0) chunk_end = chunk + 1;
-  const uint32_t rank = kLevel == LV_WARP ? lane_id() : (kLevel == LV_GRID ? vblock() * kPT + threadIdx.x : threadIdx.x);
-  const uint32_t gsize = kLevel == LV_WARP ? 32 : (kLevel == LV_GRID ? vgrid() * kPT : kPT);
-  auto sync = [&]() -> bool {
-    if (kLevel == LV_WARP) { __syncwarp(); return true; }
-    if (kLevel == LV_BLOCK) { __syncthreads(); return true; }
-    return grid_barrier(ctl);
+__device__ void wing_item(const Lists& G, const Work& W, Ctl* ctl, const uint4& E, uint32_t* keys, Shared& S,
+                          WarpQueue& Q, Acc& A, uint32_t chunk, uint32_t nchunks, uint32_t chunk_end) {
+  constexpr uint32_t cap = kLevel == LV_WARP ? kWingWarpSlots : kWingSlots;
+  const uint32_t rank = kLevel == LV_WARP ? lane_id() : threadIdx.x;
+  constexpr uint32_t gsize = kLevel == LV_WARP ? 32 : kPT;
+  auto sync = [] {
+    if (kLevel == LV_WARP) __syncwarp();
+    else __syncthreads();
   };
-  // Probe set: N(u) (keys: centres) when walking from v, else N(v) (keys: count-side ids).
-  uint32_t pb, pe;
-  if (E.from_v) { pb = G.offK[E.u]; pe = G.offK[E.u + 1]; }
-  else { pb = G.offC[E.v]; pe = G.offC[E.v + 1]; }
-  const uint32_t psize = pe - pb;
-  const bool hash = kLevel != LV_GRID && 2 * psize <= slots;
-  uint32_t* mark = kLevel == LV_GRID ? W.gshared : W.gscratch + (size_t)blockIdx.x * (size_t)W.gscratch_len;
-  const uint32_t tsize = hash ? max(64u, np2(2u * psize)) : 0u;
-  const uint32_t mask = tsize - 1;
+  // Side A holds the probe set N(a) and the second-level lists, side B the first level N(b).
+  const bool from_v = (E.y & kInfoFromV) != 0;
+  const uint32_t* offA = from_v ? G.offK : G.offC;
+  const uint32_t* edgA = from_v ? G.edgK : G.edgC;
+  const uint32_t* eidA = from_v ? G.eidK : G.eidC;
+  const uint32_t* offB = from_v ? G.offC : G.offK;
+  const uint32_t* edgB = from_v ? G.edgC : G.edgK;
+  const uint32_t* eidB = from_v ? G.eidC : G.eidK;
+  const uint32_t e1 = E.x, a = E.y & ~kInfoFromV, b = E.z;
+  const uint32_t pb = offA[a], pe = offA[a + 1], psize = pe - pb;
+  const uint32_t b1 = offB[b], d1 = offB[b + 1] - b1;
+  const bool hash = kLevel == LV_WARP || psize <= kWingSet;
+  uint32_t* mark = W.gscratch + (size_t)blockIdx.x * (size_t)W.gscratch_len;
+  const uint32_t tsize = hash ? max(64u, min(2 * psize, cap)) : 0u;
+  uint32_t* vals = keys + cap;
   // hits[slot]: butterflies found through a probe-set edge, charged to it in one decrement once
-  // the intersections are done (the table area holds keys, edges and hits).
-  uint32_t* hits = vals + slots;
-  if (hash)
-    for (uint32_t s = rank; s < tsize; s += gsize) {
-      keys[s] = kEmpty;
-      hits[s] = 0;
-    }
-  if (!sync()) return false;
+  // the intersections are done.
+  uint32_t* hits = vals + cap;
+  for (uint32_t s = rank; s < tsize; s += gsize) {
+    keys[s] = kEmpty;
+    hits[s] = 0;
+  }
+  sync();
   for (uint32_t p = pb + rank; p < pe; p += gsize) {
-    uint32_t key, e;
-    if (E.from_v) { key = G.edgK[p]; e = G.eidK[p]; }
-    else { key = G.edgC[p]; e = G.eidC[p]; }
-    if (edge_gone(W, e)) continue;
-    if (hash) t_put(keys, vals, mask, key, e, ctl);
-    else mark[key] = e + 1;
+    const uint32_t key = edgA[p], e = eidA[p];
+    const uint32_t es = edge_status(W, e, e1);
+    if (es == ES_GONE) continue;
+    const uint32_t val = es == ES_KEEP ? (e | kKeepBit) : e;
+    if (hash) t_put(keys, vals, tsize, key, val, ctl);
+    else mark[key] = val + 1;
   }
-  if (!sync()) return false;
-  // e: the probe-set edge of key; slot: its table slot (kEmpty for the dense markers).
-  auto probe = [&](uint32_t key, uint32_t& e, uint32_t& slot) -> bool {
-    if (hash) {
-      slot = t_slot(keys, mask, key);
-      if (slot == kEmpty) return false;
-      e = vals[slot];
-      return true;
-    }
-    slot = kEmpty;
-    const uint32_t x = mark[key];
-    if (!x) return false;
-    e = x - 1;
-    return true;
-  };
-  PosAcc acc;
-  unsigned long long my_work = 0, my_rev = 0;
-  auto flush = [&]() {
-    if (acc.j != kEmpty && acc.acc) dec(W, ctl, par, E.from_v ? G.eidC[acc.j] : G.eidK[acc.j], acc.acc);
-    acc.acc = 0;
-  };
-  // Each (first-level vertex x, probe set) intersection runs in one of two directions: scan
-  // N(x) and probe the probe-set table, or (when the probe set is much shorter than N(x))
-  // walk the probe set and binary-search N(x), which is sorted.  The direction rides in the
+  sync();
+  // The chunk's first-level edge of this thread (position j0 + rank).
+  uint32_t f_edge = 0, f_st = ES_GONE;
+  uint32_t* accp = kLevel == LV_WARP ? S.acc + (threadIdx.x & ~31u) : S.acc;
+  // Each (first-level vertex y, probe set) intersection runs in one of two directions: scan
+  // N(y) and probe the probe-set table, or (when the probe set is much shorter than N(y))
+  // walk the probe set and binary-search N(y), which is sorted.  The direction rides in the
   // top bit of the second-level position.
-  // One butterfly: e_list (unique to it) loses 1 now; the probe-set edge e_set loses 1 through
-  // its hit counter when it has a table slot; the first-level edge through the accumulator.
-  auto found = [&](uint32_t j, uint32_t e_list, uint32_t e_set, uint32_t slot) {
-    dec(W, ctl, par, e_list, 1);
-    if (slot != kEmpty) atomicAdd(&hits[slot], 1u);
-    else dec(W, ctl, par, e_set, 1);
-    if (j != acc.j) { flush(); acc.j = j; }
-    acc.acc += 1;
+  uint32_t j_chunk = 0;
+  auto first = [&](uint32_t j, bool valid, uint32_t& L, uint32_t& sb) {
+    f_st = ES_GONE;
+    accp[rank] = 0;
+    j_chunk = j - rank;
+    if (!valid) return;
+    const uint32_t y = edgB[j];
+    f_edge = eidB[j];
+    const uint32_t b2 = offA[y], d2 = offA[y + 1] - b2;
+    f_st = edge_status(W, f_edge, e1);
+    if (y == a || f_st == ES_GONE) return;
+    if (reverse_cheaper(psize, d2)) { sb = pb | kRevFlag; L = psize; }
+    else { sb = b2; L = d2; }
   };
-  // Second-level entries (and the probe set walked in the reverse direction) come from one list
-  // array per orientation: N(u2) / N(u) in the count side's lists when walking from v, N(v2) /
-  // N(v) in the centre side's lists when walking from u.
-  const uint32_t* arr = E.from_v ? G.edgK : G.edgC;
-  auto run = [&](uint32_t b, uint32_t e, auto&& first, auto&& f) {
-    if (kLevel == LV_WARP) {
-      warp_iter(b, e, first, f, arr);
-    } else if (kLevel == LV_BLOCK) {
-      block_iter(b, e, *S, first, f, arr);
+  // One butterfly found through second-level entry q: its edge loses 1 now; the probe-set edge
+  // loses 1 through its hit counter when it has a table slot; the first-level edge through the
+  // chunk's accumulator.
+  auto charge = [&](unsigned long long x) {
+    const uint32_t q = (uint32_t)(x >> 32), slot = (uint32_t)x & kNoSlot, lo = ((uint32_t)x >> 14) & 511u;
+    const uint32_t e3 = eidA[q];
+    const uint32_t es = edge_status(W, e3, e1);
+    if (es == ES_GONE) return;
+    if (es == ES_CHARGE) dec_known(W, ctl, A, e3, 1);
+    if (slot != kNoSlot) {
+      atomicAdd(&hits[slot], 1u);
     } else {
-      const uint64_t T = block_total(b, e, *S, first);
-      const uint64_t lo = T * vblock() / vgrid(), hi = T * (vblock() + 1) / vgrid();
-      block_iter_range(b, e, *S, first, f, lo, hi, arr);
+      const uint32_t val = mark[edgA[q]] - 1u;
+      if (!(val & kKeepBit)) dec_known(W, ctl, A, val, 1);
     }
+    atomicAdd(&accp[lo], 1u);
   };
-  if (E.from_v) {
-    auto first = [&](uint32_t p, uint32_t& L, uint32_t& sb) {
-      const uint32_t u2 = G.edgC[p];
-      if (u2 == E.u || skip_edge(W, G.eidC[p], E.e1)) { L = 0; sb = 0; return; }
-      const uint32_t b2 = G.offK[u2], d2 = G.offK[u2 + 1] - b2;
-      if (reverse_cheaper(psize, d2)) { sb = pb | kRevFlag; L = psize; }
-      else { sb = b2; L = d2; }
-    };
-    auto f = [&](uint32_t p, uint32_t q, uint32_t v2) {  // v2 = G.edgK[q without the flag]
-      ++my_work;
-      if (q & kRevFlag) {  // walk N(u), binary-search N(u2)
+  unsigned my_work = 0, my_rev = 0;
+  auto pair = [&](bool valid, uint32_t lo, uint32_t q, uint32_t z) {
+    bool hit = false;
+    unsigned long long ent = 0;
+    if (valid) ++my_work;
+    if (valid && z != b) {
+      if (q & kRevFlag) {  // walk N(a), binary-search N(y)
         ++my_rev;
-        const uint32_t pos = q & ~kRevFlag;
-        if (v2 == E.v) return;
-        const uint32_t e4 = G.eidK[pos];
-        if (skip_edge(W, e4, E.e1)) return;
-        const uint32_t u2 = G.edgC[p];
-        const uint32_t hi = G.offK[u2 + 1];
-        const uint32_t at = lower_bound_u32(G.edgK, G.offK[u2], hi, v2);
-        if (at == hi || G.edgK[at] != v2) return;
-        const uint32_t e3 = G.eidK[at];
-        if (skip_edge(W, e3, E.e1)) return;
-        found(p, e3, e4, kEmpty);
-        return;
+        const uint32_t e4 = eidA[q & ~kRevFlag];
+        const uint32_t s4 = edge_status(W, e4, e1);
+        if (s4 != ES_GONE) {
+          const uint32_t y = edgB[j_chunk + lo];
+          const uint32_t end = offA[y + 1];
+          const uint32_t at = lower_bound_u32(edgA, offA[y], end, z);
+          if (at != end && edgA[at] == z) {
+            const uint32_t e3 = eidA[at];
+            const uint32_t s3 = edge_status(W, e3, e1);
+            if (s3 != ES_GONE) {
+              if (s3 == ES_CHARGE) dec_known(W, ctl, A, e3, 1);
+              if (s4 == ES_CHARGE) dec_known(W, ctl, A, e4, 1);
+              atomicAdd(&accp[lo], 1u);
+            }
+          }
+        }
+      } else if (hash) {
+        const uint32_t slot = t_slot(keys, tsize, z);
+        hit = slot != kEmpty;
+        ent = ((unsigned long long)q << 32) | (lo << 14) | (slot & kNoSlot);
+      } else {
+        hit = mark[z] != 0;
+        ent = ((unsigned long long)q << 32) | (lo << 14) | kNoSlot;
       }
-      if (v2 == E.v) return;
-      uint32_t e4, slot;
-      if (!probe(v2, e4, slot)) return;  // most probes miss: test the table before any global read
-      const uint32_t e3 = G.eidK[q];
-      if (skip_edge(W, e3, E.e1) || active_before(W, e4, E.e1)) return;
-      found(p, e3, e4, slot);
-    };
-    const uint32_t b1 = G.offC[E.v], d1 = G.offC[E.v + 1] - b1;
-    run(b1 + (uint32_t)((uint64_t)d1 * chunk / nchunks), b1 + (uint32_t)((uint64_t)d1 * chunk_end / nchunks), first, f);
-  } else {
-    auto first = [&](uint32_t q, uint32_t& L, uint32_t& sb) {
-      const uint32_t v2 = G.edgK[q];
-      if (v2 == E.v || skip_edge(W, G.eidK[q], E.e1)) { L = 0; sb = 0; return; }
-      const uint32_t b2 = G.offC[v2], d2 = G.offC[v2 + 1] - b2;
-      if (reverse_cheaper(psize, d2)) { sb = pb | kRevFlag; L = psize; }
-      else { sb = b2; L = d2; }
-    };
-    auto f = [&](uint32_t q, uint32_t p3, uint32_t u2) {  // u2 = G.edgC[p3 without the flag]
-      ++my_work;
-      if (p3 & kRevFlag) {  // walk N(v), binary-search N(v2)
-        ++my_rev;
-        const uint32_t pos = p3 & ~kRevFlag;
-        if (u2 == E.u) return;
-        const uint32_t e2 = G.eidC[pos];
-        if (skip_edge(W, e2, E.e1)) return;
-        const uint32_t v2 = G.edgK[q];
-        const uint32_t hi = G.offC[v2 + 1];
-        const uint32_t at = lower_bound_u32(G.edgC, G.offC[v2], hi, u2);
-        if (at == hi || G.edgC[at] != u2) return;
-        const uint32_t e3 = G.eidC[at];
-        if (skip_edge(W, e3, E.e1)) return;
-        found(q, e3, e2, kEmpty);
-        return;
-      }
-      if (u2 == E.u) return;
-      uint32_t e2, slot;
-      if (!probe(u2, e2, slot)) return;
-      const uint32_t e3 = G.eidC[p3];
-      if (skip_edge(W, e3, E.e1) || active_before(W, e2, E.e1)) return;
-      found(q, e3, e2, slot);
-    };
-    const uint32_t b1 = G.offK[E.u], d1 = G.offK[E.u + 1] - b1;
-    run(b1 + (uint32_t)((uint64_t)d1 * chunk / nchunks), b1 + (uint32_t)((uint64_t)d1 * chunk_end / nchunks), first, f);
-  }
-  flush();
-  work += my_work;
-  if (hash) {  // the probe-set edges' decrements, one per edge
-    if (!sync()) return false;
-    for (uint32_t s = rank; s < tsize; s += gsize) {
-      const uint32_t h = hits[s];
-      if (h && keys[s] != kEmpty) dec(W, ctl, par, vals[s], (int64_t)h);
     }
+    Q.push(hit, ent, charge);
+  };
+  auto done = [&] {
+    Q.flush(charge);
+    sync();
+    const uint32_t got = accp[rank];
+    if (got && f_st == ES_CHARGE) dec_known(W, ctl, A, f_edge, (int64_t)got);
+  };
+  const uint32_t fb = b1 + (uint32_t)((uint64_t)d1 * chunk / nchunks);
+  const uint32_t fe = b1 + (uint32_t)((uint64_t)d1 * chunk_end / nchunks);
+  if (kLevel == LV_WARP) warp_iter(fb, fe, edgA, first, pair, done);
+  else block_iter(fb, fe, S, edgA, first, pair, done);
+  // The probe-set edges' decrements, one per edge.
+  for (uint32_t s0 = 0; s0 < tsize; s0 += gsize) {
+    const uint32_t s = s0 + rank;
+    const uint32_t h = s < tsize ? hits[s] : 0u;
+    const uint32_t val = h ? vals[s] : kKeepBit;
+    Q.push(!(val & kKeepBit), ((unsigned long long)h << 32) | val,
+           [&](unsigned long long x) { dec_known(W, ctl, A, (uint32_t)x, (int64_t)(x >> 32)); });
   }
-  {
-    const int mode = kLevel == LV_WARP ? 0 : (kLevel == LV_GRID ? 3 : (hash ? 1 : 2));
-    const unsigned long long w = warp_sum((unsigned long long)my_work);
-    const unsigned long long rw = warp_sum((unsigned long long)my_rev);
-    if (lane_id() == 0) {
-      if (w) atomicAdd(&ctl->mode_work[mode], w);
-      if (rw) atomicAdd(&ctl->rev_work, rw);
-    }
-    if (rank == 0) atomicAdd(&ctl->mode_items[mode], 1ull);
-  }
-  if (!sync()) return false;
+  Q.flush([&](unsigned long long x) { dec_known(W, ctl, A, (uint32_t)x, (int64_t)(x >> 32)); });
   if (!hash) {  // clear the dense markers
-    for (uint32_t p = pb + rank; p < pe; p += gsize) mark[E.from_v ? G.edgK[p] : G.edgC[p]] = 0;
+    for (uint32_t p = pb + rank; p < pe; p += gsize) mark[edgA[p]] = 0;
   }
-  return sync();
-}
-
-// Huge tip item: every CTA aggregates one slice of u's two-hop list into grid-shared dense
-// counters; a second pass reads and clears them (atomicExch), crediting each distinct u2 once.
-__device__ bool tip_item_grid(const Lists& G, const Work& W, Ctl* ctl, unsigned par, uint32_t u, Shared& S,
-                              unsigned long long& work) {
-  auto first = [&](uint32_t j, uint32_t& L, uint32_t& sb) {
-    const uint32_t v = G.edgK[j];
-    sb = G.offC[v];
-    L = G.offC[v + 1] - sb;
-  };
-  const uint64_t T = (uint64_t)G.wk[u] + (G.offK[u + 1] - G.offK[u]);
-  const uint64_t lo = T * vblock() / vgrid(), hi = T * (vblock() + 1) / vgrid();
-  uint32_t* cnt = W.gshared;
-  block_iter_range(G.offK[u], G.offK[u + 1], S, first, [&](uint32_t, uint32_t, uint32_t u2) {
-    if (u2 != u) atomicAdd(&cnt[u2], 1u);
-  }, lo, hi, G.edgC);
-  if (!grid_barrier(ctl)) return false;
-  block_iter_range(G.offK[u], G.offK[u + 1], S, first, [&](uint32_t, uint32_t, uint32_t u2) {
-    if (u2 == u) return;
-    const int64_t w = atomicExch(&cnt[u2], 0u);
-    if (w >= 2) dec(W, ctl, par, u2, w * (w - 1) / 2);
-  }, lo, hi, G.edgC);
-  if (vblock() == 0 && threadIdx.x == 0) work += T;
-  return grid_barrier(ctl);
-}
-
-// The same for a group of gs CTAs (this CTA is number lb in it) with its own counter slice and
-// barrier: several heavy tip items of a round run at once, one per group.  The caller's grid
-// barrier after the group's item separates it from the next use of the slice.
-__device__ bool tip_item_group(const Lists& G, const Work& W, Ctl* ctl, unsigned par, uint32_t u, Shared& S,
-                               unsigned long long& work, unsigned lb, unsigned gs, unsigned slot, uint32_t* cnt) {
-  auto first = [&](uint32_t j, uint32_t& L, uint32_t& sb) {
-    const uint32_t v = G.edgK[j];
-    sb = G.offC[v];
-    L = G.offC[v + 1] - sb;
-  };
-  const uint64_t T = (uint64_t)G.wk[u] + (G.offK[u + 1] - G.offK[u]);
-  const uint64_t lo = T * lb / gs, hi = T * (lb + 1) / gs;
-  block_iter_range(G.offK[u], G.offK[u + 1], S, first, [&](uint32_t, uint32_t, uint32_t u2) {
-    if (u2 != u) atomicAdd(&cnt[u2], 1u);
-  }, lo, hi, G.edgC);
-  if (!group_barrier(ctl, slot, gs)) return false;
-  block_iter_range(G.offK[u], G.offK[u + 1], S, first, [&](uint32_t, uint32_t, uint32_t u2) {
-    if (u2 == u) return;
-    const int64_t w = atomicExch(&cnt[u2], 0u);
-    if (w >= 2) dec(W, ctl, par, u2, w * (w - 1) / 2);
-  }, lo, hi, G.edgC);
-  if (lb == 0 && threadIdx.x == 0) work += T;
-  return true;
+  A.work += my_work;
+  {
+    const int mode = kLevel == LV_WARP ? 0 : (hash ? 1 : 2);
+    const unsigned w = __reduce_add_sync(0xffffffffu, my_work);
+    const unsigned rw = __reduce_add_sync(0xffffffffu, my_rev);
+    if (lane_id() == 0) {
+      if (w) atomicAdd(&s_st.mode_work[mode], (unsigned long long)w);
+      if (rw) atomicAdd(&s_st.rev_work, (unsigned long long)rw);
+    }
+    if (rank == 0) atomicAdd(&s_st.mode_items[mode], 1ull);
+  }
+  sync();
 }
 
 // ---- the persistent kernel ------------------------------------------------------------------
 // Wing items run on one warp when their work is small and their probe set fits a warp table.
 struct Classify {
   int64_t small_work;
-  int64_t huge_work;   // items above this run on the whole grid
+  int64_t huge_work;   // tip items above this run on the whole grid
   int64_t chunk_work;  // target probes per work unit of a CTA-level wing item
   int64_t units_per_cta;  // work units per CTA a round's CTA-level wing work is cut into
   int64_t warp_units;     // wing: every item with a warp-sized probe set runs as warp units
 
   __device__ __forceinline__ bool tip_small(const Lists& G, uint32_t u) const {
-    return G.wk[u] <= kWarpSlots / 2 && G.wk[u] <= small_work;
+    return G.wk[u] <= kTipWarpSlots / 2 && G.wk[u] <= small_work;
   }
   // Estimated probes from each side: the two-hop list sizes, capped by deg(u)*deg(v) times a
   // binary-search factor (the reverse-direction intersections).
@@ -866,9 +875,6 @@ struct Classify {
   __device__ __forceinline__ int64_t cost_u(const Lists& G, uint32_t v, uint32_t u) const {
     const int64_t du = G.offK[u + 1] - G.offK[u], dv = G.offC[v + 1] - G.offC[v];
     return min(G.S[u], du * dv * 16);
-  }
-  __device__ __forceinline__ bool wing_from_v(const Lists& G, uint32_t v, uint32_t u) const {
-    return cost_v(G, v, u) <= cost_u(G, v, u);
   }
   __device__ __forceinline__ bool tip_huge(const Lists& G, uint32_t u) const { return G.wk[u] > huge_work; }
 };
@@ -897,6 +903,31 @@ struct Instances {
   uint32_t n;
 };
 
+// Adds the CTA's statistics to the control block (CTA 0 also its rounds and phase times).
+__device__ void flush_stats(Ctl* ctl) {
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    if (s_st.mode_items[threadIdx.x]) atomicAdd(&ctl->mode_items[threadIdx.x], s_st.mode_items[threadIdx.x]);
+    if (s_st.mode_work[threadIdx.x]) atomicAdd(&ctl->mode_work[threadIdx.x], s_st.mode_work[threadIdx.x]);
+  }
+  if (threadIdx.x == 3 && s_st.rev_work) atomicAdd(&ctl->rev_work, s_st.rev_work);
+  if (vblock() != 0) return;
+  if (threadIdx.x < 42) {
+    ctl->pbin_ns[threadIdx.x] += s_st.pbin_ns[threadIdx.x];
+    ctl->pbin_rounds[threadIdx.x] += s_st.pbin_rounds[threadIdx.x];
+    ctl->pbin_est[threadIdx.x] += s_st.pbin_est[threadIdx.x];
+  }
+  if (threadIdx.x < 3) ctl->phase_ns[threadIdx.x] += s_st.phase_ns[threadIdx.x];
+  if (threadIdx.x == 0) {
+    ctl->rounds += s_st.rounds;
+    ctl->scanned += s_st.scanned;
+    ctl->n_small += s_st.n_small;
+    ctl->n_big += s_st.n_big;
+    ctl->n_huge += s_st.n_huge;
+    ctl->advances += s_st.advances;
+  }
+}
+
 // All rounds of one peel instance, run by its CTAs; false when a bounded wait ran out or an
 // invariant broke (recorded in ctl->err).
 template <bool kWing>
@@ -905,41 +936,78 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
   Shared& S = *reinterpret_cast<Shared*>(smem_raw);
   uint32_t* pool = reinterpret_cast<uint32_t*>(smem_raw + ((sizeof(Shared) + 15) & ~size_t(15)));
   const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  uint32_t* wkeys = pool + warp * (3 * kWarpSlots);  // keys, values, hit counters
-  uint32_t* wvals = wkeys + kWarpSlots;
+  uint32_t* wkeys = pool + warp * (kWing ? 3 * kWingWarpSlots : 2 * kTipWarpSlots);
   const unsigned gtid = vblock() * kPT + threadIdx.x;
   const unsigned gthreads = vgrid() * kPT;
+  const bool cta0 = vblock() == 0;
+  WarpQueue Q{S.queue[warp], 0u};
+  for (unsigned i = threadIdx.x; i < sizeof(Stats) / 8; i += kPT) reinterpret_cast<unsigned long long*>(&s_st)[i] = 0;
+  if (threadIdx.x == 0) {
+    s_bar_target = *(volatile unsigned long long*)&ctl->bar_base;
+    s_bar_timeout = ctl->barrier_timeout_ns;
+    s_skip_arrival = vblock() == 0 ? ctl->test_skip_arrival : 0u;
+    s_err = 0;
+  }
   unsigned alist_cur = *(volatile unsigned*)&ctl->alist_cur;
   const bool range = *(volatile unsigned*)&ctl->range_mode != 0;
+  const bool trace = cta0 && ctl->trace != 0;
   unsigned part_idx = *(volatile unsigned*)&ctl->npart;  // partitions opened (range mode)
+  unsigned alive = *(volatile unsigned*)&ctl->alive;     // kept per CTA: every CTA sees the frontier sizes
+  unsigned near_done = *(volatile unsigned*)&ctl->near_done;
+  const unsigned at_compact = *(volatile unsigned*)&ctl->alive_at_compact;
+  const unsigned min_gain = *(volatile unsigned*)&ctl->min_gain;
+  // Near items a window opens with: near_min, but no more than four per thread (a round scans the
+  // near list once, so on few CTAs a long list costs more than the advances it saves).
+  const unsigned near_min = min(ctl->near_min, 4u * gthreads);
+  const unsigned near_div = max(1u, ctl->near_div);
   unsigned long long work = 0;
+  __syncthreads();
   if (!*(volatile unsigned*)&ctl->started) {
     for (int64_t x = gtid; x < W.N; x += gthreads)
       W.alist[0][x] = W.items ? W.items[W.item0 + x] : W.item0 + (uint32_t)x;
     if (!grid_barrier(ctl)) return false;
-    if (vblock() == 0 && threadIdx.x == 0) ctl->started = 1;
+    if (cta0 && threadIdx.x == 0) ctl->started = 1;
   }
+  const bool trace_est = ctl->trace != 0;
+  // What the last barrier of a round hands to the next one: the next minimum and the near list's
+  // length; the window bound changes only in an advance; the frontier sizes of the last round.
+  const unsigned long long r0 = *(volatile unsigned long long*)&ctl->round;
+  unsigned long long next_k = *(volatile unsigned long long*)&ctl->nm[r0 & 1ull];
+  unsigned near_len = (unsigned)*(volatile unsigned long long*)&ctl->near_len;
+  unsigned long long win_hi = *(volatile unsigned long long*)&ctl->win_hi;
+  unsigned ps = (unsigned)(*(volatile unsigned long long*)&ctl->fsmall[(r0 & 1ull) ^ 1ull] >> 32);
+  unsigned pg = (unsigned)(*(volatile unsigned long long*)&ctl->fbig[(r0 & 1ull) ^ 1ull] >> 32);
+  unsigned ph = (unsigned)(*(volatile unsigned long long*)&ctl->fhuge[(r0 & 1ull) ^ 1ull] >> 32);
+  // Tip: flat items of the previous round whose counters are still to be cleared.
+  unsigned clear_n = 0, clear_nh = 0;
 
-  for (unsigned long long r = *(volatile unsigned long long*)&ctl->round;; ++r) {
+  for (unsigned long long r = r0;; ++r) {
     const unsigned par = (unsigned)(r & 1ull), npar = par ^ 1u;
-    const unsigned alive = *(volatile unsigned*)&ctl->alive;
-    if (alive == 0) break;
     // Pause at a round boundary once enough items have been peeled since the lists were last
-    // compacted; the host compacts them and relaunches (all CTAs see the same values here).
-    const unsigned at_compact = *(volatile unsigned*)&ctl->alive_at_compact;
-    if (2u * alive < at_compact && at_compact - alive >= *(volatile unsigned*)&ctl->min_gain) {
-      if (vblock() == 0 && threadIdx.x == 0) {
+    // compacted; the host compacts them and relaunches (all CTAs hold the same values here).
+    const bool pause = alive != 0 && 2u * alive < at_compact && at_compact - alive >= min_gain;
+    if (alive == 0 || pause) {
+      if (!kWing && clear_n) {
+        Acc none{kInf, 0};
+        tip_items_flat(G, W, ctl, W.fhuge[npar], clear_nh, W.front[npar] + (W.N - 1), clear_n, true, S, none);
+      }
+      if (cta0 && threadIdx.x == 0) {
         ctl->round = r;
         ctl->alist_cur = alist_cur;
+        ctl->alive = alive;
+        ctl->near_done = near_done;
+        ctl->bar_base = s_bar_target;
+        ctl->part_done += s_st.part_done;
       }
       break;
     }
-    unsigned long long k = *(volatile unsigned long long*)&ctl->nm[par];
+    unsigned long long k = next_k;
     if (k == kInf) {
       unsigned long long part_target_next = 0, part_ratio_next = 0;  // range mode
       // ---- window advance (no unpeeled item left in the near list): compact the alive list
       // and take its minimum; a log2 histogram of distances to the minimum picks the window
-      // bound; the near list is rebuilt from the alive list.
+      // bound; the near list is rebuilt from the alive list.  Unpeeled items lie above the old
+      // bound here: their bucket is their count.
       const unsigned na = alist_cur ^ 1u;
       const unsigned alen = *(volatile unsigned*)&ctl->alen[alist_cur];
       unsigned long long mn = kInf;
@@ -947,43 +1015,48 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
         const uint32_t x = W.alist[alist_cur][q];
         if (W.state[x] != ALIVE) continue;
         W.alist[na][atomicAdd(&ctl->alen[na], 1u)] = x;
-        // No unpeeled item is in the near list here, and items outside it were queued only
-        // when they fell below the bound: their bucket is their count.
         const int64_t c = W.cnt[x];
-        W.D[x] = c;
+        if (range) W.D[x] = c;
         mn = min(mn, (unsigned long long)c);
       }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
       if (lane == 0 && mn != kInf) atomicMin(&ctl->k_lo, mn);
       if (threadIdx.x < 66) S.hist[threadIdx.x] = 0;
-      if (vblock() == 0) {
+      if (cta0) {
         // The previous advance's histograms were last read before two barriers ago.
         if (threadIdx.x < 66) {
           ctl->hist[threadIdx.x] = 0;
           ctl->whist[threadIdx.x] = 0;
         }
         if (range && threadIdx.x < 256) ctl->wsub[threadIdx.x] = 0;
-        if (threadIdx.x == 0) ctl->near_len = 0;
+        if (threadIdx.x == 0) {
+          ctl->near_len = 0;
+          if (range) {
+            ctl->part_done += s_st.part_done;
+            s_st.part_done = 0;
+          }
+        }
       }
       if (!grid_barrier(ctl)) return false;
+      near_done = 0;
       if (range) {
         ++part_idx;  // the window opened here is partition part_idx - 1
-        if (vblock() == 0 && threadIdx.x == 0) ctl->npart = part_idx;
+        if (cta0 && threadIdx.x == 0) ctl->npart = part_idx;
       }
       const unsigned long long klo = *(volatile unsigned long long*)&ctl->k_lo;
       const unsigned alen2 = *(volatile unsigned*)&ctl->alen[na];
       unsigned long long hi = kInf;
       if (!range) {
         for (unsigned q = gtid; q < alen2; q += gthreads) {
-          const unsigned long long d = (unsigned long long)W.D[W.alist[na][q]] - klo;
+          const unsigned long long d = (unsigned long long)W.cnt[W.alist[na][q]] - klo;
           atomicAdd(&S.hist[d ? 64 - __clzll(d) : 0], 1u);
         }
         __syncthreads();
         if (threadIdx.x < 66 && S.hist[threadIdx.x]) atomicAdd(&ctl->hist[threadIdx.x], S.hist[threadIdx.x]);
         if (!grid_barrier(ctl)) return false;
         // Every CTA derives the same bound: the smallest B with >= target items at distance < 2^B.
-        const unsigned target = max(ctl->near_min, alen2 / max(1u, ctl->near_div));
+        const unsigned target = max(near_min, alen2 / near_div);
         unsigned cum = 0;
         int B = 0;
         for (; B < 65; ++B) {
@@ -1003,7 +1076,7 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
         __syncthreads();
         for (unsigned q = gtid; q < alen2; q += gthreads) {
           const uint32_t x = W.alist[na][q];
-          const unsigned long long d = (unsigned long long)W.D[x] - klo;
+          const unsigned long long d = (unsigned long long)W.cnt[x] - klo;
           atomicAdd(&wh[d ? 64 - __clzll(d) : 0], (unsigned long long)W.wgt[x]);
         }
         __syncthreads();
@@ -1014,8 +1087,8 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
         const unsigned long long used = *(volatile unsigned long long*)&ctl->part_used;
         unsigned long long ratio_q = *(volatile unsigned long long*)&ctl->part_ratio_q;
         if (used > 0 && done > 0) {
-          const unsigned long long r = min(done * 256ull / used, 256ull * 4096ull);
-          ratio_q = ratio_q ? (ratio_q + r) / 2 : r;
+          const unsigned long long rq = min(done * 256ull / used, 256ull * 4096ull);
+          ratio_q = ratio_q ? (ratio_q + rq) / 2 : rq;
         }
         const unsigned long long target = max(1ull, ratio_q > 256 ? base * 256ull / ratio_q : base);
         part_target_next = target;
@@ -1036,7 +1109,7 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
           __syncthreads();
           for (unsigned q = gtid; q < alen2; q += gthreads) {
             const uint32_t x = W.alist[na][q];
-            const unsigned long long d = (unsigned long long)W.D[x] - klo;
+            const unsigned long long d = (unsigned long long)W.cnt[x] - klo;
             if (d >= lo_d && d < lo_d + width)
               atomicAdd(&wh[(unsigned)((d - lo_d) * 256ull / width)], (unsigned long long)W.wgt[x]);
           }
@@ -1055,376 +1128,273 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
       }
       for (unsigned q = gtid; q < alen2; q += gthreads) {
         const uint32_t x = W.alist[na][q];
-        if (hi == kInf || (unsigned long long)W.D[x] < hi) {
-          W.in_near[x] = 1;
-          W.near[atomicAdd(&ctl->near_len, 1u)] = x;
-        }
+        if (hi == kInf || (unsigned long long)W.cnt[x] < hi) W.near[atomicAdd(&ctl->near_len, 1ull)] = x;
       }
-      if (vblock() == 0 && threadIdx.x == 0) {
+      if (cta0 && threadIdx.x == 0) {
         ctl->win_hi = hi;
         ctl->alen[alist_cur] = 0;  // read by every CTA before the first barrier
         ctl->k_lo = kInf;          // read by every CTA right after the first barrier
+        s_st.advances += 1;
       }
       alist_cur = na;
-      if (!grid_barrier(ctl)) return false;
-      phase_mark(ctl, 0);
-      if (vblock() == 0 && threadIdx.x == 0) {
-        ctl->advances += 1;
-        if (range) {  // every CTA read the previous values before this barrier
-          ctl->part_used = part_target_next;
-          ctl->part_ratio_q = part_ratio_next;
-          ctl->part_done = 0;
-        }
+      if (!grid_barrier(ctl, &ctl->near_len)) return false;
+      near_len = (unsigned)s_words[0];
+      win_hi = hi;
+      phase_mark(trace, 0);
+      if (range && cta0 && threadIdx.x == 0) {  // every CTA read the previous values before this barrier
+        ctl->part_used = part_target_next;
+        ctl->part_ratio_q = part_ratio_next;
+        ctl->part_done = 0;
       }
       k = klo;
     }
-    const unsigned long long win_hi = *(volatile unsigned long long*)&ctl->win_hi;
-    if (threadIdx.x == 0) s_win_hi = win_hi;
-    __syncthreads();
-    // ---- phase F: the frontier is every near item in bucket k; the minimum of the other near
-    // items is the first part of the next round's minimum.
+    const unsigned char act = (unsigned char)(1u + par);
+    if (threadIdx.x == 0) {
+      s_win_hi = win_hi;
+      s_k = (long long)k;
+      s_act = act;
+    }
+    // ---- phase F: the frontier is every near item in bucket k (range mode: every near item not
+    // taken yet); the minimum of the other near items is the first part of the next round's
+    // minimum.  Four items per thread are loaded at a time.
     {
-      const unsigned nl = *(volatile unsigned*)&ctl->near_len;
+      const unsigned nl = near_len;
+      // The previous round's frontier (ps, pg, ph items) becomes PEELED.
       unsigned long long mn = kInf;
-      for (unsigned q = gtid; q < nl; q += gthreads) {
-        const uint32_t x = W.near[q];
-        if (W.state[x] != ALIVE) continue;
-        const unsigned long long d = (unsigned long long)W.D[x];
-        if (range || d == k) {
-          W.state[x] = ACTIVE;
-          bool small, huge;
-          int64_t cost;
-          uint32_t wunits_of = 1;
+      unsigned long long est = 0;
+      for (unsigned q0 = near_done + gtid; q0 < nl; q0 += 4 * gthreads) {
+        uint32_t xs[4];
+        uint8_t st[4];
+        long long cs[4];
+#pragma unroll
+        for (unsigned i = 0; i < 4; ++i) {
+          const unsigned q = q0 + i * gthreads;
+          xs[i] = q < nl ? W.near[q] : kEmpty;
+        }
+#pragma unroll
+        for (unsigned i = 0; i < 4; ++i) {
+          st[i] = PEELED;
+          cs[i] = 0;
+          if (xs[i] != kEmpty) {
+            st[i] = W.state[xs[i]];
+            cs[i] = W.cnt[xs[i]];
+          }
+        }
+#pragma unroll 1
+        for (unsigned i = 0; i < 4; ++i) {
+          const uint32_t x = xs[0];
+          const uint8_t sx = st[0];
+          const long long c = cs[0];
+          xs[0] = xs[1]; xs[1] = xs[2]; xs[2] = xs[3];
+          st[0] = st[1]; st[1] = st[2]; st[2] = st[3];
+          cs[0] = cs[1]; cs[1] = cs[2]; cs[2] = cs[3];
+          if (sx != ALIVE) continue;
+          if (!range && c > (long long)k) {
+            mn = min(mn, (unsigned long long)c);
+            continue;
+          }
+          W.state[x] = act;
+          if (range) W.part_out[x] = part_idx - 1;
+          else W.D[x] = (int64_t)k;
+          // An item without live butterflies gets no units: nothing is left to remove.
           if (kWing) {
-            const uint32_t v = G.center_of[x], u = G.u_of[x];
-            const int64_t cv = cls.cost_v(G, v, u), cu = cls.cost_u(G, v, u);
-            const bool fv = cv <= cu;
-            cost = fv ? cv : cu;
-            const uint32_t psize = fv ? G.offK[u + 1] - G.offK[u] : G.offC[v + 1] - G.offC[v];
-            // Warp-unit setting: every item whose probe set fits a warp table runs on warps, cut
-            // into warp units of about chunk_work probes (first-level slices).  Otherwise only
-            // items of at most small_work probes run on warps, whole.
-            small = 2 * psize <= (uint32_t)kWarpSlots && (cls.warp_units || cost <= cls.small_work);
-            huge = !small && cost > cls.huge_work && W.gshared != nullptr;
-            if (small && cls.warp_units) {
-              const int64_t d1 = fv ? G.offC[v + 1] - G.offC[v] : G.offK[u + 1] - G.offK[u];
-              int64_t units = (cost + cls.chunk_work - 1) / cls.chunk_work;
-              units = min(units, min(d1, (int64_t)4096));
-              wunits_of = (uint32_t)max(units, (int64_t)1);
-            }
+            const uint32_t inf = G.info[x], v = G.center_of[x], u = G.u_of[x];
+            const bool fv = (inf & kInfoFromV) != 0;
+            const unsigned long long add = (1ull << 32) | (c != 0 ? inf & kInfoUnits : 0u);
+            const bool small = (inf & kInfoSmall) != 0;
+            const unsigned long long at = atomicAdd(small ? &ctl->fsmall[par] : &ctl->fbig[par], add);
+            const uint32_t pos = (uint32_t)(at >> 32);
+            W.front[par][small ? (int64_t)pos : W.N - 1 - pos] =
+                make_uint4(x, (fv ? u : v) | (inf & kInfoFromV), fv ? v : u, (uint32_t)at);
+            if (range || trace_est) est += item_weight<kWing>(G, cls, x) - 1ull;
           } else {
-            cost = G.wk[x];
-            small = cls.tip_small(G, x);
-            huge = !small && cls.tip_huge(G, x) && W.gshared != nullptr;
+            const int64_t wk = G.wk[x];
+            const uint32_t b = G.offK[x], d = G.offK[x + 1] - b;
+            const unsigned long long pairs = c != 0 ? (unsigned long long)wk + d : 0ull;
+            const uint4 it = make_uint4(x, b, d, (uint32_t)min(pairs, 0xFFFFFFFFull));
+            const unsigned long long add = (1ull << 32) | 1ull;
+            if (cls.tip_small(G, x)) {
+              W.front[par][atomicAdd(&ctl->fsmall[par], add) >> 32] = it;
+            } else if (cls.tip_huge(G, x) && W.gshared != nullptr) {
+              W.fhuge[par][atomicAdd(&ctl->fhuge[par], add) >> 32] = it;
+            } else {
+              W.front[par][W.N - 1 - (int64_t)(atomicAdd(&ctl->fbig[par], add) >> 32)] = it;
+            }
+            est += (unsigned long long)(wk > 0 ? wk : 0);
           }
-          atomicAdd(&ctl->round_est[par], (unsigned long long)(cost > 0 ? cost : 0));
-          if (small) {
-            const unsigned at = atomicAdd(&ctl->flen_small[par], 1u);
-            W.fsmall[par][at] = x;
-            if (kWing) W.fwchunks[par][at] = wunits_of;
-          }
-          else if (huge) W.fhuge[par][atomicAdd(&ctl->flen_huge[par], 1u)] = x;
-          else {
-            const unsigned at = atomicAdd(&ctl->flen_big[par], 1u);
-            W.fbig[par][at] = x;
-            const int64_t c = cost < 1 ? 1 : (cost > 0x7fffffff ? 0x7fffffff : cost);
-            W.fchunks[par][at] = (uint32_t)c;  // cost for now; CTA 0 turns it into a unit count
-            atomicAdd(&ctl->round_cost[par], (unsigned long long)c);
-          }
-        } else {
-          mn = min(mn, d);
         }
       }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
       if (lane == 0 && mn != kInf) atomicMin(&ctl->nm[npar], mn);
-      if (vblock() == 0 && threadIdx.x == 0) {  // slots of the previous round, no longer read
-        ctl->flen_small[npar] = 0;
-        ctl->flen_big[npar] = 0;
-        ctl->flen_huge[npar] = 0;
-        ctl->round_cost[npar] = 0;
-        ctl->round_est[npar] = 0;
-        ctl->tlen[npar] = 0;
-        ctl->cur_small[npar] = 0;
-        ctl->cur_big[npar] = 0;
-        ctl->scanned += nl;
+      if ((range || trace_est) && __any_sync(0xffffffffu, est != 0)) {
+        est = warp_sum(est);
+        if (lane == 0) atomicAdd(&ctl->round_est[par], est);
       }
+      for (unsigned q = gtid; q < ps + pg + ph; q += gthreads) {
+        const uint32_t x = q < ps ? W.front[npar][q].x
+                                  : (q < ps + pg ? W.front[npar][W.N - 1 - (q - ps)].x : W.fhuge[npar][q - ps - pg].x);
+        W.state[x] = PEELED;
+      }
+      if (!kWing && clear_n) {
+        Acc none{kInf, 0};
+        tip_items_flat(G, W, ctl, W.fhuge[npar], clear_nh, W.front[npar] + (W.N - 1), clear_n, true, S, none);
+        clear_n = 0;
+      }
+      if (cta0 && threadIdx.x == 0) s_st.scanned += nl - near_done;
+      if (range) near_done = nl;
     }
-    if (!grid_barrier(ctl)) return false;
-    phase_mark(ctl, 1);
+    if (!grid_barrier(ctl, &ctl->fsmall[par], &ctl->fbig[par], &ctl->fhuge[par])) return false;
+    phase_mark(trace, 1);
     // ---- phase P: process the frontier (small items per warp, then heavy items per CTA).
+    Acc A{kInf, 0};
+    const unsigned ns = (unsigned)(s_words[0] >> 32), nwu = (unsigned)s_words[0];
+    const unsigned nb = (unsigned)(s_words[1] >> 32), nu = (unsigned)s_words[1];
+    const unsigned nh = kWing ? 0u : (unsigned)(s_words[2] >> 32);
+    ps = ns;
+    pg = nb;
+    ph = nh;
+    unsigned long long round_est = 0;
+    if (cta0 && threadIdx.x == 0) {
+      if (range || trace) round_est = *(volatile unsigned long long*)&ctl->round_est[par];
+      ctl->nm[par] = kInf;  // every CTA has read it
+      // Slots of the previous round: last read in phase F.
+      ctl->fsmall[npar] = 0;
+      ctl->fbig[npar] = 0;
+      ctl->fhuge[npar] = 0;
+      ctl->round_est[npar] = 0;
+      ctl->cur_small[npar] = 0;
+      ctl->cur_big[npar] = 0;
+      s_st.rounds += 1;
+      s_st.n_small += ns;
+      s_st.n_big += nb;
+      s_st.n_huge += nh;
+      s_st.part_done += round_est;
+    }
+    alive -= ns + nb + nh;
     {
-      if (vblock() == 0 && threadIdx.x == 0) ctl->nm[par] = kInf;  // every CTA has read it
-      const unsigned ns = *(volatile unsigned*)&ctl->flen_small[par];
-      if (!kWing) {
-        while (true) {
-          unsigned q = 0;
-          if (lane == 0) q = atomicAdd(&ctl->cur_small[par], 1u);
-          q = __shfl_sync(0xffffffffu, q, 0);
-          if (q >= ns) break;
-          const uint32_t x = W.fsmall[par][q];
-          if (W.cnt[x] == 0) continue;  // no live butterfly contains x: nothing to remove
-          tip_item_warp(G, W, ctl, par, x, wkeys, wvals, work);
-        }
-      } else if (ns) {
-        // Warp units: the exclusive prefix of the warp items' unit counts (every CTA computes it
-        // in shared memory up to kLocalUnits items, else CTA 0 in global memory behind a
-        // barrier); warps claim runs of consecutive units and process an item's units of a
-        // run as one first-level slice, independently of the other warps.
-        const bool wlocal = ns <= kLocalUnits;
-        if (wlocal || vblock() == 0) {
-          uint32_t carry = 0;
-          for (uint32_t j0 = 0; j0 < ns; j0 += kPT) {
-            const uint32_t j = j0 + threadIdx.x;
-            const uint32_t c = j < ns ? W.fwchunks[par][j] : 0u;
-            uint32_t T;
-            const uint32_t incl = block_incl_scan(c, S.scan, T);
-            if (j < ns) {
-              if (wlocal) S.uprefix[j] = carry + incl - c;
-              else W.wprefix[j] = carry + incl - c;
-            }
-            carry += T;
-          }
-          if (threadIdx.x == 0) {
-            if (wlocal) S.uprefix[ns] = carry;
-            else {
-              W.wprefix[ns] = carry;
-              ctl->wunits = carry;
-            }
-          }
-        }
-        if (wlocal) __syncthreads();
-        else if (!grid_barrier(ctl)) return false;
-        const uint32_t* wpre = wlocal ? S.uprefix : W.wprefix;
-        const unsigned nwu = wlocal ? S.uprefix[ns] : *(volatile unsigned*)&ctl->wunits;
-        const unsigned Kw = max(1u, nwu / (4u * vgrid() * (kPT / 32)));
-        while (true) {
-          unsigned u = 0;
-          if (lane == 0) u = atomicAdd(&ctl->cur_small[par], Kw);
-          u = __shfl_sync(0xffffffffu, u, 0);
-          if (u >= nwu) break;
-          uint32_t lo = 0, hi = ns;  // the last item whose prefix <= u, 32-way search
+      // Warp-level items: warps claim runs of consecutive units and process an item's units of a
+      // run as one first-level slice, independently of the other warps (tip: an item is one
+      // unit).  The first run of a warp is its own number; the cursor hands out the later ones.
+      const unsigned gwarps = vgrid() * kPW;
+      const unsigned Kw = kWing ? max(1u, nwu / (4u * gwarps)) : 1u;
+      const uint4* const fsm = W.front[par];
+      for (unsigned u = (vblock() * kPW + warp) * Kw; u < nwu;) {
+        const unsigned uend = min(u + Kw, nwu);
+        if (kWing) {
+          uint32_t lo = 0, hi = ns;  // the last item whose first unit <= u, 32-way search
           while (hi - lo > 1) {
             const uint32_t step = (hi - lo + 31) / 32;
             const uint32_t idx = lo + lane * step;
-            const bool le = idx < hi && wpre[idx] <= u;
+            const bool le = idx < hi && fsm[idx].w <= u;
             const unsigned bal = __ballot_sync(0xffffffffu, le);
-            lo = lo + (31 - __clz(bal)) * step;
+            lo = lo + (31 - __clz(bal)) * step;  // lane 0 always qualifies
             hi = min(lo + step, hi);
           }
-          const unsigned uend = min(u + Kw, nwu);
           for (unsigned uu = u, q = lo; uu < uend; ++q) {  // uniform across the warp
-            const uint32_t base = wpre[q], next = wpre[q + 1];
+            const uint4 it = fsm[q];
+            const uint32_t next = q + 1 < ns ? fsm[q + 1].w : nwu;
             const uint32_t c1 = min(uend, next);
-            const uint32_t x = W.fsmall[par][q];
-            if (W.cnt[x] != 0) {  // no live butterfly contains x: nothing to remove
-              WingEdge E;
-              E.e1 = x;
-              E.v = G.center_of[x];
-              E.u = G.u_of[x];
-              E.from_v = cls.wing_from_v(G, E.v, E.u);
-              wing_item<LV_WARP>(G, W, ctl, par, E, wkeys, wvals, kWarpSlots, nullptr, work, uu - base, next - base,
-                                 c1 - base);
-            }
-            uu = c1;
+            if (c1 > uu) wing_item<LV_WARP>(G, W, ctl, it, wkeys, S, Q, A, uu - it.w, next - it.w, c1 - it.w);
+            uu = max(uu, c1);
           }
+        } else {
+          const uint4 it = fsm[u];
+          if (it.w) tip_item_warp(G, W, ctl, it.x, wkeys, wkeys + kTipWarpSlots, Q, A);
         }
+        if (gwarps * Kw >= nwu) break;
+        unsigned c = 0;
+        if (lane == 0) c = atomicAdd(&ctl->cur_small[par], Kw);
+        u = gwarps * Kw + __shfl_sync(0xffffffffu, c, 0);
       }
-      __syncthreads();  // warp tables and the CTA table share memory
-      const unsigned nb = *(volatile unsigned*)&ctl->flen_big[par];
-      if (nb) {
-        // Units: the exclusive prefix of the items' unit counts; every CTA then pulls units
-        // (item, slice) from a shared cursor.  Up to kLocalUnits items every CTA computes the
-        // same prefix in its shared memory (from the costs phase F froze), so no grid barrier
-        // is needed; beyond that CTA 0 lays it out in global memory behind a barrier.
-        const bool local = nb <= kLocalUnits;
-        if (local || vblock() == 0) {
-          uint32_t carry = 0;
-          // Unit size: about cls.units_per_cta units per CTA over the round's CTA-level work,
-          // never below cls.chunk_work probes or four probe-set sizes (each unit rebuilds its
-          // probe table).
-          const unsigned long long rc = *(volatile unsigned long long*)&ctl->round_cost[par];
-          const int64_t target =
-              max((int64_t)cls.chunk_work, (int64_t)(rc / ((unsigned long long)cls.units_per_cta * vgrid())));
-          for (uint32_t j0 = 0; j0 < nb; j0 += kPT) {
-            const uint32_t j = j0 + threadIdx.x;
-            uint32_t c = 0;
-            if (j < nb) {
-              if (kWing) {
-                const uint32_t x = W.fbig[par][j];
-                const uint32_t v = G.center_of[x], u = G.u_of[x];
-                const bool fv = cls.wing_from_v(G, v, u);
-                const int64_t psize = fv ? G.offK[u + 1] - G.offK[u] : G.offC[v + 1] - G.offC[v];
-                const int64_t d1 = fv ? G.offC[v + 1] - G.offC[v] : G.offK[u + 1] - G.offK[u];
-                const int64_t unit = max(target, 4 * psize);
-                int64_t k = ((int64_t)W.fchunks[par][j] + unit - 1) / unit;
-                k = min(k, min(d1, (int64_t)4096));
-                c = (uint32_t)max(k, (int64_t)1);
-              } else {
-                c = 1;
-              }
-              if (!local) W.fchunks[par][j] = c;
-            }
-            uint32_t T;
-            const uint32_t incl = block_incl_scan(c, S.scan, T);
-            if (j < nb) {
-              if (local) S.uprefix[j] = carry + incl - c;
-              else W.uprefix[j] = carry + incl - c;
-            }
-            carry += T;
-          }
-          if (threadIdx.x == 0) {
-            if (local) {
-              S.uprefix[nb] = carry;
-            } else {
-              W.uprefix[nb] = carry;
-              ctl->units = carry;
-            }
-          }
-        }
-        if (local) __syncthreads();
-        else if (!grid_barrier(ctl)) return false;
-        const uint32_t* upre = local ? S.uprefix : W.uprefix;
-        const unsigned nu = local ? S.uprefix[nb] : *(volatile unsigned*)&ctl->units;
+      if (ns) __syncthreads();  // warp tables and the CTA table share memory
+      // Tip items: the huge ones run over the whole grid, in waves of up to ngroups; when the
+      // round has so few CTA-level items that one wave holds them all, they run there too (one
+      // CTA per item leaves the rest of the grid idle: rounds of 2^12 wedges took 40 us in phase
+      // P on one CTA each, 24 us spread over the grid).
+      const unsigned ng = kWing ? 0u : (W.gshared ? min(W.ngroups, kMaxGroups) : 0u);
+      const bool flat_all = !kWing && vgrid() >= 8 && nb + nh > 0 && nb + nh <= ng;
+      if (nu && !flat_all) {
         // CTAs claim runs of K consecutive units (wing: about a quarter of a CTA's share; tip: one
         // unit, which is one item); the units of one item inside a run are processed as one
-        // slice, so the item's probe table is built once per run, not once per unit.
-        const unsigned K = kWing ? max(1u, nu / (4u * vgrid())) : 1u;
-        while (true) {
-          if (threadIdx.x < 32) {  // warp 0: take a run, find the item of its first unit, 32-way
-            unsigned u = 0;
-            if (lane == 0) u = atomicAdd(&ctl->cur_big[par], K);
-            u = __shfl_sync(0xffffffffu, u, 0);
-            uint32_t lo = 0, hi = nb;  // answer in [lo, hi): the last item whose prefix <= u
-            if (u < nu) {
-              while (hi - lo > 1) {
-                const uint32_t step = (hi - lo + 31) / 32;
-                const uint32_t idx = lo + lane * step;
-                const bool le = idx < hi && upre[idx] <= u;
-                const unsigned bal = __ballot_sync(0xffffffffu, le);
-                const uint32_t last = 31 - __clz(bal);  // lane 0 always qualifies (prefix[lo] <= u)
-                lo = lo + last * step;
-                hi = min(lo + step, hi);
-              }
-            }
-            if (lane == 0) {
-              S.item = u;
-              S.hist[0] = lo;
-            }
-          }
-          __syncthreads();
-          const unsigned u0 = S.item, q0 = S.hist[0];
-          __syncthreads();
-          if (u0 >= nu) break;
+        // slice, so the item's probe table is built once per run, not once per unit.  The first
+        // run of a CTA is its own number; the cursor hands out the later ones.
+        const uint4* const fbg = W.front[par] + (W.N - 1);  // item q: fbg[-q]
+        const unsigned K = kWing ? max(1u, (unsigned)(nu / ((unsigned)cls.units_per_cta * vgrid()))) : 1u;
+        const bool more = vgrid() * K < nu;  // some run is left for the cursor
+        for (unsigned u0 = vblock() * K; u0 < nu;) {
           const unsigned uend = min(u0 + K, nu);
-          for (unsigned uu = u0, q = q0; uu < uend; ++q) {  // uniform across the CTA
-            const uint32_t base = upre[q], next = upre[q + 1];
-            const uint32_t c1 = min(uend, next);
-            const uint32_t x = W.fbig[par][q];
-            if (W.cnt[x] != 0) {  // no live butterfly contains x: nothing to remove
-              if (kWing) {
-                WingEdge E;
-                E.e1 = x;
-                E.v = G.center_of[x];
-                E.u = G.u_of[x];
-                E.from_v = cls.wing_from_v(G, E.v, E.u);
-                wing_item<LV_BLOCK>(G, W, ctl, par, E, pool, pool + kBlockSlots, kBlockSlots, &S, work, uu - base,
-                                    next - base, c1 - base);
-              } else {
-                tip_item_block(G, W, ctl, par, x, pool, S, work);
-              }
+          if (more && threadIdx.x == 0) S.item = atomicAdd(&ctl->cur_big[par], K);
+          if (kWing) {
+            uint32_t lo = 0, hi = nb;  // the last item whose first unit <= u0, 32-way search by every warp
+            while (hi - lo > 1) {
+              const uint32_t step = (hi - lo + 31) / 32;
+              const uint32_t idx = lo + lane * step;
+              const bool le = idx < hi && fbg[-(int64_t)idx].w <= u0;
+              const unsigned bal = __ballot_sync(0xffffffffu, le);
+              lo = lo + (31 - __clz(bal)) * step;  // lane 0 always qualifies
+              hi = min(lo + step, hi);
             }
-            uu = c1;
+            for (unsigned uu = u0, q = lo; uu < uend; ++q) {  // uniform across the CTA
+              const uint4 it = fbg[-(int64_t)q];
+              const uint32_t next = q + 1 < nb ? fbg[-(int64_t)(q + 1)].w : nu;
+              const uint32_t c1 = min(uend, next);
+              if (c1 > uu) wing_item<LV_BLOCK>(G, W, ctl, it, pool, S, Q, A, uu - it.w, next - it.w, c1 - it.w);
+              uu = max(uu, c1);
+            }
+          } else {
+            const uint4 it = fbg[-(int64_t)u0];
+            if (it.w) tip_item_block(G, W, ctl, it.x, pool, S, Q, A);
+          }
+          if (!more) break;
+          __syncthreads();
+          u0 = vgrid() * K + S.item;
+          __syncthreads();
+        }
+      }
+      if constexpr (!kWing) if (nh || flat_all) {
+        const unsigned total = flat_all ? nb + nh : nh;
+        for (unsigned w0 = 0; w0 < total; w0 += ng) {
+          const unsigned n = min(ng, total - w0);
+          const unsigned in_huge = nh > w0 ? min(n, nh - w0) : 0u;
+          const uint4* hl = W.fhuge[par] + w0;
+          tip_items_flat(G, W, ctl, hl, in_huge, W.front[par] + (W.N - 1), n, false, S, A);
+          if (w0 + ng < total) {  // the slices are reused by the next wave
+            if (!grid_barrier(ctl)) return false;
+            tip_items_flat(G, W, ctl, hl, in_huge, W.front[par] + (W.N - 1), n, true, S, A);
+            if (!grid_barrier(ctl)) return false;
+          } else {
+            clear_n = n;
+            clear_nh = in_huge;
           }
         }
-      }
-      // Huge items: tip items in waves of up to ngroups at once, one per CTA group (equal
-      // splits of the instance's CTAs); otherwise one at a time over every CTA.
-      const unsigned nh = *(volatile unsigned*)&ctl->flen_huge[par];
-      const unsigned ng = kWing ? 1u : min(W.ngroups, vgrid());
-      if (!kWing && nh > 1 && ng > 1) {
-        const unsigned vg = vgrid(), vb = vblock();
-        for (unsigned w0 = 0; w0 < nh; w0 += ng) {
-          const unsigned gn = min(ng, nh - w0);
-          const unsigned grp = vb * gn / vg;
-          const unsigned g0 = (grp * vg + gn - 1) / gn, g1 = ((grp + 1) * vg + gn - 1) / gn;
-          const uint32_t x = W.fhuge[par][w0 + grp];
-          if (W.cnt[x] != 0 &&  // uniform across the group
-              !tip_item_group(G, W, ctl, par, x, S, work, vb - g0, g1 - g0, grp,
-                              W.gshared + (size_t)grp * (size_t)W.gshared_stride))
-            return false;
-          if (w0 + ng < nh && !grid_barrier(ctl)) return false;  // the slices are reused next wave
+        // The last wave's counters are cleared by the next round (its lists start at w0 = 0 when
+        // there was one wave; later waves are cleared here).
+        if (total > ng) {
+          const unsigned w0 = (total - 1) / ng * ng;
+          if (!grid_barrier(ctl)) return false;
+          tip_items_flat(G, W, ctl, W.fhuge[par] + w0, clear_nh, W.front[par] + (W.N - 1), clear_n, true, S, A);
+          clear_n = 0;
         }
-      }
-      for (unsigned q = 0; q < nh && (kWing || nh == 1 || ng <= 1); ++q) {
-        const uint32_t x = W.fhuge[par][q];
-        if (W.cnt[x] == 0) continue;  // frontier counts do not change during the phase
-        bool ok;
-        if (kWing) {
-          WingEdge E;
-          E.e1 = x;
-          E.v = G.center_of[x];
-          E.u = G.u_of[x];
-          E.from_v = cls.wing_from_v(G, E.v, E.u);
-          ok = wing_item<LV_GRID>(G, W, ctl, par, E, nullptr, nullptr, 0, &S, work);
-        } else {
-          ok = tip_item_grid(G, W, ctl, par, x, S, work);
-        }
-        if (!ok) return false;
       }
     }
-    if (!grid_barrier(ctl)) return false;
-    phase_mark(ctl, 2, vblock() == 0 && threadIdx.x == 0 ? *(volatile unsigned long long*)&ctl->round_est[par] : 0);
-    // ---- phase U: touched items move to bucket max(count, k) (all unpeeled items are above
-    // k here); those entering the window join the near list and feed the next minimum.
     {
-      const unsigned nt = *(volatile unsigned*)&ctl->tlen[par];
-      unsigned long long mn = kInf;
-      for (unsigned q = gtid; q < nt; q += gthreads) {
-        const uint32_t x = W.tlist[par][q];
-        W.touched[x] = 0;
-        if (W.state[x] != ALIVE) continue;
-        const int64_t c = W.cnt[x];
-        // Range mode keeps D (the count at the partition's start) and queues by count.
-        const int64_t nd = range ? c : (c > (int64_t)k ? c : (int64_t)k);
-        if (!range) W.D[x] = nd;
-        if ((unsigned long long)nd < win_hi) {
-          mn = min(mn, (unsigned long long)nd);
-          if (!W.in_near[x]) {
-            W.in_near[x] = 1;
-            W.near[atomicAdd(&ctl->near_len, 1u)] = x;
-          }
-        }
-      }
+      unsigned long long mn = A.mn;
+      if (__any_sync(0xffffffffu, mn != kInf)) {
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-      if (lane == 0 && mn != kInf) atomicMin(&ctl->nm[npar], mn);
-      const unsigned ns = *(volatile unsigned*)&ctl->flen_small[par];
-      const unsigned nb = *(volatile unsigned*)&ctl->flen_big[par];
-      const unsigned nh = *(volatile unsigned*)&ctl->flen_huge[par];
-      for (unsigned q = gtid; q < ns + nb + nh; q += gthreads) {
-        const uint32_t x = q < ns ? W.fsmall[par][q] : (q < ns + nb ? W.fbig[par][q - ns] : W.fhuge[par][q - ns - nb]);
-        W.state[x] = PEELED;
-        if (range) W.part_out[x] = part_idx - 1;
+        for (int o = 16; o > 0; o >>= 1) mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+        if (lane == 0) atomicMin(&ctl->nm[npar], mn);
       }
-      if (vblock() == 0 && threadIdx.x == 0) {
-        ctl->alive -= ns + nb + nh;
-        ctl->rounds += 1;
-        ctl->touched_total += nt;
-        ctl->n_small += ns;
-        ctl->n_big += nb;
-        ctl->n_huge += nh;
-        ctl->prev_items = ns + nb + nh;  // read by the next round's phase F after two barriers
-        if (range) ctl->part_done += *(volatile unsigned long long*)&ctl->round_est[par];
-      }
+      work += A.work;
     }
-    if (!grid_barrier(ctl)) return false;
-    phase_mark(ctl, 3);
+    if (!grid_barrier(ctl, &ctl->nm[npar], &ctl->near_len)) return false;
+    next_k = s_words[0];
+    near_len = (unsigned)s_words[1];
+    phase_mark(trace, 2, round_est);
   }
-  unsigned long long w = work;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-  if (lane == 0 && w) atomicAdd(&ctl->work, w);
+  work = warp_sum(work);
+  if (lane == 0 && work) atomicAdd(&ctl->work, work);
+  flush_stats(ctl);
   return true;
 }
 
@@ -1456,14 +1426,12 @@ __global__ void __launch_bounds__(kPT, kMinBlocks) peel_kernel(Lists G, const Li
 
 // ---- set-up kernels -------------------------------------------------------------------------
 __global__ void peel_init_kernel(const int64_t* __restrict__ counts, int64_t N, int64_t* D, int64_t* cnt,
-                                 uint8_t* state, uint8_t* in_near, uint32_t* touched) {
+                                 uint8_t* state) {
   for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < N; x += (int64_t)gridDim.x * blockDim.x) {
     const int64_t c = counts[x];
     D[x] = c;
     cnt[x] = c;
     state[x] = ALIVE;
-    in_near[x] = 0;
-    touched[x] = 0;
   }
 }
 
@@ -1530,7 +1498,7 @@ __global__ void live_degree_kernel(const uint32_t* __restrict__ off, const uint3
   for (int64_t x = warp; x < n; x += nwarps) {
     uint32_t c = 0;
     for (uint32_t p = off[x] + lane; p < off[x + 1]; p += 32)
-      c += state[kByEdge ? eid[p] : nbr[p]] != PEELED;
+      c += state[kByEdge ? eid[p] : nbr[p]] == ALIVE;
     c = warp_sum(c);
     if (lane == 0) deg[x] = c;
   }
@@ -1554,7 +1522,7 @@ __global__ void compact_lists_kernel(const uint32_t* __restrict__ off, const uin
       if (p < e) {
         y = nbr[p];
         id = eid ? eid[p] : 0u;
-        live = state[kByEdge ? id : y] != PEELED;
+        live = state[kByEdge ? id : y] == ALIVE;
       }
       const unsigned bal = __ballot_sync(0xffffffffu, live);
       if (live) {
@@ -1641,6 +1609,39 @@ __global__ void item_weight_kernel(Lists G, Classify cls, int64_t N, uint32_t* w
     const unsigned long long w = item_weight<kWing>(G, cls, (uint32_t)x);
     wgt[x] = (uint32_t)min(w, 0xFFFFFFFFull);
   }
+}
+
+// info[e]: how the item of edge e is peeled, from the current lists (the live lists shrink between
+// launches).  Units are slices of about `chunk` estimated probes, never below twice the probe set
+// (each unit rebuilds the probe table), at most one per first-level entry and 4096 in all;
+// chunk grows with the summed cost (*total) so that a frontier of all items stays below 2^32 units.
+// Warp-unit setting: every item whose probe set fits a warp table runs on warps, cut into units;
+// otherwise only items of at most small_work probes run on warps, whole.
+__global__ void wing_info_kernel(Lists G, Classify cls, int64_t N, const unsigned long long* __restrict__ total,
+                                 uint32_t* info) {
+  const int64_t chunk = max((int64_t)cls.chunk_work, (int64_t)(*total >> 30));
+  for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < N; x += (int64_t)gridDim.x * blockDim.x) {
+    const uint32_t v = G.center_of[x], u = G.u_of[x];
+    const int64_t cv = cls.cost_v(G, v, u), cu = cls.cost_u(G, v, u);
+    const bool fv = cv <= cu;
+    const int64_t cost = fv ? cv : cu;
+    const int64_t du = G.offK[u + 1] - G.offK[u], dv = G.offC[v + 1] - G.offC[v];
+    const int64_t psize = fv ? du : dv, d1 = fv ? dv : du;
+    const bool small = psize <= (int64_t)kWingWarpSet && (cls.warp_units || cost <= cls.small_work);
+    const int64_t unit = small ? chunk : max(chunk, 2 * psize);
+    int64_t units = small && !cls.warp_units ? 1 : (cost + unit - 1) / unit;
+    units = max((int64_t)1, min(units, min(d1, (int64_t)4096)));
+    info[x] = (uint32_t)units | (small ? kInfoSmall : 0u) | (fv ? kInfoFromV : 0u);
+  }
+}
+
+template <bool kWing>
+__global__ void total_weight_kernel(Lists G, Classify cls, int64_t N, unsigned long long* total) {
+  unsigned long long s = 0;
+  for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < N; x += (int64_t)gridDim.x * blockDim.x)
+    s += item_weight<kWing>(G, cls, (uint32_t)x);
+  s = warp_sum(s);
+  if ((threadIdx.x & 31) == 0 && s) atomicAdd(total, s);
 }
 
 // gid[x] = i for the items x in [base[i], base[i + 1]) (one CTA per range).
@@ -1772,8 +1773,12 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
   const bool two_phase_batch = batch && two_phase_req && g_recorder == nullptr;
 
   DevBuf<int64_t> cnt(N, s);
-  DevBuf<uint32_t> eti, iota, center_of, touched(N, s), alist0(N, s), alist1(N, s), nearl(N, s);
-  DevBuf<uint32_t> fs0(N, s), fs1(N, s), fb0(N, s), fb1(N, s), fh0(N, s), fh1(N, s), tl0(N, s), tl1(N, s);
+  DevBuf<uint32_t> eti, iota, center_of, alist0(N, s), alist1(N, s), nearl(N, s);
+  DevBuf<uint4> fr0(N, s), fr1(N, s), fh0, fh1;
+  if (!kWing) {
+    fh0.alloc(N, s);
+    fh1.alloc(N, s);
+  }
   // Independent instances (the graphs of a batch) or the whole input as one.
   std::vector<int64_t> pbase{0}, psize{N};
   std::vector<double> pweight{1.0};
@@ -1789,14 +1794,17 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
     }
     if (pbase.empty()) return res;
   }
-  // Grid-shared dense counters: tip peeling keeps one slice per CTA group (heavy items of a round
-  // run concurrently), up to 32 slices within kGsharedBudget.
+  // Grid-shared dense counters: tip peeling keeps one slice per heavy item of a wave (they run
+  // concurrently), up to 32 slices within kGsharedBudget.
   const int64_t gstride = std::max(G.nK, G.nC) + 1;
   const unsigned ngroups =
-      kWing ? 1u : (unsigned)std::max<int64_t>(1, std::min<int64_t>(kMaxGroups, kGsharedBudget / (4 * gstride)));
-  DevBuf<uint32_t> gshared((size_t)gstride * ngroups, s);
-  PB_CUDA_TRY(cudaMemsetAsync(gshared.get(), 0, gshared.bytes(), s));
-  DevBuf<uint8_t> state(N, s), in_near(N, s);
+      (unsigned)std::max<int64_t>(1, std::min<int64_t>(kMaxGroups, kGsharedBudget / (4 * gstride)));
+  DevBuf<uint32_t> gshared;
+  if (!kWing) {
+    gshared.alloc((size_t)gstride * ngroups, s);
+    PB_CUDA_TRY(cudaMemsetAsync(gshared.get(), 0, gshared.bytes(), s));
+  }
+  DevBuf<uint8_t> state(N, s);
   LiveSide liveK, liveC;
   liveK.n = G.nK;
   liveC.n = G.nC;
@@ -1808,10 +1816,19 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
     part.alloc(N, s);
   }
   PB_LAUNCH(peel_init_kernel, grid_for(N), 256, 0, s, counts, N, (two_phase || two_phase_batch) ? snap.get() : out,
-            cnt.get(), state.get(), in_near.get(), touched.get());
+            cnt.get(), state.get());
+  Classify cls{tune.small_work, tune.huge_work, tune.chunk_work, std::max<int64_t>(1, tune.units_per_cta),
+               tune.warp_units ? 1 : 0};
+  if (const char* e = getenv("PB_PEEL_WARP_UNITS")) cls.warp_units = atoi(e) != 0;  // diagnostic hook
+  // Thresholds may be lowered through the environment (tests use this to drive small graphs
+  // through the CTA- and grid-level paths).
+  if (const char* e = getenv("PB_PEEL_SMALL_WORK")) cls.small_work = atoll(e);
+  if (const char* e = getenv("PB_PEEL_HUGE_WORK")) cls.huge_work = atoll(e);
+  if (const char* e = getenv("PB_PEEL_CHUNK_WORK")) cls.chunk_work = atoll(e);
   // Work estimates of the lists a version holds: neighbour-degree sums (wing) or two-hop wedges
   // (tip).
   std::vector<std::unique_ptr<DevBuf<int64_t>>> work_bufs;
+  std::vector<std::unique_ptr<DevBuf<uint32_t>>> info_bufs;
   auto refresh_work = [&](Lists& L) {
     auto buf = std::make_unique<DevBuf<int64_t>>(kWing ? L.nK + L.nC : L.nK, s);
     if (kWing) {
@@ -1819,6 +1836,14 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
       if (L.nC)
         PB_LAUNCH(nbr_degree_sum_kernel, grid_for(L.nC * 32), 256, 0, s, L.offC, L.edgC, L.offK, L.nC, buf->get() + L.nK);
       L.S = buf->get();
+      auto info = std::make_unique<DevBuf<uint32_t>>(N, s);
+      DevBuf<unsigned long long> total(1, s);
+      PB_CUDA_TRY(cudaMemsetAsync(total.get(), 0, sizeof(unsigned long long), s));
+      PB_LAUNCH(total_weight_kernel<kWing>, grid_for(N), 256, 0, s, L, cls, N, total.get());
+      PB_LAUNCH(wing_info_kernel, grid_for(N), 256, 0, s, L, cls, N, total.get(), info->get());
+      L.info = info->get();
+      if (!two_phase) info_bufs.clear();
+      info_bufs.push_back(std::move(info));
     } else {
       PB_LAUNCH(tip_work_kernel, grid_for(L.nK * 32), 256, 0, s, L.offK, L.edgK, L.offC, L.nK, buf->get());
       L.wk = buf->get();
@@ -1840,7 +1865,7 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
     G.center_of = center_of.get();
     G.u_of = edgC0;  // edge ids are positions in the centre side's original lists
     refresh_work(G);
-    need_scratch = 2ull * g.max_deg > (uint64_t)kBlockSlots;
+    need_scratch = g.max_deg > kWingSet;
     scratch_len = std::max(G.nK, G.nC);
   } else {
     refresh_work(G);
@@ -1849,12 +1874,12 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
     PB_LAUNCH(max_i64_kernel, grid_for(G.nK), 256, 0, s, G.wk, G.nK, mx.get());
     unsigned long long hmx = 0;
     readback(&hmx, mx.get(), sizeof(hmx), s);
-    need_scratch = 2ull * hmx > (uint64_t)kBlockSlots;
+    need_scratch = 2ull * hmx > (uint64_t)kTipSlots;
     scratch_len = G.nK;
   }
   const Lists G0 = G;  // the full lists (version 0)
 
-  const size_t smem = ((sizeof(Shared) + 15) & ~size_t(15)) + (size_t)kBlockSlots * 3 * sizeof(uint32_t);
+  const size_t smem = ((sizeof(Shared) + 15) & ~size_t(15)) + (size_t)kPoolWords * sizeof(uint32_t);
   void (*kern)(Lists, const Lists*, Instances, Ctl*, Classify) = peel_kernel<kWing, 2>;
   if constexpr (!kWing) {
     if (!batch) kern = peel_kernel<false, 1>;
@@ -1875,39 +1900,20 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
     gscratch.alloc((size_t)grid * (size_t)scratch_len, s);
     PB_CUDA_TRY(cudaMemsetAsync(gscratch.get(), 0, gscratch.bytes(), s));
   }
-  DevBuf<uint32_t> fc0(N, s), fc1(N, s), upre(N + (int64_t)pbase.size() + 1, s);
-  DevBuf<uint32_t> fw0, fw1, wpre;  // warp units of wing items
-  if (kWing) {
-    fw0.alloc(N, s);
-    fw1.alloc(N, s);
-    wpre.alloc(N + (int64_t)pbase.size() + 1, s);
-  }
   Work W{};
   W.D = (two_phase || two_phase_batch) ? snap.get() : out;
   W.cnt = cnt.get();
   W.state = state.get();
-  W.in_near = in_near.get();
-  W.touched = touched.get();
   W.alist[0] = alist0.get();
   W.alist[1] = alist1.get();
   W.near = nearl.get();
-  W.fsmall[0] = fs0.get();
-  W.fsmall[1] = fs1.get();
-  W.fbig[0] = fb0.get();
-  W.fbig[1] = fb1.get();
-  W.fchunks[0] = fc0.get();
-  W.fchunks[1] = fc1.get();
-  W.uprefix = upre.get();
-  W.fwchunks[0] = fw0.get();
-  W.fwchunks[1] = fw1.get();
-  W.wprefix = wpre.get();
+  W.front[0] = fr0.get();
+  W.front[1] = fr1.get();
   W.fhuge[0] = fh0.get();
   W.fhuge[1] = fh1.get();
   W.gshared = gshared.get();
   W.gshared_stride = gstride;
   W.ngroups = ngroups;
-  W.tlist[0] = tl0.get();
-  W.tlist[1] = tl1.get();
   W.gscratch = gscratch.get();
   W.gscratch_len = scratch_len;
   W.N = N;
@@ -1927,6 +1933,11 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
   // host cannot step in between launches of a CUDA graph); so do per-graph instances.
   if (g_recorder != nullptr || batch) hctl.min_gain = 0xFFFFFFFFu;
   hctl.barrier_timeout_ns = kBarrierTimeoutNs;
+  const bool trace = [] {
+    const char* tr = getenv("PB_TRACE");
+    return tr && *tr && *tr != '0';
+  }();
+  hctl.trace = trace ? 1u : 0u;
   hctl.near_min = (unsigned)tune.near_min;
   hctl.near_div = (unsigned)tune.near_div;
   // Diagnostic hooks for the window size.
@@ -1937,14 +1948,6 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
   // wait runs out; checks that a timeout comes back as PB_ETIMEOUT with the context usable.
   if (const char* e = getenv("PB_PEEL_TEST_STUCK_BARRIER"))
     if (*e && *e != '0') hctl.test_skip_arrival = 1;
-  Classify cls{tune.small_work, tune.huge_work, tune.chunk_work, std::max<int64_t>(1, tune.units_per_cta),
-               tune.warp_units ? 1 : 0};
-  if (const char* e = getenv("PB_PEEL_WARP_UNITS")) cls.warp_units = atoi(e) != 0;  // diagnostic hook
-  // Thresholds may be lowered through the environment (tests use this to drive small graphs
-  // through the CTA- and grid-level paths).
-  if (const char* e = getenv("PB_PEEL_SMALL_WORK")) cls.small_work = atoll(e);
-  if (const char* e = getenv("PB_PEEL_HUGE_WORK")) cls.huge_work = atoll(e);
-  if (const char* e = getenv("PB_PEEL_CHUNK_WORK")) cls.chunk_work = atoll(e);
   DevBuf<unsigned> status(2, s);
   DevBuf<uint32_t> wgt;  // coarse passes: static per-item work estimates
   if (two_phase || two_phase_batch) {
@@ -2033,22 +2036,10 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
       x.alist[0] = alist0.get() + b;
       x.alist[1] = alist1.get() + b;
       x.near = nearl.get() + b;
-      x.fsmall[0] = fs0.get() + b;
-      x.fsmall[1] = fs1.get() + b;
-      x.fbig[0] = fb0.get() + b;
-      x.fbig[1] = fb1.get() + b;
-      x.fchunks[0] = fc0.get() + b;
-      x.fchunks[1] = fc1.get() + b;
-      x.uprefix = upre.get() + b + i;
-      if (kWing) {
-        x.fwchunks[0] = fw0.get() + b;
-        x.fwchunks[1] = fw1.get() + b;
-        x.wprefix = wpre.get() + b + i;
-      }
-      x.fhuge[0] = fh0.get() + b;
-      x.fhuge[1] = fh1.get() + b;
-      x.tlist[0] = tl0.get() + b;
-      x.tlist[1] = tl1.get() + b;
+      x.front[0] = fr0.get() + b;
+      x.front[1] = fr1.get() + b;
+      x.fhuge[0] = kWing ? nullptr : fh0.get() + b;
+      x.fhuge[1] = kWing ? nullptr : fh1.get() + b;
       x.N = n;
       x.item0 = (uint32_t)b;
       Ctl& c = cs[i];
@@ -2124,8 +2115,7 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
     PB_CUDA_TRY(cudaMemcpyAsync(hcnt.data(), pcnt.get(), sizeof(unsigned) * ntot, cudaMemcpyDeviceToHost, s));
     PB_CUDA_TRY(cudaMemcpyAsync(hwork.data(), pwork.get(), sizeof(unsigned long long) * ntot, cudaMemcpyDeviceToHost, s));
     PB_CUDA_TRY(cudaStreamSynchronize(s));
-    PB_LAUNCH(peel_init_kernel, grid_for(N), 256, 0, s, (const int64_t*)snap.get(), N, out, cnt.get(), state.get(),
-              in_near.get(), touched.get());
+    PB_LAUNCH(peel_init_kernel, grid_for(N), 256, 0, s, (const int64_t*)snap.get(), N, out, cnt.get(), state.get());
     std::vector<Work> fws;
     std::vector<Ctl> fcs;
     std::vector<double> fw;
@@ -2144,16 +2134,10 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
         x.alist[0] = alist0.get() + b;
         x.alist[1] = alist1.get() + b;
         x.near = nearl.get() + b;
-        x.fsmall[0] = fs0.get() + b;
-        x.fsmall[1] = fs1.get() + b;
-        x.fbig[0] = fb0.get() + b;
-        x.fbig[1] = fb1.get() + b;
-        x.fchunks[0] = fc0.get() + b;
-        x.fchunks[1] = fc1.get() + b;
-        x.fhuge[0] = fh0.get() + b;
-        x.fhuge[1] = fh1.get() + b;
-        x.tlist[0] = tl0.get() + b;
-        x.tlist[1] = tl1.get() + b;
+        x.front[0] = fr0.get() + b;
+        x.front[1] = fr1.get() + b;
+        x.fhuge[0] = kWing ? nullptr : fh0.get() + b;
+        x.fhuge[1] = kWing ? nullptr : fh1.get() + b;
         x.N = n;
         x.item0 = (uint32_t)b;
         fws.push_back(x);
@@ -2168,23 +2152,13 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
       }
     }
     PB_REQUIRE(b == N, PB_ECUDA, "two-phase peel: partition sizes do not add up");
-    DevBuf<uint32_t> upre2(N + (int64_t)fws.size() + 1, s), wpre2;
-    if (kWing) wpre2.alloc(N + (int64_t)fws.size() + 1, s);
-    for (size_t i = 0; i < fws.size(); ++i) {
-      fws[i].uprefix = upre2.get() + fws[i].item0 + i;
-      if (kWing) {
-        fws[i].fwchunks[0] = fw0.get() + fws[i].item0;
-        fws[i].fwchunks[1] = fw1.get() + fws[i].item0;
-        fws[i].wprefix = wpre2.get() + fws[i].item0 + i;
-      }
-    }
     const int64_t gstride_b = gstride;
     const int64_t slices = std::max<int64_t>(1, kGsharedBudget / (4 * gstride_b));
     std::vector<std::unique_ptr<DevBuf<uint32_t>>> gsl;
     auto per_slot = [&](Work& x, uint32_t ncta) {
       x.gshared = nullptr;
       x.ngroups = 1;
-      if (ncta >= 2 && (int64_t)gsl.size() < slices) {
+      if (!kWing && ncta >= 2 && (int64_t)gsl.size() < slices) {
         gsl.push_back(std::make_unique<DevBuf<uint32_t>>((size_t)gstride_b, s));
         PB_CUDA_TRY(cudaMemsetAsync(gsl.back()->get(), 0, gsl.back()->bytes(), s));
         x.gshared = gsl.back()->get();
@@ -2287,23 +2261,19 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
   }
   res.rounds = (int64_t)hctl.rounds;
   res.work = (int64_t)hctl.work;
-  const bool trace = [] {
-    const char* tr = getenv("PB_TRACE");
-    return tr && *tr && *tr != '0';
-  }();
   if (trace) {
     fprintf(stderr,
-            "[pb] peel %s%s: rounds %llu launches %d advances %llu | ms advance %.1f F %.1f P %.1f U %.1f | "
-            "near scanned %llu touched %llu items small %llu big %llu huge %llu work %llu\n",
+            "[pb] peel %s%s: rounds %llu launches %d advances %llu | ms advance %.1f F %.1f P %.1f | "
+            "near scanned %llu items small %llu big %llu huge %llu work %llu\n",
             kWing ? "wing" : "tip", two_phase ? " (coarse pass)" : "", hctl.rounds, launches, hctl.advances,
-            hctl.phase_ns[0] / 1e6, hctl.phase_ns[1] / 1e6, hctl.phase_ns[2] / 1e6, hctl.phase_ns[3] / 1e6,
-            hctl.scanned, hctl.touched_total, hctl.n_small, hctl.n_big, hctl.n_huge, hctl.work);
+            hctl.phase_ns[0] / 1e6, hctl.phase_ns[1] / 1e6, hctl.phase_ns[2] / 1e6, hctl.scanned, hctl.n_small,
+            hctl.n_big, hctl.n_huge, hctl.work);
     if (kWing)
       fprintf(stderr,
               "[pb]   wing items / probes: warp %llu / %llu, CTA table %llu / %llu, dense markers %llu / %llu, "
-              "grid %llu / %llu; reverse-direction probes %llu\n",
+              "reverse-direction probes %llu\n",
               hctl.mode_items[0], hctl.mode_work[0], hctl.mode_items[1], hctl.mode_work[1], hctl.mode_items[2],
-              hctl.mode_work[2], hctl.mode_items[3], hctl.mode_work[3], hctl.rev_work);
+              hctl.mode_work[2], hctl.rev_work);
     for (int b = 0; b < 42; ++b)
       if (hctl.pbin_rounds[b])
         fprintf(stderr, "[pb]   P rounds with est work in [2^%d, 2^%d): %llu rounds, %.1f ms, est %.3g (%.3g/s)\n",
@@ -2336,8 +2306,7 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
   PB_CUDA_TRY(cudaMemcpyAsync(hwork.data(), pwork.get(), sizeof(unsigned long long) * nparts, cudaMemcpyDeviceToHost, s));
   PB_CUDA_TRY(cudaStreamSynchronize(s));
   // Fresh per-item state: every partition starts from the counts its items had when it opened.
-  PB_LAUNCH(peel_init_kernel, grid_for(N), 256, 0, s, (const int64_t*)snap.get(), N, out, cnt.get(), state.get(),
-            in_near.get(), touched.get());
+  PB_LAUNCH(peel_init_kernel, grid_for(N), 256, 0, s, (const int64_t*)snap.get(), N, out, cnt.get(), state.get());
   DevBuf<Lists> dlevels(levels.size(), s);
   PB_CUDA_TRY(cudaMemcpyAsync(dlevels.get(), levels.data(), sizeof(Lists) * levels.size(), cudaMemcpyHostToDevice, s));
   Ctl c0;
@@ -2368,16 +2337,10 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
     x.alist[0] = alist0.get() + b;
     x.alist[1] = alist1.get() + b;
     x.near = nearl.get() + b;
-    x.fsmall[0] = fs0.get() + b;
-    x.fsmall[1] = fs1.get() + b;
-    x.fbig[0] = fb0.get() + b;
-    x.fbig[1] = fb1.get() + b;
-    x.fchunks[0] = fc0.get() + b;
-    x.fchunks[1] = fc1.get() + b;
-    x.fhuge[0] = fh0.get() + b;
-    x.fhuge[1] = fh1.get() + b;
-    x.tlist[0] = tl0.get() + b;
-    x.tlist[1] = tl1.get() + b;
+    x.front[0] = fr0.get() + b;
+    x.front[1] = fr1.get() + b;
+    x.fhuge[0] = kWing ? nullptr : fh0.get() + b;
+    x.fhuge[1] = kWing ? nullptr : fh1.get() + b;
     x.N = n;
     x.item0 = (uint32_t)b;
     ws.push_back(x);
@@ -2390,17 +2353,6 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
     b += n;
   }
   PB_REQUIRE(b == N, PB_ECUDA, "two-phase peel: partition sizes do not add up");
-  // Unit prefixes: N + 1 slots per instance (n + 1 each).
-  DevBuf<uint32_t> upre2(N + (int64_t)ws.size() + 1, s), wpre2;
-  if (kWing) wpre2.alloc(N + (int64_t)ws.size() + 1, s);
-  for (size_t i = 0; i < ws.size(); ++i) {
-    ws[i].uprefix = upre2.get() + ws[i].item0 + i;
-    if (kWing) {
-      ws[i].fwchunks[0] = fw0.get() + ws[i].item0;
-      ws[i].fwchunks[1] = fw1.get() + ws[i].item0;
-      ws[i].wprefix = wpre2.get() + ws[i].item0 + i;
-    }
-  }
   const int64_t coarse_work = res.work;
   res.rounds = 0;
   res.work = 0;
@@ -2412,7 +2364,7 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
   auto per_slot = [&](Work& x, uint32_t ncta) {
     x.gshared = nullptr;
     x.ngroups = 1;
-    if (ncta >= 2 && (int64_t)gsl.size() < slices) {
+    if (!kWing && ncta >= 2 && (int64_t)gsl.size() < slices) {
       gsl.push_back(std::make_unique<DevBuf<uint32_t>>((size_t)gstride, s));
       PB_CUDA_TRY(cudaMemsetAsync(gsl.back()->get(), 0, gsl.back()->bytes(), s));
       x.gshared = gsl.back()->get();
