@@ -138,6 +138,7 @@ struct Lists {
   int64_t nK, nC;
 };
 // Lists::info: work units of the item, whether it runs on warps, whether it walks from the centre.
+constexpr int64_t kUnitSets = 2;
 constexpr uint32_t kInfoUnits = 0x1FFFu, kInfoSmall = 1u << 13, kInfoFromV = 1u << 31;
 
 struct Work {
@@ -698,11 +699,14 @@ __device__ __forceinline__ uint32_t edge_status(const Work& W, uint32_t e, uint3
 }
 
 enum Level { LV_WARP = 0, LV_BLOCK = 1 };
+constexpr unsigned kOneSlice = 128;          // rounds of at most this many CTA-level items: one slice per CTA
 constexpr uint32_t kKeepBit = 0x80000000u;   // probe-set edges that are not charged (m < 2^31)
 constexpr uint32_t kNoSlot = 0x3FFFu;        // queue entries found through the dense markers
 
-// The units [chunk, chunk_end) of nchunks (slices of the first level) of one frontier edge, by one
-// warp or one CTA.
+// The units [chunk, chunk_end) of nchunks of one frontier edge, by one warp or one CTA.  Unit s holds
+// the first-level positions s, s + nchunks, s + 2 nchunks, ...: list lengths vary smoothly with the
+// position (ids are ordered alike in every list), so strided units are of nearly equal work where
+// contiguous slices are not.
 template <int kLevel>
 __device__ void wing_item(const Lists& G, const Work& W, Ctl* ctl, const uint4& E, uint32_t* keys, Shared& S,
                           WarpQueue& Q, Acc& A, uint32_t chunk, uint32_t nchunks, uint32_t chunk_end) {
@@ -731,40 +735,74 @@ __device__ void wing_item(const Lists& G, const Work& W, Ctl* ctl, const uint4& 
   // hits[slot]: butterflies found through a probe-set edge, charged to it in one decrement once
   // the intersections are done.
   uint32_t* hits = vals + cap;
-  for (uint32_t s = rank; s < tsize; s += gsize) {
-    keys[s] = kEmpty;
-    hits[s] = 0;
-  }
-  sync();
-  for (uint32_t p = pb + rank; p < pe; p += gsize) {
-    const uint32_t key = edgA[p], e = eidA[p];
-    const uint32_t es = edge_status(W, e, e1);
-    if (es == ES_GONE) continue;
-    const uint32_t val = es == ES_KEEP ? (e | kKeepBit) : e;
-    if (hash) t_put(keys, vals, tsize, key, val, ctl);
-    else mark[key] = val + 1;
-  }
-  sync();
-  // The chunk's first-level edge of this thread (position j0 + rank).
-  uint32_t f_edge = 0, f_st = ES_GONE;
+  // The slice's positions are numbered t = 0 .. fn - 1: rows of `width` of every nchunks positions.
+  const uint32_t width = chunk_end - chunk, rows = d1 / nchunks, rest = d1 - rows * nchunks;
+  const uint32_t fn = rows * width + (rest > chunk ? min(rest - chunk, width) : 0u);
+  auto pos_of = [&](uint32_t t) {
+    const uint32_t row = width == 1 ? t : t / width;
+    return b1 + row * nchunks + chunk + (t - row * width);
+  };
+  // The chunk's first-level edge of this thread (number t0 + rank).
+  uint32_t f_edge = 0, f_st = ES_GONE, f_len = 0, f_beg = 0;
   uint32_t* accp = kLevel == LV_WARP ? S.acc + (threadIdx.x & ~31u) : S.acc;
   // Each (first-level vertex y, probe set) intersection runs in one of two directions: scan
   // N(y) and probe the probe-set table, or (when the probe set is much shorter than N(y))
   // walk the probe set and binary-search N(y), which is sorted.  The direction rides in the
   // top bit of the second-level position.
-  uint32_t j_chunk = 0;
-  auto first = [&](uint32_t j, bool valid, uint32_t& L, uint32_t& sb) {
-    f_st = ES_GONE;
-    accp[rank] = 0;
-    j_chunk = j - rank;
-    if (!valid) return;
-    const uint32_t y = edgB[j];
-    f_edge = eidB[j];
+  uint32_t t_chunk = 0;
+  auto load_first = [&](uint32_t y, uint32_t e) {
+    f_edge = e;
     const uint32_t b2 = offA[y], d2 = offA[y + 1] - b2;
-    f_st = edge_status(W, f_edge, e1);
+    f_st = edge_status(W, e, e1);
+    f_len = 0;
     if (y == a || f_st == ES_GONE) return;
-    if (reverse_cheaper(psize, d2)) { sb = pb | kRevFlag; L = psize; }
-    else { sb = b2; L = d2; }
+    if (reverse_cheaper(psize, d2)) { f_beg = pb | kRevFlag; f_len = psize; }
+    else { f_beg = b2; f_len = d2; }
+  };
+  // The first probe-set entry and the first chunk's first-level entry of this thread are loaded
+  // together, before the table is built: one chain of round trips instead of two.
+  uint32_t key0 = 0, e0 = 0, st0 = ES_GONE, y0 = 0, g0 = 0;
+  if (pb + rank < pe) {
+    key0 = edgA[pb + rank];
+    e0 = eidA[pb + rank];
+  }
+  if (rank < fn) {
+    const uint32_t j = pos_of(rank);
+    y0 = edgB[j];
+    g0 = eidB[j];
+  }
+  for (uint32_t s = rank; s < tsize; s += gsize) {
+    keys[s] = kEmpty;
+    hits[s] = 0;
+  }
+  if (pb + rank < pe) st0 = edge_status(W, e0, e1);
+  if (rank < fn) load_first(y0, g0);
+  sync();
+  auto put = [&](uint32_t key, uint32_t e, uint32_t es) {
+    if (es == ES_GONE) return;
+    const uint32_t val = es == ES_KEEP ? (e | kKeepBit) : e;
+    if (hash) t_put(keys, vals, tsize, key, val, ctl);
+    else mark[key] = val + 1;
+  };
+  put(key0, e0, st0);
+  for (uint32_t p = pb + rank + gsize; p < pe; p += gsize) {
+    const uint32_t key = edgA[p], e = eidA[p];
+    put(key, e, edge_status(W, e, e1));
+  }
+  sync();
+  auto first = [&](uint32_t t, bool valid, uint32_t& L, uint32_t& sb) {
+    accp[rank] = 0;
+    t_chunk = t - rank;
+    if (t_chunk) {
+      f_st = ES_GONE;
+      f_len = 0;
+      if (valid) {
+        const uint32_t j = pos_of(t);
+        load_first(edgB[j], eidB[j]);
+      }
+    }
+    L = f_len;
+    sb = f_beg;
   };
   // One butterfly found through second-level entry q: its edge loses 1 now; the probe-set edge
   // loses 1 through its hit counter when it has a table slot; the first-level edge through the
@@ -794,7 +832,7 @@ __device__ void wing_item(const Lists& G, const Work& W, Ctl* ctl, const uint4& 
         const uint32_t e4 = eidA[q & ~kRevFlag];
         const uint32_t s4 = edge_status(W, e4, e1);
         if (s4 != ES_GONE) {
-          const uint32_t y = edgB[j_chunk + lo];
+          const uint32_t y = edgB[pos_of(t_chunk + lo)];
           const uint32_t end = offA[y + 1];
           const uint32_t at = lower_bound_u32(edgA, offA[y], end, z);
           if (at != end && edgA[at] == z) {
@@ -818,25 +856,27 @@ __device__ void wing_item(const Lists& G, const Work& W, Ctl* ctl, const uint4& 
     }
     Q.push(hit, ent, charge);
   };
+  // Summed decrements of one edge: (edge, amount).
+  auto charge_sum = [&](unsigned long long x) { dec_known(W, ctl, A, (uint32_t)x, (int64_t)(x >> 32)); };
+  // The first-level edges' decrements; those of the last chunk wait in the queue and are charged
+  // together with the probe set's.
   auto done = [&] {
     Q.flush(charge);
     sync();
-    const uint32_t got = accp[rank];
-    if (got && f_st == ES_CHARGE) dec_known(W, ctl, A, f_edge, (int64_t)got);
+    const uint32_t got = f_st == ES_CHARGE ? accp[rank] : 0u;
+    Q.push(got != 0, ((unsigned long long)got << 32) | f_edge, charge_sum);
+    if (t_chunk + gsize < fn) Q.flush(charge_sum);
   };
-  const uint32_t fb = b1 + (uint32_t)((uint64_t)d1 * chunk / nchunks);
-  const uint32_t fe = b1 + (uint32_t)((uint64_t)d1 * chunk_end / nchunks);
-  if (kLevel == LV_WARP) warp_iter(fb, fe, edgA, first, pair, done);
-  else block_iter(fb, fe, S, edgA, first, pair, done);
+  if (kLevel == LV_WARP) warp_iter(0, fn, edgA, first, pair, done);
+  else block_iter(0, fn, S, edgA, first, pair, done);
   // The probe-set edges' decrements, one per edge.
   for (uint32_t s0 = 0; s0 < tsize; s0 += gsize) {
     const uint32_t s = s0 + rank;
     const uint32_t h = s < tsize ? hits[s] : 0u;
     const uint32_t val = h ? vals[s] : kKeepBit;
-    Q.push(!(val & kKeepBit), ((unsigned long long)h << 32) | val,
-           [&](unsigned long long x) { dec_known(W, ctl, A, (uint32_t)x, (int64_t)(x >> 32)); });
+    Q.push(!(val & kKeepBit), ((unsigned long long)h << 32) | val, charge_sum);
   }
-  Q.flush([&](unsigned long long x) { dec_known(W, ctl, A, (uint32_t)x, (int64_t)(x >> 32)); });
+  Q.flush(charge_sum);
   if (!hash) {  // clear the dense markers
     for (uint32_t p = pb + rank; p < pe; p += gsize) mark[edgA[p]] = 0;
   }
@@ -1315,41 +1355,69 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
       const unsigned ng = kWing ? 0u : (W.gshared ? min(W.ngroups, kMaxGroups) : 0u);
       const bool flat_all = !kWing && vgrid() >= 8 && nb + nh > 0 && nb + nh <= ng;
       if (nu && !flat_all) {
-        // CTAs claim runs of K consecutive units (wing: about a quarter of a CTA's share; tip: one
-        // unit, which is one item); the units of one item inside a run are processed as one
-        // slice, so the item's probe table is built once per run, not once per unit.  The first
-        // run of a CTA is its own number; the cursor hands out the later ones.
         const uint4* const fbg = W.front[par] + (W.N - 1);  // item q: fbg[-q]
-        const unsigned K = kWing ? max(1u, (unsigned)(nu / ((unsigned)cls.units_per_cta * vgrid()))) : 1u;
-        const bool more = vgrid() * K < nu;  // some run is left for the cursor
-        for (unsigned u0 = vblock() * K; u0 < nu;) {
-          const unsigned uend = min(u0 + K, nu);
-          if (more && threadIdx.x == 0) S.item = atomicAdd(&ctl->cur_big[par], K);
-          if (kWing) {
-            uint32_t lo = 0, hi = nb;  // the last item whose first unit <= u0, 32-way search by every warp
-            while (hi - lo > 1) {
-              const uint32_t step = (hi - lo + 31) / 32;
-              const uint32_t idx = lo + lane * step;
-              const bool le = idx < hi && fbg[-(int64_t)idx].w <= u0;
-              const unsigned bal = __ballot_sync(0xffffffffu, le);
-              lo = lo + (31 - __clz(bal)) * step;  // lane 0 always qualifies
-              hi = min(lo + step, hi);
+        if (kWing && nb <= kOneSlice && 2 * nb <= vgrid()) {
+          // Light rounds: K units make a slice such that every CTA gets at most one slice (of one
+          // item).  Each warp derives the layout from the items' unit counts by itself.
+          const unsigned K = (nu + vgrid() - nb - 1) / (vgrid() - nb);
+          unsigned carry = 0;
+          for (unsigned q0 = 0; q0 < nb; q0 += 32) {
+            const unsigned q = q0 + lane;
+            uint4 it = make_uint4(0, 0, 0, nu);
+            if (q < nb) it = fbg[-(int64_t)q];
+            unsigned next = __shfl_down_sync(0xffffffffu, it.w, 1);
+            if (lane == 31) next = q + 1 < nb ? fbg[-(int64_t)(q + 1)].w : nu;
+            const unsigned units = q < nb ? next - it.w : 0u, slices = (units + K - 1) / K;
+            const unsigned end = carry + warp_inclusive_scan(slices);
+            const unsigned m = __ballot_sync(0xffffffffu, slices && vblock() >= end - slices && vblock() < end);
+            if (m) {  // this CTA's slice: units sl, sl + n, ... of the item of lane l, as one of n slices
+              const int l = __ffs(m) - 1;
+              it.x = __shfl_sync(0xffffffffu, it.x, l);
+              it.y = __shfl_sync(0xffffffffu, it.y, l);
+              it.z = __shfl_sync(0xffffffffu, it.z, l);
+              const unsigned n = __shfl_sync(0xffffffffu, slices, l);
+              const unsigned sl = vblock() - (__shfl_sync(0xffffffffu, end, l) - n);
+              wing_item<LV_BLOCK>(G, W, ctl, it, pool, S, Q, A, sl, n, sl + 1);
+              break;
             }
-            for (unsigned uu = u0, q = lo; uu < uend; ++q) {  // uniform across the CTA
-              const uint4 it = fbg[-(int64_t)q];
-              const uint32_t next = q + 1 < nb ? fbg[-(int64_t)(q + 1)].w : nu;
-              const uint32_t c1 = min(uend, next);
-              if (c1 > uu) wing_item<LV_BLOCK>(G, W, ctl, it, pool, S, Q, A, uu - it.w, next - it.w, c1 - it.w);
-              uu = max(uu, c1);
-            }
-          } else {
-            const uint4 it = fbg[-(int64_t)u0];
-            if (it.w) tip_item_block(G, W, ctl, it.x, pool, S, Q, A);
+            carry = __shfl_sync(0xffffffffu, end, 31);
           }
-          if (!more) break;
-          __syncthreads();
-          u0 = vgrid() * K + S.item;
-          __syncthreads();
+        } else {
+          // CTAs claim runs of K consecutive units (wing: a units_per_cta-th of a CTA's share; tip:
+          // one unit, which is one item); the units of one item inside a run are processed as one
+          // slice, so the item's probe table is built once per run, not once per unit.  The first
+          // run of a CTA is its own number; the cursor hands out the later ones.
+          const unsigned K = kWing ? max(1u, nu / ((unsigned)cls.units_per_cta * vgrid())) : 1u;
+          const bool more = vgrid() * K < nu;  // some run is left for the cursor
+          for (unsigned u0 = vblock() * K; u0 < nu;) {
+            const unsigned uend = min(u0 + K, nu);
+            if (more && threadIdx.x == 0) S.item = atomicAdd(&ctl->cur_big[par], K);
+            if (kWing) {
+              uint32_t lo = 0, hi = nb;  // the last item whose first unit <= u0, 32-way search by every warp
+              while (hi - lo > 1) {
+                const uint32_t step = (hi - lo + 31) / 32;
+                const uint32_t idx = lo + lane * step;
+                const bool le = idx < hi && fbg[-(int64_t)idx].w <= u0;
+                const unsigned bal = __ballot_sync(0xffffffffu, le);
+                lo = lo + (31 - __clz(bal)) * step;  // lane 0 always qualifies
+                hi = min(lo + step, hi);
+              }
+              for (unsigned uu = u0, q = lo; uu < uend; ++q) {  // uniform across the CTA
+                const uint4 it = fbg[-(int64_t)q];
+                const uint32_t next = q + 1 < nb ? fbg[-(int64_t)(q + 1)].w : nu;
+                const uint32_t c1 = min(uend, next);
+                if (c1 > uu) wing_item<LV_BLOCK>(G, W, ctl, it, pool, S, Q, A, uu - it.w, next - it.w, c1 - it.w);
+                uu = max(uu, c1);
+              }
+            } else {
+              const uint4 it = fbg[-(int64_t)u0];
+              if (it.w) tip_item_block(G, W, ctl, it.x, pool, S, Q, A);
+            }
+            if (!more) break;
+            __syncthreads();
+            u0 = vgrid() * K + S.item;
+            __syncthreads();
+          }
         }
       }
       if constexpr (!kWing) if (nh || flat_all) {
@@ -1400,9 +1468,12 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
 
 // kMinBlocks: CTAs per SM the register allocation must allow.  2 caps a thread at 64 registers
 // (some spill); 1 leaves about 108 and no spills, at half the resident warps.  The single-
-// instance tip peel runs faster on the latter (fewer CTAs also shorten its grid barriers: R-MAT
-// 2^24, one round at a time, 2.36 s -> 1.60 s); wing peeling and batches keep two CTAs per SM
-// (the wing peel's intersections need the warps: 18.5 s against 19.6 s).
+// instance tip peel runs faster on the latter (light rounds: fewer CTAs also shorten its grid
+// barriers), and so does the wing peel while its rounds are light; with more edges the rounds are
+// heavy and the intersections need the warps.  Wing peel of R-MAT graphs, one against two CTAs:
+// 2^18 edges 220 / 243 ms, 2^20 665 / 724, 2^21 1254 / 1303, 2^22 2491 / 2424, 2^24 11369 / 9881.
+// Batches keep two (more graphs at a time).
+constexpr int64_t kWingOneCta = int64_t(3) << 20;
 template <bool kWing, int kMinBlocks>
 __global__ void __launch_bounds__(kPT, kMinBlocks) peel_kernel(Lists G, const Lists* levels, Instances I, Ctl* ctls,
                                                                Classify cls) {
@@ -1628,7 +1699,7 @@ __global__ void wing_info_kernel(Lists G, Classify cls, int64_t N, const unsigne
     const int64_t du = G.offK[u + 1] - G.offK[u], dv = G.offC[v + 1] - G.offC[v];
     const int64_t psize = fv ? du : dv, d1 = fv ? dv : du;
     const bool small = psize <= (int64_t)kWingWarpSet && (cls.warp_units || cost <= cls.small_work);
-    const int64_t unit = small ? chunk : max(chunk, 2 * psize);
+    const int64_t unit = small ? chunk : max(chunk, kUnitSets * psize / 2);
     int64_t units = small && !cls.warp_units ? 1 : (cost + unit - 1) / unit;
     units = max((int64_t)1, min(units, min(d1, (int64_t)4096)));
     info[x] = (uint32_t)units | (small ? kInfoSmall : 0u) | (fv ? kInfoFromV : 0u);
@@ -1883,6 +1954,8 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
   void (*kern)(Lists, const Lists*, Instances, Ctl*, Classify) = peel_kernel<kWing, 2>;
   if constexpr (!kWing) {
     if (!batch) kern = peel_kernel<false, 1>;
+  } else {
+    if (!two_phase && g.m <= kWingOneCta) kern = peel_kernel<true, 1>;
   }
   PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per_sm = 0;
