@@ -7,9 +7,9 @@
 // (the -m option, getNextWedgeIdx, butterfly_utils.h:1700-1714).
 //
 // Device version.  A batch of endpoints [i0, i1) is flattened: wedge t of the batch lives at
-// position t, with key ((i - i0) << 32) | u2, the slot j of (i, v) and the slot of (v, u2) in
-// side arrays.  Warps materialise chunks of consecutive wedges (one binary search over the
-// per-slot wedge prefix per chunk, then a forward walk).
+// position t, with key ((i - i0) << bits of u2) | u2 (32-bit keys when they fit), the slot j of
+// (i, v) and the slot of (v, u2) in side arrays.  Warps materialise chunks of consecutive wedges,
+// 32 slots at a time.
 //   SORT: stable LSD radix sort of (key, position) pairs; run boundaries give w.
 //   HIST: one radix pass on the top bits of a key hash groups each key's wedges into one
 //         bucket; one CTA per bucket builds the bucket's histogram in a shared-memory table,
@@ -18,6 +18,7 @@
 // Credits then follow the ranked semantics: C(w,2) per distinct pair to tagged endpoints (and to
 // the total), w-1 per wedge to tagged centres (VERT) or to both wedge edges (EDGE).
 #include <algorithm>
+#include <type_traits>
 
 #include "pb_engine.cuh"
 #include "pb_prims.cuh"
@@ -27,67 +28,86 @@ namespace pb {
 namespace {
 
 enum Per { VERT = 0, EDGE = 1, TOTAL = 2 };
-constexpr uint32_t kChunk = 1024;  // wedges per materialising warp
+constexpr uint32_t kChunk = 512;  // wedges per materialising warp
 
-__global__ void widen_pref_kernel(const uint32_t* __restrict__ pref, int64_t m2, int64_t* out) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m2; i += (int64_t)gridDim.x * blockDim.x)
-    out[i] = pref[i];
+// Per slot: its row and its wedges as 64-bit numbers (scanned afterwards).
+__global__ void slot_rows_kernel(const uint32_t* __restrict__ off, const uint32_t* __restrict__ pref, int64_t n,
+                                 uint32_t* rowid, int64_t* wide) {
+  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const unsigned lane = threadIdx.x & 31u;
+  for (int64_t r = warp; r < n; r += nwarps) {
+    const uint32_t e = off[r + 1];
+    for (uint32_t j = off[r] + lane; j < e; j += 32) {
+      rowid[j] = (uint32_t)r;
+      wide[j] = pref[j];
+    }
+  }
 }
 
-// First index s in [lo, hi) with a[s + 1] > t, i.e. the segment of a (exclusive prefix) holding t.
-__device__ __forceinline__ int64_t seg_of(const int64_t* __restrict__ a, int64_t lo, int64_t hi, int64_t t) {
+// The last index s in [lo, hi) with a[s] <= t (a ascending, a[lo] <= t): 32-way search by a warp.
+__device__ __forceinline__ int64_t warp_last_le(const int64_t* __restrict__ a, int64_t lo, int64_t hi, int64_t t) {
   while (hi - lo > 1) {
-    const int64_t mid = (lo + hi) >> 1;
-    if (a[mid] <= t) lo = mid;
-    else hi = mid;
+    const int64_t step = (hi - lo + 31) / 32;
+    const int64_t idx = lo + lane_id() * step;
+    const unsigned le = __ballot_sync(0xffffffffu, idx < hi && a[idx] <= t);
+    lo += (31 - __clz(le)) * step;  // lane 0 always qualifies
+    hi = min(lo + step, hi);
   }
   return lo;
 }
 
 // Materialises wedges [t_begin, t_end) (global flattened indices) at positions t - t_begin.
+// Bound by its writes (20 bytes a wedge).  A warp takes kChunk wedges and walks their slots 32 at
+// a time: lanes load 32 slots at once, every wedge finds its slot by a search over the lanes'
+// prefixes, so neighbouring lanes write neighbouring positions.  Groups of 32 slots without wedges
+// are left by a search over the prefix (most slots of the low ranks hold none: walking them one by
+// one took 129 ms for the 1e7 wedges of a uniform graph with 1e6 edges, this walk 0.1 ms).
+template <class K>
 __global__ void materialize_kernel(const uint32_t* __restrict__ off, const uint32_t* __restrict__ adj,
-                                   const uint32_t* __restrict__ pref, const int64_t* __restrict__ spre, int64_t n,
-                                   int64_t m2, int64_t t_begin, int64_t t_end, uint32_t i0, uint64_t* keys,
-                                   uint32_t* vals, uint32_t* jarr, uint32_t* s2arr) {
+                                   const uint32_t* __restrict__ pref, const int64_t* __restrict__ spre,
+                                   const uint32_t* __restrict__ rowid, int64_t m2, int64_t t_begin, int64_t t_end,
+                                   uint32_t i0, int ubits, K* keys, uint32_t* vals, uint32_t* jarr, uint32_t* s2arr) {
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const unsigned lane = threadIdx.x & 31u;
   for (int64_t c0 = t_begin + warp * (int64_t)kChunk; c0 < t_end; c0 += nwarps * (int64_t)kChunk) {
     const int64_t c1 = min(c0 + (int64_t)kChunk, t_end);
-    int64_t s = 0, row = 0;
-    if (lane == 0) {
-      s = seg_of(spre, 0, m2, c0);  // slot holding wedge c0 (slots of zero length are skipped)
-      int64_t lo = 0, hi = n;       // row of slot s: last r with off[r] <= s
-      while (hi - lo > 1) {
-        const int64_t mid = (lo + hi) >> 1;
-        if ((int64_t)off[mid] <= s) lo = mid;
-        else hi = mid;
+    int64_t s = warp_last_le(spre, 0, m2, c0), t = c0;
+    while (t < c1) {
+      const int64_t j = s + lane;
+      int64_t base = c1, end = c1;  // lanes beyond the last slot hold nothing
+      uint32_t vs = 0, row = 0;
+      if (j < m2) {
+        base = spre[j];
+        end = base + pref[j];
+        vs = off[adj[j] >> 1];
+        row = rowid[j];
       }
-      row = lo;
-    }
-    s = __shfl_sync(0xffffffffu, s, 0);
-    row = __shfl_sync(0xffffffffu, row, 0);
-    int64_t t = c0;
-    while (t < c1 && s < m2) {
-      while ((int64_t)off[row + 1] <= s) ++row;
-      const uint32_t L = pref[s];
-      const int64_t base = spre[s];
-      if (base + L > t) {  // slots are visited in order; zero-length ones are passed over
-        const uint32_t vt = adj[s];
-        const uint32_t vs = off[vt >> 1];
-        const int64_t kb = t - base, ke = min((int64_t)L, c1 - base);
-        for (int64_t k = kb + lane; k < ke; k += 32) {
-          const uint32_t slot2 = vs + (uint32_t)k;
-          const uint32_t u2 = adj[slot2] >> 1;
-          const int64_t pos = base + k - t_begin;
-          keys[pos] = ((uint64_t)((uint32_t)row - i0) << 32) | u2;
+      const int64_t gend = min(c1, __shfl_sync(0xffffffffu, end, 31));
+      for (int64_t t0 = t; t0 < gend; t0 += 32) {
+        const int64_t x = t0 + lane;
+        uint32_t lo = 0;  // the last lane whose slot begins at or before x (it holds x)
+#pragma unroll
+        for (uint32_t step = 16; step > 0; step >>= 1)
+          if (__shfl_sync(0xffffffffu, base, lo + step) <= x) lo += step;
+        const int64_t b = __shfl_sync(0xffffffffu, base, lo);
+        const uint32_t v0 = __shfl_sync(0xffffffffu, vs, lo), r = __shfl_sync(0xffffffffu, row, lo);
+        if (x < gend) {
+          const uint32_t slot2 = v0 + (uint32_t)(x - b);
+          const int64_t pos = x - t_begin;
+          keys[pos] = ((K)(r - i0) << ubits) | (K)(adj[slot2] >> 1);
           vals[pos] = (uint32_t)pos;
-          jarr[pos] = (uint32_t)s;
+          jarr[pos] = (uint32_t)(s + lo);
           s2arr[pos] = slot2;
         }
-        t = base + ke;
       }
-      ++s;
+      if (gend > t) {
+        t = gend;
+        s += 32;
+      } else {
+        s = warp_last_le(spre, s, m2, t);
+      }
     }
   }
 }
@@ -98,6 +118,7 @@ struct Credit {
   const uint32_t* eout;
   int per;
   uint32_t i0;
+  int ubits;  // key = (endpoint - i0) << ubits | u2
   int64_t* out;
   uint32_t* out32;
   unsigned long long* total;
@@ -105,6 +126,8 @@ struct Credit {
     if (out32) atomicAdd(&out32[idx], (uint32_t)v);
     else atomic_add_i64(&out[idx], v);
   }
+  __device__ __forceinline__ uint32_t endpoint(uint64_t key) const { return i0 + (uint32_t)(key >> ubits); }
+  __device__ __forceinline__ uint32_t end2(uint64_t key) const { return (uint32_t)(key & ((1ull << ubits) - 1ull)); }
   // One wedge of multiplicity w: centre / edge credits.
   __device__ __forceinline__ void wedge(uint32_t i, uint32_t j, uint32_t slot2, int64_t w) const {
     if (w < 2) return;
@@ -130,18 +153,22 @@ struct Credit {
 };
 
 // SORT: sorted keys -> run heads.
-__global__ void run_heads_kernel(const uint64_t* __restrict__ keys, int64_t n, uint32_t* head) {
+template <class K>
+__global__ void run_heads_kernel(const K* __restrict__ keys, int64_t n, uint32_t* head) {
   for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x)
     head[p] = (p == 0 || keys[p] != keys[p - 1]) ? 1u : 0u;
 }
 
+// start[r]: first position of run r; start[number of runs] = n.
 __global__ void run_starts_kernel(const uint32_t* __restrict__ head, const uint32_t* __restrict__ rid, int64_t n,
                                   uint32_t* start) {
   for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x)
     if (head[p]) start[rid[p]] = (uint32_t)p;
+  if (blockIdx.x == 0 && threadIdx.x == 0) start[rid[n]] = (uint32_t)n;
 }
 
-__global__ void sort_credit_kernel(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ vals,
+template <class K>
+__global__ void sort_credit_kernel(const K* __restrict__ keys, const uint32_t* __restrict__ vals,
                                    const uint32_t* __restrict__ jarr, const uint32_t* __restrict__ s2arr,
                                    const uint32_t* __restrict__ head, const uint32_t* __restrict__ rid,
                                    const uint32_t* __restrict__ start, int64_t n, Credit C) {
@@ -149,7 +176,7 @@ __global__ void sort_credit_kernel(const uint64_t* __restrict__ keys, const uint
     const uint32_t r = rid[p] - (head[p] ? 0u : 1u);  // rid = heads strictly before p
     const int64_t w = (int64_t)start[r + 1] - start[r];
     const uint64_t key = keys[p];
-    const uint32_t i = C.i0 + (uint32_t)(key >> 32), u2 = (uint32_t)key;
+    const uint32_t i = C.endpoint(key), u2 = C.end2(key);
     const uint32_t pos = vals[p];
     const uint32_t j = jarr[pos];
     C.wedge(i, j, s2arr[pos], w);
@@ -251,12 +278,12 @@ __global__ void __launch_bounds__(kHistThreads) hist_bucket_kernel(const uint64_
       const uint64_t k = keys[q];
       const int64_t w = h64_get(tk, tc, kHistSlots - 1, k);
       const uint32_t pos = vals[q];
-      C.wedge(C.i0 + (uint32_t)(k >> 32), jarr[pos], s2arr[pos], w);
+      C.wedge(C.endpoint(k), jarr[pos], s2arr[pos], w);
     }
     for (uint32_t s = threadIdx.x; s < kHistSlots; s += kHistThreads) {
       const unsigned long long k = tk[s];
       if (k == kNoKey) continue;
-      C.pair(C.i0 + (uint32_t)(k >> 32), (uint32_t)k, tc[s]);
+      C.pair(C.endpoint(k), C.end2(k), tc[s]);
     }
     __syncthreads();
   }
@@ -286,10 +313,10 @@ __global__ void hist_global_kernel(const uint64_t* __restrict__ keys, const uint
     for (uint32_t q = p0 + threadIdx.x; q < p1; q += blockDim.x) {
       const uint64_t k = keys[q];
       const uint32_t pos = vals[q];
-      C.wedge(C.i0 + (uint32_t)(k >> 32), jarr[pos], s2arr[pos], h64_get(tk, tc, mask, k));
+      C.wedge(C.endpoint(k), jarr[pos], s2arr[pos], h64_get(tk, tc, mask, k));
     }
     for (uint32_t s = threadIdx.x; s <= mask; s += blockDim.x)
-      if (tk[s] != kNoKey) C.pair(C.i0 + (uint32_t)(tk[s] >> 32), (uint32_t)tk[s], tc[s]);
+      if (tk[s] != kNoKey) C.pair(C.endpoint(tk[s]), C.end2(tk[s]), tc[s]);
     __syncthreads();
   }
 }
@@ -303,6 +330,11 @@ __global__ void gather_keys_kernel(const uint64_t* __restrict__ keys, const uint
 __global__ void widen_kernel(const uint32_t* __restrict__ in, int64_t n, int64_t* out) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     out[i] = (int64_t)in[i];
+}
+
+// One warp per chunk of wedges, all of them resident at most eight times over.
+int materialize_grid(int64_t cnt) {
+  return std::max(1, std::min(ceil_div(cnt, (int64_t)kChunk * 8), sm_count() * 32));
 }
 
 int grid_for(int64_t n) { return std::max(1, std::min(ceil_div(n, 256), sm_count() * 16)); }
@@ -326,16 +358,22 @@ CountResult count_ranked_materialized(const Ranked& R, int per, int64_t* out, bo
   PB_CUDA_TRY(cudaEventCreate(&e0));
   PB_CUDA_TRY(cudaEventCreate(&e1));
   PB_CUDA_TRY(cudaEventRecord(e0, s));
-  // Per-slot exclusive wedge prefix (the flattened wedge index of each slot's first wedge).
+  // Per-slot rows and exclusive wedge prefix (the flattened wedge index of each slot's first wedge).
   DevBuf<int64_t> spre(m2 + 1, s);
-  PB_LAUNCH(widen_pref_kernel, grid_for(m2), 256, 0, s, R.pref.get(), m2, spre.get());
+  DevBuf<uint32_t> rowid(m2, s);
+  PB_LAUNCH(slot_rows_kernel, grid_for(n * 32), 256, 0, s, R.off.get(), R.pref.get(), n, rowid.get(), spre.get());
   exclusive_scan_i64(spre.get(), spre.get(), m2, s);
-  // Endpoint wedge prefix on the host, to cut batches at endpoint boundaries.
-  std::vector<int64_t> wsum(n + 1);
-  PB_CUDA_TRY(cudaMemcpyAsync(wsum.data(), R.wsum.get(), sizeof(int64_t) * (n + 1), cudaMemcpyDeviceToHost, s));
-  PB_CUDA_TRY(cudaStreamSynchronize(s));
   // Batch budget: -m, capped so that one batch's arrays stay within a few GiB.
   const int64_t cap = std::min<int64_t>(max_wedges > 0 ? max_wedges : (int64_t)1 << 27, (int64_t)1 << 27);
+  // Endpoint wedge prefix on the host, to cut batches at endpoint boundaries (one batch: its ends).
+  const bool one_batch = R.w_rank <= cap;
+  std::vector<int64_t> wsum;
+  if (!one_batch) {
+    wsum.resize(n + 1);
+    PB_CUDA_TRY(cudaMemcpyAsync(wsum.data(), R.wsum.get(), sizeof(int64_t) * (n + 1), cudaMemcpyDeviceToHost, s));
+    PB_CUDA_TRY(cudaStreamSynchronize(s));
+  }
+  const int ubits = std::max(1, bits_for((uint64_t)(n - 1)));
   const uint64_t md = R.max_deg > 0 ? R.max_deg - 1 : 0;
   DevBuf<uint32_t> out32;
   if (per == EDGE && md * md < (1ull << 32)) {
@@ -344,49 +382,59 @@ CountResult count_ranked_materialized(const Ranked& R, int per, int64_t* out, bo
   }
   DevBuf<unsigned long long> total(1, s);
   PB_CUDA_TRY(cudaMemsetAsync(total.get(), 0, sizeof(unsigned long long), s));
+  // SORT on keys of one width: sorted runs give the multiplicities.
+  auto sort_batch = [&](auto* keys, auto* keys2, int64_t cnt, int64_t tb, int key_bits, const Credit& C) {
+    using K = std::remove_pointer_t<decltype(keys)>;
+    DevBuf<uint32_t> vals(cnt, s), vals2(cnt, s), jarr(cnt, s), s2arr(cnt, s);
+    PB_LAUNCH(materialize_kernel<K>, materialize_grid(cnt), 256, 0, s, R.off.get(), R.adj.get(), R.pref.get(),
+              spre.get(), rowid.get(), m2, tb, tb + cnt, C.i0, ubits, keys, vals.get(), jarr.get(), s2arr.get());
+    bool alt;
+    if constexpr (sizeof(K) == 4) alt = radix_sort_pairs_u32(keys, vals.get(), keys2, vals2.get(), cnt, 0, key_bits, s);
+    else alt = radix_sort_pairs_u64(keys, vals.get(), keys2, vals2.get(), cnt, 0, key_bits, s);
+    K* k = alt ? keys2 : keys;
+    uint32_t* v = alt ? vals2.get() : vals.get();
+    DevBuf<uint32_t> head(cnt, s), rid(cnt + 1, s), start(cnt + 1, s);
+    PB_LAUNCH(run_heads_kernel<K>, grid_for(cnt), 256, 0, s, k, cnt, head.get());
+    exclusive_scan_u32(head.get(), rid.get(), cnt, s);
+    PB_LAUNCH(run_starts_kernel, grid_for(cnt), 256, 0, s, head.get(), rid.get(), cnt, start.get());
+    PB_LAUNCH(sort_credit_kernel<K>, grid_for(cnt), 256, 0, s, k, v, jarr.get(), s2arr.get(), head.get(), rid.get(),
+              start.get(), cnt, C);
+  };
   int64_t i0 = 0;
   while (i0 < n) {
     // Largest i1 with wsum[i1] - wsum[i0] <= cap (at least one endpoint).
-    int64_t i1 = std::upper_bound(wsum.begin() + i0 + 1, wsum.end(), wsum[i0] + cap) - wsum.begin() - 1;
-    if (i1 <= i0) i1 = i0 + 1;
-    const int64_t tb = wsum[i0], te = wsum[i1], cnt = te - tb;
+    int64_t i1 = n;
+    if (!one_batch) {
+      i1 = std::upper_bound(wsum.begin() + i0 + 1, wsum.end(), wsum[i0] + cap) - wsum.begin() - 1;
+      if (i1 <= i0) i1 = i0 + 1;
+    }
+    const int64_t tb = one_batch ? 0 : wsum[i0], te = one_batch ? R.w_rank : wsum[i1], cnt = te - tb;
     PB_REQUIRE(cnt < (int64_t)UINT32_MAX, PB_ETOOBIG, "a single endpoint's wedges exceed 2^32");
     if (cnt > 0) {
-      DevBuf<uint64_t> keys(cnt, s), keys2(cnt, s);
-      DevBuf<uint32_t> vals(cnt, s), vals2(cnt, s), jarr(cnt, s), s2arr(cnt, s);
-      PB_LAUNCH(materialize_kernel, std::max(1, std::min(ceil_div(cnt, (int64_t)kChunk * 8), sm_count() * 32)), 256, 0,
-                s, R.off.get(), R.adj.get(), R.pref.get(), spre.get(), n, m2, tb, te, (uint32_t)i0, keys.get(),
-                vals.get(), jarr.get(), s2arr.get());
-      Credit C{R.off.get(), R.adj.get(), R.eout.get(), per, (uint32_t)i0, out, out32.get(), total.get()};
-      const int key_bits = 32 + bits_for((uint64_t)(i1 - i0));
-      if (!hist) {
-        const bool alt = radix_sort_pairs_u64(keys.get(), vals.get(), keys2.get(), vals2.get(), cnt, 0, key_bits, s);
-        uint64_t* k = alt ? keys2.get() : keys.get();
-        uint32_t* v = alt ? vals2.get() : vals.get();
-        DevBuf<uint32_t> head(cnt, s), rid(cnt + 1, s), start(cnt + 1, s);
-        PB_LAUNCH(run_heads_kernel, grid_for(cnt), 256, 0, s, k, cnt, head.get());
-        exclusive_scan_u32(head.get(), rid.get(), cnt, s);
-        PB_LAUNCH(run_starts_kernel, grid_for(cnt), 256, 0, s, head.get(), rid.get(), cnt, start.get());
-        uint32_t nruns = 0;
-        PB_CUDA_TRY(cudaMemcpyAsync(&nruns, rid.get() + cnt, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-        PB_CUDA_TRY(cudaStreamSynchronize(s));
-        const uint32_t cnt32 = (uint32_t)cnt;
-        PB_CUDA_TRY(cudaMemcpyAsync(start.get() + nruns, &cnt32, sizeof(uint32_t), cudaMemcpyHostToDevice, s));
-        PB_LAUNCH(sort_credit_kernel, grid_for(cnt), 256, 0, s, k, v, jarr.get(), s2arr.get(), head.get(),
-                  rid.get(), start.get(), cnt, C);
-        PB_CUDA_TRY(cudaStreamSynchronize(s));
+      Credit C{R.off.get(), R.adj.get(), R.eout.get(), per, (uint32_t)i0, ubits, out, out32.get(), total.get()};
+      const int key_bits = ubits + bits_for((uint64_t)(i1 - i0 - 1));
+      if (!hist && key_bits <= 32) {
+        DevBuf<uint32_t> keys(cnt, s), keys2(cnt, s);
+        sort_batch(keys.get(), keys2.get(), cnt, tb, key_bits, C);
+      } else if (!hist) {
+        DevBuf<uint64_t> keys(cnt, s), keys2(cnt, s);
+        sort_batch(keys.get(), keys2.get(), cnt, tb, key_bits, C);
       } else {
+        DevBuf<uint64_t> keys(cnt, s), keys2(cnt, s);
+        DevBuf<uint32_t> vals(cnt, s), jarr(cnt, s), s2arr(cnt, s);
+        PB_LAUNCH(materialize_kernel<uint64_t>, materialize_grid(cnt), 256, 0, s, R.off.get(), R.adj.get(),
+                  R.pref.get(), spre.get(), rowid.get(), m2, tb, te, (uint32_t)i0, ubits, keys.get(), vals.get(),
+                  jarr.get(), s2arr.get());
         // Semisort: bucket keys by hash (about 1024 wedges per bucket), one stable radix pass.
         int bits = bits_for((uint64_t)std::max<int64_t>(1, cnt / 1024));
         bits = std::max(1, std::min(bits, 24));
         const uint32_t nb = 1u << bits;
-        DevBuf<uint32_t> bkey(cnt, s), bkey2(cnt, s), perm(cnt, s), perm2(cnt, s);
+        DevBuf<uint32_t> bkey(cnt, s), bkey2(cnt, s), perm2(cnt, s);
         PB_LAUNCH(bucket_keys_kernel, grid_for(cnt), 256, 0, s, keys.get(), cnt, bits, bkey.get());
         // sort (bucket, original position) pairs; positions double as the permutation
-        PB_CUDA_TRY(cudaMemcpyAsync(perm.get(), vals.get(), sizeof(uint32_t) * cnt, cudaMemcpyDeviceToDevice, s));
-        const bool alt = radix_sort_pairs_u32(bkey.get(), perm.get(), bkey2.get(), perm2.get(), cnt, 0, bits, s);
+        const bool alt = radix_sort_pairs_u32(bkey.get(), vals.get(), bkey2.get(), perm2.get(), cnt, 0, bits, s);
         uint32_t* bs = alt ? bkey2.get() : bkey.get();
-        uint32_t* pm = alt ? perm2.get() : perm.get();
+        uint32_t* pm = alt ? perm2.get() : vals.get();
         DevBuf<uint32_t> bstart(nb + 1, s);
         PB_LAUNCH(bucket_bounds_kernel, grid_for(cnt), 256, 0, s, bs, cnt, nb, bstart.get());
         // gather keys into bucket order
