@@ -10,16 +10,21 @@
 // Endpoint and centre are on opposite sides, so for one endpoint either the centre credits or
 // the endpoint credits matter, never both.
 //
-// Aggregators (the multiplicity table w):
-//   warp  : endpoints with W_i <= small_w; one warp, an open-addressing table in shared memory
-//           (keys u2, values w), linear probing, insert by atomicCAS / atomicAdd.
-//   block : larger endpoints, one CTA per endpoint taken from a global work counter; the table
-//           is a dense shared-memory window over [0, i) (BATCHS-style dense counters), a
-//           shared-memory hash table, or a per-CTA dense array in global scratch memory when
-//           neither fits.
-// The wedge list of an endpoint is flattened: each chunk of neighbours gets an inclusive scan
-// of its prefix lengths, and lane/thread t locates its neighbour by a branchless binary search
-// over that scan, so consecutive threads read consecutive entries of N(v) (coalesced).
+// Aggregators (the multiplicity table w), by the wedges W_i of the endpoint:
+//   warp : W_i <= small_w; one warp, an open-addressing table in shared memory.
+//   mid  : W_i <= mid_w and the table fits a CTA of 128 threads; many such CTAs share an SM, since
+//          an endpoint of this size is a chain of a few round trips, not a throughput problem.
+//   block: larger endpoints, one CTA of 512 threads per endpoint taken from a global work counter.
+// The CTA kernels choose among dense counters over [0, i) (BATCHS-style; 16 bits wide when the
+// degree allows), a hash table, dense counters for the low ranks with a hash table for the rest,
+// and a per-CTA dense array in global scratch memory when none of them holds the endpoint.
+// Hash entries are one 32-bit word (key and count) whenever the count fits beside the key, so an
+// insertion is one shared-memory atomic.
+// The wedge list of an endpoint is cut into pieces of neighbour lists, each walked by a warp, so
+// consecutive lanes read consecutive entries of N(v) (coalesced).
+// Per-edge credits are gathered per slot of the ranked CSR, where the wedges of a piece lie next to
+// each other (one 128-byte atomic request per 32 wedges instead of 32 scattered ones), and moved to
+// output edge order once at the end.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -34,8 +39,11 @@ namespace pb {
 namespace {
 
 constexpr uint32_t kEmpty = 0xFFFFFFFFu;
-constexpr int kWarpTable = 1024;  // slots per warp (keys + values = 8 KiB)
+constexpr int kWarpTable = 1024;  // slots per warp
 constexpr int kWarpsPerBlockSmall = 8;
+constexpr uint32_t kHotRanks = 256;   // count_warp_kernel: vertex counts gathered per CTA
+constexpr uint32_t kWarpRow = 1024;   // longer rows take a CTA
+constexpr uint32_t kMidRow = 16384;   // longer rows take a large CTA
 
 enum Per { VERT = 0, EDGE = 1, TOTAL = 2 };
 
@@ -43,7 +51,6 @@ struct Params {
   const uint32_t* __restrict__ off;
   const uint32_t* __restrict__ adj;
   const uint32_t* __restrict__ pref;
-  const uint32_t* __restrict__ eout;
   const int64_t* __restrict__ wsum;
   int64_t n;
   int per;
@@ -51,11 +58,12 @@ struct Params {
   int64_t out_len;  // entries of out
   int64_t m2;       // slots of the ranked CSR
   uint32_t* err;    // record of the first bounds violation {code, index lo, index hi, aux}
-  uint32_t* out32;  // per-edge counts accumulated in 32 bits when every count fits (else null)
+  uint32_t* sacc32;             // per-edge counts per slot: 32 bits wide when every count fits,
+  unsigned long long* sacc64;   // else 64 (the other is null)
   unsigned long long* mstats;  // per mode (dense, hash, hybrid, global): endpoints, wedges
-  // Scheduler hooks of the block aggregator (all null on the plain path):
-  const uint8_t* modes;        // modes[q]: aggregation mode of item q chosen by the scheduler
-  uint8_t* mode_out;           // mode_out[q]: mode item q ran with
+  // Block aggregator (null for the mid kernel):
+  const uint8_t* modes;        // modes[q]: aggregation mode of item q
+  uint8_t* mode_out;           // mode_out[q]: mode item q ran with (scheduler hooks)
   unsigned long long* cycles;  // cycles[q]: SM cycles item q took (clock64, thread 0)
 };
 
@@ -72,8 +80,7 @@ __device__ __noinline__ void record_violation(uint32_t* err, uint32_t code, uint
 // (and reported as an error by the host) instead of being accessed.
 __device__ __forceinline__ void credit(const Params& P, uint64_t idx, int64_t v, uint32_t code) {
   if (idx >= (uint64_t)P.out_len) { record_violation(P.err, code, idx, 0); return; }
-  if (P.out32) atomicAdd(&P.out32[idx], (uint32_t)v);  // L2-resident 32-bit accumulation
-  else atomic_add_i64(&P.out[idx], v);
+  atomic_add_i64(&P.out[idx], v);
 }
 
 __device__ __forceinline__ bool slot_ok(const Params& P, uint64_t slot, uint32_t code) {
@@ -81,143 +88,221 @@ __device__ __forceinline__ bool slot_ok(const Params& P, uint64_t slot, uint32_t
   return true;
 }
 
-// Fibonacci hashing: the high bits of key * 2^32/phi, folded into the table size.
-__device__ __forceinline__ uint32_t hash_slot(uint32_t key, uint32_t mask) {
-  return __umulhi(key * 0x9E3779B1u, mask + 1u) & mask;
+// Per-edge credit of a slot (checked by the caller).
+__device__ __forceinline__ void credit_slot(const Params& P, uint32_t slot, uint32_t v) {
+  if (P.sacc32) atomicAdd(&P.sacc32[slot], v);
+  else atomicAdd(&P.sacc64[slot], (unsigned long long)v);
 }
 
-// Insert-or-increment.  Tables are sized to at least twice the wedge count, so a probe
-// sequence never exceeds the table size; the bound turns a broken invariant into a recorded
-// error instead of an endless loop.
-__device__ __forceinline__ bool table_insert(uint32_t* keys, uint32_t* vals, uint32_t mask, uint32_t key) {
-  uint32_t h = hash_slot(key, mask);
-  for (uint32_t probes = 0; probes <= mask; ++probes) {
-    uint32_t k = keys[h];
-    if (k == key) { atomicAdd(&vals[h], 1u); return true; }
+// Fibonacci hashing: the high bits of key * 2^32/phi, folded into the table size (any size).
+__device__ __forceinline__ uint32_t hash_slot(uint32_t key, uint32_t size) { return __umulhi(key * 0x9E3779B1u, size); }
+
+// Tables.  kOne: one word per slot, key << cb | count (cb count bits; the caller guarantees counts
+// of at most 2^cb - 2, so no entry equals kEmpty).  Otherwise keys and counts in two arrays of
+// `size` words (cb is 0).  Insert-or-increment; tables hold at most 3/4 of their slots, so a probe
+// sequence never exceeds the table size; the bound turns a broken invariant into a recorded error
+// instead of an endless loop.
+template <bool kOne>
+__device__ __forceinline__ bool table_insert(uint32_t* tab, uint32_t size, int cb, uint32_t key) {
+  uint32_t h = hash_slot(key, size);
+  for (uint32_t probes = 0; probes < size; ++probes) {
+    uint32_t k = tab[h];
     if (k == kEmpty) {
-      uint32_t prev = atomicCAS(&keys[h], kEmpty, key);
-      if (prev == kEmpty || prev == key) { atomicAdd(&vals[h], 1u); return true; }
+      k = atomicCAS(&tab[h], kEmpty, kOne ? (key << cb) | 1u : key);
+      if (k == kEmpty) {
+        if (!kOne) atomicAdd(&tab[size + h], 1u);
+        return true;
+      }
     }
-    h = (h + 1) & mask;
+    if ((kOne ? k >> cb : k) == key) {
+      atomicAdd(&tab[kOne ? h : size + h], 1u);
+      return true;
+    }
+    h = h + 1 == size ? 0u : h + 1;
   }
   return false;
 }
 
-__device__ __forceinline__ uint32_t table_find(const uint32_t* keys, const uint32_t* vals, uint32_t mask,
-                                               uint32_t key) {
-  uint32_t h = hash_slot(key, mask);
-  for (uint32_t probes = 0; probes <= mask; ++probes) {
-    uint32_t k = keys[h];
-    if (k == key) return vals[h];
+template <bool kOne>
+__device__ __forceinline__ uint32_t table_find(const uint32_t* tab, uint32_t size, int cb, uint32_t key) {
+  uint32_t h = hash_slot(key, size);
+  for (uint32_t probes = 0; probes < size; ++probes) {
+    const uint32_t k = tab[h];
+    if ((kOne ? k >> cb : k) == key) return kOne ? k & ((1u << cb) - 1u) : tab[size + h];
     if (k == kEmpty) return 0;  // unreachable for keys that were inserted
-    h = (h + 1) & mask;
+    h = h + 1 == size ? 0u : h + 1;
   }
   return 0;
 }
 
-__device__ __forceinline__ uint32_t next_pow2(uint32_t x) { return x <= 1 ? 1u : 1u << (32 - __clz(x - 1)); }
+// Entry of slot s: its key and count (count 0 when empty).
+__device__ __forceinline__ uint32_t table_entry(const uint32_t* tab, uint32_t size, int cb, uint32_t s, uint32_t& key) {
+  const uint32_t k = tab[s];
+  key = k >> cb;
+  return k == kEmpty ? 0u : (cb ? k & ((1u << cb) - 1u) : tab[size + s]);
+}
 
-// Iterates every wedge of endpoint i (slots [b, e) of the ranked CSR) with one warp.
-// f(j, vt, slot2, u2t): j = slot of (i, v), vt = tagged v, slot2 = slot of (v, u2), u2t = tagged u2.
-template <class F>
-__device__ __forceinline__ void warp_wedges(uint32_t b, uint32_t e, const Params& P, F&& f) {
+// Endpoint lists: {endpoint, first slot, end slot, wedges (saturated)}.
+__device__ __forceinline__ unsigned list_at(uint32_t* counter, bool have) {
+  const unsigned bal = __ballot_sync(0xffffffffu, have);
+  unsigned base = 0;
+  if (bal && lane_id() == (unsigned)(__ffs(bal) - 1)) base = atomicAdd(counter, (uint32_t)__popc(bal));
+  base = __shfl_sync(0xffffffffu, base, bal ? __ffs(bal) - 1 : 0);
+  return base + __popc(bal & ((1u << lane_id()) - 1u));
+}
+
+// One slot of an endpoint's row, as a lane holds it: the wedges of the slot, the tagged neighbour
+// and where the neighbour's row begins.
+struct SlotRow {
+  uint32_t L, vt, vs;
+};
+
+__device__ __forceinline__ SlotRow load_slot(uint32_t j, uint32_t e, const Params& P) {
+  SlotRow r{0, kEmpty, 0};
+  if (j < e) {
+    r.L = P.pref[j];
+    r.vt = P.adj[j];
+    if ((r.vt >> 1) < P.n) r.vs = P.off[r.vt >> 1];
+    else { record_violation(P.err, 28, r.vt, j); r.L = 0; }
+  }
+  return r;
+}
+
+// Iterates every wedge of an endpoint (slots [b, e) of the ranked CSR) with one warp, 32 slots and
+// then four steps of 32 wedges at a time (their loads are issued together).  `row` holds the first
+// group's slots.  slots(): all lanes, once per group; f(lo, slot2, u2): lo = lane of the wedge's
+// slot; group_end(j, vt): all lanes, with this lane's slot (vt = kEmpty beyond the end).
+template <class Slots, class F, class End>
+__device__ __forceinline__ void warp_wedges(uint32_t b, uint32_t e, SlotRow row, const Params& P, Slots&& slots, F&& f,
+                                            End&& group_end) {
   const unsigned lane = lane_id();
   for (uint32_t j0 = b; j0 < e; j0 += 32) {
-    const uint32_t j = j0 + lane;
-    uint32_t L = 0, vt = 0, vs = 0;
-    if (j < e) {
-      L = P.pref[j];
-      vt = P.adj[j];
-      if ((vt >> 1) < P.n) vs = P.off[vt >> 1];
-      else { record_violation(P.err, 28, vt, j); L = 0; }
-    }
-    const uint32_t incl = warp_inclusive_scan(L);
-    const uint32_t excl = incl - L;
+    if (j0 != b) row = load_slot(j0 + lane, e, P);
+    slots();
+    const uint32_t incl = warp_inclusive_scan(row.L);
+    const uint32_t from = row.vs - (incl - row.L);  // slot2 = from + t
     const uint32_t T = __shfl_sync(0xffffffffu, incl, 31);
-    for (uint32_t t0 = 0; t0 < T; t0 += 32) {
-      const uint32_t t = t0 + lane;
-      uint32_t lo = 0;
+    for (uint32_t t0 = 0; t0 < T; t0 += 128) {
+      uint32_t at[4], s2[4], x[4];
 #pragma unroll
-      for (uint32_t step = 16; step > 0; step >>= 1) {
-        uint32_t x = __shfl_sync(0xffffffffu, incl, lo + step - 1);
-        if (x <= t) lo += step;
+      for (int r = 0; r < 4; ++r) {
+        const uint32_t t = t0 + 32 * r + lane;
+        uint32_t lo = 0;
+#pragma unroll
+        for (uint32_t step = 16; step > 0; step >>= 1) {
+          const uint32_t y = __shfl_sync(0xffffffffu, incl, lo + step - 1);
+          if (y <= t) lo += step;
+        }
+        at[r] = lo;
+        s2[r] = __shfl_sync(0xffffffffu, from, lo) + t;
+        x[r] = kEmpty;
+        if (t < T && slot_ok(P, s2[r], 20)) x[r] = P.adj[s2[r]];
       }
-      const uint32_t ex = __shfl_sync(0xffffffffu, excl, lo);
-      const uint32_t vsj = __shfl_sync(0xffffffffu, vs, lo);
-      const uint32_t vtj = __shfl_sync(0xffffffffu, vt, lo);
-      if (t < T) {
-        const uint32_t slot2 = vsj + (t - ex);
-        if (slot_ok(P, slot2, 20)) f(j0 + lo, vtj, slot2, P.adj[slot2]);
-      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        if (x[r] != kEmpty) f(at[r], s2[r], x[r] >> 1);
     }
+    __syncwarp();
+    group_end(j0 + lane, row.vt);
   }
 }
 
-// Per-thread accumulator of per-(i,v) credits, flushed when the neighbour slot changes.
-struct SlotAcc {
-  uint32_t j = kEmpty;
-  int64_t acc = 0;
-  __device__ __forceinline__ void flush(const Params& P) {
-    if (j != kEmpty && acc) {
-      if (!slot_ok(P, j, 10)) return;
-      if (P.per == VERT) credit(P, P.adj[j] >> 1, acc, 11);
-      else credit(P, P.eout[j], acc, 12);
-    }
-    acc = 0;
-  }
-  __device__ __forceinline__ void add(const Params& P, uint32_t jj, int64_t x) {
-    if (jj != j) { flush(P); j = jj; }
-    acc += x;
-  }
-};
-
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) count_warp_kernel(Params P, int small_w) {
-  extern __shared__ uint32_t smem_w[];
+// Small endpoints: a warp each.  Bound by latency: an endpoint is a chain of round trips for a few
+// dozen to 512 wedges, so what counts is the number of warps (48 per SM with one-word tables of
+// 4 KiB; 24 with two-array tables) and that the next endpoint's list entry and first slots are
+// loaded while this one is counted.
+// The vertices of the lowest ranks share wedges with most endpoints: their counts are gathered per
+// CTA (1e6 endpoints adding to one address took 5.2 ms on the power-law graph of 1e7 edges, the
+// aggregation as a whole 12.2 ms; 6.5 ms with this).
+// kOneWord false: two-array tables (more than 2^22 vertices leave no room for a count of 512).
+template <bool kOneWord>
+__global__ void __launch_bounds__(256, kOneWord ? 6 : 3) count_warp_kernel(Params P, const uint4* __restrict__ items,
+                                                                         const uint32_t* __restrict__ n_items_dev,
+                                                                         int count_bits) {
+  extern __shared__ __align__(16) uint32_t smem_w[];
   const unsigned lane = lane_id();
   const int wib = threadIdx.x >> 5;
-  uint32_t* keys = smem_w + wib * (2 * kWarpTable);
-  uint32_t* vals = keys + kWarpTable;
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const int cb = kOneWord ? count_bits : 0;
+  uint32_t* hot = smem_w;  // low and high words of the lowest ranks' counts
+  for (uint32_t s = threadIdx.x; s < 2 * kHotRanks; s += blockDim.x) hot[s] = 0;
+  __syncthreads();
+  uint32_t* tab = smem_w + 2 * kHotRanks + wib * ((kOneWord ? 1 : 2) * kWarpTable + 32);
+  uint32_t* acc = tab + (kOneWord ? 1 : 2) * kWarpTable;  // credits of the group's 32 slots
+  const uint32_t n_items = *n_items_dev;
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   int64_t total = 0;
-  for (int64_t i = warp; i < P.n; i += nwarps) {
-    const int64_t W = P.wsum[i + 1] - P.wsum[i];
-    if (W <= 0 || W > small_w) {
-      if (W < 0 && lane == 0) record_violation(P.err, 34, (uint64_t)i, 0);
-      continue;
+  uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  // Two list entries ahead, one row ahead.
+  uint4 next = q < n_items ? items[q] : make_uint4(0, 0, 0, 0);
+  uint4 after = q + nwarps < n_items ? items[q + nwarps] : make_uint4(0, 0, 0, 0);
+  SlotRow next_row = load_slot(next.y + lane, next.z, P);
+  for (; q < n_items; q += nwarps) {
+    const uint4 it = next;
+    const SlotRow row = next_row;
+    const uint32_t i = it.x, b = it.y, e = it.z;
+    next = after;
+    after = q + 2 * nwarps < n_items ? items[q + 2 * nwarps] : make_uint4(0, 0, 0, 0);
+    // The next endpoint's first slots: issued here, their row starts (a dependent load) below.
+    next_row = SlotRow{0, kEmpty, 0};
+    if (next.y + lane < next.z) {
+      next_row.L = P.pref[next.y + lane];
+      next_row.vt = P.adj[next.y + lane];
     }
-    const uint32_t b = P.off[i], e = P.off[i + 1];
-    const bool tag_i = !(P.adj[b] & 1u);
+    const bool tag_i = !(__shfl_sync(0xffffffffu, row.vt, 0) & 1u);
     const bool need_center = P.per == EDGE || (P.per == VERT && !tag_i);
-    const uint32_t tsize = max(64u, next_pow2(2u * (uint32_t)W));
-    const uint32_t mask = tsize - 1;
-    for (uint32_t s = lane; s < tsize; s += 32) { keys[s] = kEmpty; vals[s] = 0; }
+    const uint32_t tsize = max(64u, (2u * it.w + 3u) & ~3u);
+    const uint32_t words = kOneWord ? tsize : 2 * tsize;
+    for (uint32_t s = lane * 4; s < words; s += 128) {
+      const uint32_t x = s < tsize ? kEmpty : 0u;
+      *reinterpret_cast<uint4*>(tab + s) = make_uint4(x, x, x, x);
+    }
     __syncwarp();
-    warp_wedges(b, e, P, [&](uint32_t, uint32_t, uint32_t, uint32_t u2t) {
-      if (!table_insert(keys, vals, mask, u2t >> 1)) record_violation(P.err, 25, u2t >> 1, (uint32_t)i);
-    });
+    warp_wedges(b, e, row, P, [] {}, [&](uint32_t, uint32_t, uint32_t u2) {
+      if (!table_insert<kOneWord>(tab, tsize, cb, u2)) record_violation(P.err, 25, u2, i);
+    }, [](uint32_t, uint32_t) {});
     __syncwarp();
+    if (next_row.vt != kEmpty) {
+      if ((next_row.vt >> 1) < P.n) next_row.vs = P.off[next_row.vt >> 1];
+      else { record_violation(P.err, 28, next_row.vt, next.y + lane); next_row.L = 0; }
+    }
     if (need_center) {
-      SlotAcc acc;
-      warp_wedges(b, e, P, [&](uint32_t jj, uint32_t, uint32_t slot2, uint32_t u2t) {
-        const uint32_t w = table_find(keys, vals, mask, u2t >> 1);
-        if (w > 1) {
-          if (P.per == EDGE) credit(P, P.eout[slot2], (int64_t)(w - 1), 13);
-          acc.add(P, jj, (int64_t)(w - 1));
-        }
-      });
-      acc.flush(P);
+      warp_wedges(b, e, row, P,
+                  [&] {
+                    acc[lane] = 0;
+                    __syncwarp();
+                  },
+                  [&](uint32_t lo, uint32_t slot2, uint32_t u2) {
+                    const uint32_t w = table_find<kOneWord>(tab, tsize, cb, u2);
+                    if (w > 1) {
+                      if (P.per == EDGE) credit_slot(P, slot2, w - 1);
+                      atomicAdd(&acc[lo], w - 1);
+                    }
+                  },
+                  [&](uint32_t j, uint32_t vt) {
+                    const uint32_t a = acc[lane];
+                    if (a && vt != kEmpty) {
+                      if (P.per == EDGE) credit_slot(P, j, a);
+                      else credit(P, vt >> 1, a, 11);
+                    }
+                    __syncwarp();
+                  });
     } else {
       int64_t mine = 0;
       for (uint32_t s = lane; s < tsize; s += 32) {
-        const uint32_t k = keys[s];
-        if (k == kEmpty) continue;
-        const int64_t w = vals[s];
+        uint32_t k;
+        const int64_t w = table_entry(tab, tsize, cb, s, k);
         if (w < 2) continue;
         const int64_t bf = w * (w - 1) / 2;
         mine += bf;
-        if (P.per == VERT) credit(P, k, bf, 14);
+        if (P.per == VERT) {
+          if (k < kHotRanks) {
+            const uint32_t old = atomicAdd(&hot[k], (uint32_t)bf);
+            if (old + (uint32_t)bf < old) atomicAdd(&hot[kHotRanks + k], 1u);
+          } else {
+            credit(P, k, bf, 14);
+          }
+        }
       }
       if (P.per == VERT) {
         mine = warp_sum(mine);
@@ -231,38 +316,33 @@ __global__ void __launch_bounds__(256) count_warp_kernel(Params P, int small_w) 
   if (P.per == TOTAL) {
     total = warp_sum(total);
     if (lane == 0 && total) atomic_add_i64(P.out, total);
+  } else if (P.per == VERT) {
+    __syncthreads();
+    for (uint32_t s = threadIdx.x; s < kHotRanks; s += blockDim.x) {
+      const int64_t v = ((int64_t)hot[kHotRanks + s] << 32) | hot[s];
+      if (v) credit(P, s, v, 17);
+    }
   }
 }
 
 // ---------------------------------------------------------------------------------------------
-constexpr int kBlock = 512;
+constexpr int kBlock = 512;    // threads of the block aggregator
+constexpr int kBlockPerSm = 3; // with 72 KiB of shared memory each (pb_engine.cuh): aggregation of
+                               // the R-MAT graph of 2^24 edges, per edge: 18.6 ms; 512 threads x 2
+                               // per SM 22.0, 256 x 4 21.5, 256 x 6 21.7, 1024 x 1 27.2
+constexpr int kMidBlock = 128; // threads of the mid aggregator
 
+template <int NT>
 struct BlockShared {
-  uint32_t incl[kBlock];
-  uint32_t vs[kBlock];
-  uint32_t vt[kBlock];
-  uint32_t len[kBlock];
-  uint32_t scan[32];
+  uint32_t vs[NT];
+  uint32_t vt[NT];
+  uint32_t len[NT];
+  uint16_t list[NT];
   int64_t red[32];
-  uint32_t item;
-  uint32_t cursor;
+  uint32_t item, n_short, n_long;
 };
-
-__device__ __forceinline__ uint32_t block_inclusive_scan_u32(uint32_t x, uint32_t* smem, uint32_t& total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  uint32_t incl = warp_inclusive_scan(x);
-  if (lane == 31) smem[warp] = incl;
-  __syncthreads();
-  if (warp == 0) {
-    uint32_t v = lane < nwarps ? smem[lane] : 0u;
-    v = warp_inclusive_scan(v);
-    smem[lane] = v;
-  }
-  __syncthreads();
-  incl += warp > 0 ? smem[warp - 1] : 0u;
-  total = smem[nwarps - 1];
-  return incl;
-}
+template <int NT>
+constexpr size_t shared_fixed() { return (sizeof(BlockShared<NT>) + 15) & ~size_t(15); }
 
 __device__ __forceinline__ int64_t block_sum_i64(int64_t x, int64_t* smem) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
@@ -278,17 +358,30 @@ __device__ __forceinline__ int64_t block_sum_i64(int64_t x, int64_t* smem) {
   return t;  // valid in thread 0
 }
 
-// Iterates every wedge of endpoint i with the whole CTA.  Per chunk of kBlock neighbours, each
-// neighbour's prefix N(v)[0, L) is cut into pieces of at most kPiece wedges; warps claim pieces
-// from a shared-memory counter, locate a piece's neighbour once (binary search over the
-// chunk's inclusive piece counts) and walk it with 32 lanes, so consecutive lanes read
-// consecutive entries of N(v) and no per-wedge search is needed.
-constexpr uint32_t kPiece = 256;
+// Iterates every wedge of an endpoint with the whole CTA, NT neighbours at a time.  Neighbours with
+// prefixes N(v)[0, L) of up to kLong wedges go to the warps in turn, longer ones are walked by all
+// warps together.  Lane t of a walk takes entries t, t + 32, ... with four loads in flight, so loads
+// and atomics on the entries' slots are coalesced.  f(slot2, u2) per wedge; part_end(j, vt): all
+// lanes of a warp, after its part of neighbour slot j.
+constexpr uint32_t kLong = 512;
 
-template <class F>
-__device__ __forceinline__ void block_wedges(uint32_t b, uint32_t e, const Params& P, BlockShared& S, F&& f) {
+template <uint32_t kStride, class F>
+__device__ __forceinline__ void walk_prefix(const uint32_t* __restrict__ adj, uint32_t beg, uint32_t end, F&& f) {
+  for (uint32_t s0 = beg; s0 < end; s0 += 4 * kStride) {
+    uint32_t x[4];
+#pragma unroll
+    for (uint32_t r = 0; r < 4; ++r) x[r] = s0 + r * kStride < end ? __ldg(adj + s0 + r * kStride) : kEmpty;
+#pragma unroll
+    for (uint32_t r = 0; r < 4; ++r)
+      if (x[r] != kEmpty) f(s0 + r * kStride, x[r] >> 1);
+  }
+}
+
+template <int NT, class F, class End>
+__device__ __forceinline__ void block_wedges(uint32_t b, uint32_t e, const Params& P, BlockShared<NT>& S, F&& f,
+                                             End&& part_end) {
   const uint32_t tid = threadIdx.x, lane = tid & 31u;
-  for (uint32_t j0 = b; j0 < e; j0 += kBlock) {
+  for (uint32_t j0 = b; j0 < e; j0 += NT) {
     const uint32_t j = j0 + tid;
     uint32_t L = 0, vt = 0, vs = 0;
     if (j < e) {
@@ -296,229 +389,256 @@ __device__ __forceinline__ void block_wedges(uint32_t b, uint32_t e, const Param
       vt = P.adj[j];
       if ((vt >> 1) < P.n) vs = P.off[vt >> 1];
       else { record_violation(P.err, 29, vt, j); L = 0; }
+      if (L && !slot_ok(P, (uint64_t)vs + L - 1, 21)) L = 0;
     }
-    uint32_t T;
-    const uint32_t incl = block_inclusive_scan_u32((L + kPiece - 1) / kPiece, S.scan, T);
-    S.incl[tid] = incl;
     S.vs[tid] = vs;
     S.vt[tid] = vt;
     S.len[tid] = L;
-    if (tid == 0) S.cursor = 0;
+    // Neighbours without wedges are left out: slots k of the chunk, in any order.
+    const unsigned some = __ballot_sync(0xffffffffu, L > 0 && L <= kLong);
+    unsigned at = 0;
+    if (lane == 0 && some) at = atomicAdd(&S.n_short, (uint32_t)__popc(some));
+    at = __shfl_sync(0xffffffffu, at, 0) + __popc(some & ((1u << lane) - 1u));
+    if (L > 0 && L <= kLong) S.list[at] = (uint16_t)tid;
+    if (L > kLong) S.list[NT - 1 - atomicAdd(&S.n_long, 1u)] = (uint16_t)tid;
     __syncthreads();
-    while (true) {
-      uint32_t p = 0;
-      if (lane == 0) p = atomicAdd(&S.cursor, 1u);
-      p = __shfl_sync(0xffffffffu, p, 0);
-      if (p >= T) break;
-      uint32_t lo = 0;
-#pragma unroll
-      for (uint32_t step = kBlock / 2; step > 0; step >>= 1)
-        if (S.incl[lo + step - 1] <= p) lo += step;
-      const uint32_t first_piece = lo ? S.incl[lo - 1] : 0u;
-      const uint32_t k0 = (p - first_piece) * kPiece;
-      const uint32_t kend = min(k0 + kPiece, S.len[lo]);
-      const uint32_t vsj = S.vs[lo], vtj = S.vt[lo];
-      // Vectorised walk: lane t takes the aligned group of four entries at g + 4t (one 16-byte
-      // load; the adjacency array is 16-byte aligned and padded to whole groups), and uses the
-      // entries inside the piece [vsj + k0, vsj + kend).
-      const uint32_t pbeg = vsj + k0, pend = vsj + kend;
-      for (uint32_t g = (pbeg & ~3u) + 4u * lane; g < pend; g += 128u) {
-        if (!slot_ok(P, g, 21)) break;
-        const uint4 q = __ldg(reinterpret_cast<const uint4*>(P.adj + g));
-        const uint32_t x[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-        for (uint32_t r = 0; r < 4; ++r) {
-          const uint32_t slot2 = g + r;
-          if (slot2 >= pbeg && slot2 < pend && slot_ok(P, slot2, 21)) f(j0 + lo, vtj, slot2, x[r]);
-        }
-      }
+    const uint32_t ns = S.n_short, nl = S.n_long;
+    for (uint32_t p = tid >> 5; p < ns; p += NT / 32) {
+      const uint32_t k = S.list[p], beg = S.vs[k];
+      walk_prefix<32>(P.adj, beg + lane, beg + S.len[k], f);
+      __syncwarp();
+      part_end(j0 + k, S.vt[k]);
+    }
+    for (uint32_t p = 0; p < nl; ++p) {
+      const uint32_t k = S.list[NT - 1 - p], beg = S.vs[k];
+      walk_prefix<NT>(P.adj, beg + tid, beg + S.len[k], f);
+      __syncwarp();
+      part_end(j0 + k, S.vt[k]);
     }
     __syncthreads();
+    if (tid == 0) S.n_short = S.n_long = 0;  // the next chunk's adds come after a barrier below
+    if (j0 + NT < e) __syncthreads();
   }
 }
 
+// The mid aggregator: CTAs of 128 threads with a table of about 18 KiB, ten to an SM.
+constexpr int kMidSmem = 22 << 10;
+constexpr int kMidPerSm = 10;
+constexpr int64_t kMidWedges = 2047;
+
 enum Mode : uint32_t { MODE_DENSE = 0, MODE_HASH = 1, MODE_GLOBAL = 2, MODE_HYBRID = 3 };
-// A scheduler mode entry that leaves the item to the plain rule (items too light for the
-// choice to matter are not scored by the learned scheduler).
-constexpr uint8_t kPlainRule = 0xFF;
 // Items with fewer wedges are left to the plain rule when the learned scheduler runs.
 constexpr int64_t kSchedMinWedges = 2048;
 
-__global__ void __launch_bounds__(kBlock) count_block_kernel(Params P, const uint32_t* __restrict__ items,
-                                                             const uint32_t* __restrict__ n_items_dev,
-                                                             uint32_t* cursor, uint32_t* gscratch,
-                                                             uint32_t cap_dense, uint32_t cap_hash,
-                                                             uint32_t hy_dense, uint32_t hy_hash) {
+// What a CTA's table area of tw words can hold.  Counts of an endpoint are at most its degree.
+struct Geom {
+  uint32_t tw;      // words of the table area
+  uint32_t hy_words;  // hybrid: words of the dense counters (16 bits each); the hash takes the rest
+  int cb;           // count bits of a one-word hash entry
+
+  __device__ __forceinline__ int bits(uint32_t deg) const { return deg < (1u << cb) - 1u ? cb : 0; }
+  __device__ __forceinline__ bool wide(uint32_t deg) const { return deg > 0xFFFFu; }
+  __device__ __forceinline__ bool dense_ok(uint32_t i, uint32_t deg) const { return i <= (wide(deg) ? tw : 2 * tw); }
+  __device__ __forceinline__ bool hash_ok(uint64_t W, uint32_t deg) const { return W * (bits(deg) ? 2 : 4) <= tw; }
+  __device__ __forceinline__ uint32_t hy_dense() const { return 2 * hy_words; }
+  __device__ __forceinline__ uint32_t hy_slots(uint32_t deg) const { return (tw - hy_words) / (bits(deg) ? 1 : 2); }
+  __device__ __forceinline__ bool hybrid_ok(uint64_t hi, uint32_t deg) const {
+    return !wide(deg) && 4 * hi <= 3ull * hy_slots(deg);
+  }
+  // The plain rule.  Dense counters when clearing and scanning them costs less than the wedges do;
+  // else a hash table; dense counters again; low ranks dense and the rest hashed; global scratch.
+  __device__ __forceinline__ Mode rule(uint32_t i, uint64_t W, uint32_t deg, uint64_t hi) const {
+    if (dense_ok(i, deg) && (uint64_t)i <= 4 * W) return MODE_DENSE;
+    if (hash_ok(W, deg)) return MODE_HASH;
+    if (dense_ok(i, deg)) return MODE_DENSE;
+    return hybrid_ok(hi, deg) ? MODE_HYBRID : MODE_GLOBAL;
+  }
+};
+
+// Wedges of an endpoint that end at or above rank d, counted by one warp (valid in lane 0): per
+// neighbour, the prefix length minus the entries below d (one binary search each).
+__device__ __forceinline__ uint64_t warp_high_wedges(const Params& P, const uint4& it, int64_t W, uint32_t d) {
+  unsigned long long lo_w = 0;
+  for (uint32_t j = it.y + lane_id(); j < it.z; j += 32) {
+    const uint32_t v = P.adj[j] >> 1;
+    if (v >= P.n) continue;
+    const uint32_t vb = P.off[v];
+    lo_w += min(lower_bound_u32(P.adj, vb, P.off[v + 1], d << 1) - vb, P.pref[j]);
+  }
+  return (uint64_t)(W - (int64_t)warp_sum(lo_w));
+}
+
+// The plain rule's mode of every block-aggregator item (one warp each); *n_global counts those
+// that need global scratch.
+__global__ void plain_modes_kernel(Params P, const uint4* __restrict__ items, const uint32_t* __restrict__ n_items_dev,
+                                   Geom G, uint8_t* modes, uint32_t* n_global) {
+  const uint32_t n_items = *n_items_dev;
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < n_items; q += nwarps) {
+    const uint4 it = items[q];
+    const int64_t W = P.wsum[it.x + 1] - P.wsum[it.x];
+    const uint32_t deg = it.z - it.y;
+    uint64_t hi = 0;
+    if (!G.dense_ok(it.x, deg) && !G.hash_ok(W, deg)) hi = warp_high_wedges(P, it, W, G.hy_dense());
+    if (lane_id() == 0) {
+      const Mode m = G.rule(it.x, W, deg, hi);
+      modes[q] = (uint8_t)m;
+      if (m == MODE_GLOBAL) atomicAdd(n_global, 1u);
+    }
+  }
+}
+
+// One CTA of NT threads per endpoint.  Bound by shared-memory atomics and latency; the two table
+// walks read 4 bytes a wedge each, mostly from L2.
+template <int NT, int kMinBlocks>
+__global__ void __launch_bounds__(NT, kMinBlocks) count_block_kernel(Params P, const uint4* __restrict__ items,
+                                                                     const uint32_t* __restrict__ n_items_dev,
+                                                                     uint32_t* cursor, uint32_t* gscratch, Geom G) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  BlockShared& S = *reinterpret_cast<BlockShared*>(smem_raw);
-  uint32_t* table = reinterpret_cast<uint32_t*>(smem_raw + ((sizeof(BlockShared) + 15) & ~size_t(15)));
+  BlockShared<NT>& S = *reinterpret_cast<BlockShared<NT>*>(smem_raw);
+  uint32_t* table = reinterpret_cast<uint32_t*>(smem_raw + shared_fixed<NT>());
   uint32_t* gcnt = gscratch ? gscratch + (size_t)blockIdx.x * (size_t)P.n : nullptr;
   const uint32_t n_items = *n_items_dev;
+  const unsigned lane = lane_id();
   int64_t total = 0;
-  while (true) {
-    if (threadIdx.x == 0) S.item = atomicAdd(cursor, 1u);
-    __syncthreads();
-    const uint32_t q = S.item;
-    __syncthreads();
-    if (q >= n_items) break;
+  if (threadIdx.x == 0) S.n_short = S.n_long = 0;
+  // The first item of a CTA is its own number; the cursor hands out the later ones.
+  for (uint32_t q = blockIdx.x; q < n_items;) {
+    if (threadIdx.x == 0) S.item = gridDim.x + atomicAdd(cursor, 1u);
     const long long t_item = clock64();
-    const uint32_t i = items[q];
-    const int64_t W = P.wsum[i + 1] - P.wsum[i];
-    const uint32_t b = P.off[i], e = P.off[i + 1];
+    const uint4 it = items[q];
+    const uint32_t i = it.x, b = it.y, e = it.z, deg = e - b;
+    const int64_t W = NT == kMidBlock ? (int64_t)it.w : P.wsum[i + 1] - P.wsum[i];
     const bool tag_i = !(P.adj[b] & 1u);
     const bool need_center = P.per == EDGE || (P.per == VERT && !tag_i);
     Mode mode;
-    if (P.modes && P.modes[q] != kPlainRule) mode = (Mode)(P.modes[q] & 3u);
-    else if (i <= cap_dense && (uint64_t)i <= 4ull * (uint64_t)W) mode = MODE_DENSE;
-    else if ((uint64_t)2 * W <= cap_hash) mode = MODE_HASH;
-    else if (i <= cap_dense) mode = MODE_DENSE;
-    else {
-      // Hybrid: dense counters for u2 < hy_dense (the low ranks, where R-MAT-like graphs put
-      // most wedge ends) plus a hash table for the rest, when the rest is small enough.  The
-      // number of wedges ending at or above hy_dense is exact: per neighbour, the prefix length
-      // minus the entries below hy_dense (one binary search each).
-      unsigned long long lo_w = 0;
-      for (uint32_t j = b + threadIdx.x; j < e; j += kBlock) {
-        const uint32_t v = P.adj[j] >> 1;
-        if (v >= P.n) continue;
-        const uint32_t vb = P.off[v];
-        const uint32_t below = lower_bound_u32(P.adj, vb, P.off[v + 1], hy_dense << 1) - vb;
-        lo_w += min(below, P.pref[j]);
-      }
-      const int64_t lo_total = block_sum_i64((int64_t)lo_w, S.red);
-      if (threadIdx.x == 0) S.item = (uint32_t)(W - lo_total > 0x7fffffff ? 0x7fffffff : W - lo_total);
-      __syncthreads();
-      const uint32_t hi_w = S.item;
-      __syncthreads();
-      mode = (2ull * hi_w <= hy_hash) ? MODE_HYBRID : MODE_GLOBAL;
-    }
+    if (NT == kMidBlock) mode = G.rule(i, W, deg, 0);
+    else mode = (Mode)(P.modes[q] & 3u);
     if (threadIdx.x == 0 && P.mstats) {
       atomicAdd(&P.mstats[mode], 1ull);
       atomicAdd(&P.mstats[4 + mode], (unsigned long long)W);
     }
-    uint32_t tsize = 0, mask = 0;
-    uint32_t* keys = table;
-    uint32_t* vals = table + cap_hash;
-    if (mode == MODE_HYBRID) {
-      keys = table + hy_dense;
-      vals = keys + hy_hash;
-      tsize = hy_hash;
-      mask = tsize - 1;
-    }
-    if (mode == MODE_DENSE) {
-      for (uint32_t s = threadIdx.x; s < i; s += kBlock) table[s] = 0;
-    } else if (mode == MODE_HASH) {
-      tsize = max(64u, next_pow2(2u * (uint32_t)W));
-      mask = tsize - 1;
-      for (uint32_t s = threadIdx.x; s < tsize; s += kBlock) { keys[s] = kEmpty; vals[s] = 0; }
-    } else if (mode == MODE_HYBRID) {
-      for (uint32_t s = threadIdx.x; s < hy_dense; s += kBlock) table[s] = 0;
-      for (uint32_t s = threadIdx.x; s < tsize; s += kBlock) { keys[s] = kEmpty; vals[s] = 0; }
+    const bool wide = G.wide(deg);
+    const int cb = G.bits(deg);
+    // Dense counters (dense, hybrid): u2 below dlim; hash table (hash, hybrid) of tsize slots.
+    const uint32_t dlim = mode == MODE_DENSE ? i : (mode == MODE_HYBRID ? G.hy_dense() : 0u);
+    uint32_t* tab = mode == MODE_HYBRID ? table + G.hy_words : table;
+    const uint32_t tsize = mode == MODE_HASH ? max(64u, 2u * (uint32_t)W) : (mode == MODE_HYBRID ? G.hy_slots(deg) : 0u);
+    const uint32_t dwords = mode == MODE_HYBRID ? G.hy_words : (wide ? dlim : (dlim + 1) / 2);
+    for (uint32_t s = threadIdx.x; s < dwords; s += NT) table[s] = 0;
+    for (uint32_t s = threadIdx.x; s < tsize; s += NT) {
+      tab[s] = kEmpty;
+      if (!cb) tab[tsize + s] = 0;
     }
     __syncthreads();
-    // Phase 1: multiplicities.
-    if (mode == MODE_DENSE) {
-      block_wedges(b, e, P, S, [&](uint32_t, uint32_t, uint32_t, uint32_t u2t) {
-        if ((u2t >> 1) >= i) { record_violation(P.err, 22, u2t >> 1, i); return; }
-        atomicAdd(&table[u2t >> 1], 1u);
-      });
-    } else if (mode == MODE_HASH) {
-      block_wedges(b, e, P, S, [&](uint32_t, uint32_t, uint32_t, uint32_t u2t) {
-        if (!table_insert(keys, vals, mask, u2t >> 1)) record_violation(P.err, 26, u2t >> 1, i);
-      });
-    } else if (mode == MODE_HYBRID) {
-      block_wedges(b, e, P, S, [&](uint32_t, uint32_t, uint32_t, uint32_t u2t) {
-        const uint32_t u2 = u2t >> 1;
-        if (u2 < hy_dense) atomicAdd(&table[u2], 1u);
-        else if (!table_insert(keys, vals, mask, u2)) record_violation(P.err, 35, u2, i);
-      });
+    // Phase 1: multiplicities.  The two common modes have loops of their own.
+    const auto nothing = [](uint32_t, uint32_t) {};
+    if (mode == MODE_DENSE && !wide) {
+      block_wedges<NT>(b, e, P, S, [&](uint32_t, uint32_t u2) {
+        if (u2 < dlim) atomicAdd(&table[u2 >> 1], 1u << (16 * (u2 & 1u)));
+        else record_violation(P.err, 22, u2, i);
+      }, nothing);
+    } else if (mode == MODE_HASH && cb) {
+      block_wedges<NT>(b, e, P, S, [&](uint32_t, uint32_t u2) {
+        if (!table_insert<true>(tab, tsize, cb, u2)) record_violation(P.err, 26, u2, i);
+      }, nothing);
     } else {
-      block_wedges(b, e, P, S, [&](uint32_t, uint32_t, uint32_t, uint32_t u2t) {
-        if ((u2t >> 1) >= P.n) { record_violation(P.err, 23, u2t >> 1, i); return; }
-        atomicAdd(&gcnt[u2t >> 1], 1u);
-      });
+      block_wedges<NT>(b, e, P, S, [&](uint32_t, uint32_t u2) {
+        if (u2 < dlim) {
+          if (wide) atomicAdd(&table[u2], 1u);
+          else atomicAdd(&table[u2 >> 1], 1u << (16 * (u2 & 1u)));
+        } else if (tsize) {
+          if (!(cb ? table_insert<true>(tab, tsize, cb, u2) : table_insert<false>(tab, tsize, 0, u2)))
+            record_violation(P.err, 35, u2, i);
+        } else if (mode == MODE_GLOBAL && u2 < P.n) {
+          atomicAdd(&gcnt[u2], 1u);
+        } else {
+          record_violation(P.err, 23, u2, i);
+        }
+      }, nothing);
     }
     __syncthreads();
     if (need_center) {
       // Phase 2: centre / edge credits.
-      SlotAcc acc;
-      block_wedges(b, e, P, S, [&](uint32_t jj, uint32_t, uint32_t slot2, uint32_t u2t) {
-        const uint32_t u2 = u2t >> 1;
-        uint32_t w;
-        if (u2 >= (mode == MODE_DENSE ? i : (uint32_t)P.n)) { record_violation(P.err, 24, u2, i); return; }
-        if (mode == MODE_DENSE) w = table[u2];
-        else if (mode == MODE_HASH) w = table_find(keys, vals, mask, u2);
-        else if (mode == MODE_HYBRID) w = u2 < hy_dense ? table[u2] : table_find(keys, vals, mask, u2);
-        else w = gcnt[u2];
+      uint32_t mine = 0;
+      auto charge = [&](uint32_t slot2, uint32_t w) {
         if (w > 1) {
-          if (P.per == EDGE) credit(P, P.eout[slot2], (int64_t)(w - 1), 13);
-          acc.add(P, jj, (int64_t)(w - 1));
+          if (P.per == EDGE) credit_slot(P, slot2, w - 1);
+          mine += w - 1;
         }
-      });
-      acc.flush(P);
-      __syncthreads();
+      };
+      auto part_end = [&](uint32_t j, uint32_t vt) {
+        const uint32_t s = __reduce_add_sync(0xffffffffu, mine);
+        mine = 0;
+        if (lane == 0 && s) {
+          if (P.per == EDGE) credit_slot(P, j, s);
+          else credit(P, vt >> 1, s, 11);
+        }
+      };
+      if (mode == MODE_DENSE && !wide) {
+        block_wedges<NT>(b, e, P, S, [&](uint32_t slot2, uint32_t u2) {
+          if (u2 < dlim) charge(slot2, (table[u2 >> 1] >> (16 * (u2 & 1u))) & 0xFFFFu);
+        }, part_end);
+      } else if (mode == MODE_HASH && cb) {
+        block_wedges<NT>(b, e, P, S, [&](uint32_t slot2, uint32_t u2) {
+          charge(slot2, table_find<true>(tab, tsize, cb, u2));
+        }, part_end);
+      } else {
+        block_wedges<NT>(b, e, P, S, [&](uint32_t slot2, uint32_t u2) {
+          uint32_t w = 0;
+          if (u2 < dlim) w = wide ? table[u2] : (table[u2 >> 1] >> (16 * (u2 & 1u))) & 0xFFFFu;
+          else if (tsize) w = cb ? table_find<true>(tab, tsize, cb, u2) : table_find<false>(tab, tsize, 0, u2);
+          else if (mode == MODE_GLOBAL && u2 < P.n) w = gcnt[u2];
+          charge(slot2, w);
+        }, part_end);
+      }
       if (mode == MODE_GLOBAL) {  // restore the zero invariant of the scratch array
-        block_wedges(b, e, P, S, [&](uint32_t, uint32_t, uint32_t, uint32_t u2t) {
-          if ((u2t >> 1) < P.n) gcnt[u2t >> 1] = 0;
-        });
-        __syncthreads();
+        block_wedges<NT>(b, e, P, S, [&](uint32_t, uint32_t u2) {
+          if (u2 < P.n) gcnt[u2] = 0;
+        }, nothing);
       }
     } else {
       // Phase 3: endpoint credits, once per distinct u2.
       int64_t mine = 0;
-      if (mode == MODE_DENSE) {
-        for (uint32_t s = threadIdx.x; s < i; s += kBlock) {
-          const int64_t w = table[s];
-          if (w >= 2) {
-            const int64_t bf = w * (w - 1) / 2;
-            mine += bf;
-            if (P.per == VERT) credit(P, s, bf, 16);
-          }
+      auto pair = [&](uint32_t u2, int64_t w) {
+        if (w < 2) return;
+        const int64_t bf = w * (w - 1) / 2;
+        mine += bf;
+        if (P.per == VERT) credit(P, u2, bf, 16);
+      };
+      for (uint32_t s = threadIdx.x; s < dwords; s += NT) {
+        const uint32_t x = table[s];
+        if (wide) {
+          pair(s, x);
+        } else if (x) {
+          pair(2 * s, x & 0xFFFFu);
+          pair(2 * s + 1, x >> 16);
         }
-      } else if (mode == MODE_HASH || mode == MODE_HYBRID) {
-        if (mode == MODE_HYBRID) {
-          for (uint32_t s = threadIdx.x; s < hy_dense; s += kBlock) {
-            const int64_t w = table[s];
-            if (w >= 2) {
-              const int64_t bf = w * (w - 1) / 2;
-              mine += bf;
-              if (P.per == VERT) credit(P, s, bf, 36);
-            }
-          }
-        }
-        for (uint32_t s = threadIdx.x; s < tsize; s += kBlock) {
-          const uint32_t k = keys[s];
-          if (k == kEmpty) continue;
-          const int64_t w = vals[s];
-          if (w >= 2) {
-            const int64_t bf = w * (w - 1) / 2;
-            mine += bf;
-            if (P.per == VERT) credit(P, k, bf, 17);
-          }
-        }
-      } else {
-        block_wedges(b, e, P, S, [&](uint32_t, uint32_t, uint32_t, uint32_t u2t) {
-          if ((u2t >> 1) >= P.n) { record_violation(P.err, 27, u2t >> 1, i); return; }
-          const int64_t w = atomicExch(&gcnt[u2t >> 1], 0u);
-          if (w >= 2) {
-            const int64_t bf = w * (w - 1) / 2;
-            mine += bf;
-            if (P.per == VERT) credit(P, u2t >> 1, bf, 18);
-          }
-        });
       }
+      for (uint32_t s = threadIdx.x; s < tsize; s += NT) {
+        uint32_t k;
+        const uint32_t w = table_entry(tab, tsize, cb, s, k);
+        pair(k, w);
+      }
+      if (mode == MODE_GLOBAL)
+        block_wedges<NT>(b, e, P, S, [&](uint32_t, uint32_t u2) {
+          if (u2 >= P.n) { record_violation(P.err, 27, u2, i); return; }
+          pair(u2, atomicExch(&gcnt[u2], 0u));
+        }, nothing);
       if (P.per == VERT) {
         const int64_t s = block_sum_i64(mine, S.red);
         if (threadIdx.x == 0 && s) credit(P, i, s, 19);
       } else {
         total += mine;
       }
-      __syncthreads();
     }
+    __syncthreads();
     if (threadIdx.x == 0) {
       if (P.mode_out) P.mode_out[q] = (uint8_t)mode;
       if (P.cycles) P.cycles[q] = (unsigned long long)(clock64() - t_item);
     }
+    q = S.item;
+    __syncthreads();
   }
   if (P.per == TOTAL) {
     const int64_t s = block_sum_i64(total, S.red);
@@ -526,20 +646,39 @@ __global__ void __launch_bounds__(kBlock) count_block_kernel(Params P, const uin
   }
 }
 
-__global__ void widen_u32_kernel(const uint32_t* __restrict__ in, int64_t n, int64_t* out) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    out[i] = (int64_t)in[i];
+// Per-edge results: the credits of an edge's two slots, added at its output index.
+__global__ void edge_gather_kernel(Params P, const uint32_t* __restrict__ eout) {
+  for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < P.m2; s += (int64_t)gridDim.x * blockDim.x) {
+    const unsigned long long v = P.sacc32 ? (unsigned long long)P.sacc32[s] : P.sacc64[s];
+    if (v) credit(P, eout[s], (int64_t)v, 12);
+  }
 }
 
-__global__ void classify_endpoints_kernel(const int64_t* __restrict__ wsum, int64_t n, int small_w, uint32_t cap_dense,
-                                          uint32_t cap_hash, uint32_t* items, uint32_t* counts /* [0]=big [1]=global */) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t W = wsum[i + 1] - wsum[i];
-    if (W <= small_w) continue;
-    items[atomicAdd(&counts[0], 1u)] = (uint32_t)i;
-    const bool dense_ok = (uint64_t)i <= cap_dense;
-    const bool hash_ok = (uint64_t)2 * W <= cap_hash;
-    if (!dense_ok && !hash_ok) atomicAdd(&counts[1], 1u);
+// Splits the endpoints with wedges into the warp, mid and block lists.
+// counts: [0] block, [1] global scratch, [2] block cursor, [3] warp, [4] mid, [5] mid cursor.
+__global__ void classify_endpoints_kernel(const int64_t* __restrict__ wsum, const uint32_t* __restrict__ off, int64_t n,
+                                          int small_w, int64_t mid_w, Geom mid, uint4* small_items, uint4* mid_items,
+                                          uint4* items, uint32_t* counts, uint32_t* err) {
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  const int64_t rounds = (n + step - 1) / step;
+  for (int64_t r = 0; r < rounds; ++r) {
+    const int64_t i = r * step + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    int64_t W = 0;
+    uint4 it = make_uint4(0, 0, 0, 0);
+    if (i < n) {
+      W = wsum[i + 1] - wsum[i];
+      if (W < 0) record_violation(err, 34, (uint64_t)i, 0);
+      it = make_uint4((uint32_t)i, off[i], off[i + 1], (uint32_t)min(W, (int64_t)0xFFFFFFFFll));
+    }
+    const uint32_t deg = it.z - it.y;
+    // A long row takes a CTA however few wedges it has: a warp would walk its slots alone.
+    const bool small = W > 0 && W <= small_w && deg <= kWarpRow;
+    const bool fits = W > 0 && !small && W <= mid_w && deg <= kMidRow && (mid.dense_ok(it.x, deg) || mid.hash_ok(W, deg));
+    const bool big = W > 0 && !small && !fits;
+    const unsigned a = list_at(&counts[3], small), c = list_at(&counts[4], fits), d = list_at(&counts[0], big);
+    if (small) small_items[a] = it;
+    else if (fits) mid_items[c] = it;
+    else if (big) items[d] = it;
   }
 }
 
@@ -548,16 +687,15 @@ constexpr int kItemFeatures = 12;  // features per item; 4 one-hot mode slots fo
 
 // One warp per block-aggregator item: cost-model features and the valid modes (bit m set when
 // mode m can hold the item's multiplicity table; the global mode always can).
-__global__ void item_features_kernel(Params P, const uint32_t* __restrict__ items, uint32_t n_items,
-                                     uint32_t cap_dense, uint32_t cap_hash, uint32_t hy_dense, uint32_t hy_hash,
-                                     float* F, uint8_t* valid) {
+__global__ void item_features_kernel(Params P, const uint4* __restrict__ items, uint32_t n_items, Geom G, float* F,
+                                     uint8_t* valid) {
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const unsigned lane = threadIdx.x & 31u;
   for (int64_t q = warp; q < n_items; q += nwarps) {
-    const uint32_t i = items[q];
+    const uint32_t i = items[q].x, b = items[q].y, e = items[q].z;
     const int64_t W = P.wsum[i + 1] - P.wsum[i];
-    const uint32_t b = P.off[i], e = P.off[i + 1];
+    const uint32_t hy_dense = G.hy_dense();
     unsigned long long lo_w = 0, sumdeg = 0;
     for (uint32_t j = b + lane; j < e; j += 32) {
       const uint32_t v = P.adj[j] >> 1;
@@ -586,16 +724,12 @@ __global__ void item_features_kernel(Params P, const uint32_t* __restrict__ item
       f[7] = P.per == EDGE ? 1.f : 0.f;
       f[8] = log2f(1.f + (float)P.n);
       f[9] = f[1] - f[0];
-      f[10] = P.out32 ? 1.f : 0.f;
+      f[10] = P.sacc32 ? 1.f : 0.f;
       f[11] = log2f(1.f + (float)W / (float)(deg ? deg : 1u));
       for (int k = kItemFeatures; k < kMlpIn; ++k) f[k] = 0.f;
-      const bool dense_ok = i <= cap_dense, hash_ok = (uint64_t)2 * W <= cap_hash, hybrid_ok = 2ull * hi_c <= hy_hash;
-      // The plain rule's choice (count_block_kernel) rides in the top bits.
-      const uint32_t rule = (dense_ok && (uint64_t)i <= 4ull * (uint64_t)W) ? MODE_DENSE
-                            : hash_ok                                     ? MODE_HASH
-                            : dense_ok                                    ? MODE_DENSE
-                            : hybrid_ok                                   ? MODE_HYBRID
-                                                                          : MODE_GLOBAL;
+      const bool dense_ok = G.dense_ok(i, deg), hash_ok = G.hash_ok(W, deg), hybrid_ok = G.hybrid_ok(hi_c, deg);
+      // The plain rule's choice rides in the top bits.
+      const uint32_t rule = G.rule(i, W, deg, hi_c);
       valid[q] = (uint8_t)((dense_ok ? 1u : 0u) | (hash_ok ? 2u : 0u) | 4u | (hybrid_ok ? 8u : 0u) | (rule << 4));
     }
   }
@@ -645,16 +779,16 @@ __global__ void sched_choose_kernel(const float* __restrict__ y, const uint8_t* 
 }
 
 // sub[k]: the positions q of block-aggregator items with at least min_w wedges.
-__global__ void heavy_items_kernel(const uint32_t* __restrict__ items, uint32_t n_items,
+__global__ void heavy_items_kernel(const uint4* __restrict__ items, uint32_t n_items,
                                    const int64_t* __restrict__ wsum, int64_t min_w, uint32_t* sub, uint32_t* n_sub) {
   for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n_items; q += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t i = items[q];
+    const uint32_t i = items[q].x;
     if (wsum[i + 1] - wsum[i] >= min_w) sub[atomicAdd(n_sub, 1u)] = (uint32_t)q;
   }
 }
 
-__global__ void gather_u32_kernel(const uint32_t* __restrict__ src, const uint32_t* __restrict__ idx, uint32_t n,
-                                  uint32_t* dst) {
+__global__ void gather_items_kernel(const uint4* __restrict__ src, const uint32_t* __restrict__ idx, uint32_t n,
+                                    uint4* dst) {
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
     dst[k] = src[idx[k]];
 }
@@ -703,8 +837,16 @@ CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConf
   const int64_t out_len = per == VERT ? n : (per == EDGE ? R.m2 / 2 : 1);
   if (out_len > 0) PB_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(int64_t) * out_len, s));
   if (n == 0 || R.w_rank == 0) return res;
-  Params P{R.off.get(), R.adj.get(), R.pref.get(), per == EDGE ? R.eout.get() : nullptr, R.wsum.get(), n, per, out,
-           out_len, R.m2, nullptr, nullptr, nullptr};
+  Params P{};
+  P.off = R.off.get();
+  P.adj = R.adj.get();
+  P.pref = R.pref.get();
+  P.wsum = R.wsum.get();
+  P.n = n;
+  P.per = per;
+  P.out = out;
+  P.out_len = out_len;
+  P.m2 = R.m2;
   DevBuf<uint32_t> err_local;
   if (cfg.err) {
     P.err = cfg.err;
@@ -716,45 +858,70 @@ CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConf
   DevBuf<unsigned long long> mstats(8, s);
   PB_CUDA_TRY(cudaMemsetAsync(mstats.get(), 0, 8 * sizeof(unsigned long long), s));
   P.mstats = mstats.get();
-  // Per-edge counts fit 32 bits when (max degree - 1)^2 < 2^32: accumulate them in a 4-byte
-  // array (67 MB for 2^24 edges, L2-resident) and widen once at the end.
-  DevBuf<uint32_t> out32;
+  // Per-edge counts are gathered per slot, in 32 bits when they fit: (max degree - 1)^2 < 2^32.
+  DevBuf<uint32_t> sacc32;
+  DevBuf<unsigned long long> sacc64;
   const uint64_t md = R.max_deg > 0 ? R.max_deg - 1 : 0;
   const char* acc64 = getenv("PB_EDGE_ACC64");  // test hook: force 64-bit per-edge accumulation
   const bool force64 = acc64 && *acc64 == '1';
-  if (per == EDGE && out_len > 0 && md * md < (1ull << 32) && !force64) {
-    out32.alloc(out_len, s);
-    PB_CUDA_TRY(cudaMemsetAsync(out32.get(), 0, out32.bytes(), s));
-    P.out32 = out32.get();
+  if (per == EDGE) {
+    if (md * md < (1ull << 32) && !force64) {
+      sacc32.alloc(R.m2, s);
+      PB_CUDA_TRY(cudaMemsetAsync(sacc32.get(), 0, sacc32.bytes(), s));
+      P.sacc32 = sacc32.get();
+    } else {
+      sacc64.alloc(R.m2, s);
+      PB_CUDA_TRY(cudaMemsetAsync(sacc64.get(), 0, sacc64.bytes(), s));
+      P.sacc64 = sacc64.get();
+    }
   }
   const int sms = sm_count();
   int small_w = std::min(cfg.small_w, kWarpTable / 2);
   int smem_bytes = cfg.smem_bytes;
   // Test hooks: shrink the CTA table / the warp threshold so small graphs reach every CTA mode.
-  if (const char* ev = getenv("PB_COUNT_SMEM")) smem_bytes = std::max(16384, std::min(atoi(ev), cfg.smem_bytes));
+  const char* hook_smem = getenv("PB_COUNT_SMEM");
+  if (hook_smem) smem_bytes = std::max(16384, std::min(atoi(hook_smem), cfg.smem_bytes));
   if (const char* ev = getenv("PB_COUNT_SMALL_W")) small_w = std::max(0, std::min(atoi(ev), small_w));
   int blocks_per_sm = cfg.blocks_per_sm;
   if (const char* ev = getenv("PB_COUNT_BPS")) blocks_per_sm = std::max(1, std::min(atoi(ev), 4));
+  int64_t sched_min_w = kSchedMinWedges;
+  if (const char* ev = getenv("PB_SCHED_MIN_WEDGES")) sched_min_w = atoll(ev);  // test hook: score light items too
 
-  // Block aggregator geometry.
-  const size_t shared_fixed = (sizeof(BlockShared) + 15) & ~size_t(15);
-  const size_t table_bytes = (size_t)smem_bytes > shared_fixed ? (size_t)smem_bytes - shared_fixed : 0;
-  const uint32_t cap_dense = (uint32_t)(table_bytes / 4);
-  uint32_t cap_hash = 1;
-  while ((size_t)cap_hash * 2 * 8 <= table_bytes) cap_hash <<= 1;  // slots; keys + values
-  if (cap_hash < 64) cap_hash = 64;
-
-  // Hybrid mode: half the table area as dense counters, the other half as a hash table.
-  const uint32_t hy_dense = (uint32_t)(table_bytes / 2 / 4);
-  uint32_t hy_hash = 1;
-  while ((size_t)hy_hash * 2 * 8 <= table_bytes / 2) hy_hash <<= 1;
-  DevBuf<uint32_t> items(n, s), counts(3, s);
-  PB_CUDA_TRY(cudaMemsetAsync(counts.get(), 0, 3 * sizeof(uint32_t), s));
-  PB_LAUNCH(classify_endpoints_kernel, std::max(1, std::min(ceil_div(n, 256), sms * 8)), 256, 0, s, R.wsum.get(), n,
-            small_w, cap_dense, cap_hash, items.get(), counts.get());
-  uint32_t hc[2];
+  // Table geometry of the CTA aggregators.
+  int key_bits = 0;
+  while (((uint64_t)(n - 1) >> key_bits) != 0) ++key_bits;
+  const int count_bits = 32 - std::max(1, key_bits);
+  auto geom_of = [&](size_t bytes, size_t fixed) {
+    Geom g;
+    g.tw = (uint32_t)((bytes - fixed) / 4) & ~31u;
+    g.hy_words = (g.tw / 4 * 3) & ~31u;
+    g.cb = count_bits;
+    return g;
+  };
+  const Geom G = geom_of(smem_bytes, shared_fixed<kBlock>());
+  const Geom Gm = geom_of(kMidSmem, shared_fixed<kMidBlock>());
+  // Endpoints of up to mid_w wedges take the mid aggregator.  Tracing covers every item, the learned
+  // scheduler those from sched_min_w on: they see the block aggregator only.
+  SchedHooks* sh = cfg.sched;
+  int64_t mid_w = kMidWedges;
+  if (hook_smem || (sh && sh->trace_X)) mid_w = 0;
+  else if (sh && sh->model) mid_w = std::min(mid_w, sched_min_w - 1);
+  DevBuf<uint4> lists((size_t)n * 3, s);  // warp, mid and block lists
+  uint4 *small_items = lists.get(), *mid_items = small_items + n, *items = mid_items + n;
+  DevBuf<uint32_t> counts(6, s);
+  DevBuf<uint8_t> modes(n, s);
+  PB_CUDA_TRY(cudaMemsetAsync(counts.get(), 0, 6 * sizeof(uint32_t), s));
+  PB_LAUNCH(classify_endpoints_kernel, std::max(1, std::min(ceil_div(n, 256), sms * 8)), 256, 0, s, R.wsum.get(),
+            R.off.get(), n, small_w, mid_w, Gm, small_items, mid_items, items, counts.get(), P.err);
+  uint32_t hc[5];
   readback(hc, counts.get(), sizeof(hc), s);
-  res.n_big = (int)hc[0];
+  const uint32_t n_block = hc[0], n_small = hc[3], n_mid = hc[4];
+  if (n_block > 0) {
+    PB_LAUNCH(plain_modes_kernel, (int)std::min<int64_t>(ceil_div(n_block, 8), sms * 8), 256, 0, s, P, items,
+              counts.get(), G, modes.get(), counts.get() + 1);
+    readback(&hc[1], counts.get() + 1, sizeof(uint32_t), s);
+  }
+  res.n_big = (int)(n_block + n_mid);
 
   // Under graph capture nothing is timed or read back here (the recording run checked).
   const bool cap = capturing();
@@ -762,26 +929,16 @@ CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConf
   PB_CUDA_TRY(cudaEventCreate(&e0));
   PB_CUDA_TRY(cudaEventCreate(&e1));
   if (!cap) PB_CUDA_TRY(cudaEventRecord(e0, s));
-  {
-    const int smem = kWarpsPerBlockSmall * 2 * kWarpTable * (int)sizeof(uint32_t);
-    static bool attr_set = false;
-    if (!attr_set) {
-      PB_CUDA_TRY(cudaFuncSetAttribute(count_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-      attr_set = true;
-    }
-    PB_LAUNCH(count_warp_kernel, sms * 3, kWarpsPerBlockSmall * 32, smem, s, P, small_w);
-  }
   // Scheduler: per-item modes (learned or exploring) and the record of what each item ran
   // with and how long it took.
-  SchedHooks* sh = cfg.sched;
-  const bool sched_on = sh && hc[0] > 0 && (sh->model || sh->explore || sh->trace_X);
+  const bool sched_on = sh && n_block > 0 && (sh->model || sh->explore || sh->trace_X);
   DevBuf<float> sF, sPred;
-  DevBuf<uint8_t> sValid, sModes, sUsed;
+  DevBuf<uint8_t> sValid, sUsed;
   DevBuf<uint32_t> sNG;
   DevBuf<unsigned long long> sCyc;
   bool need_global = hc[1] > 0;
   if (sched_on) {
-    const uint32_t ni = hc[0];
+    const uint32_t ni = n_block;
     cudaEvent_t a0, a1;
     PB_CUDA_TRY(cudaEventCreate(&a0));
     PB_CUDA_TRY(cudaEventCreate(&a1));
@@ -798,56 +955,49 @@ CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConf
     if (sh->model && !sh->trace_X) {
       DevBuf<uint32_t> sub(ni, s), nsub(1, s);
       PB_CUDA_TRY(cudaMemsetAsync(nsub.get(), 0, sizeof(uint32_t), s));
-      int64_t min_w = kSchedMinWedges;
-      if (const char* ev = getenv("PB_SCHED_MIN_WEDGES")) min_w = atoll(ev);  // test hook: score light items too
-      PB_LAUNCH(heavy_items_kernel, g1, 256, 0, s, items.get(), ni, R.wsum.get(), min_w, sub.get(), nsub.get());
+      PB_LAUNCH(heavy_items_kernel, g1, 256, 0, s, items, ni, R.wsum.get(), sched_min_w, sub.get(), nsub.get());
       uint32_t nh = 0;
       readback(&nh, nsub.get(), sizeof(nh), s);
-      sModes.alloc(ni, s);
       sPred.alloc(ni, s);
-      PB_CUDA_TRY(cudaMemsetAsync(sModes.get(), kPlainRule, ni, s));
       PB_CUDA_TRY(cudaMemsetAsync(sPred.get(), 0xFF, sizeof(float) * ni, s));  // NaN: no prediction
       PB_CUDA_TRY(cudaMemsetAsync(sF.get(), 0, sF.bytes(), s));
       if (nh > 0) {
-        DevBuf<uint32_t> hitems(nh, s);
+        DevBuf<uint4> hitems(nh, s);
         DevBuf<float> hF((size_t)nh * kMlpIn, s), hPr(nh, s);
         DevBuf<uint8_t> hValid(nh, s), hModes(nh, s);
         const int gh = std::max(1, std::min(ceil_div(nh, 256), sms * 8));
-        PB_LAUNCH(gather_u32_kernel, gh, 256, 0, s, items.get(), sub.get(), nh, hitems.get());
+        PB_LAUNCH(gather_items_kernel, gh, 256, 0, s, items, sub.get(), nh, hitems.get());
         PB_LAUNCH(item_features_kernel, std::max(1, std::min(ceil_div((int64_t)nh * 32, 256), sms * 8)), 256, 0, s, P,
-                  hitems.get(), nh, cap_dense, cap_hash, hy_dense, hy_hash, hF.get(), hValid.get());
+                  hitems.get(), nh, G, hF.get(), hValid.get());
         DevBuf<float> X((size_t)nh * 3 * kMlpIn, s), y((size_t)nh * 3, s);
         PB_LAUNCH(sched_candidates_kernel, std::max(1, std::min(ceil_div((int64_t)nh * 3 * kMlpIn, 256), sms * 8)), 256,
                   0, s, hF.get(), nh, X.get());
         sh->model->predict_dev(X.get(), (int64_t)nh * 3, y.get(), s);
         PB_LAUNCH(sched_choose_kernel, gh, 256, 0, s, y.get(), hValid.get(), nh, hModes.get(), hPr.get(), sNG.get());
-        PB_LAUNCH(scatter_scored_kernel, gh, 256, 0, s, sub.get(), nh, hModes.get(), hPr.get(), hF.get(), sModes.get(),
+        PB_LAUNCH(scatter_scored_kernel, gh, 256, 0, s, sub.get(), nh, hModes.get(), hPr.get(), hF.get(), modes.get(),
                   sPred.get(), sF.get());
       }
     } else {
       PB_LAUNCH(item_features_kernel, std::max(1, std::min(ceil_div((int64_t)ni * 32, 256), sms * 8)), 256, 0, s, P,
-                items.get(), ni, cap_dense, cap_hash, hy_dense, hy_hash, sF.get(), sValid.get());
+                items, ni, G, sF.get(), sValid.get());
     }
     if (sh->model && sh->trace_X) {
       DevBuf<float> X((size_t)ni * 3 * kMlpIn, s), y((size_t)ni * 3, s);
       PB_LAUNCH(sched_candidates_kernel, std::max(1, std::min(ceil_div((int64_t)ni * 3 * kMlpIn, 256), sms * 8)), 256,
                 0, s, sF.get(), ni, X.get());
       sh->model->predict_dev(X.get(), (int64_t)ni * 3, y.get(), s);
-      sModes.alloc(ni, s);
       sPred.alloc(ni, s);
-      PB_LAUNCH(sched_choose_kernel, g1, 256, 0, s, y.get(), sValid.get(), ni, sModes.get(), sPred.get(), sNG.get());
+      PB_LAUNCH(sched_choose_kernel, g1, 256, 0, s, y.get(), sValid.get(), ni, modes.get(), sPred.get(), sNG.get());
     } else if (sh->explore) {
-      sModes.alloc(ni, s);
-      PB_LAUNCH(sched_explore_kernel, g1, 256, 0, s, sValid.get(), ni, sh->seed, sModes.get(), sNG.get());
+      PB_LAUNCH(sched_explore_kernel, g1, 256, 0, s, sValid.get(), ni, sh->seed, modes.get(), sNG.get());
     }
-    P.modes = sModes.get();  // null when only the plain choices are traced
     P.mode_out = sUsed.get();
     P.cycles = sCyc.get();
     uint32_t ng = 0;
     PB_CUDA_TRY(cudaMemcpyAsync(&ng, sNG.get(), sizeof(ng), cudaMemcpyDeviceToHost, s));
     PB_CUDA_TRY(cudaEventRecord(a1, s));
     PB_CUDA_TRY(cudaEventSynchronize(a1));
-    if (P.modes) need_global = ng > 0 || hc[1] > 0;  // unscored items follow the plain rule
+    need_global = ng > 0 || hc[1] > 0;  // unscored items follow the plain rule
     float ms = 0;
     PB_CUDA_TRY(cudaEventElapsedTime(&ms, a0, a1));
     sh->ms = ms;
@@ -855,8 +1005,8 @@ CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConf
     cudaEventDestroy(a1);
   }
   DevBuf<uint32_t> gscratch;
-  if (hc[0] > 0) {
-    int grid = (int)std::min<int64_t>(hc[0], (int64_t)sms * blocks_per_sm);
+  if (n_block > 0) {
+    int grid = (int)std::min<int64_t>(n_block, (int64_t)sms * blocks_per_sm);
     if (need_global) {
       // One dense counter array of n entries per CTA: at very large n (the 1e9-edge R-MAT) the
       // CTA count is capped so the arrays stay within half of the free device memory (64 GB at
@@ -869,12 +1019,31 @@ CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConf
       gscratch.alloc((size_t)grid * (size_t)n, s);
       PB_CUDA_TRY(cudaMemsetAsync(gscratch.get(), 0, gscratch.bytes(), s));
     }
-    PB_CUDA_TRY(cudaFuncSetAttribute(count_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
-    PB_LAUNCH(count_block_kernel, grid, kBlock, smem_bytes, s, P, items.get(), counts.get(), counts.get() + 2,
-              gscratch.get(), cap_dense, cap_hash, hy_dense, hy_hash);
+    P.modes = modes.get();
+    auto kern = count_block_kernel<kBlock, kBlockPerSm>;
+    PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
+    PB_LAUNCH(kern, grid, kBlock, smem_bytes, s, P, items, counts.get(), counts.get() + 2, gscratch.get(), G);
   }
-  if (P.out32)
-    PB_LAUNCH(widen_u32_kernel, std::max(1, std::min(ceil_div(out_len, 256), sms * 8)), 256, 0, s, P.out32, out_len, out);
+  P.modes = nullptr;
+  P.mode_out = nullptr;
+  P.cycles = nullptr;
+  if (n_mid > 0) {
+    auto kern = count_block_kernel<kMidBlock, kMidPerSm>;
+    PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMidSmem));
+    PB_LAUNCH(kern, (int)std::min<int64_t>(n_mid, (int64_t)sms * kMidPerSm), kMidBlock, kMidSmem, s, P, mid_items,
+              counts.get() + 4, counts.get() + 5, (uint32_t*)nullptr, Gm);
+  }
+  if (n_small > 0) {
+    const bool one_word = (uint32_t)small_w <= (1u << count_bits) - 2u;
+    auto kern = one_word ? count_warp_kernel<true> : count_warp_kernel<false>;
+    const int smem =
+        (2 * (int)kHotRanks + kWarpsPerBlockSmall * ((one_word ? 1 : 2) * kWarpTable + 32)) * (int)sizeof(uint32_t);
+    PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    PB_LAUNCH(kern, (int)std::min<int64_t>(ceil_div(n_small, kWarpsPerBlockSmall), (int64_t)sms * (one_word ? 6 : 3)),
+              kWarpsPerBlockSmall * 32, smem, s, P, small_items, counts.get() + 3, count_bits);
+  }
+  if (per == EDGE)
+    PB_LAUNCH(edge_gather_kernel, std::max(1, std::min(ceil_div(R.m2, 256), sms * 8)), 256, 0, s, P, R.eout.get());
   if (cap) {
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
@@ -895,7 +1064,7 @@ CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConf
                    std::to_string(((uint64_t)h[2] << 32) | h[1]) + " aux " + std::to_string(h[3]));
   }
   if (sched_on) {
-    const uint32_t ni = hc[0];
+    const uint32_t ni = n_block;
     std::vector<float> hF((size_t)ni * kMlpIn), hPred;
     std::vector<uint8_t> hUsed(ni);
     std::vector<unsigned long long> hCyc(ni);

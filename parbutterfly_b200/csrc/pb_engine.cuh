@@ -67,8 +67,8 @@ struct CountConfig {
   int strategy = STRAT_AUTO;
   int small_w = 512;          // endpoints with W_i <= small_w go to the warp aggregator
   int block_threads = 512;    // threads of the block aggregator
-  int smem_bytes = 48 * 1024;   // dynamic shared memory of the block aggregator
-  int blocks_per_sm = 4;
+  int smem_bytes = 72 * 1024;   // dynamic shared memory of the block aggregator
+  int blocks_per_sm = 3;
   int split_w = 0;            // endpoints above this many wedges are split across CTAs (0: auto)
   uint32_t* err = nullptr;    // checked mode: device record of the first bounds violation
   SchedHooks* sched = nullptr;
