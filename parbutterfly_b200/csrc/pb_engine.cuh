@@ -35,6 +35,8 @@ struct Ranked {
   DevBuf<int64_t> wsum;    // n+1: exclusive prefix of per-endpoint wedge counts
   int64_t w_rank = 0;
   uint32_t max_deg = 0;
+  DevBuf<uint8_t> co;      // control block of the co-core ranking kernel (its error word is checked
+                           // with the wedge scan's readback)
 };
 
 // Ranking stage (pb_rank.cu).

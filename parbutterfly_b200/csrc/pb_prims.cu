@@ -105,7 +105,10 @@ void exclusive_scan_impl(const T* in, T* out, int64_t n, cudaStream_t s) {
 // ---------------------------------------------------------------------------------------------
 // Stable LSD radix sort, 8-bit digits.  A tile is 256 threads x 16 items; warp w of a tile owns
 // items [w*512, (w+1)*512) in 16 rounds of 32, so (warp, round, lane) order is input order.
-// Per-item ranks inside a warp come from __match_any_sync on the digit (warp multisplit).
+// Per-item ranks inside a warp come from __match_any_sync on the digit (warp multisplit).  Bound by
+// memory: a tile is ordered in shared memory first, so that its runs of equal digits (16 items on
+// average) leave as whole sectors; writing every item from its own lane took 128 us a pass for 1e7
+// pairs, this 95.
 constexpr int kRadixThreads = 256;
 constexpr int kRadixRounds = 16;
 constexpr int kRadixWarps = kRadixThreads / 32;
@@ -127,74 +130,104 @@ __global__ void radix_upsweep_kernel(const K* __restrict__ keys, int64_t n, int 
 }
 
 template <class K>
-__global__ void radix_downsweep_kernel(const K* __restrict__ keys, const uint32_t* __restrict__ vals, int64_t n,
-                                       int shift, int64_t tiles, const uint32_t* __restrict__ offsets,
-                                       K* __restrict__ keys_out, uint32_t* __restrict__ vals_out) {
-  __shared__ uint32_t wcnt[kRadixWarps][256];
-  __shared__ uint32_t toff[256];
+size_t radix_smem(bool vals, bool vals2) {
+  return (size_t)kRadixTile * (sizeof(K) + (vals ? 4 : 0) + (vals2 ? 4 : 0)) +
+         (size_t)(kRadixWarps * 256 + 2 * 256 + 32) * sizeof(uint32_t);
+}
+
+// vals and vals2 may be null (no payload / one payload).
+template <class K>
+__global__ void __launch_bounds__(kRadixThreads) radix_downsweep_kernel(
+    const K* __restrict__ keys, const uint32_t* __restrict__ vals, const uint32_t* __restrict__ vals2, int64_t n, int shift,
+    int64_t tiles, const uint32_t* __restrict__ offsets, K* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
+    uint32_t* __restrict__ vals2_out) {
+  extern __shared__ __align__(16) unsigned char radix_smem_raw[];
+  K* skeys = reinterpret_cast<K*>(radix_smem_raw);
+  uint32_t* svals = reinterpret_cast<uint32_t*>(skeys + kRadixTile);
+  uint32_t* svals2 = svals + (vals ? kRadixTile : 0);
+  uint32_t(*wcnt)[256] = reinterpret_cast<uint32_t(*)[256]>(svals2 + (vals2 ? kRadixTile : 0));
+  uint32_t* toff = &wcnt[kRadixWarps][0];   // global position of the tile's first item of a digit ...
+  uint32_t* dstart = toff + 256;            // ... and its position within the tile
+  uint32_t* scan = dstart + 256;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int d = threadIdx.x; d < kRadixWarps * 256; d += kRadixThreads) (&wcnt[0][0])[d] = 0;
   toff[threadIdx.x] = offsets[(int64_t)threadIdx.x * tiles + blockIdx.x];
   __syncthreads();
-  const int64_t base = (int64_t)blockIdx.x * kRadixTile + (int64_t)warp * (32 * kRadixRounds);
+  const int64_t tile0 = (int64_t)blockIdx.x * kRadixTile;
+  const int64_t base = tile0 + (int64_t)warp * (32 * kRadixRounds);
   K kreg[kRadixRounds];
-  uint32_t vreg[kRadixRounds];
   uint32_t rank[kRadixRounds];
   const unsigned lt = (1u << lane) - 1u;
 #pragma unroll
   for (int r = 0; r < kRadixRounds; ++r) {
-    int64_t idx = base + r * 32 + lane;
-    bool valid = idx < n;
-    K key = valid ? keys[idx] : K(0);
-    kreg[r] = key;
-    vreg[r] = (valid && vals) ? vals[idx] : 0u;
-    uint32_t d = valid ? ((uint32_t)(key >> shift) & 255u) : 256u;
-    unsigned peers = __match_any_sync(0xffffffffu, d);
-    uint32_t pre = valid ? wcnt[warp][d] : 0u;
+    const int64_t idx = base + r * 32 + lane;
+    kreg[r] = idx < n ? keys[idx] : K(0);
+  }
+#pragma unroll
+  for (int r = 0; r < kRadixRounds; ++r) {
+    const bool valid = base + r * 32 + lane < n;
+    const uint32_t d = valid ? ((uint32_t)(kreg[r] >> shift) & 255u) : 256u;
+    const unsigned peers = __match_any_sync(0xffffffffu, d);
+    const uint32_t pre = valid ? wcnt[warp][d] : 0u;
     __syncwarp();
     if (valid && lane == __ffs(peers) - 1) wcnt[warp][d] = pre + __popc(peers);
     __syncwarp();
     rank[r] = pre + __popc(peers & lt);
   }
   __syncthreads();
-  {  // exclusive prefix over warps, per digit
+  {  // exclusive prefix over warps, per digit, and over digits
     uint32_t run = 0;
     for (int w = 0; w < kRadixWarps; ++w) {
-      uint32_t c = wcnt[w][threadIdx.x];
+      const uint32_t c = wcnt[w][threadIdx.x];
       wcnt[w][threadIdx.x] = run;
       run += c;
     }
+    uint32_t total;
+    dstart[threadIdx.x] = block_exclusive_scan(run, scan, total);
   }
   __syncthreads();
 #pragma unroll
   for (int r = 0; r < kRadixRounds; ++r) {
-    int64_t idx = base + r * 32 + lane;
+    const int64_t idx = base + r * 32 + lane;
     if (idx < n) {
-      uint32_t d = (uint32_t)(kreg[r] >> shift) & 255u;
-      uint32_t pos = toff[d] + wcnt[warp][d] + rank[r];
-      keys_out[pos] = kreg[r];
-      if (vals) vals_out[pos] = vreg[r];
+      const uint32_t d = (uint32_t)(kreg[r] >> shift) & 255u;
+      const uint32_t at = dstart[d] + wcnt[warp][d] + rank[r];
+      skeys[at] = kreg[r];
+      if (vals) svals[at] = vals[idx];
+      if (vals2) svals2[at] = vals2[idx];
     }
+  }
+  __syncthreads();
+  const int cnt = (int)min((int64_t)kRadixTile, n - tile0);
+  for (int x = threadIdx.x; x < cnt; x += kRadixThreads) {
+    const K key = skeys[x];
+    const uint32_t d = (uint32_t)(key >> shift) & 255u;
+    const uint32_t pos = toff[d] + ((uint32_t)x - dstart[d]);
+    keys_out[pos] = key;
+    if (vals) vals_out[pos] = svals[x];
+    if (vals2) vals2_out[pos] = svals2[x];
   }
 }
 
 template <class K>
 bool radix_sort_impl(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt, int64_t n, int begin_bit,
-                     int end_bit, cudaStream_t s) {
+                     int end_bit, cudaStream_t s, uint32_t* vals2 = nullptr, uint32_t* vals2_alt = nullptr) {
   if (n <= 1 || end_bit <= begin_bit) return false;
   PB_REQUIRE(n < (int64_t)UINT32_MAX, PB_ETOOBIG, "radix sort supports < 2^32 items");
   const int64_t tiles = (n + kRadixTile - 1) / kRadixTile;
   DevBuf<uint32_t> counts(256 * tiles + 1, s);
+  const size_t smem = radix_smem<K>(vals != nullptr, vals2 != nullptr);
+  PB_CUDA_TRY(cudaFuncSetAttribute(radix_downsweep_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)radix_smem<K>(true, true)));
   bool alt = false;
   for (int shift = begin_bit; shift < end_bit; shift += 8) {
     K* kin = alt ? keys_alt : keys;
     K* kout = alt ? keys : keys_alt;
-    uint32_t* vin = vals ? (alt ? vals_alt : vals) : nullptr;
-    uint32_t* vout = vals ? (alt ? vals : vals_alt) : nullptr;
     PB_LAUNCH(radix_upsweep_kernel<K>, (unsigned)tiles, kRadixThreads, 0, s, kin, n, shift, tiles, counts.get());
     exclusive_scan_u32(counts.get(), counts.get(), 256 * tiles, s);
-    PB_LAUNCH(radix_downsweep_kernel<K>, (unsigned)tiles, kRadixThreads, 0, s, kin, vin, n, shift, tiles,
-              counts.get(), kout, vout);
+    PB_LAUNCH(radix_downsweep_kernel<K>, (unsigned)tiles, kRadixThreads, smem, s, kin, alt ? vals_alt : vals,
+              alt ? vals2_alt : vals2, n, shift, tiles, counts.get(), kout, alt ? vals : vals_alt,
+              alt ? vals2 : vals2_alt);
     alt = !alt;
   }
   return alt;
@@ -341,8 +374,8 @@ bool radix_sort_pairs_u64(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, ui
   return radix_sort_impl<uint64_t>(keys, vals, keys_alt, vals_alt, n, begin_bit, end_bit, s);
 }
 bool radix_sort_pairs_u32(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt, int64_t n,
-                          int begin_bit, int end_bit, cudaStream_t s) {
-  return radix_sort_impl<uint32_t>(keys, vals, keys_alt, vals_alt, n, begin_bit, end_bit, s);
+                          int begin_bit, int end_bit, cudaStream_t s, uint32_t* vals2, uint32_t* vals2_alt) {
+  return radix_sort_impl<uint32_t>(keys, vals, keys_alt, vals_alt, n, begin_bit, end_bit, s, vals2, vals2_alt);
 }
 
 void segmented_sort_rows(const uint32_t* off, int64_t nrows, uint32_t* keys, uint32_t* vals, int key_bits,

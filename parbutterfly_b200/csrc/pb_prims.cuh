@@ -12,11 +12,12 @@ void exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, cudaStream
 
 // Stable LSD radix sort of (key, value) pairs on key bits [begin_bit, end_bit).  Sorted data
 // ends in (keys, vals) or (keys_alt, vals_alt); the return value says which (true = alt).
-// vals may be null (keys only).
+// vals may be null (keys only); vals2 is a second payload of the same kind (null: none).
 bool radix_sort_pairs_u64(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t* vals_alt, int64_t n,
                           int begin_bit, int end_bit, cudaStream_t s);
 bool radix_sort_pairs_u32(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt, int64_t n,
-                          int begin_bit, int end_bit, cudaStream_t s);
+                          int begin_bit, int end_bit, cudaStream_t s, uint32_t* vals2 = nullptr,
+                          uint32_t* vals2_alt = nullptr);
 
 // Sorts every row r of a CSR (off[r]..off[r+1]) ascending by key, carrying an optional
 // payload.  Keys within a row are distinct.  key_bits bounds the key values (< 2^key_bits).

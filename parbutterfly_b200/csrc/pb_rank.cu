@@ -62,57 +62,131 @@ __global__ void order_keys_kernel(const uint32_t* __restrict__ deg, int64_t n, i
   }
 }
 
-__global__ void cocore_init_kernel(const uint32_t* __restrict__ deg, int64_t n, int approx, uint32_t* key,
-                                   uint32_t* dact, uint8_t* done) {
-  for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x) {
-    dact[x] = deg[x];
-    key[x] = approx ? log_key(deg[x]) : deg[x];
-    done[x] = 0;
-  }
-}
+// The bucket rounds of getCoCoreRanks / getApproxCoCoreRanks (butterfly_utils.h:448-559), all in
+// one cooperative launch: every undone vertex whose key equals the current maximum k is finished;
+// each neighbour with key < k (undone, outside the bucket) loses one degree per finished neighbour
+// and its key becomes f(new degree) (min with k is implied, since f(new) <= key < k).  Keys only
+// decrease, so atomicMin of f over all decrements leaves f(final degree).
+// Two barriers a round: the scan that collects bucket k also takes the maximum of the other keys;
+// the updates that follow can only lower them, so the next round's k is that maximum or the round
+// is empty.  A finished vertex's list is cut into units of kCoUnit entries, so that the hubs of the
+// first rounds are not one warp's work.  One launch pair and a host readback per round with one warp
+// per vertex took 5.2 ms (R-MAT 2^24 edges, 15 rounds) and 1.8 ms (46 rounds of a uniform graph with
+// 1e6 edges); this takes 0.97 ms and 0.45 ms.
+struct CoCtl {
+  unsigned long long bar;
+  uint32_t err, kmax[2], len[2];
+};
+constexpr uint32_t kCoDone = 0x80000000u;  // finished (keys are degrees or their logarithms, below 2^23)
+constexpr uint32_t kCoUnit = 256;
+constexpr int kCoThreads = 1024;
+constexpr unsigned long long kCoTimeoutNs = 60ull * 1000000000ull;
 
-__global__ void cocore_max_kernel(const uint32_t* __restrict__ key, const uint8_t* __restrict__ done, int64_t n,
-                                  uint32_t* out /* [0]=max key+1 of undone (0: none) */) {
-  uint32_t m = 0;
-  for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x)
-    if (!done[x]) m = max(m, key[x] + 1u);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0 && m) atomicMax(out, m);
-}
-
-// One bucket round of getCoCoreRanks / getApproxCoCoreRanks (butterfly_utils.h:448-559):
-// every undone vertex with key k is finished; each neighbour with key < k (undone, outside
-// the bucket) loses one degree per finished neighbour and its key becomes f(new degree)
-// (min with k is implied, since f(new) <= key < k).  Keys only decrease, so atomicMin of
-// f over all decrements leaves f(final degree).
-__global__ void cocore_round_kernel(Lists L, int64_t n, int approx, const uint32_t* __restrict__ kbuf, uint32_t* key,
-                                    uint32_t* dact, uint8_t* done) {
-  const uint32_t k = kbuf[0] - 1u;
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const unsigned lane = threadIdx.x & 31u;
-  for (int64_t x = warp; x < n; x += nwarps) {
-    if (done[x] || key[x] != k) continue;
-    uint32_t b, e; const uint32_t* a; int64_t sh;
-    L.get(x, b, e, a, sh);
-    for (uint32_t j = b + lane; j < e; j += 32) {
-      int64_t y = (int64_t)a[j] + sh;
-      if (key[y] < k) {
-        uint32_t old = atomicSub(&dact[y], 1u);
-        uint32_t nd = old - 1u;
-        atomicMin(&key[y], approx ? log_key(nd) : nd);
+// Grid barrier of a cooperative launch: arrivals are counted in a word that is never reset.
+// Bounded: on expiry sets err and returns false in every CTA.
+__device__ bool co_barrier(CoCtl* c, unsigned long long target) {
+  __syncthreads();
+  int bad = 0;
+  if (threadIdx.x == 0) {
+    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&c->bar), "l"(1ull) : "memory");
+    unsigned long long seen, t0 = 0;
+    for (unsigned polls = 0;;) {
+      asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(seen) : "l"(&c->bar) : "memory");
+      if (seen >= target) break;
+      if ((++polls & 63u) == 0) {
+        unsigned long long now;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+        if (!t0) t0 = now;
+        else if (now - t0 > kCoTimeoutNs) {
+          atomicExch(&c->err, 1u);
+          atomicOr(&c->bar, 1ull << 63);
+        }
       }
     }
-    __syncwarp();
-    if (lane == 0) done[x] = 1;
+    bad = (seen >> 63) != 0;
+  }
+  return __syncthreads_or(bad) == 0;
+}
+
+__global__ void __launch_bounds__(kCoThreads, 1) cocore_kernel(Lists L, int64_t n, int approx, uint32_t* key, uint32_t* dact,
+                                                              uint2* units, CoCtl* ctl) {
+  __shared__ uint32_t s_k, s_len;
+  const unsigned lane = threadIdx.x & 31u;
+  const int64_t gtid = (int64_t)blockIdx.x * kCoThreads + threadIdx.x, gthreads = (int64_t)gridDim.x * kCoThreads;
+  unsigned long long target = 0;
+  auto post_max = [&](uint32_t m, uint32_t* to) {
+    m = __reduce_max_sync(0xffffffffu, m);
+    if (lane == 0 && m) atomicMax(to, m);
+  };
+  {
+    uint32_t m = 0;
+    for (int64_t x = gtid; x < n; x += gthreads) {
+      uint32_t b, e; const uint32_t* a; int64_t sh;
+      L.get(x, b, e, a, sh);
+      const uint32_t k = approx ? log_key(e - b) : e - b;
+      dact[x] = e - b;
+      key[x] = k;
+      m = max(m, k + 1u);
+    }
+    post_max(m, &ctl->kmax[0]);
+  }
+  if (!co_barrier(ctl, target += gridDim.x)) return;
+  for (unsigned par = 0;; par ^= 1u) {
+    if (threadIdx.x == 0) s_k = *(volatile uint32_t*)&ctl->kmax[par];
+    __syncthreads();
+    if (s_k == 0) break;
+    const uint32_t k = s_k - 1u;
+    uint32_t m = 0;
+    for (int64_t x0 = gtid - lane; x0 < n; x0 += gthreads) {  // whole warps
+      const int64_t x = x0 + lane;
+      const uint32_t kx = x < n ? key[x] : kCoDone;
+      const bool mine = kx == k;
+      if (kx < k) m = max(m, kx + 1u);
+      if (!__any_sync(0xffffffffu, mine)) continue;
+      uint32_t nu = 0;
+      if (mine) {
+        key[x] = k | kCoDone;
+        uint32_t b, e; const uint32_t* a; int64_t sh;
+        L.get(x, b, e, a, sh);
+        nu = (e - b + kCoUnit - 1) / kCoUnit;
+      }
+      const uint32_t incl = warp_inclusive_scan(nu);
+      uint32_t at = 0;
+      if (lane == 31 && incl) at = atomicAdd(&ctl->len[par], incl);
+      at = __shfl_sync(0xffffffffu, at, 31) + incl - nu;
+      for (uint32_t c = 0; c < nu; ++c) units[at + c] = make_uint2((uint32_t)x, c);
+    }
+    post_max(m, &ctl->kmax[par ^ 1u]);
+    if (!co_barrier(ctl, target += gridDim.x)) return;
+    if (threadIdx.x == 0) s_len = *(volatile uint32_t*)&ctl->len[par];
+    __syncthreads();
+    if (blockIdx.x == 0 && threadIdx.x == 0) {  // every CTA has read kmax[par]; len[par ^ 1] is the last round's
+      ctl->kmax[par] = 0;
+      ctl->len[par ^ 1u] = 0;
+    }
+    const uint32_t len = s_len;
+    for (uint32_t q = (uint32_t)(gtid >> 5); q < len; q += (uint32_t)(gthreads >> 5)) {
+      const uint2 u = units[q];
+      uint32_t b, e; const uint32_t* a; int64_t sh;
+      L.get(u.x, b, e, a, sh);
+      b += u.y * kCoUnit;
+      e = min(e, b + kCoUnit);
+      for (uint32_t j = b + lane; j < e; j += 32) {
+        const int64_t y = (int64_t)a[j] + sh;
+        if (key[y] < k) {
+          const uint32_t nd = atomicSub(&dact[y], 1u) - 1u;
+          atomicMin(&key[y], approx ? log_key(nd) : nd);
+        }
+      }
+    }
+    if (!co_barrier(ctl, target += gridDim.x)) return;
   }
 }
 
 __global__ void cocore_keys_kernel(const uint32_t* __restrict__ key, int64_t n, uint32_t kmax, uint32_t* skeys,
                                    uint32_t* ids) {
   for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x) {
-    skeys[x] = kmax - key[x];
+    skeys[x] = kmax - (key[x] & ~kCoDone);
     ids[x] = (uint32_t)x;
   }
 }
@@ -128,42 +202,83 @@ __global__ void ranked_degrees_kernel(const uint32_t* __restrict__ order, const 
     rdeg[r] = deg[order[r]];
 }
 
-// Fills row r of the ranked CSR with (rank(y) << 1 | on_count_side(y)) for every neighbour y
-// of order[r] (rankGraph, butterfly_utils.h:579-623).  With eout, also the output edge index
-// of each slot (CountERank's conversion, butterfly_ecount.h:1728-1738): slots whose neighbour
-// is on the count side index the center side's lists directly; the others hold the index of
-// the same edge in the neighbour's (center side) list, found by binary search (edgeToIdxs,
-// butterfly_utils.h:2034-2062).
+// Calls f(valid, slot, row) for every slot of [s0, s1) of a CSR (row: the slot's row), 32 slots of
+// one warp at a time: work is cut by slots, not rows, since rows are as uneven as degrees (one
+// warp per row left the last hubs running alone: the wedge scan of the power-law graph with 1e7 edges
+// took 4.4 ms, in chunks of slots 0.29; its fill 1.2 and 0.14).
+template <class F>
+__device__ __forceinline__ void warp_slots(const uint32_t* __restrict__ off, int64_t n, uint32_t s0, uint32_t s1, F&& f) {
+  const unsigned lane = threadIdx.x & 31u;
+  int64_t lo = 0, hi = n;  // the last row with off[row] <= s0, 32-way search
+  while (hi - lo > 1) {
+    const int64_t step = (hi - lo + 31) / 32, idx = lo + lane * step;
+    const unsigned le = __ballot_sync(0xffffffffu, idx < hi && off[idx] <= s0);
+    lo += (31 - __clz(le)) * step;  // lane 0 always qualifies
+    hi = min(lo + step, hi);
+  }
+  uint32_t r = (uint32_t)lo;
+  for (uint32_t s = s0; s < s1; s += 32) {
+    const uint32_t slot = s + lane;
+    uint32_t row = r;
+    for (uint32_t base = r;; base += 32) {
+      // Starts of rows base + 1 .. base + 32 (off[n] lies above every slot).
+      const uint32_t bnd = off[min((int64_t)base + 1 + lane, n)];
+      uint32_t c = 0;  // how many of them are at or before this lane's slot
+#pragma unroll
+      for (uint32_t step = 16; step > 0; step >>= 1)
+        if (__shfl_sync(0xffffffffu, bnd, c + step - 1) <= slot) c += step;
+      if (__shfl_sync(0xffffffffu, bnd, c) <= slot) ++c;
+      if (slot < s1 && row == base) row = base + c;
+      if (!__any_sync(0xffffffffu, slot < s1 && row == base + 32)) break;
+    }
+    f(slot < s1, slot, row);
+    r = __shfl_sync(0xffffffffu, row, 31);
+  }
+}
+// Slots a warp takes at a time: 256 share the search for the first row, 32 while that many warps are
+// all resident (small graphs are bound by one warp's chain).
+constexpr uint32_t kSlotChunk = 256;
+
+// The neighbours of the ranked graph, slot by slot in rank order (rankGraph,
+// butterfly_utils.h:579-623): row r is the vertex x = order[r], y its neighbour of the slot.
+// With eout, also the output edge index of the slot (CountERank's conversion,
+// butterfly_ecount.h:1728-1738): slots whose neighbour is on the count side index the centre side's
+// lists directly; the others hold the index of the same edge in the neighbour's (centre side) list,
+// found by binary search (edgeToIdxs, butterfly_utils.h:2034-2062).
+// Large graphs (dest != null): dest = rank(y), adj = (r << 1 | on_count_side(x)), to be sorted by dest
+// into the rows of y; otherwise adj = (rank(y) << 1 | on_count_side(y)), to be sorted within the row.
 __global__ void ranked_fill_kernel(Lists L, const uint32_t* __restrict__ order, const uint32_t* __restrict__ rank,
-                                   const uint32_t* __restrict__ roff, int64_t n, int use_v, uint32_t* adj,
-                                   uint32_t* eout) {
+                                   const uint32_t* __restrict__ roff, int64_t n, int64_t m2, uint32_t chunk, int use_v, uint32_t* dest,
+                                   uint32_t* adj, uint32_t* eout) {
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const unsigned lane = threadIdx.x & 31u;
-  for (int64_t r = warp; r < n; r += nwarps) {
-    const int64_t x = order[r];
-    uint32_t b, e; const uint32_t* a; int64_t sh;
-    L.get(x, b, e, a, sh);
-    const uint32_t dst = roff[r];
-    const uint32_t x_local = (uint32_t)(x < L.nv ? x : x - L.nv);
-    for (uint32_t j = b + lane; j < e; j += 32) {
+  for (int64_t c = warp * chunk; c < m2; c += nwarps * chunk) {
+    warp_slots(roff, n, (uint32_t)c, (uint32_t)min(c + (int64_t)chunk, m2), [&](bool valid, uint32_t s, uint32_t r) {
+      if (!valid) return;
+      const int64_t x = order[r];
+      uint32_t b, e; const uint32_t* a; int64_t sh;
+      L.get(x, b, e, a, sh);
+      const uint32_t j = b + (s - roff[r]);
       const uint32_t yl = a[j];
       const int64_t y = (int64_t)yl + sh;
       const bool y_v = y < L.nv;
       const uint32_t tag = use_v ? (y_v ? 0u : 1u) : (y_v ? 1u : 0u);
-      adj[dst + (j - b)] = (rank[y] << 1) | tag;
+      if (dest) {
+        dest[s] = rank[y];
+        adj[s] = (r << 1) | (tag ^ 1u);
+      } else {
+        adj[s] = (rank[y] << 1) | tag;
+      }
       if (eout) {
-        uint32_t o;
-        if (tag) {
-          o = j;
-        } else {
+        uint32_t o = j;
+        if (!tag) {
           const uint32_t* yo = y_v ? L.offV : L.offU;
           const uint32_t* ya = y_v ? L.edgV : L.edgU;
-          o = lower_bound_u32(ya, yo[yl], yo[yl + 1], x_local);
+          o = lower_bound_u32(ya, yo[yl], yo[yl + 1], (uint32_t)(x < L.nv ? x : x - L.nv));
         }
-        eout[dst + (j - b)] = o;
+        eout[s] = o;
       }
-    }
+    });
   }
 }
 
@@ -180,27 +295,35 @@ __global__ void below_self_kernel(const uint32_t* __restrict__ off, const uint32
 // slot (i, v) the wedges are the u2 in N(v) with u2 < min(i, v).  Lists are ascending, so that
 // prefix length is a binary search for i in N(v) (when i < v) or the per-vertex below[v].
 __global__ void wedge_scan_kernel(const uint32_t* __restrict__ off, const uint32_t* __restrict__ adj,
-                                  const uint32_t* __restrict__ below, int64_t n, uint32_t* pref, int64_t* wcount) {
+                                  const uint32_t* __restrict__ below, int64_t n, int64_t m2, uint32_t chunk, uint32_t* pref,
+                                  int64_t* wcount) {
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const unsigned lane = threadIdx.x & 31u;
-  for (int64_t i = warp; i < n; i += nwarps) {
-    const uint32_t b = off[i], e = off[i + 1];
-    int64_t sum = 0;
-    for (uint32_t j = b + lane; j < e; j += 32) {
-      const uint32_t v = adj[j] >> 1;
-      uint32_t L;
-      if ((uint32_t)i < v) {
-        const uint32_t vb = off[v];
-        L = lower_bound_u32(adj, vb, off[v + 1], (uint32_t)i << 1) - vb;
-      } else {
-        L = below[v];
+  for (int64_t c = warp * chunk; c < m2; c += nwarps * chunk) {
+    warp_slots(off, n, (uint32_t)c, (uint32_t)min(c + (int64_t)chunk, m2), [&](bool valid, uint32_t j, uint32_t i) {
+      uint32_t L = 0;
+      if (valid) {
+        const uint32_t v = adj[j] >> 1;
+        if (i < v) {
+          const uint32_t vb = off[v];
+          L = lower_bound_u32(adj, vb, off[v + 1], i << 1) - vb;
+        } else {
+          L = below[v];
+        }
+        pref[j] = L;
       }
-      pref[j] = L;
-      sum += L;
-    }
-    sum = warp_sum(sum);
-    if (lane == 0) wcount[i] = sum;
+      // One add per row and group of 32 slots (a row's slots are neighbouring lanes).
+      const int64_t incl = warp_inclusive_scan((int64_t)L);
+      const uint32_t row = valid ? i : 0xFFFFFFFFu;
+      const uint32_t prev = __shfl_up_sync(0xffffffffu, row, 1);
+      const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || row != prev);
+      const int first = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+      const int64_t before = __shfl_sync(0xffffffffu, incl, first > 0 ? first - 1 : 0);
+      const uint32_t next = __shfl_down_sync(0xffffffffu, row, 1);
+      const int64_t sum = incl - (first > 0 ? before : 0);
+      if (valid && (lane == 31 || next != row) && sum) atomic_add_i64(&wcount[i], sum);
+    });
   }
 }
 
@@ -250,6 +373,11 @@ __global__ void validate_uses_kernel(const uint32_t* __restrict__ uses, int64_t 
     if (uses[i] != 2u && atomicCAS(&err[0], 0u, 33u) == 0u) { err[1] = (uint32_t)i; err[3] = uses[i]; }
 }
 
+// Slots from which the ranked rows are built by one radix sort of (row, neighbour) pairs over the
+// whole CSR instead of a sort within each row.  Relabel of R-MAT graphs, per vertex, radix against row
+// sort: 2^18 slots 0.115 / 0.098 ms, 2^19 0.119 / 0.121, 2^20 0.125 / 0.190, 2^23 0.449 / 1.033.
+constexpr int64_t kRankSort = int64_t(1) << 19;
+
 int bits_for(uint64_t x) {
   int b = 0;
   while (b < 64 && (x >> b) != 0) ++b;
@@ -259,6 +387,8 @@ int bits_for(uint64_t x) {
 Lists lists_of(const pb_graph& g) {
   return Lists{g.offV.get(), g.edgV.get(), g.offU.get(), g.edgU.get(), g.nv};
 }
+
+uint32_t slot_chunk(int64_t m2) { return m2 <= (int64_t)sm_count() * 64 * 32 ? 32u : kSlotChunk; }
 
 int grid_for(int64_t n, int per_block = 256) { return std::max(1, std::min(ceil_div(n, per_block), sm_count() * 16)); }
 
@@ -297,19 +427,21 @@ void vertex_order(const pb_graph& g, int rank_type, int use_v, Ranked& R, cudaSt
   uint32_t* ids = R.order.get();
   if (rank_type == PB_COCORE || rank_type == PB_ACOCORE) {
     const int approx = rank_type == PB_ACOCORE;
-    DevBuf<uint32_t> key(n, s), dact(n, s), kbuf(1, s);
-    DevBuf<uint8_t> done(n, s);
-    PB_LAUNCH(cocore_init_kernel, grid_for(n), 256, 0, s, deg.get(), n, approx, key.get(), dact.get(), done.get());
-    while (true) {
-      PB_CUDA_TRY(cudaMemsetAsync(kbuf.get(), 0, sizeof(uint32_t), s));
-      PB_LAUNCH(cocore_max_kernel, grid_for(n), 256, 0, s, key.get(), done.get(), n, kbuf.get());
-      uint32_t k1 = 0;
-      readback(&k1, kbuf.get(), sizeof(uint32_t), s);
-      if (k1 == 0) break;
-      kmax = std::max(kmax, k1 - 1);
-      PB_LAUNCH(cocore_round_kernel, grid_for(n * 32), 256, 0, s, lists_of(g), n, approx, kbuf.get(), key.get(),
-                dact.get(), done.get());
-    }
+    DevBuf<uint32_t> key(n, s), dact(n, s);
+    DevBuf<uint2> units((size_t)(n + 2 * g.m / kCoUnit + 1), s);
+    R.co.alloc(sizeof(CoCtl), s);
+    CoCtl* ctl = reinterpret_cast<CoCtl*>(R.co.get());
+    PB_CUDA_TRY(cudaMemsetAsync(ctl, 0, sizeof(CoCtl), s));
+    kmax = approx ? (g.max_deg ? 32u - (uint32_t)__builtin_clz(g.max_deg) : 0u) : g.max_deg;
+    Lists lists = lists_of(g);
+    int64_t nn = n;
+    int ap = approx;
+    uint32_t *kp = key.get(), *dp = dact.get();
+    uint2* up = units.get();
+    void* args[] = {&lists, &nn, &ap, &kp, &dp, &up, &ctl};
+    const int grid = std::max(1, std::min(sm_count(), ceil_div(n, kCoThreads)));
+    PB_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)cocore_kernel, dim3(grid), dim3(kCoThreads), args, 0, s));
+    if (g_launch_counter) ++*g_launch_counter;
     PB_LAUNCH(cocore_keys_kernel, grid_for(n), 256, 0, s, key.get(), n, kmax, keys.get(), ids);
     nbits = bits_for(kmax);
   } else {
@@ -345,10 +477,24 @@ void build_ranked_csr(const pb_graph& g, Ranked& R, bool with_eout, cudaStream_t
     exclusive_scan_u32(rdeg.get(), R.off.get(), n, s);
   }
   if (R.m2 == 0) return;
-  PB_LAUNCH(ranked_fill_kernel, grid_for(n * 32), 256, 0, s, lists_of(g), R.order.get(), R.rank.get(), R.off.get(), n,
-            R.use_v, R.adj.get(), with_eout ? R.eout.get() : nullptr);
-  segmented_sort_rows(R.off.get(), n, R.adj.get(), with_eout ? R.eout.get() : nullptr, bits_for((uint64_t)(2 * n)),
-                      g.max_deg, s);
+  const uint32_t chunk = slot_chunk(R.m2);
+  const int grid = grid_for((R.m2 + chunk - 1) / chunk * 32);
+  if (R.m2 < kRankSort) {
+    PB_LAUNCH(ranked_fill_kernel, grid, 256, 0, s, lists_of(g), R.order.get(), R.rank.get(), R.off.get(), n, R.m2, chunk, R.use_v,
+              (uint32_t*)nullptr, R.adj.get(), with_eout ? R.eout.get() : nullptr);
+    segmented_sort_rows(R.off.get(), n, R.adj.get(), with_eout ? R.eout.get() : nullptr, bits_for((uint64_t)(2 * n)),
+                        g.max_deg, s);
+    return;
+  }
+  DevBuf<uint32_t> dest(R.m2, s), dest2(R.m2, s), adj2(R.adj.n, s), eout2;
+  if (with_eout) eout2.alloc(R.m2, s);
+  PB_LAUNCH(ranked_fill_kernel, grid, 256, 0, s, lists_of(g), R.order.get(), R.rank.get(), R.off.get(), n, R.m2, chunk, R.use_v,
+            dest.get(), R.adj.get(), with_eout ? R.eout.get() : nullptr);
+  if (radix_sort_pairs_u32(dest.get(), R.adj.get(), dest2.get(), adj2.get(), R.m2, 0, bits_for((uint64_t)(n - 1)), s,
+                           R.eout.get(), eout2.get())) {
+    std::swap(R.adj.p, adj2.p);
+    std::swap(R.eout.p, eout2.p);
+  }
 }
 
 void wedge_scan(Ranked& R, cudaStream_t s) {
@@ -362,11 +508,19 @@ void wedge_scan(Ranked& R, cudaStream_t s) {
   }
   DevBuf<uint32_t> below(n, s);
   DevBuf<int64_t> wc(n, s);
+  PB_CUDA_TRY(cudaMemsetAsync(wc.get(), 0, wc.bytes(), s));
   PB_LAUNCH(below_self_kernel, grid_for(n), 256, 0, s, R.off.get(), R.adj.get(), n, below.get());
-  PB_LAUNCH(wedge_scan_kernel, grid_for(n * 32), 256, 0, s, R.off.get(), R.adj.get(), below.get(), n, R.pref.get(),
-            wc.get());
+  const uint32_t chunk = slot_chunk(R.m2);
+  if (R.m2 > 0)
+    PB_LAUNCH(wedge_scan_kernel, grid_for((R.m2 + chunk - 1) / chunk * 32), 256, 0, s, R.off.get(), R.adj.get(),
+              below.get(), n, R.m2, chunk, R.pref.get(), wc.get());
   exclusive_scan_i64(wc.get(), R.wsum.get(), n, s);
   readback(&R.w_rank, R.wsum.get() + n, sizeof(int64_t), s);
+  if (R.co.get()) {
+    uint32_t err = 0;
+    readback(&err, &reinterpret_cast<CoCtl*>(R.co.get())->err, sizeof(err), s);
+    PB_REQUIRE(err == 0, PB_ETIMEOUT, "ranking: a grid barrier wait ran out of time");
+  }
 }
 
 bool check_mode() {

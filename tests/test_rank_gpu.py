@@ -1,0 +1,43 @@
+"""The ranked CSR at the edges of its builders: slots around the line between the row sort and the
+radix sort, rows that begin and end inside a 256-slot chunk, long runs of empty rows, and co-core
+ranking with lists around multiples of its 256-entry units.  The order is checked through the ranked
+wedge count (equal to the oracle's only for the same order), the rows through the counts."""
+import numpy as np
+import pytest
+
+import oracle
+from parbutterfly_b200 import butterflies as pb
+from parbutterfly_b200.graph import BipartiteGraph
+
+pytestmark = pytest.mark.gpu
+
+
+def _hubs():
+    """Stars of 255, 256, 257, 512 and 513 leaves that share leaves, and isolated vertices between."""
+    v, u = [], []
+    for k, d in enumerate((255, 256, 257, 512, 513)):
+        v.append(np.full(d, 40 * k))
+        u.append(np.arange(d) * 3)
+    return BipartiteGraph.from_edges(400, 2000, np.concatenate(v), np.concatenate(u))
+
+
+GRAPHS = {
+    "slots_below": lambda: BipartiteGraph.uniform(9_000, 7_000, (1 << 18) - 1, 31),
+    "slots_at": lambda: BipartiteGraph.rmat(14, 12, 1 << 18, 0.55, 0.15, 0.15, 0.15, 32),
+    "slots_above": lambda: BipartiteGraph.powerlaw_u(5_000, 30_000, (1 << 18) + 1, 2.0, 5_000, 33),
+    "hubs": _hubs,
+    "sparse": lambda: BipartiteGraph.uniform(200_000, 150_000, 3_000, 34),
+    "one_row": lambda: BipartiteGraph.from_edges(3, 700, np.r_[np.zeros(700, int), 1, 1], np.r_[np.arange(700), 0, 699]),
+}
+
+
+@pytest.mark.parametrize("rank", ["SIDE", "COCORE", "ACOCORE", "DEG", "ADEG"])
+@pytest.mark.parametrize("name", sorted(GRAPHS))
+def test_ranked_csr(ctx, name, rank):
+    g = GRAPHS[name]()
+    dg = ctx.upload(g)
+    want, w_rank = oracle.count(g, "VERT", rank)
+    assert np.array_equal(pb.count(dg, "HASH", rank), want)
+    assert ctx.stats()["w_rank"] == w_rank
+    assert np.array_equal(pb.count_e(dg, "BATCHS", rank), oracle.count(g, "EDGE", rank)[0])
+    dg.close()
