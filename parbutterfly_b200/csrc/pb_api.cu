@@ -59,6 +59,9 @@ struct pb_ctx {
   int trace_mode = PB_TRACE_OFF;
   uint64_t trace_seed = 0;
   uint64_t peel_sweep[2] = {0, 0};  // explore-mode position in the setting grid (tip, wing)
+  // Timing events, made at the first use and kept until the context goes.
+  cudaEvent_t ev[8] = {};
+  pb::CountTail* tail = nullptr;  // pinned host copy of a counting call's tail
   std::vector<float> trace_X[2], trace_y[2];
 };
 
@@ -217,14 +220,12 @@ struct Trace {
 };
 
 struct Timer {
-  cudaEvent_t ev[8];
+  cudaEvent_t* ev;
   int k = 0;
   cudaStream_t s;
-  explicit Timer(cudaStream_t st) : s(st) {
-    for (auto& e : ev) PB_CUDA_TRY(cudaEventCreate(&e));
-  }
-  ~Timer() {
-    for (auto& e : ev) cudaEventDestroy(e);
+  explicit Timer(pb_ctx* ctx) : ev(ctx->ev), s(ctx->stream) {
+    for (int i = 0; i < 8; ++i)
+      if (!ev[i]) PB_CUDA_TRY(cudaEventCreate(&ev[i]));
   }
   void mark() { PB_CUDA_TRY(cudaEventRecord(ev[k++], s)); }
   double ms(int a, int b) {
@@ -240,18 +241,19 @@ int64_t out_len_of(const pb_graph* g, int per, int use_v) {
   return 1;
 }
 
-// The whole counting pipeline; result (dense int64, length out_len_of) in out_dev.
-void run_count(pb_ctx* ctx, const pb_graph* g, const pb_opts& o, int per, int use_v, int64_t* out_dev) {
+// The whole counting pipeline for count side use_v; result (dense int64, length out_len_of) in
+// out_dev, and copied to out_host when that is not null.
+void run_count(pb_ctx* ctx, const pb_graph* g, const pb_opts& o, int per, int use_v, int64_t* out_dev,
+               int64_t* out_host = nullptr) {
   cudaStream_t s = ctx->stream;
   pb_stats& st = ctx->stats;
   std::memset(&st, 0, sizeof(st));
-  int uv = 0;
-  int64_t wmin = 0, wv = 0, wu = 0;
-  cmp_wedge_counts(*g, &uv, &wmin, &wv, &wu, s);
-  if (use_v < 0) use_v = uv;
-  st.w_side = use_v ? wv : wu;
   st.use_v = use_v;
-  Timer T(s);
+  // The side's wedge count is only reported: it comes back with the call's last readback.
+  DevBuf<CountTail> tail(1, s);
+  PB_CUDA_TRY(cudaMemsetAsync(tail.get(), 0, sizeof(CountTail), s));
+  side_wedge_sums(*g, tail.get()->sides, s);
+  Timer T(ctx);
   Trace tr(s);
   Ranked R;
   T.mark();
@@ -337,15 +339,13 @@ void run_count(pb_ctx* ctx, const pb_graph* g, const pb_opts& o, int per, int us
     rc.alloc(R.n > 0 ? R.n : 1, s);
     target = rc.get();
   }
+  cfg.tail = tail.get();
+  cfg.ev = ctx->ev + 6;
   CountResult cr = cfg.strategy == STRAT_SORT   ? count_ranked_materialized(R, per, target, false, o.max_wedges, s)
                    : cfg.strategy == STRAT_HIST ? count_ranked_materialized(R, per, target, true, o.max_wedges, s)
                                                 : count_ranked(R, per, target, cfg, s);
   T.mark();
   tr.stage("count");
-  if (trace_on())
-    fprintf(stderr, "[pb] CTA modes (endpoints / wedges): dense %llu/%llu hash %llu/%llu global %llu/%llu hybrid %llu/%llu\n",
-            cr.mode_items[0], cr.mode_wedges[0], cr.mode_items[1], cr.mode_wedges[1], cr.mode_items[2],
-            cr.mode_wedges[2], cr.mode_items[3], cr.mode_wedges[3]);
   if (chk.get()) {
     uint32_t h[4];
     PB_CUDA_TRY(cudaMemcpyAsync(h, chk.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
@@ -362,7 +362,17 @@ void run_count(pb_ctx* ctx, const pb_graph* g, const pb_opts& o, int per, int us
                 R.rank.get(), base, nc, out_dev);
   }
   T.mark();
+  CountTail& h = *ctx->tail;
+  PB_CUDA_TRY(cudaMemcpyAsync(&h, tail.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
+  if (out_host)
+    PB_CUDA_TRY(cudaMemcpyAsync(out_host, out_dev, sizeof(int64_t) * out_len_of(g, per, use_v), cudaMemcpyDeviceToHost, s));
   PB_CUDA_TRY(cudaStreamSynchronize(s));
+  if (cr.pending) finish_count(cr, h, cfg.ev);
+  if (trace_on())
+    fprintf(stderr, "[pb] CTA modes (endpoints / wedges): dense %llu/%llu hash %llu/%llu global %llu/%llu hybrid %llu/%llu\n",
+            cr.mode_items[0], cr.mode_wedges[0], cr.mode_items[1], cr.mode_wedges[1], cr.mode_items[2],
+            cr.mode_wedges[2], cr.mode_items[3], cr.mode_wedges[3]);
+  st.w_side = (int64_t)h.sides[use_v ? 0 : 1];
   st.w_rank = R.w_rank;
   st.n_big = cr.n_big;
   st.ms_rank = T.ms(0, 1);
@@ -573,6 +583,13 @@ pb_status pb_ctx_create(int device, void* stream, pb_ctx** out) {
     }
     c->own_stream = true;
   }
+  if (cudaMallocHost((void**)&c->tail, sizeof(pb::CountTail)) != cudaSuccess) {
+    cudaGetLastError();
+    if (c->own_stream) cudaStreamDestroy(c->stream);
+    delete c;
+    cudaSetDevice(prev);
+    return PB_ENOMEM;
+  }
   cudaMemPool_t pool;
   if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) {
     uint64_t thr = UINT64_MAX;
@@ -590,6 +607,9 @@ pb_status pb_ctx_destroy(pb_ctx* ctx) {
   cudaGetDevice(&prev);
   cudaSetDevice(ctx->device);
   cudaStreamSynchronize(ctx->stream);
+  for (cudaEvent_t e : ctx->ev)
+    if (e) cudaEventDestroy(e);
+  cudaFreeHost(ctx->tail);
   if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
   cudaSetDevice(prev);
   delete ctx;
@@ -769,16 +789,13 @@ static pb_status count_entry(pb_ctx* ctx, const pb_graph* g, const pb_opts* opts
       use_v = uv;
     }
     const int64_t len = out_len_of(g, per, use_v);
-    if (per == PB_TOTAL && len > 0 && !is_device_ptr(out)) {
-      DevBuf<int64_t> tmp(1, ctx->stream);
-      run_count(ctx, g, o, per, use_v, tmp.get());
-      PB_CUDA_TRY(cudaMemcpyAsync(out, tmp.get(), sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
-      PB_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-      return;
+    if (len <= 0) return;
+    if (is_device_ptr(out)) {
+      run_count(ctx, g, o, per, use_v, out);
+    } else {
+      DevBuf<int64_t> tmp(len, ctx->stream);
+      run_count(ctx, g, o, per, use_v, tmp.get(), out);
     }
-    with_output(ctx, out, len, [&](int64_t* dev) {
-      if (dev) run_count(ctx, g, o, per, use_v, dev);
-    });
   });
 }
 
@@ -815,7 +832,7 @@ static pb_status peel_entry(pb_ctx* ctx, const pb_graph* g, const pb_opts* opts,
       PB_CUDA_TRY(cudaMemcpyAsync(cin.get(), counts, sizeof(int64_t) * len, cudaMemcpyHostToDevice, s));
       cdev = cin.get();
     }
-    Timer T(s);
+    Timer T(ctx);
     std::vector<float> row;
     float pred = 0.f;
     const PeelTuning tune = peel_setting(ctx, *g, use_v, edges, cdev, o, row, &pred);
@@ -875,7 +892,7 @@ pb_status pb_peel_vert_batch(pb_ctx* ctx, const pb_graph* const* gs, int32_t k, 
       if (ksize[g])
         PB_CUDA_TRY(cudaMemcpyAsync(cin.get() + kbase[g], counts[g], sizeof(int64_t) * ksize[g], cudaMemcpyDefault, s));
     }
-    Timer T(s);
+    Timer T(ctx);
     std::vector<float> row;
     float pred = 0.f;
     const PeelTuning tune = peel_setting(ctx, U, 1, false, cin.get(), o, row, &pred);
@@ -963,7 +980,7 @@ pb_status pb_batch_run(pb_ctx* ctx, pb_batch* b, int64_t* const* counts, int64_t
     PB_REQUIRE(b && b->exec, PB_EINVAL, "null batch");
     PB_REQUIRE(b->device == ctx->device, PB_EINVAL, "batch and context are on different devices");
     cudaStream_t s = ctx->stream;
-    Timer T(s);
+    Timer T(ctx);
     b->rec.status[0] = 0xFFFFFFFFu;
     T.mark();
     PB_CUDA_TRY(cudaGraphLaunch(b->exec, s));

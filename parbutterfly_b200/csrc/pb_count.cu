@@ -847,17 +847,19 @@ CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConf
   P.out = out;
   P.out_len = out_len;
   P.m2 = R.m2;
-  DevBuf<uint32_t> err_local;
-  if (cfg.err) {
-    P.err = cfg.err;
+  DevBuf<CountTail> own_tail;
+  CountTail* tail = cfg.tail;
+  if (!tail) {
+    own_tail.alloc(1, s);
+    tail = own_tail.get();
+    PB_CUDA_TRY(cudaMemsetAsync(tail, 0, sizeof(CountTail), s));
   } else {
-    err_local.alloc(4, s);
-    PB_CUDA_TRY(cudaMemsetAsync(err_local.get(), 0, 4 * sizeof(uint32_t), s));
-    P.err = err_local.get();
+    // (the autotuner runs several counts on one tail)
+    PB_CUDA_TRY(cudaMemsetAsync(tail->counts, 0, sizeof(tail->counts), s));
   }
-  DevBuf<unsigned long long> mstats(8, s);
-  PB_CUDA_TRY(cudaMemsetAsync(mstats.get(), 0, 8 * sizeof(unsigned long long), s));
-  P.mstats = mstats.get();
+  P.err = cfg.err ? cfg.err : tail->err;
+  P.mstats = tail->mstats;
+  uint32_t* const counts = tail->counts;
   // Per-edge counts are gathered per slot, in 32 bits when they fit: (max degree - 1)^2 < 2^32.
   DevBuf<uint32_t> sacc32;
   DevBuf<unsigned long long> sacc64;
@@ -908,27 +910,28 @@ CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConf
   else if (sh && sh->model) mid_w = std::min(mid_w, sched_min_w - 1);
   DevBuf<uint4> lists((size_t)n * 3, s);  // warp, mid and block lists
   uint4 *small_items = lists.get(), *mid_items = small_items + n, *items = mid_items + n;
-  DevBuf<uint32_t> counts(6, s);
   DevBuf<uint8_t> modes(n, s);
-  PB_CUDA_TRY(cudaMemsetAsync(counts.get(), 0, 6 * sizeof(uint32_t), s));
   PB_LAUNCH(classify_endpoints_kernel, std::max(1, std::min(ceil_div(n, 256), sms * 8)), 256, 0, s, R.wsum.get(),
-            R.off.get(), n, small_w, mid_w, Gm, small_items, mid_items, items, counts.get(), P.err);
+            R.off.get(), n, small_w, mid_w, Gm, small_items, mid_items, items, counts, P.err);
   uint32_t hc[5];
-  readback(hc, counts.get(), sizeof(hc), s);
+  readback(hc, counts, sizeof(hc), s);
   const uint32_t n_block = hc[0], n_small = hc[3], n_mid = hc[4];
   if (n_block > 0) {
     PB_LAUNCH(plain_modes_kernel, (int)std::min<int64_t>(ceil_div(n_block, 8), sms * 8), 256, 0, s, P, items,
-              counts.get(), G, modes.get(), counts.get() + 1);
-    readback(&hc[1], counts.get() + 1, sizeof(uint32_t), s);
+              counts, G, modes.get(), counts + 1);
+    readback(&hc[1], counts + 1, sizeof(uint32_t), s);
   }
   res.n_big = (int)(n_block + n_mid);
 
   // Under graph capture nothing is timed or read back here (the recording run checked).
   const bool cap = capturing();
-  cudaEvent_t e0, e1;
-  PB_CUDA_TRY(cudaEventCreate(&e0));
-  PB_CUDA_TRY(cudaEventCreate(&e1));
-  if (!cap) PB_CUDA_TRY(cudaEventRecord(e0, s));
+  cudaEvent_t ev[2] = {nullptr, nullptr};
+  if (!cap) {
+    if (cfg.ev) std::copy(cfg.ev, cfg.ev + 2, ev);
+    else
+      for (auto& e : ev) PB_CUDA_TRY(cudaEventCreate(&e));
+    PB_CUDA_TRY(cudaEventRecord(ev[0], s));
+  }
   // Scheduler: per-item modes (learned or exploring) and the record of what each item ran
   // with and how long it took.
   const bool sched_on = sh && n_block > 0 && (sh->model || sh->explore || sh->trace_X);
@@ -1022,7 +1025,7 @@ CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConf
     P.modes = modes.get();
     auto kern = count_block_kernel<kBlock, kBlockPerSm>;
     PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
-    PB_LAUNCH(kern, grid, kBlock, smem_bytes, s, P, items, counts.get(), counts.get() + 2, gscratch.get(), G);
+    PB_LAUNCH(kern, grid, kBlock, smem_bytes, s, P, items, counts, counts + 2, gscratch.get(), G);
   }
   P.modes = nullptr;
   P.mode_out = nullptr;
@@ -1031,7 +1034,7 @@ CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConf
     auto kern = count_block_kernel<kMidBlock, kMidPerSm>;
     PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMidSmem));
     PB_LAUNCH(kern, (int)std::min<int64_t>(n_mid, (int64_t)sms * kMidPerSm), kMidBlock, kMidSmem, s, P, mid_items,
-              counts.get() + 4, counts.get() + 5, (uint32_t*)nullptr, Gm);
+              counts + 4, counts + 5, (uint32_t*)nullptr, Gm);
   }
   if (n_small > 0) {
     const bool one_word = (uint32_t)small_w <= (1u << count_bits) - 2u;
@@ -1040,29 +1043,20 @@ CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConf
         (2 * (int)kHotRanks + kWarpsPerBlockSmall * ((one_word ? 1 : 2) * kWarpTable + 32)) * (int)sizeof(uint32_t);
     PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     PB_LAUNCH(kern, (int)std::min<int64_t>(ceil_div(n_small, kWarpsPerBlockSmall), (int64_t)sms * (one_word ? 6 : 3)),
-              kWarpsPerBlockSmall * 32, smem, s, P, small_items, counts.get() + 3, count_bits);
+              kWarpsPerBlockSmall * 32, smem, s, P, small_items, counts + 3, count_bits);
   }
   if (per == EDGE)
     PB_LAUNCH(edge_gather_kernel, std::max(1, std::min(ceil_div(R.m2, 256), sms * 8)), 256, 0, s, P, R.eout.get());
-  if (cap) {
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
+  if (cap) return res;
+  PB_CUDA_TRY(cudaEventRecord(ev[1], s));
+  if (cfg.tail && cfg.ev && !sched_on) {
+    res.pending = true;
     return res;
   }
-  PB_CUDA_TRY(cudaEventRecord(e1, s));
-  PB_CUDA_TRY(cudaEventSynchronize(e1));
-  {
-    unsigned long long h[8];
-    PB_CUDA_TRY(cudaMemcpy(h, P.mstats, sizeof(h), cudaMemcpyDeviceToHost));
-    for (int k = 0; k < 4; ++k) { res.mode_items[k] = h[k]; res.mode_wedges[k] = h[4 + k]; }
-  }
-  {
-    uint32_t h[4];
-    PB_CUDA_TRY(cudaMemcpy(h, P.err, sizeof(h), cudaMemcpyDeviceToHost));
-    PB_REQUIRE(h[0] == 0, PB_ECUDA,
-               "aggregation: bounds violation code " + std::to_string(h[0]) + " index " +
-                   std::to_string(((uint64_t)h[2] << 32) | h[1]) + " aux " + std::to_string(h[3]));
-  }
+  CountTail h;
+  PB_CUDA_TRY(cudaMemcpyAsync(&h, tail, sizeof(h), cudaMemcpyDeviceToHost, s));
+  PB_CUDA_TRY(cudaStreamSynchronize(s));
+  finish_count(res, h, ev);
   if (sched_on) {
     const uint32_t ni = n_block;
     std::vector<float> hF((size_t)ni * kMlpIn), hPred;
@@ -1098,12 +1092,24 @@ CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConf
     sh->pred_cycles = pc;
     sh->mae_log2 = npred ? mae / npred : 0.0;
   }
-  float ms = 0;
-  PB_CUDA_TRY(cudaEventElapsedTime(&ms, e0, e1));
-  res.agg_ms = ms;
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
+  if (!cfg.ev)
+    for (auto& e : ev) cudaEventDestroy(e);
   return res;
+}
+
+void finish_count(CountResult& res, const CountTail& tail, const cudaEvent_t* ev) {
+  for (int k = 0; k < 4; ++k) {
+    res.mode_items[k] = tail.mstats[k];
+    res.mode_wedges[k] = tail.mstats[4 + k];
+  }
+  res.pending = false;
+  float ms = 0;
+  PB_CUDA_TRY(cudaEventElapsedTime(&ms, ev[0], ev[1]));
+  res.agg_ms = ms;
+  const uint32_t* e = tail.err;
+  PB_REQUIRE(e[0] == 0, PB_ECUDA,
+             "aggregation: bounds violation code " + std::to_string(e[0]) + " index " +
+                 std::to_string(((uint64_t)e[2] << 32) | e[1]) + " aux " + std::to_string(e[3]));
 }
 
 }  // namespace pb

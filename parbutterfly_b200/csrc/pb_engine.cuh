@@ -28,6 +28,7 @@ struct Ranked {
   int use_v = 1;
   DevBuf<uint32_t> order;  // order[r] = combined id (V ids 0..nv-1, then nv + U id)
   DevBuf<uint32_t> rank;   // rank[combined id]
+  DevBuf<uint32_t> rdeg;   // degrees in rank order (until the ranked CSR is built)
   DevBuf<uint32_t> off;    // n+1
   DevBuf<uint32_t> adj;    // 2m tagged ranks
   DevBuf<uint32_t> eout;   // 2m output edge index (per-edge counting only)
@@ -40,7 +41,8 @@ struct Ranked {
 };
 
 // Ranking stage (pb_rank.cu).
-void degrees_combined(const pb_graph& g, uint32_t* deg, cudaStream_t s);
+// sums[0] / sums[1]: wedges centred on V / on U (device memory), not waited for.
+void side_wedge_sums(const pb_graph& g, unsigned long long* sums, cudaStream_t s);
 void cmp_wedge_counts(const pb_graph& g, int* use_v, int64_t* w_min, int64_t* wv, int64_t* wu, cudaStream_t s);
 void vertex_order(const pb_graph& g, int rank_type, int use_v, Ranked& R, cudaStream_t s);
 void build_ranked_csr(const pb_graph& g, Ranked& R, bool with_eout, cudaStream_t s);
@@ -65,6 +67,13 @@ struct SchedHooks {
   int64_t items = 0;
   double pred_cycles = 0, meas_cycles = 0, mae_log2 = 0, ms = 0;
 };
+// What a counting call reads back besides its result, in one device block: one fill, one copy.
+struct CountTail {
+  unsigned long long mstats[8];  // per mode (dense, hash, global, hybrid): endpoints, wedges
+  unsigned long long sides[2];   // side_wedge_sums
+  uint32_t err[4];               // first bounds violation {code, index lo, index hi, aux}
+  uint32_t counts[6];            // classify_endpoints_kernel
+};
 struct CountConfig {
   int strategy = STRAT_AUTO;
   int small_w = 512;          // endpoints with W_i <= small_w go to the warp aggregator
@@ -74,6 +83,11 @@ struct CountConfig {
   int split_w = 0;            // endpoints above this many wedges are split across CTAs (0: auto)
   uint32_t* err = nullptr;    // checked mode: device record of the first bounds violation
   SchedHooks* sched = nullptr;
+  // The caller's zeroed tail and two events for the aggregation's time: count_ranked then leaves
+  // reading them (finish_count) to the caller, who has a wait of its own to come, unless the
+  // scheduler needs the call's cycles.  Null: count_ranked uses its own and waits.
+  CountTail* tail = nullptr;
+  cudaEvent_t* ev = nullptr;
 };
 
 // Checked mode (PB_CHECK=1): kernels bounds-check indices read from memory and record the
@@ -87,7 +101,11 @@ struct CountResult {
   // CTA aggregator modes (dense, hash, global scratch, hybrid): endpoints and wedges.
   unsigned long long mode_items[4] = {0, 0, 0, 0};
   unsigned long long mode_wedges[4] = {0, 0, 0, 0};
+  bool pending = false;  // finish_count is still to be called
 };
+// Fills the result from the tail's host copy and the (completed) events; throws on a recorded
+// bounds violation.
+void finish_count(CountResult& res, const CountTail& tail, const cudaEvent_t* ev);
 CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConfig& cfg, cudaStream_t s);
 // SORT (hist = false) and HIST (hist = true) aggregators over materialised wedge batches of at
 // most max_wedges wedges (pb_agg_sort.cu).

@@ -135,7 +135,7 @@ size_t radix_smem(bool vals, bool vals2) {
          (size_t)(kRadixWarps * 256 + 2 * 256 + 32) * sizeof(uint32_t);
 }
 
-// vals and vals2 may be null (no payload / one payload).
+// vals and vals2 may be null (no payload / one payload); offsets null: the input is one tile.
 template <class K>
 __global__ void __launch_bounds__(kRadixThreads) radix_downsweep_kernel(
     const K* __restrict__ keys, const uint32_t* __restrict__ vals, const uint32_t* __restrict__ vals2, int64_t n, int shift,
@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(kRadixThreads) radix_downsweep_kernel(
   uint32_t* scan = dstart + 256;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int d = threadIdx.x; d < kRadixWarps * 256; d += kRadixThreads) (&wcnt[0][0])[d] = 0;
-  toff[threadIdx.x] = offsets[(int64_t)threadIdx.x * tiles + blockIdx.x];
+  if (offsets) toff[threadIdx.x] = offsets[(int64_t)threadIdx.x * tiles + blockIdx.x];
   __syncthreads();
   const int64_t tile0 = (int64_t)blockIdx.x * kRadixTile;
   const int64_t base = tile0 + (int64_t)warp * (32 * kRadixRounds);
@@ -184,6 +184,7 @@ __global__ void __launch_bounds__(kRadixThreads) radix_downsweep_kernel(
     }
     uint32_t total;
     dstart[threadIdx.x] = block_exclusive_scan(run, scan, total);
+    if (!offsets) toff[threadIdx.x] = dstart[threadIdx.x];  // one tile
   }
   __syncthreads();
 #pragma unroll
@@ -215,7 +216,8 @@ bool radix_sort_impl(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt, i
   if (n <= 1 || end_bit <= begin_bit) return false;
   PB_REQUIRE(n < (int64_t)UINT32_MAX, PB_ETOOBIG, "radix sort supports < 2^32 items");
   const int64_t tiles = (n + kRadixTile - 1) / kRadixTile;
-  DevBuf<uint32_t> counts(256 * tiles + 1, s);
+  DevBuf<uint32_t> counts;
+  if (tiles > 1) counts.alloc(256 * tiles + 1, s);
   const size_t smem = radix_smem<K>(vals != nullptr, vals2 != nullptr);
   PB_CUDA_TRY(cudaFuncSetAttribute(radix_downsweep_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)radix_smem<K>(true, true)));
@@ -223,8 +225,10 @@ bool radix_sort_impl(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt, i
   for (int shift = begin_bit; shift < end_bit; shift += 8) {
     K* kin = alt ? keys_alt : keys;
     K* kout = alt ? keys : keys_alt;
-    PB_LAUNCH(radix_upsweep_kernel<K>, (unsigned)tiles, kRadixThreads, 0, s, kin, n, shift, tiles, counts.get());
-    exclusive_scan_u32(counts.get(), counts.get(), 256 * tiles, s);
+    if (tiles > 1) {
+      PB_LAUNCH(radix_upsweep_kernel<K>, (unsigned)tiles, kRadixThreads, 0, s, kin, n, shift, tiles, counts.get());
+      exclusive_scan_u32(counts.get(), counts.get(), 256 * tiles, s);
+    }
     PB_LAUNCH(radix_downsweep_kernel<K>, (unsigned)tiles, kRadixThreads, smem, s, kin, alt ? vals_alt : vals,
               alt ? vals2_alt : vals2, n, shift, tiles, counts.get(), kout, alt ? vals : vals_alt,
               alt ? vals2 : vals2_alt);

@@ -24,38 +24,40 @@ struct Lists {
   }
 };
 
-__global__ void degrees_kernel(Lists L, int64_t n, uint32_t* deg) {
-  for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x) {
-    uint32_t b, e; const uint32_t* a; int64_t sh;
-    L.get(x, b, e, a, sh);
-    deg[x] = e - b;
-  }
+__device__ __forceinline__ uint32_t degree_of(const Lists& L, int64_t x) {
+  uint32_t b, e; const uint32_t* a; int64_t sh;
+  L.get(x, b, e, a, sh);
+  return e - b;
 }
 
 // wedgeF (butterfly_utils.h:1061-1070): (v_deg * (v_deg - 1)) / 2 in 32-bit unsigned
 // arithmetic, summed per side in 64 bits (cmpWedgeCounts, :1080-1086).
-__global__ void side_wedges_kernel(const uint32_t* __restrict__ off, int64_t n, unsigned long long* acc) {
+// Both sides in one launch (blockIdx.y: 0 V, 1 U).
+__global__ void side_wedges_kernel(const uint32_t* __restrict__ offV, int64_t nv, const uint32_t* __restrict__ offU,
+                                   int64_t nu, unsigned long long* acc) {
+  const uint32_t* off = blockIdx.y ? offU : offV;
+  const int64_t n = blockIdx.y ? nu : nv;
   unsigned long long s = 0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     uint32_t d = off[i + 1] - off[i];
     s += (unsigned long long)((uint32_t)(d * (d - 1u)) / 2u);
   }
   s = warp_sum(s);
-  if ((threadIdx.x & 31) == 0 && s) atomicAdd(acc, s);
+  if ((threadIdx.x & 31) == 0 && s) atomicAdd(&acc[blockIdx.y], s);
 }
 
 // Sort key (ascending = earlier rank) for the degree-based orders.
-__global__ void order_keys_kernel(const uint32_t* __restrict__ deg, int64_t n, int64_t nv, int rank_type, int use_v,
-                                  uint32_t kmax, uint32_t* keys, uint32_t* ids) {
+__global__ void order_keys_kernel(Lists L, int64_t n, int rank_type, int use_v, uint32_t kmax, uint32_t* keys,
+                                  uint32_t* ids) {
   for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x) {
     uint32_t k;
     if (rank_type == PB_SIDE) {
-      bool on_count = use_v ? (x >= nv) : (x < nv);
+      bool on_count = use_v ? (x >= L.nv) : (x < L.nv);
       k = on_count ? 0u : 1u;
     } else if (rank_type == PB_DEG) {
-      k = kmax - deg[x];
+      k = kmax - degree_of(L, x);
     } else {  // PB_ADEG
-      k = kmax - log_key(deg[x]);
+      k = kmax - log_key(degree_of(L, x));
     }
     keys[x] = k;
     ids[x] = (uint32_t)x;
@@ -191,15 +193,14 @@ __global__ void cocore_keys_kernel(const uint32_t* __restrict__ key, int64_t n, 
   }
 }
 
-__global__ void invert_order_kernel(const uint32_t* __restrict__ order, int64_t n, uint32_t* rank) {
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x)
-    rank[order[r]] = (uint32_t)r;
-}
-
-__global__ void ranked_degrees_kernel(const uint32_t* __restrict__ order, const uint32_t* __restrict__ deg, int64_t n,
-                                      uint32_t* rdeg) {
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x)
-    rdeg[r] = deg[order[r]];
+// rank[order[r]] = r and the degrees in rank order.
+__global__ void invert_order_kernel(Lists L, const uint32_t* __restrict__ order, int64_t n, uint32_t* rank,
+                                    uint32_t* rdeg) {
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
+    const uint32_t x = order[r];
+    rank[x] = (uint32_t)r;
+    rdeg[r] = degree_of(L, x);
+  }
 }
 
 // Calls f(valid, slot, row) for every slot of [s0, s1) of a CSR (row: the slot's row), 32 slots of
@@ -309,7 +310,8 @@ __global__ void wedge_scan_kernel(const uint32_t* __restrict__ off, const uint32
           const uint32_t vb = off[v];
           L = lower_bound_u32(adj, vb, off[v + 1], i << 1) - vb;
         } else {
-          L = below[v];
+          const uint32_t vb = below ? 0u : off[v];
+          L = below ? below[v] : lower_bound_u32(adj, vb, off[v + 1], v << 1) - vb;
         }
         pref[j] = L;
       }
@@ -388,23 +390,26 @@ Lists lists_of(const pb_graph& g) {
   return Lists{g.offV.get(), g.edgV.get(), g.offU.get(), g.edgU.get(), g.nv};
 }
 
+// Wedge scan stage of R-MAT graphs with the below[] kernel against without: 2^14 slots 39 / 35 us,
+// 2^18 54 / 50, 2^20 78 / 77, 2^21 85 / 93.
+constexpr int64_t kSmallSlots = int64_t(1) << 18;
+
 uint32_t slot_chunk(int64_t m2) { return m2 <= (int64_t)sm_count() * 64 * 32 ? 32u : kSlotChunk; }
 
 int grid_for(int64_t n, int per_block = 256) { return std::max(1, std::min(ceil_div(n, per_block), sm_count() * 16)); }
 
 }  // namespace
 
-void degrees_combined(const pb_graph& g, uint32_t* deg, cudaStream_t s) {
-  const int64_t n = g.nv + g.nu;
-  if (n == 0) return;
-  PB_LAUNCH(degrees_kernel, grid_for(n), 256, 0, s, lists_of(g), n, deg);
+void side_wedge_sums(const pb_graph& g, unsigned long long* sums, cudaStream_t s) {
+  PB_CUDA_TRY(cudaMemsetAsync(sums, 0, 2 * sizeof(unsigned long long), s));
+  if (g.nv + g.nu)
+    PB_LAUNCH(side_wedges_kernel, dim3(grid_for(std::max(g.nv, g.nu)), 2), 256, 0, s, g.offV.get(), g.nv, g.offU.get(), g.nu,
+              sums);
 }
 
 void cmp_wedge_counts(const pb_graph& g, int* use_v, int64_t* w_min, int64_t* wv, int64_t* wu, cudaStream_t s) {
   DevBuf<unsigned long long> acc(2, s);
-  PB_CUDA_TRY(cudaMemsetAsync(acc.get(), 0, 2 * sizeof(unsigned long long), s));
-  if (g.nv) PB_LAUNCH(side_wedges_kernel, grid_for(g.nv), 256, 0, s, g.offV.get(), g.nv, acc.get());
-  if (g.nu) PB_LAUNCH(side_wedges_kernel, grid_for(g.nu), 256, 0, s, g.offU.get(), g.nu, acc.get() + 1);
+  side_wedge_sums(g, acc.get(), s);
   unsigned long long h[2];
   readback(h, acc.get(), sizeof(h), s);
   *wv = (int64_t)h[0];
@@ -420,8 +425,7 @@ void vertex_order(const pb_graph& g, int rank_type, int use_v, Ranked& R, cudaSt
   R.order.alloc(n, s);
   R.rank.alloc(n, s);
   if (n == 0) return;
-  DevBuf<uint32_t> deg(n, s), keys(n, s), keys2(n, s), ids2(n, s);
-  degrees_combined(g, deg.get(), s);
+  DevBuf<uint32_t> keys(n, s), keys2(n, s), ids2(n, s);
   uint32_t kmax = 0;
   int nbits = 0;
   uint32_t* ids = R.order.get();
@@ -448,13 +452,14 @@ void vertex_order(const pb_graph& g, int rank_type, int use_v, Ranked& R, cudaSt
     if (rank_type == PB_DEG) kmax = g.max_deg;
     else if (rank_type == PB_ADEG) kmax = g.max_deg ? 32u - (uint32_t)__builtin_clz(g.max_deg) : 0u;
     else kmax = 1;
-    PB_LAUNCH(order_keys_kernel, grid_for(n), 256, 0, s, deg.get(), n, g.nv, rank_type, use_v, kmax, keys.get(), ids);
+    PB_LAUNCH(order_keys_kernel, grid_for(n), 256, 0, s, lists_of(g), n, rank_type, use_v, kmax, keys.get(), ids);
     nbits = bits_for(kmax);
   }
   // Stable sort by key: ties keep combined-id order.
   bool alt = radix_sort_pairs_u32(keys.get(), ids, keys2.get(), ids2.get(), n, 0, nbits, s);
-  if (alt) PB_CUDA_TRY(cudaMemcpyAsync(ids, ids2.get(), sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s));
-  PB_LAUNCH(invert_order_kernel, grid_for(n), 256, 0, s, R.order.get(), n, R.rank.get());
+  if (alt) std::swap(R.order.p, ids2.p);
+  R.rdeg.alloc(n, s);
+  PB_LAUNCH(invert_order_kernel, grid_for(n), 256, 0, s, lists_of(g), R.order.get(), n, R.rank.get(), R.rdeg.get());
 }
 
 void build_ranked_csr(const pb_graph& g, Ranked& R, bool with_eout, cudaStream_t s) {
@@ -470,12 +475,8 @@ void build_ranked_csr(const pb_graph& g, Ranked& R, bool with_eout, cudaStream_t
     PB_CUDA_TRY(cudaMemsetAsync(R.off.get(), 0, sizeof(uint32_t), s));
     return;
   }
-  {
-    DevBuf<uint32_t> deg(n, s), rdeg(n, s);
-    degrees_combined(g, deg.get(), s);
-    PB_LAUNCH(ranked_degrees_kernel, grid_for(n), 256, 0, s, R.order.get(), deg.get(), n, rdeg.get());
-    exclusive_scan_u32(rdeg.get(), R.off.get(), n, s);
-  }
+  exclusive_scan_u32(R.rdeg.get(), R.off.get(), n, s);
+  R.rdeg.release();
   if (R.m2 == 0) return;
   const uint32_t chunk = slot_chunk(R.m2);
   const int grid = grid_for((R.m2 + chunk - 1) / chunk * 32);
@@ -506,10 +507,15 @@ void wedge_scan(Ranked& R, cudaStream_t s) {
     R.w_rank = 0;
     return;
   }
-  DevBuf<uint32_t> below(n, s);
+  // Small graphs look below[v] up slot by slot: the second search costs less than a launch.
+  const bool with_below = R.m2 > kSmallSlots;
+  DevBuf<uint32_t> below;
   DevBuf<int64_t> wc(n, s);
   PB_CUDA_TRY(cudaMemsetAsync(wc.get(), 0, wc.bytes(), s));
-  PB_LAUNCH(below_self_kernel, grid_for(n), 256, 0, s, R.off.get(), R.adj.get(), n, below.get());
+  if (with_below) {
+    below.alloc(n, s);
+    PB_LAUNCH(below_self_kernel, grid_for(n), 256, 0, s, R.off.get(), R.adj.get(), n, below.get());
+  }
   const uint32_t chunk = slot_chunk(R.m2);
   if (R.m2 > 0)
     PB_LAUNCH(wedge_scan_kernel, grid_for((R.m2 + chunk - 1) / chunk * 32), 256, 0, s, R.off.get(), R.adj.get(),

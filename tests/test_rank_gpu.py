@@ -25,6 +25,9 @@ GRAPHS = {
     "slots_below": lambda: BipartiteGraph.uniform(9_000, 7_000, (1 << 18) - 1, 31),
     "slots_at": lambda: BipartiteGraph.rmat(14, 12, 1 << 18, 0.55, 0.15, 0.15, 0.15, 32),
     "slots_above": lambda: BipartiteGraph.powerlaw_u(5_000, 30_000, (1 << 18) + 1, 2.0, 5_000, 33),
+    "one_tile": lambda: BipartiteGraph.uniform(2_000, 2_096, 9_000, 35),    # 4096 vertices: one radix tile
+    "two_tiles": lambda: BipartiteGraph.uniform(2_000, 2_097, 9_000, 36),
+    "search_below": lambda: BipartiteGraph.uniform(3_000, 2_000, (1 << 17) + 1, 37),  # 2^18 + 2 slots
     "hubs": _hubs,
     "sparse": lambda: BipartiteGraph.uniform(200_000, 150_000, 3_000, 34),
     "one_row": lambda: BipartiteGraph.from_edges(3, 700, np.r_[np.zeros(700, int), 1, 1], np.r_[np.arange(700), 0, 699]),
