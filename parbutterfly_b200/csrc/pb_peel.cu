@@ -112,7 +112,8 @@ struct Ctl {
   // probes that walked the probe set against a binary search (the reverse direction).
   unsigned long long mode_items[3], mode_work[3], rev_work;
 };
-constexpr unsigned kMaxGroups = 32;
+constexpr unsigned kMaxGroups = 128;  // heavy tip items of one wave
+constexpr unsigned kFlatAll = 32;     // rounds of at most this many CTA-level tip items run as one wave
 // Pairs per CTA below which tip_items_flat uses fewer CTAs.
 constexpr unsigned long long kFlatPairs = 1024;
 // Device memory for grid-shared dense counters (one n-sized slice per concurrent heavy tip
@@ -331,9 +332,11 @@ struct Shared {
   uint32_t sb[kPT];
   uint32_t len[kPT];
   uint32_t acc[kPT];  // butterflies found through each first-level position of the chunk
-  uint4 flat[32];     // tip_items_flat: the items of the wave
+  uint4 flat[kMaxGroups];  // tip_items_flat: the items of the wave
+  unsigned long long flat_end[kMaxGroups];
   uint32_t scan[32];
   uint32_t item;
+  uint32_t flat_steps, flat_item;  // tip_items_flat: steps of this CTA's slice, item of a one-step slice
   unsigned hist[66];
 };
 
@@ -368,6 +371,64 @@ struct WarpQueue {
     __syncwarp();
   }
 };
+
+// Position of this lane's entry in a list of *len entries that the lanes with `have` append to: one
+// add per warp (all lanes call it).
+template <class T>
+__device__ __forceinline__ T warp_append(T* len, bool have) {
+  const unsigned bal = __ballot_sync(0xffffffffu, have);
+  T base = 0;
+  if (bal && lane_id() == (unsigned)(__ffs(bal) - 1)) base = atomicAdd(len, (T)__popc(bal));
+  base = __shfl_sync(0xffffffffu, base, bal ? __ffs(bal) - 1 : 0);
+  return base + (T)__popc(bal & ((1u << lane_id()) - 1u));
+}
+
+// bins[bin] += w (bin < 0: nothing), equal bins of a warp in one shared-memory add: neighbouring
+// items lie in few bins, and 64-bit shared-memory adds to one address are served one by one.
+__device__ __forceinline__ void warp_bin_add(unsigned long long* bins, int bin, uint32_t w) {
+  const unsigned peers = __match_any_sync(0xffffffffu, bin);
+  const uint32_t lo = __reduce_add_sync(peers, w & 0xFFFFu), hi = __reduce_add_sync(peers, w >> 16);
+  if (bin >= 0 && lane_id() == (unsigned)(__ffs(peers) - 1))
+    atomicAdd(&bins[bin], ((unsigned long long)hi << 16) + lo);
+}
+
+// The first of `nbins` control-block bins whose running sum (from `cum` on) reaches target, nbins when
+// none does, for the whole CTA; cum becomes the sum of the bins before it.  One warp loads the bins
+// together: walked one by one, every bin is a round trip (84 us of an advance).
+__shared__ unsigned s_bin;
+__shared__ unsigned long long s_cum;
+template <class T>
+__device__ __forceinline__ unsigned find_bin(const T* bins, unsigned nbins, unsigned long long target,
+                                             unsigned long long& cum) {
+  if (threadIdx.x < 32) {
+    const unsigned per = (nbins + 31) / 32, b0 = threadIdx.x * per;
+    T v[8];
+    unsigned long long sum = 0;
+#pragma unroll
+    for (unsigned i = 0; i < 8; ++i) {
+      v[i] = i < per && b0 + i < nbins ? *(const volatile T*)&bins[b0 + i] : T(0);
+      sum += v[i];
+    }
+    const unsigned long long incl = warp_inclusive_scan(sum) + cum;
+    const unsigned reach = __ballot_sync(0xffffffffu, incl >= target);
+    if (reach ? threadIdx.x == (unsigned)(__ffs(reach) - 1) : threadIdx.x == 31) {
+      unsigned long long run = incl - sum;
+      unsigned b = nbins;
+#pragma unroll
+      for (unsigned i = 0; i < 8; ++i) {
+        if (b == nbins && i < per && b0 + i < nbins) {
+          if (run + v[i] >= target) b = b0 + i;
+          else run += v[i];
+        }
+      }
+      s_bin = b;
+      s_cum = run;
+    }
+  }
+  __syncthreads();
+  cum = s_cum;
+  return s_bin;
+}
 
 // Flattened two-level iteration by one warp: first(j, L, sb) gives the second-level range
 // [sb, sb + L) of first-level position j in [b, e) (all lanes call it; valid: j < e); f(valid, lo,
@@ -618,28 +679,45 @@ __device__ void tip_item_block(const Lists& G, const Work& W, Ctl* ctl, uint32_t
 // CTA-level ones read back from `big`): their flattened two-hop lists are cut into equal slices
 // over the instance's CTAs.  Every wedge adds one to the item's grid-shared dense counter of u2;
 // the add that returns j removes j butterflies from u2 at once (0 + 1 + ... + (w - 1) = C(w, 2)),
-// so one pass and no barrier is needed.  clear: the same walk resets the counters (after a
-// barrier), on the CTAs from the other end of the grid: those at this end scan the near list.
+// so one pass and no barrier is needed.  clear: every CTA resets the counters of its slice (after a
+// barrier): a slice of one step is remembered in `kept` (4 entries per thread of shared memory, so
+// clearing costs no loads: light rounds wait for it), a longer one is walked again.
 __device__ void tip_items_flat(const Lists& G, const Work& W, Ctl* ctl, const uint4* huge, unsigned nh, const uint4* big,
-                               unsigned n, bool clear, Shared& S, Acc& A) {
-  if (threadIdx.x < 32) {
-    unsigned long long t = 0;
-    uint4 d = make_uint4(0, 0, 0, 0);
-    if (threadIdx.x < n) {
-      d = threadIdx.x < nh ? huge[threadIdx.x] : big[-(int)(threadIdx.x - nh)];
-      t = d.w == 0xFFFFFFFFu ? (unsigned long long)G.wk[d.x] + d.z : d.w;
+                               unsigned n, bool clear, Shared& S, uint32_t* kept, Acc& A) {
+  if (clear && S.flat_steps <= 1) {  // uniform across the CTA; set by the walk
+    if (S.flat_steps == 1) {
+      uint32_t* cnt = W.gshared + (size_t)S.flat_item * (size_t)W.gshared_stride;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const uint32_t x = kept[r * kPT + threadIdx.x];
+        if (x != kEmpty) cnt[x] = 0u;
+      }
     }
-    S.flat[threadIdx.x] = d;
-    S.red[threadIdx.x] = warp_inclusive_scan(t);
+    return;
+  }
+  if (threadIdx.x < 32) {
+    unsigned long long carry = 0;
+    for (unsigned i0 = 0; i0 < n; i0 += 32) {
+      const unsigned i = i0 + threadIdx.x;
+      unsigned long long t = 0;
+      if (i < n) {
+        const uint4 d = i < nh ? huge[i] : big[-(int)(i - nh)];
+        t = d.w == 0xFFFFFFFFu ? (unsigned long long)G.wk[d.x] + d.z : d.w;
+        S.flat[i] = d;
+      }
+      t = warp_inclusive_scan(t) + carry;
+      if (i < n) S.flat_end[i] = t;
+      carry = __shfl_sync(0xffffffffu, t, 31);
+    }
   }
   __syncthreads();
-  const unsigned long long T = S.red[31];
+  unsigned steps = 0;
+  const unsigned long long T = S.flat_end[n - 1];
   const unsigned nuse = (unsigned)min((unsigned long long)vgrid(), T / kFlatPairs + 1ull);
-  const unsigned vb = clear ? vgrid() - 1u - vblock() : vblock();
-  if (T && vb < nuse) {
-    const unsigned long long lo = T * vb / nuse, hi = T * (vb + 1) / nuse;
+  if (T && vblock() < nuse) {
+    const unsigned long long lo = T * vblock() / nuse, hi = T * (vblock() + 1) / nuse;
     for (unsigned i = 0; i < n; ++i) {
-      const unsigned long long tb = i ? S.red[i - 1] : 0ull, te = S.red[i];
+      const unsigned long long tb = i ? S.flat_end[i - 1] : 0ull, te = S.flat_end[i];
       if (te <= lo || tb >= hi) continue;  // uniform across the CTA
       const uint32_t u = S.flat[i].x, b = S.flat[i].y;
       uint32_t* cnt = W.gshared + (size_t)i * (size_t)W.gshared_stride;
@@ -651,6 +729,12 @@ __device__ void tip_items_flat(const Lists& G, const Work& W, Ctl* ctl, const ui
                              if (x[r] != kEmpty) cnt[x[r]] = 0u;
                            return;
                          }
+                         if (steps == 0) {
+#pragma unroll
+                           for (int r = 0; r < 4; ++r) kept[r * kPT + threadIdx.x] = x[r];
+                           if (threadIdx.x == 0) S.flat_item = i;
+                         }
+                         ++steps;
                          uint32_t j[4];
                          uint8_t st[4];
 #pragma unroll
@@ -668,8 +752,11 @@ __device__ void tip_items_flat(const Lists& G, const Work& W, Ctl* ctl, const ui
                        });
     }
   }
-  if (!clear && vblock() == 0 && threadIdx.x == 0) A.work += T;
-  __syncthreads();  // S.red is reused
+  if (!clear && threadIdx.x == 0) {
+    S.flat_steps = steps;
+    if (vblock() == 0) A.work += T;
+  }
+  __syncthreads();
 }
 
 // ---- wing: process one frontier edge --------------------------------------------------------
@@ -976,6 +1063,7 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
   Shared& S = *reinterpret_cast<Shared*>(smem_raw);
   uint32_t* pool = reinterpret_cast<uint32_t*>(smem_raw + ((sizeof(Shared) + 15) & ~size_t(15)));
   const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint32_t* kept = pool + kPoolWords - 4 * kPT;  // beyond the tip tables and the advance's bins
   uint32_t* wkeys = pool + warp * (kWing ? 3 * kWingWarpSlots : 2 * kTipWarpSlots);
   const unsigned gtid = vblock() * kPT + threadIdx.x;
   const unsigned gthreads = vgrid() * kPT;
@@ -987,6 +1075,7 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
     s_bar_timeout = ctl->barrier_timeout_ns;
     s_skip_arrival = vblock() == 0 ? ctl->test_skip_arrival : 0u;
     s_err = 0;
+    S.flat_steps = 0;
   }
   unsigned alist_cur = *(volatile unsigned*)&ctl->alist_cur;
   const bool range = *(volatile unsigned*)&ctl->range_mode != 0;
@@ -1029,7 +1118,7 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
     if (alive == 0 || pause) {
       if (!kWing && clear_n) {
         Acc none{kInf, 0};
-        tip_items_flat(G, W, ctl, W.fhuge[npar], clear_nh, W.front[npar] + (W.N - 1), clear_n, true, S, none);
+        tip_items_flat(G, W, ctl, W.fhuge[npar], clear_nh, W.front[npar] + (W.N - 1), clear_n, true, S, kept, none);
       }
       if (cta0 && threadIdx.x == 0) {
         ctl->round = r;
@@ -1051,14 +1140,18 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
       const unsigned na = alist_cur ^ 1u;
       const unsigned alen = *(volatile unsigned*)&ctl->alen[alist_cur];
       unsigned long long mn = kInf;
-      for (unsigned q = gtid; q < alen; q += gthreads) {
-        const uint32_t x = W.alist[alist_cur][q];
-        if (W.state[x] != ALIVE) continue;
-        W.alist[na][atomicAdd(&ctl->alen[na], 1u)] = x;
+      for (unsigned q0 = gtid - lane; q0 < alen; q0 += gthreads) {  // whole warps: one add per warp
+        const unsigned q = q0 + lane;
+        const uint32_t x = q < alen ? W.alist[alist_cur][q] : kEmpty;
+        const bool live = x != kEmpty && W.state[x] == ALIVE;
+        const unsigned at = warp_append(&ctl->alen[na], live);
+        if (!live) continue;
+        W.alist[na][at] = x;
         const int64_t c = W.cnt[x];
         if (range) W.D[x] = c;
         mn = min(mn, (unsigned long long)c);
       }
+      __syncwarp();
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
       if (lane == 0 && mn != kInf) atomicMin(&ctl->k_lo, mn);
@@ -1097,12 +1190,8 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
         if (!grid_barrier(ctl)) return false;
         // Every CTA derives the same bound: the smallest B with >= target items at distance < 2^B.
         const unsigned target = max(near_min, alen2 / near_div);
-        unsigned cum = 0;
-        int B = 0;
-        for (; B < 65; ++B) {
-          cum += *(volatile unsigned*)&ctl->hist[B];
-          if (cum >= target) break;
-        }
+        unsigned long long cum = 0;
+        const int B = (int)find_bin(ctl->hist, 65, target, cum);
         if (B < 63) {
           const unsigned long long span = 1ull << B;
           if (klo <= kInf - span) hi = klo + span;
@@ -1114,10 +1203,17 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
         unsigned long long* wh = reinterpret_cast<unsigned long long*>(pool);
         if (threadIdx.x < 66) wh[threadIdx.x] = 0;
         __syncthreads();
-        for (unsigned q = gtid; q < alen2; q += gthreads) {
-          const uint32_t x = W.alist[na][q];
-          const unsigned long long d = (unsigned long long)W.cnt[x] - klo;
-          atomicAdd(&wh[d ? 64 - __clzll(d) : 0], (unsigned long long)W.wgt[x]);
+        for (unsigned q0 = gtid - lane; q0 < alen2; q0 += gthreads) {
+          const unsigned q = q0 + lane;
+          int bin = -1;
+          uint32_t w = 0;
+          if (q < alen2) {
+            const uint32_t x = W.alist[na][q];
+            const unsigned long long d = (unsigned long long)W.cnt[x] - klo;
+            bin = d ? 64 - __clzll(d) : 0;
+            w = W.wgt[x];
+          }
+          warp_bin_add(wh, bin, w);
         }
         __syncthreads();
         if (threadIdx.x < 66 && wh[threadIdx.x]) atomicAdd(&ctl->whist[threadIdx.x], wh[threadIdx.x]);
@@ -1134,12 +1230,7 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
         part_target_next = target;
         part_ratio_next = ratio_q;
         unsigned long long cum = 0;
-        int B = 0;
-        for (; B < 65; ++B) {
-          const unsigned long long w = *(volatile unsigned long long*)&ctl->whist[B];
-          if (cum + w >= target) break;
-          cum += w;
-        }
+        const int B = (int)find_bin(ctl->whist, 65, target, cum);
         if (B == 0) {
           hi = klo + 1;
         } else if (B < 63) {
@@ -1147,28 +1238,35 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
           __syncthreads();
           if (threadIdx.x < 256) wh[threadIdx.x] = 0;
           __syncthreads();
-          for (unsigned q = gtid; q < alen2; q += gthreads) {
-            const uint32_t x = W.alist[na][q];
-            const unsigned long long d = (unsigned long long)W.cnt[x] - klo;
-            if (d >= lo_d && d < lo_d + width)
-              atomicAdd(&wh[(unsigned)((d - lo_d) * 256ull / width)], (unsigned long long)W.wgt[x]);
+          for (unsigned q0 = gtid - lane; q0 < alen2; q0 += gthreads) {
+            const unsigned q = q0 + lane;
+            int bin = -1;
+            uint32_t w = 0;
+            if (q < alen2) {
+              const uint32_t x = W.alist[na][q];
+              const unsigned long long d = (unsigned long long)W.cnt[x] - klo;
+              if (d >= lo_d && d < lo_d + width) {
+                bin = (int)((d - lo_d) * 256ull / width);
+                w = W.wgt[x];
+              }
+            }
+            warp_bin_add(wh, bin, w);
           }
           __syncthreads();
           if (threadIdx.x < 256 && wh[threadIdx.x]) atomicAdd(&ctl->wsub[threadIdx.x], wh[threadIdx.x]);
           if (!grid_barrier(ctl)) return false;
-          unsigned j = 0;
-          for (; j < 255; ++j) {
-            cum += *(volatile unsigned long long*)&ctl->wsub[j];
-            if (cum >= target) break;
-          }
+          const unsigned j = find_bin(ctl->wsub, 255, target, cum);
           // Bin j covers distances [lo_d + ceil(j w / 256), lo_d + ceil((j + 1) w / 256)).
           const unsigned long long end_d = lo_d + ((unsigned long long)(j + 1) * width + 255ull) / 256ull;
           if (klo <= kInf - end_d) hi = klo + end_d;
         }
       }
-      for (unsigned q = gtid; q < alen2; q += gthreads) {
-        const uint32_t x = W.alist[na][q];
-        if (hi == kInf || (unsigned long long)W.cnt[x] < hi) W.near[atomicAdd(&ctl->near_len, 1ull)] = x;
+      for (unsigned q0 = gtid - lane; q0 < alen2; q0 += gthreads) {
+        const unsigned q = q0 + lane;
+        const uint32_t x = q < alen2 ? W.alist[na][q] : kEmpty;
+        const bool in = x != kEmpty && (hi == kInf || (unsigned long long)W.cnt[x] < hi);
+        const unsigned at = (unsigned)warp_append(&ctl->near_len, in);
+        if (in) W.near[at] = x;
       }
       if (cta0 && threadIdx.x == 0) {
         ctl->win_hi = hi;
@@ -1278,7 +1376,7 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
       }
       if (!kWing && clear_n) {
         Acc none{kInf, 0};
-        tip_items_flat(G, W, ctl, W.fhuge[npar], clear_nh, W.front[npar] + (W.N - 1), clear_n, true, S, none);
+        tip_items_flat(G, W, ctl, W.fhuge[npar], clear_nh, W.front[npar] + (W.N - 1), clear_n, true, S, kept, none);
         clear_n = 0;
       }
       if (cta0 && threadIdx.x == 0) s_st.scanned += nl - near_done;
@@ -1353,7 +1451,7 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
       // CTA per item leaves the rest of the grid idle: rounds of 2^12 wedges took 40 us in phase
       // P on one CTA each, 24 us spread over the grid).
       const unsigned ng = kWing ? 0u : (W.gshared ? min(W.ngroups, kMaxGroups) : 0u);
-      const bool flat_all = !kWing && vgrid() >= 8 && nb + nh > 0 && nb + nh <= ng;
+      const bool flat_all = !kWing && vgrid() >= 8 && nb + nh > 0 && nb + nh <= min(ng, kFlatAll);
       if (nu && !flat_all) {
         const uint4* const fbg = W.front[par] + (W.N - 1);  // item q: fbg[-q]
         if (kWing && nb <= kOneSlice && 2 * nb <= vgrid()) {
@@ -1426,10 +1524,10 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
           const unsigned n = min(ng, total - w0);
           const unsigned in_huge = nh > w0 ? min(n, nh - w0) : 0u;
           const uint4* hl = W.fhuge[par] + w0;
-          tip_items_flat(G, W, ctl, hl, in_huge, W.front[par] + (W.N - 1), n, false, S, A);
+          tip_items_flat(G, W, ctl, hl, in_huge, W.front[par] + (W.N - 1), n, false, S, kept, A);
           if (w0 + ng < total) {  // the slices are reused by the next wave
             if (!grid_barrier(ctl)) return false;
-            tip_items_flat(G, W, ctl, hl, in_huge, W.front[par] + (W.N - 1), n, true, S, A);
+            tip_items_flat(G, W, ctl, hl, in_huge, W.front[par] + (W.N - 1), n, true, S, kept, A);
             if (!grid_barrier(ctl)) return false;
           } else {
             clear_n = n;
@@ -1441,7 +1539,7 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
         if (total > ng) {
           const unsigned w0 = (total - 1) / ng * ng;
           if (!grid_barrier(ctl)) return false;
-          tip_items_flat(G, W, ctl, W.fhuge[par] + w0, clear_nh, W.front[par] + (W.N - 1), clear_n, true, S, A);
+          tip_items_flat(G, W, ctl, W.fhuge[par] + w0, clear_nh, W.front[par] + (W.N - 1), clear_n, true, S, kept, A);
           clear_n = 0;
         }
       }
@@ -1968,9 +2066,20 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
   if (const char* e = getenv("PB_PEEL_CTAS")) cap = atoll(e);  // diagnostic hook
   if (cap > 0) grid = (int)std::max<int64_t>(1, std::min<int64_t>(grid, cap));
 
+  // The fine pass of a two-phase tip peel runs many small instances: two CTAs per SM give each of
+  // them a CTA of its own (R-MAT 2^22 edges, 296 partitions asked for: 64.2 ms against 66.3).
+  auto fine_kern = kern;
+  int fine_grid = grid;
+  if (!kWing && two_phase && cap <= 0) {
+    fine_kern = peel_kernel<kWing, 2>;
+    PB_CUDA_TRY(cudaFuncSetAttribute(fine_kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fine_kern, kPT, smem));
+    fine_grid = sm_count() * std::max(1, per_sm);
+  }
+
   DevBuf<uint32_t> gscratch;
   if (need_scratch) {
-    gscratch.alloc((size_t)grid * (size_t)scratch_len, s);
+    gscratch.alloc((size_t)std::max(grid, fine_grid) * (size_t)scratch_len, s);
     PB_CUDA_TRY(cudaMemsetAsync(gscratch.get(), 0, gscratch.bytes(), s));
   }
   Work W{};
@@ -2034,10 +2143,12 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
   auto launch_instances = [&](const std::vector<Work>& wproto, const std::vector<Ctl>& cproto,
                               const std::vector<double>& weights, const Lists* levels_dev,
                               const std::function<void(Work&, uint32_t)>& per_slot,
-                              std::vector<Ctl>* inst_out = nullptr) {
+                              std::vector<Ctl>* inst_out = nullptr, bool fine = false) {
+    const auto lkern = fine ? fine_kern : kern;
+    const int lgrid = fine ? fine_grid : grid;
     std::vector<int> inst_of;
     std::vector<uint32_t> first, ncta, cbeg, cend;
-    assign_ctas(weights, grid, inst_of, first, ncta, cbeg, cend);
+    assign_ctas(weights, lgrid, inst_of, first, ncta, cbeg, cend);
     const int n_slots = (int)inst_of.size();
     std::vector<Work> ws(n_slots);
     std::vector<Ctl> hctls(n_slots);
@@ -2048,7 +2159,7 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
     }
     DevBuf<Ctl> ctls(n_slots, s);
     DevBuf<Work> dws(n_slots, s);
-    DevBuf<uint32_t> meta(2 * (size_t)n_slots + 2 * (size_t)grid, s);
+    DevBuf<uint32_t> meta(2 * (size_t)n_slots + 2 * (size_t)lgrid, s);
     std::vector<uint32_t> hmeta;
     hmeta.insert(hmeta.end(), first.begin(), first.end());
     hmeta.insert(hmeta.end(), ncta.begin(), ncta.end());
@@ -2072,12 +2183,12 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
     PB_CUDA_TRY(cudaMemcpyAsync(dws.get(), src_w, sizeof(Work) * n_slots, cudaMemcpyHostToDevice, s));
     PB_CUDA_TRY(cudaMemcpyAsync(meta.get(), src_m, sizeof(uint32_t) * hmeta.size(), cudaMemcpyHostToDevice, s));
     Instances I{dws.get(), meta.get(), meta.get() + n_slots, meta.get() + 2 * n_slots,
-                meta.get() + 2 * n_slots + grid, (uint32_t)n_slots};
+                meta.get() + 2 * n_slots + lgrid, (uint32_t)n_slots};
     Ctl* cp = ctls.get();
     Lists Gk = G0;
     const Lists* lv = levels_dev;
     void* args[] = {&Gk, &lv, &I, &cp, &cls};
-    PB_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3(kPT), args, smem, s));
+    PB_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)lkern, dim3(lgrid), dim3(kPT), args, smem, s));
     if (g_launch_counter) ++*g_launch_counter;
     PB_LAUNCH(ctl_status_kernel, 1, 32, 0, s, cp, (unsigned)n_slots, status.get());
     if (capturing()) {
@@ -2443,7 +2554,7 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
       x.gshared = gsl.back()->get();
     }
   };
-  launch_instances(ws, cs, weights, dlevels.get(), per_slot);
+  launch_instances(ws, cs, weights, dlevels.get(), per_slot, nullptr, true);
   res.work += coarse_work;
   res.parts = (int64_t)ws.size();
   if (trace)
