@@ -51,6 +51,7 @@ constexpr int kPW = kPT / 32;
 constexpr uint32_t kPoolWords = 21504;
 constexpr uint32_t kWingSlots = kPoolWords / 3;            // 7168 slots, probe sets up to kWingSet
 constexpr uint32_t kWingSet = 4096;
+constexpr uint32_t kWingLoad = 4;  // slots per probe-set entry, while they fit
 constexpr uint32_t kWingWarpSlots = kPoolWords / 3 / kPW;  // 448 slots, probe sets up to kWingWarpSet
 constexpr uint32_t kWingWarpSet = 256;
 constexpr uint32_t kTipSlots = 8192;      // two-hop lists of up to 4096 wedges
@@ -188,7 +189,7 @@ __shared__ unsigned long long s_win_hi;
 __shared__ long long s_k;
 __shared__ unsigned s_act;  // state mark of this round's frontier
 __shared__ unsigned long long s_bar_target, s_bar_timeout;
-__shared__ unsigned s_err, s_skip_arrival;
+__shared__ unsigned s_err, s_skip_arrival, s_trace;
 
 // Statistics of CTA 0 (phase times, round counts) and of every CTA (wing probes), written to the
 // control block when the instance ends or pauses.
@@ -310,6 +311,17 @@ __device__ __forceinline__ void t_put(uint32_t* keys, uint32_t* vals, uint32_t s
   raise_err(ctl, ERR_TABLE);
 }
 
+// The same from slot h on, which neither matched nor was empty.
+__device__ __forceinline__ uint32_t t_slot_next(const uint32_t* keys, uint32_t size, uint32_t key, uint32_t h) {
+  for (uint32_t probes = 1; probes < size; ++probes) {
+    h = h + 1 == size ? 0u : h + 1;
+    const uint32_t k = keys[h];
+    if (k == key) return h;
+    if (k == kEmpty) return kEmpty;
+  }
+  return kEmpty;
+}
+
 // Slot of key, or kEmpty when absent.
 __device__ __forceinline__ uint32_t t_slot(const uint32_t* keys, uint32_t size, uint32_t key) {
   uint32_t h = hslot(key, size);
@@ -336,6 +348,7 @@ struct Shared {
   unsigned long long flat_end[kMaxGroups];
   uint32_t scan[32];
   uint32_t item;
+  uint32_t list_steps[kPW], list_item[kPW];  // tip_items_lists: the same per warp
   uint32_t flat_steps, flat_item;  // tip_items_flat: steps of this CTA's slice, item of a one-step slice
   unsigned hist[66];
 };
@@ -470,33 +483,55 @@ __device__ __forceinline__ void warp_iter(uint32_t b, uint32_t e, const uint32_t
   }
 }
 
+// Inclusive scan over the CTA; smem (32 words) may be used again after the caller's next barrier.
 __device__ __forceinline__ uint32_t block_incl_scan(uint32_t x, uint32_t* smem, uint32_t& total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  uint32_t incl = warp_inclusive_scan(x);
+  const uint32_t incl = warp_inclusive_scan(x);
   if (lane == 31) smem[warp] = incl;
   __syncthreads();
-  if (warp == 0) {
-    uint32_t v = lane < nwarps ? smem[lane] : 0u;
-    v = warp_inclusive_scan(v);
-    smem[lane] = v;
-  }
-  __syncthreads();
-  incl += warp > 0 ? smem[warp - 1] : 0u;
-  total = smem[nwarps - 1];
-  __syncthreads();
-  return incl;
+  const uint32_t v = warp_inclusive_scan(lane < nwarps ? smem[lane] : 0u);  // by every warp
+  total = __shfl_sync(0xffffffffu, v, nwarps - 1);
+  const uint32_t before = __shfl_sync(0xffffffffu, v, warp > 0 ? warp - 1 : 0);
+  return incl + (warp > 0 ? before : 0u);
 }
 
 // The same iteration by the whole CTA.  Each chunk of kPT first-level positions has its
 // second-level ranges cut into pieces of at most kPiece entries; pieces go to the warps in turn
-// (they are of one size, so no counter is needed), a warp locates a piece's position once (binary
-// search over the chunk's inclusive piece counts) and walks it with 32 lanes, so consecutive lanes
-// read consecutive entries.
+// (they are of one size, so no counter is needed), a warp locates a piece's position once (two
+// ballots over the chunk's inclusive piece counts) and walks it with 32 lanes, so consecutive lanes
+// read consecutive entries.  piece(lo, k, q, n, x): a piece of position j0 + lo; this lane holds its
+// entries k, k + 32, ... below n, at list positions q, q + 32, ..., with values x[0 .. 3] (kEmpty
+// beyond the end).
 constexpr uint32_t kPiece = 128;
 
-template <class First, class F, class Done>
-__device__ __forceinline__ void block_iter(uint32_t b, uint32_t e, Shared& S, const uint32_t* __restrict__ arr,
-                                           First&& first, F&& f, Done&& done) {
+// One warp's part of the pieces of up to 32 positions (lens / starts in shared memory): every warp
+// scans the piece counts by itself, so no barrier is needed.
+template <class Piece>
+__device__ __forceinline__ void few_pieces(uint32_t n, const uint32_t* lens, const uint32_t* starts,
+                                           const uint32_t* __restrict__ arr, Piece&& piece) {
+  const uint32_t lane = lane_id();
+  const uint32_t len = lane < n ? lens[lane] : 0u, beg = lane < n ? starts[lane] : 0u;
+  const uint32_t incl = warp_inclusive_scan((len + kPiece - 1) / kPiece);
+  const uint32_t T = __shfl_sync(0xffffffffu, incl, 31);
+  for (uint32_t p = threadIdx.x >> 5; p < T; p += kPW) {
+    const uint32_t lo = (uint32_t)__ffs(__ballot_sync(0xffffffffu, incl > p)) - 1u;
+    const uint32_t before = __shfl_sync(0xffffffffu, incl, lo > 0 ? lo - 1 : 0);
+    const uint32_t k0 = (p - (lo > 0 ? before : 0u)) * kPiece;
+    const uint32_t kend = min(k0 + kPiece, __shfl_sync(0xffffffffu, len, lo));
+    const uint32_t sbj = __shfl_sync(0xffffffffu, beg, lo), base = sbj & ~kRevFlag;
+    uint32_t x[kPiece / 32];
+#pragma unroll
+    for (uint32_t r = 0; r < kPiece / 32; ++r) {
+      const uint32_t k = k0 + lane + 32 * r;
+      x[r] = k < kend ? arr[base + k] : kEmpty;
+    }
+    piece(lo, k0 + lane, sbj + k0 + lane, kend, x);
+  }
+}
+
+template <class First, class Piece, class Done>
+__device__ __forceinline__ void block_pieces(uint32_t b, uint32_t e, Shared& S, const uint32_t* __restrict__ arr,
+                                             First&& first, Piece&& piece, Done&& done) {
   const uint32_t tid = threadIdx.x, lane = tid & 31u;
   for (uint32_t j0 = b; j0 < e; j0 += kPT) {
     const uint32_t j = j0 + tid;
@@ -509,10 +544,11 @@ __device__ __forceinline__ void block_iter(uint32_t b, uint32_t e, Shared& S, co
     S.len[tid] = L;
     __syncthreads();
     for (uint32_t p = tid >> 5; p < T; p += kPW) {
-      uint32_t lo = 0;
-#pragma unroll
-      for (uint32_t step = kPT / 2; step > 0; step >>= 1)
-        if (S.incl[lo + step - 1] <= p) lo += step;
+      // The first position whose inclusive count exceeds p, in two ballots.
+      const unsigned ge = __ballot_sync(0xffffffffu, S.incl[lane * kPW + kPW - 1] > p);
+      uint32_t lo = (__ffs(ge) - 1) * kPW;
+      const unsigned in = __ballot_sync(0xffffffffu, lane < kPW && S.incl[lo + (lane & (kPW - 1))] > p);
+      lo += __ffs(in) - 1;
       const uint32_t k0 = (p - (lo ? S.incl[lo - 1] : 0u)) * kPiece;
       const uint32_t kend = min(k0 + kPiece, S.len[lo]);
       const uint32_t sbj = S.sb[lo], base = sbj & ~kRevFlag;
@@ -521,14 +557,24 @@ __device__ __forceinline__ void block_iter(uint32_t b, uint32_t e, Shared& S, co
 #pragma unroll
       for (uint32_t r = 0; r < kPiece / 32; ++r) {
         const uint32_t k = k0 + lane + 32 * r;
-        x[r] = k < kend ? arr[base + k] : 0u;
+        x[r] = k < kend ? arr[base + k] : kEmpty;
       }
-#pragma unroll
-      for (uint32_t r = 0; r < kPiece / 32; ++r)
-        if (k0 + 32 * r < kend) f(k0 + lane + 32 * r < kend, lo, sbj + k0 + lane + 32 * r, x[r]);
+      piece(lo, k0 + lane, sbj + k0 + lane, kend, x);
     }
     done();
   }
+}
+
+
+// The same with f(valid, lo, q, x) per step of 32 entries.
+template <class First, class F, class Done>
+__device__ __forceinline__ void block_iter(uint32_t b, uint32_t e, Shared& S, const uint32_t* __restrict__ arr,
+                                           First&& first, F&& f, Done&& done) {
+  block_pieces(b, e, S, arr, first, [&](uint32_t lo, uint32_t k, uint32_t q, uint32_t n, const uint32_t* x) {
+#pragma unroll
+    for (uint32_t r = 0; r < kPiece / 32; ++r)
+      if ((k & ~31u) + 32 * r < n) f(k + 32 * r < n, lo, q + 32 * r, x[r]);
+  }, done);
 }
 
 // The same iteration restricted to flattened pair indices [lo, hi) (counted from the first
@@ -585,14 +631,21 @@ __device__ __forceinline__ bool mine(const Work& W, uint32_t x) { return !W.part
 // whose result first lies below the window bound adds the item to the near list (counts only
 // fall, so exactly one decrement crosses); items above the bound cannot reach the frontier before
 // the next window advance, which reads their counts.
-__device__ __forceinline__ void dec_known(const Work& W, Ctl* ctl, Acc& A, uint32_t x, int64_t amount) {
-  const long long old = (long long)atomicAdd(reinterpret_cast<unsigned long long*>(&W.cnt[x]),
-                                             (unsigned long long)(-amount));
+__device__ __forceinline__ long long dec_add(const Work& W, uint32_t x, int64_t amount) {
+  return (long long)atomicAdd(reinterpret_cast<unsigned long long*>(&W.cnt[x]), (unsigned long long)(-amount));
+}
+
+// What follows the add that returned `old`.
+__device__ __forceinline__ void dec_done(const Work& W, Ctl* ctl, Acc& A, uint32_t x, int64_t amount, long long old) {
   const unsigned long long nb = (unsigned long long)max(old - amount, s_k);
   if (nb < s_win_hi) {
     A.mn = min(A.mn, nb);
     if ((unsigned long long)max(old, s_k) >= s_win_hi) W.near[atomicAdd(&ctl->near_len, 1ull)] = x;
   }
+}
+
+__device__ __forceinline__ void dec_known(const Work& W, Ctl* ctl, Acc& A, uint32_t x, int64_t amount) {
+  dec_done(W, ctl, A, x, amount, dec_add(W, x, amount));
 }
 
 __device__ __forceinline__ void dec(const Work& W, Ctl* ctl, Acc& A, uint32_t x, int64_t amount) {
@@ -675,6 +728,22 @@ __device__ void tip_item_block(const Lists& G, const Work& W, Ctl* ctl, uint32_t
   __syncthreads();
 }
 
+// Removes j[r] butterflies from x[r] where it is unpeeled (state st[r]): all four adds are under way
+// before the first result is looked at.
+__device__ __forceinline__ void charge_four(const Work& W, Ctl* ctl, Acc& A, const uint32_t* x, const uint32_t* j,
+                                            const uint8_t* st) {
+  bool c[4];
+  long long old[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    c[r] = j[r] && st[r] == ALIVE && mine(W, x[r]);
+    old[r] = c[r] ? dec_add(W, x[r], (int64_t)j[r]) : 0;
+  }
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+    if (c[r]) dec_done(W, ctl, A, x[r], (int64_t)j[r], old[r]);
+}
+
 // Heavy tip items of a round (at most W.ngroups of them, items i < nh from `huge`, the others
 // CTA-level ones read back from `big`): their flattened two-hop lists are cut into equal slices
 // over the instance's CTAs.  Every wedge adds one to the item's grid-shared dense counter of u2;
@@ -746,9 +815,7 @@ __device__ void tip_items_flat(const Lists& G, const Work& W, Ctl* ctl, const ui
                              st[r] = W.state[x[r]];
                            }
                          }
-#pragma unroll
-                         for (int r = 0; r < 4; ++r)
-                           if (j[r] && st[r] == ALIVE && mine(W, x[r])) dec_known(W, ctl, A, x[r], (int64_t)j[r]);
+                         charge_four(W, ctl, A, x, j, st);
                        });
     }
   }
@@ -757,6 +824,85 @@ __device__ void tip_items_flat(const Lists& G, const Work& W, Ctl* ctl, const ui
     if (vblock() == 0) A.work += T;
   }
   __syncthreads();
+}
+
+// The same for light rounds (at most 32 items and kListPairs pairs; false and nothing done
+// otherwise): a warp takes a whole list N(v) of an item, or with few lists an equal share of its
+// 128-entry steps, so that no scan, search or barrier lies between the item and its wedges.  What a
+// warp did in one step is remembered in `kept`; several steps are walked again to clear.  (Tip peel
+// of the R-MAT graph with 2^20 edges: 78.0 -> 72.4 ms, of it the clearing in phase F 3.7.)
+constexpr unsigned long long kListPairs = 1ull << 15;
+__device__ bool tip_items_lists(const Lists& G, const Work& W, Ctl* ctl, const uint4* huge, unsigned nh, const uint4* big,
+                                unsigned n, bool clear, Shared& S, uint32_t* kept, Acc& A) {
+  if (n > 32) return false;
+  const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+  uint32_t* mykept = kept + warp * 128;
+  if (clear && S.list_steps[warp] <= 1) {
+    if (S.list_steps[warp] == 1) {
+      uint32_t* cnt = W.gshared + (size_t)S.list_item[warp] * (size_t)W.gshared_stride;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const uint32_t x = mykept[r * 32 + lane];
+        if (x != kEmpty) cnt[x] = 0u;
+      }
+    }
+    return true;
+  }
+  uint4 d = make_uint4(0, 0, 0, 0);
+  if (lane < n) d = lane < nh ? huge[lane] : big[-(int)(lane - nh)];
+  const unsigned long long T = warp_sum((unsigned long long)d.w);  // a saturated length is above the limit
+  if (T > kListPairs) return false;
+  const uint32_t incl = warp_inclusive_scan(d.w ? d.z : 0u);  // lists (none: no live butterfly)
+  const uint32_t D = __shfl_sync(0xffffffffu, incl, 31);
+  unsigned steps = 0, item = 0;
+  if (D) {
+    const uint32_t nw = vgrid() * kPW, share = max(1u, nw / D);
+    for (uint32_t t = warp * vgrid() + vblock(); t < D * share; t += nw) {
+      const uint32_t s = t / D, l = t - s * D;
+      const unsigned i = __ffs(__ballot_sync(0xffffffffu, incl > l)) - 1;
+      const uint32_t before = __shfl_sync(0xffffffffu, incl, i > 0 ? i - 1 : 0);
+      const uint32_t u = __shfl_sync(0xffffffffu, d.x, i);
+      const uint32_t v = G.edgK[__shfl_sync(0xffffffffu, d.y, i) + l - (i > 0 ? before : 0u)];
+      const uint32_t end = G.offC[v + 1];
+      uint32_t* cnt = W.gshared + (size_t)i * (size_t)W.gshared_stride;
+      for (uint32_t q = G.offC[v] + s * 128; q < end; q += share * 128) {
+        uint32_t x[4], j[4];
+        uint8_t st[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) x[r] = q + 32 * r + lane < end ? G.edgC[q + 32 * r + lane] : kEmpty;
+        if (clear) {
+#pragma unroll
+          for (int r = 0; r < 4; ++r)
+            if (x[r] != kEmpty) cnt[x[r]] = 0u;
+          continue;
+        }
+        if (steps == 0) {
+          item = i;
+#pragma unroll
+          for (int r = 0; r < 4; ++r) mykept[r * 32 + lane] = x[r];
+        }
+        ++steps;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          j[r] = 0;
+          st[r] = PEELED;
+          if (x[r] != kEmpty && x[r] != u) {
+            j[r] = atomicAdd(&cnt[x[r]], 1u);
+            st[r] = W.state[x[r]];
+          }
+        }
+        charge_four(W, ctl, A, x, j, st);
+      }
+    }
+  }
+  if (!clear) {
+    if (lane == 0) {
+      S.list_steps[warp] = steps;
+      S.list_item[warp] = item;
+    }
+    if (vblock() == 0 && threadIdx.x == 0) A.work += T;
+  }
+  return true;
 }
 
 // ---- wing: process one frontier edge --------------------------------------------------------
@@ -817,7 +963,7 @@ __device__ void wing_item(const Lists& G, const Work& W, Ctl* ctl, const uint4& 
   const uint32_t b1 = offB[b], d1 = offB[b + 1] - b1;
   const bool hash = kLevel == LV_WARP || psize <= kWingSet;
   uint32_t* mark = W.gscratch + (size_t)blockIdx.x * (size_t)W.gscratch_len;
-  const uint32_t tsize = hash ? max(64u, min(2 * psize, cap)) : 0u;
+  const uint32_t tsize = hash ? max(64u, min(kWingLoad * psize, cap)) : 0u;
   uint32_t* vals = keys + cap;
   // hits[slot]: butterflies found through a probe-set edge, charged to it in one decrement once
   // the intersections are done.
@@ -864,6 +1010,12 @@ __device__ void wing_item(const Lists& G, const Work& W, Ctl* ctl, const uint4& 
   }
   if (pb + rank < pe) st0 = edge_status(W, e0, e1);
   if (rank < fn) load_first(y0, g0);
+  const bool few = kLevel == LV_BLOCK && hash && fn <= 32;  // a light round's slice
+  if (few && rank < fn) {
+    S.len[rank] = f_len;
+    S.sb[rank] = f_beg;
+  }
+  accp[rank] = 0;
   sync();
   auto put = [&](uint32_t key, uint32_t e, uint32_t es) {
     if (es == ES_GONE) return;
@@ -878,9 +1030,9 @@ __device__ void wing_item(const Lists& G, const Work& W, Ctl* ctl, const uint4& 
   }
   sync();
   auto first = [&](uint32_t t, bool valid, uint32_t& L, uint32_t& sb) {
-    accp[rank] = 0;
     t_chunk = t - rank;
     if (t_chunk) {
+      accp[rank] = 0;
       f_st = ES_GONE;
       f_len = 0;
       if (valid) {
@@ -954,8 +1106,41 @@ __device__ void wing_item(const Lists& G, const Work& W, Ctl* ctl, const uint4& 
     Q.push(got != 0, ((unsigned long long)got << 32) | f_edge, charge_sum);
     if (t_chunk + gsize < fn) Q.flush(charge_sum);
   };
-  if (kLevel == LV_WARP) warp_iter(0, fn, edgA, first, pair, done);
-  else block_iter(0, fn, S, edgA, first, pair, done);
+  if (kLevel == LV_WARP) {
+    warp_iter(0, fn, edgA, first, pair, done);
+  } else if (hash) {
+    auto piece = [&](uint32_t lo, uint32_t k, uint32_t q, uint32_t n, const uint32_t* x) {
+      if (q & kRevFlag) {
+#pragma unroll 1
+        for (uint32_t r = 0; r < kPiece / 32; ++r)
+          if ((k & ~31u) + 32 * r < n) pair(k + 32 * r < n, lo, q + 32 * r, r == 0 ? x[0] : r == 1 ? x[1] : r == 2 ? x[2] : x[3]);
+        return;
+      }
+      // The four first probes of a lane are made together; only collisions go on one by one.
+      uint32_t slot[kPiece / 32], key[kPiece / 32];
+#pragma unroll
+      for (uint32_t r = 0; r < kPiece / 32; ++r) {
+        slot[r] = hslot(x[r], tsize);
+        key[r] = keys[slot[r]];
+      }
+#pragma unroll
+      for (uint32_t r = 0; r < kPiece / 32; ++r) {
+        const bool valid = x[r] != kEmpty && x[r] != b;
+        my_work += x[r] != kEmpty;
+        if (!valid || key[r] == kEmpty) slot[r] = kEmpty;
+        else if (key[r] != x[r]) slot[r] = t_slot_next(keys, tsize, x[r], slot[r]);
+        Q.push(slot[r] != kEmpty, ((unsigned long long)(q + 32 * r) << 32) | (lo << 14) | (slot[r] & kNoSlot), charge);
+      }
+    };
+    if (few) {
+      few_pieces(fn, S.len, S.sb, edgA, piece);
+      done();
+    } else {
+      block_pieces(0, fn, S, edgA, first, piece, done);
+    }
+  } else {
+    block_iter(0, fn, S, edgA, first, pair, done);
+  }
   // The probe-set edges' decrements, one per edge.
   for (uint32_t s0 = 0; s0 < tsize; s0 += gsize) {
     const uint32_t s = s0 + rank;
@@ -968,7 +1153,7 @@ __device__ void wing_item(const Lists& G, const Work& W, Ctl* ctl, const uint4& 
     for (uint32_t p = pb + rank; p < pe; p += gsize) mark[edgA[p]] = 0;
   }
   A.work += my_work;
-  {
+  if (s_trace) {
     const int mode = kLevel == LV_WARP ? 0 : (hash ? 1 : 2);
     const unsigned w = __reduce_add_sync(0xffffffffu, my_work);
     const unsigned rw = __reduce_add_sync(0xffffffffu, my_rev);
@@ -1075,6 +1260,7 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
     s_bar_timeout = ctl->barrier_timeout_ns;
     s_skip_arrival = vblock() == 0 ? ctl->test_skip_arrival : 0u;
     s_err = 0;
+    s_trace = ctl->trace;
     S.flat_steps = 0;
   }
   unsigned alist_cur = *(volatile unsigned*)&ctl->alist_cur;
@@ -1109,6 +1295,7 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
   unsigned ph = (unsigned)(*(volatile unsigned long long*)&ctl->fhuge[(r0 & 1ull) ^ 1ull] >> 32);
   // Tip: flat items of the previous round whose counters are still to be cleared.
   unsigned clear_n = 0, clear_nh = 0;
+  bool clear_lists = false;  // by tip_items_lists
 
   for (unsigned long long r = r0;; ++r) {
     const unsigned par = (unsigned)(r & 1ull), npar = par ^ 1u;
@@ -1118,7 +1305,10 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
     if (alive == 0 || pause) {
       if (!kWing && clear_n) {
         Acc none{kInf, 0};
-        tip_items_flat(G, W, ctl, W.fhuge[npar], clear_nh, W.front[npar] + (W.N - 1), clear_n, true, S, kept, none);
+        if (clear_lists)
+          tip_items_lists(G, W, ctl, W.fhuge[npar], clear_nh, W.front[npar] + (W.N - 1), clear_n, true, S, kept, none);
+        else
+          tip_items_flat(G, W, ctl, W.fhuge[npar], clear_nh, W.front[npar] + (W.N - 1), clear_n, true, S, kept, none);
       }
       if (cta0 && threadIdx.x == 0) {
         ctl->round = r;
@@ -1319,7 +1509,7 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
           }
         }
 #pragma unroll 1
-        for (unsigned i = 0; i < 4; ++i) {
+        for (unsigned i = 0; i < 4 && q0 + i * gthreads < nl; ++i) {
           const uint32_t x = xs[0];
           const uint8_t sx = st[0];
           const long long c = cs[0];
@@ -1369,14 +1559,18 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
         est = warp_sum(est);
         if (lane == 0) atomicAdd(&ctl->round_est[par], est);
       }
-      for (unsigned q = gtid; q < ps + pg + ph; q += gthreads) {
+      // (from the other end of the grid: the threads at this end had near items to look at)
+      for (unsigned q = gthreads - 1u - gtid; q < ps + pg + ph; q += gthreads) {
         const uint32_t x = q < ps ? W.front[npar][q].x
                                   : (q < ps + pg ? W.front[npar][W.N - 1 - (q - ps)].x : W.fhuge[npar][q - ps - pg].x);
         W.state[x] = PEELED;
       }
       if (!kWing && clear_n) {
         Acc none{kInf, 0};
-        tip_items_flat(G, W, ctl, W.fhuge[npar], clear_nh, W.front[npar] + (W.N - 1), clear_n, true, S, kept, none);
+        if (clear_lists)
+          tip_items_lists(G, W, ctl, W.fhuge[npar], clear_nh, W.front[npar] + (W.N - 1), clear_n, true, S, kept, none);
+        else
+          tip_items_flat(G, W, ctl, W.fhuge[npar], clear_nh, W.front[npar] + (W.N - 1), clear_n, true, S, kept, none);
         clear_n = 0;
       }
       if (cta0 && threadIdx.x == 0) s_st.scanned += nl - near_done;
@@ -1524,7 +1718,8 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
           const unsigned n = min(ng, total - w0);
           const unsigned in_huge = nh > w0 ? min(n, nh - w0) : 0u;
           const uint4* hl = W.fhuge[par] + w0;
-          tip_items_flat(G, W, ctl, hl, in_huge, W.front[par] + (W.N - 1), n, false, S, kept, A);
+          clear_lists = total <= ng && tip_items_lists(G, W, ctl, hl, in_huge, W.front[par] + (W.N - 1), n, false, S, kept, A);
+          if (!clear_lists) tip_items_flat(G, W, ctl, hl, in_huge, W.front[par] + (W.N - 1), n, false, S, kept, A);
           if (w0 + ng < total) {  // the slices are reused by the next wave
             if (!grid_barrier(ctl)) return false;
             tip_items_flat(G, W, ctl, hl, in_huge, W.front[par] + (W.N - 1), n, true, S, kept, A);
