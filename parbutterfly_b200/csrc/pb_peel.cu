@@ -55,7 +55,9 @@ constexpr uint32_t kWingLoad = 4;  // slots per probe-set entry, while they fit
 constexpr uint32_t kWingWarpSlots = kPoolWords / 3 / kPW;  // 448 slots, probe sets up to kWingWarpSet
 constexpr uint32_t kWingWarpSet = 256;
 constexpr uint32_t kTipSlots = 8192;      // two-hop lists of up to 4096 wedges
-constexpr uint32_t kTipWarpSlots = 512;   // two-hop lists of up to 256 wedges
+constexpr uint32_t kTipWarpSlots = 512;   // two-hop lists of up to 256 wedges; 512 with one-word entries
+constexpr uint32_t kTipWindow = 2 * kPoolWords;  // 16-bit counters of a window
+constexpr int64_t kTipWindows = 4, kTipWindowWedges = 4096;
 constexpr uint32_t kEmpty = 0xFFFFFFFFu;
 constexpr unsigned long long kInf = ~0ull;
 // Item states.  The frontier of round r is marked 1 + (r & 1); the next round turns the marks
@@ -72,7 +74,8 @@ struct Ctl {
   // Frontier lists per round parity: items in the high word, their work units in the low word, so
   // that one add gives an item its position and its first unit (units ascend with positions).
   unsigned long long fsmall[2], fbig[2], fhuge[2];
-  unsigned cur_small[2], cur_big[2];
+  unsigned cur_small[2], cur_big[2], cur_huge[2];
+  unsigned long long huge_sum[2], huge_max[2];  // two-hop lengths of the heavy tip items
   unsigned long long round_est[2];   // summed cost estimate of the round (range mode, tracing)
   unsigned long long near_len;
   unsigned near_done;             // range mode: near items already taken (kept across launches)
@@ -160,6 +163,7 @@ struct Work {
   unsigned ngroups;
   uint32_t* gscratch;  // per-CTA dense scratch (dense counters / probe markers)
   int64_t gscratch_len;
+  int tip_cb;          // count bits of a one-word tip table entry (beside a count-side vertex)
   int64_t N;           // items of this instance
   uint32_t item0;      // first item of this instance: its items are items[item0 .. item0 + N)
                        // (item0 .. item0 + N - 1 themselves when items is null)
@@ -294,6 +298,21 @@ __device__ __forceinline__ void t_add(uint32_t* keys, uint32_t* vals, uint32_t s
       uint32_t prev = atomicCAS(&keys[h], kEmpty, key);
       if (prev == kEmpty || prev == key) { atomicAdd(&vals[h], 1u); return; }
     }
+    h = h + 1 == size ? 0u : h + 1;
+  }
+  raise_err(ctl, ERR_TABLE);
+}
+
+// The same with one-word entries (key << cb | count; counts of at most 2^cb - 2).
+__device__ __forceinline__ void t_add1(uint32_t* tab, uint32_t size, int cb, uint32_t key, Ctl* ctl) {
+  uint32_t h = hslot(key, size);
+  for (uint32_t probes = 0; probes < size; ++probes) {
+    uint32_t k = tab[h];
+    if (k == kEmpty) {
+      k = atomicCAS(&tab[h], kEmpty, (key << cb) | 1u);
+      if (k == kEmpty) return;
+    }
+    if ((k >> cb) == key) { atomicAdd(&tab[h], 1u); return; }
     h = h + 1 == size ? 0u : h + 1;
   }
   raise_err(ctl, ERR_TABLE);
@@ -663,29 +682,43 @@ struct TipFirst {
   }
 };
 
+__device__ __forceinline__ bool tip_one_word(const Work& W, uint32_t deg) { return deg < (1u << W.tip_cb) - 1u; }
+
 // Queue entries of tip items: (u2, w) with w wedges to u2.
 __device__ __forceinline__ void tip_charge(const Work& W, Ctl* ctl, Acc& A, unsigned long long x) {
   const int64_t w = (int64_t)(x >> 32);
   dec(W, ctl, A, (uint32_t)x, w * (w - 1) / 2);
 }
 
-__device__ void tip_item_warp(const Lists& G, const Work& W, Ctl* ctl, uint32_t u, uint32_t* keys, uint32_t* vals,
-                              WarpQueue& Q, Acc& A) {
+// Table: 2 kTipWarpSlots words.  Entries are one word (u2 << cb | count) when the count, at most the
+// degree, fits beside the vertex.
+__device__ void tip_item_warp(const Lists& G, const Work& W, Ctl* ctl, const uint4& it, uint32_t* keys, WarpQueue& Q,
+                              Acc& A) {
   const unsigned lane = lane_id();
+  const uint32_t u = it.x;
   const int64_t wk = G.wk[u];
-  const uint32_t tsize = max(64u, np2(2u * (uint32_t)wk));
-  for (uint32_t s = lane; s < tsize; s += 32) { keys[s] = kEmpty; vals[s] = 0; }
+  const int cb = tip_one_word(W, it.z) ? W.tip_cb : 0;
+  uint32_t* vals = keys + kTipWarpSlots;  // two-array tables
+  const uint32_t tsize = max(64u, cb ? 2u * (uint32_t)wk : np2(2u * (uint32_t)wk));
+  for (uint32_t s = lane; s < tsize; s += 32) {
+    keys[s] = kEmpty;
+    if (!cb) vals[s] = 0;
+  }
   __syncwarp();
-  warp_iter(G.offK[u], G.offK[u + 1], G.edgC, TipFirst{G},
+  warp_iter(it.y, it.y + it.z, G.edgC, TipFirst{G},
             [&](bool valid, uint32_t, uint32_t, uint32_t u2) {
-              if (valid && u2 != u) t_add(keys, vals, tsize, u2, ctl);
+              if (!valid || u2 == u) return;
+              if (cb) t_add1(keys, tsize, cb, u2, ctl);
+              else t_add(keys, vals, tsize, u2, ctl);
             },
             [] {});
   __syncwarp();
   auto charge = [&](unsigned long long x) { tip_charge(W, ctl, A, x); };
-  for (uint32_t s = lane; s < tsize; s += 32) {
-    const uint32_t w = vals[s];
-    Q.push(w >= 2, ((unsigned long long)w << 32) | keys[s], charge);
+  for (uint32_t s0 = 0; s0 < tsize; s0 += 32) {
+    const uint32_t s = s0 + lane;
+    const uint32_t k = s < tsize ? keys[s] : kEmpty;
+    const uint32_t w = k == kEmpty ? 0u : (cb ? k & ((1u << cb) - 1u) : vals[s]);
+    Q.push(w >= 2, ((unsigned long long)w << 32) | (k >> cb), charge);
   }
   Q.flush(charge);
   if (lane == 0) A.work += (unsigned long long)wk;
@@ -695,6 +728,37 @@ __device__ void tip_item_block(const Lists& G, const Work& W, Ctl* ctl, uint32_t
                                WarpQueue& Q, Acc& A) {
   const int64_t wk = G.wk[u];
   const bool hash = (uint64_t)2 * (uint64_t)wk <= (uint64_t)kTipSlots;
+  const uint32_t deg = G.offK[u + 1] - G.offK[u];
+  // Longer lists: 16-bit counters in shared memory over windows of the vertices, when that takes few
+  // windows for the list's length (no atomic leaves the SM); else counters in global memory.
+  const int64_t nwin = (G.nK + kTipWindow - 1) / kTipWindow;
+  if (!hash && deg <= 0xFFFFu && nwin <= kTipWindows && wk > nwin * kTipWindowWedges) {
+    auto charge = [&](unsigned long long x) { tip_charge(W, ctl, A, x); };
+    for (int64_t w0 = 0; w0 < G.nK; w0 += kTipWindow) {
+      const uint32_t base = (uint32_t)w0, len = (uint32_t)min((int64_t)kTipWindow, G.nK - w0), words = (len + 1) / 2;
+      for (uint32_t s = threadIdx.x; s < words; s += kPT) table[s] = 0;
+      __syncthreads();
+      block_pieces(G.offK[u], G.offK[u + 1], S, G.edgC, TipFirst{G},
+                   [&](uint32_t, uint32_t, uint32_t, uint32_t, const uint32_t* x) {
+#pragma unroll
+                     for (uint32_t r = 0; r < kPiece / 32; ++r) {
+                       const uint32_t i = x[r] - base;  // kEmpty lies above every window
+                       if (i < len && x[r] != u) atomicAdd(&table[i >> 1], 1u << (16 * (i & 1u)));
+                     }
+                   },
+                   [] { __syncthreads(); });
+      __syncthreads();
+      for (uint32_t s0 = 0; s0 < words; s0 += kPT) {
+        const uint32_t s = s0 + threadIdx.x, c = s < words ? table[s] : 0u;
+        Q.push((c & 0xFFFFu) >= 2, ((unsigned long long)(c & 0xFFFFu) << 32) | (base + 2 * s), charge);
+        Q.push((c >> 16) >= 2, ((unsigned long long)(c >> 16) << 32) | (base + 2 * s + 1), charge);
+      }
+      Q.flush(charge);
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) A.work += (unsigned long long)wk;
+    return;
+  }
   uint32_t* keys = table;
   uint32_t* vals = table + kTipSlots;
   uint32_t* gcnt = W.gscratch + (size_t)blockIdx.x * (size_t)W.gscratch_len;
@@ -744,15 +808,26 @@ __device__ __forceinline__ void charge_four(const Work& W, Ctl* ctl, Acc& A, con
     if (c[r]) dec_done(W, ctl, A, x[r], (int64_t)j[r], old[r]);
 }
 
-// Heavy tip items of a round (at most W.ngroups of them, items i < nh from `huge`, the others
-// CTA-level ones read back from `big`): their flattened two-hop lists are cut into equal slices
+// The tip items of one wave: huge ones, then (rounds that run whole) CTA-level and warp-level ones.
+struct TipWave {
+  const uint4* huge;
+  const uint4* front;  // warp-level items from the front, CTA-level ones back from front[last]
+  int64_t last;
+  unsigned nh, nb, n;
+  __device__ __forceinline__ uint4 item(unsigned i) const {
+    return i < nh ? huge[i] : (i < nh + nb ? front[last - (int64_t)(i - nh)] : front[i - nh - nb]);
+  }
+};
+
+// The items of a wave (at most W.ngroups of them): their flattened two-hop lists are cut into equal slices
 // over the instance's CTAs.  Every wedge adds one to the item's grid-shared dense counter of u2;
 // the add that returns j removes j butterflies from u2 at once (0 + 1 + ... + (w - 1) = C(w, 2)),
 // so one pass and no barrier is needed.  clear: every CTA resets the counters of its slice (after a
 // barrier): a slice of one step is remembered in `kept` (4 entries per thread of shared memory, so
 // clearing costs no loads: light rounds wait for it), a longer one is walked again.
-__device__ void tip_items_flat(const Lists& G, const Work& W, Ctl* ctl, const uint4* huge, unsigned nh, const uint4* big,
-                               unsigned n, bool clear, Shared& S, uint32_t* kept, Acc& A) {
+__device__ void tip_items_flat(const Lists& G, const Work& W, Ctl* ctl, const TipWave& V, bool clear, Shared& S,
+                               uint32_t* kept, Acc& A) {
+  const unsigned n = V.n;
   if (clear && S.flat_steps <= 1) {  // uniform across the CTA; set by the walk
     if (S.flat_steps == 1) {
       uint32_t* cnt = W.gshared + (size_t)S.flat_item * (size_t)W.gshared_stride;
@@ -770,7 +845,7 @@ __device__ void tip_items_flat(const Lists& G, const Work& W, Ctl* ctl, const ui
       const unsigned i = i0 + threadIdx.x;
       unsigned long long t = 0;
       if (i < n) {
-        const uint4 d = i < nh ? huge[i] : big[-(int)(i - nh)];
+        const uint4 d = V.item(i);
         t = d.w == 0xFFFFFFFFu ? (unsigned long long)G.wk[d.x] + d.z : d.w;
         S.flat[i] = d;
       }
@@ -832,8 +907,9 @@ __device__ void tip_items_flat(const Lists& G, const Work& W, Ctl* ctl, const ui
 // warp did in one step is remembered in `kept`; several steps are walked again to clear.  (Tip peel
 // of the R-MAT graph with 2^20 edges: 78.0 -> 72.4 ms, of it the clearing in phase F 3.7.)
 constexpr unsigned long long kListPairs = 1ull << 15;
-__device__ bool tip_items_lists(const Lists& G, const Work& W, Ctl* ctl, const uint4* huge, unsigned nh, const uint4* big,
-                                unsigned n, bool clear, Shared& S, uint32_t* kept, Acc& A) {
+__device__ bool tip_items_lists(const Lists& G, const Work& W, Ctl* ctl, const TipWave& V, bool clear, Shared& S,
+                                uint32_t* kept, Acc& A) {
+  const unsigned n = V.n;
   if (n > 32) return false;
   const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
   uint32_t* mykept = kept + warp * 128;
@@ -849,7 +925,7 @@ __device__ bool tip_items_lists(const Lists& G, const Work& W, Ctl* ctl, const u
     return true;
   }
   uint4 d = make_uint4(0, 0, 0, 0);
-  if (lane < n) d = lane < nh ? huge[lane] : big[-(int)(lane - nh)];
+  if (lane < n) d = V.item(lane);
   const unsigned long long T = warp_sum((unsigned long long)d.w);  // a saturated length is above the limit
   if (T > kListPairs) return false;
   const uint32_t incl = warp_inclusive_scan(d.w ? d.z : 0u);  // lists (none: no live butterfly)
@@ -1175,8 +1251,8 @@ struct Classify {
   int64_t units_per_cta;  // work units per CTA a round's CTA-level wing work is cut into
   int64_t warp_units;     // wing: every item with a warp-sized probe set runs as warp units
 
-  __device__ __forceinline__ bool tip_small(const Lists& G, uint32_t u) const {
-    return G.wk[u] <= kTipWarpSlots / 2 && G.wk[u] <= small_work;
+  __device__ __forceinline__ bool tip_small(const Work& W, int64_t wk, uint32_t deg) const {
+    return wk <= (int64_t)(tip_one_word(W, deg) ? kTipWarpSlots : kTipWarpSlots / 2) && wk <= small_work;
   }
   // Estimated probes from each side: the two-hop list sizes, capped by deg(u)*deg(v) times a
   // binary-search factor (the reverse-direction intersections).
@@ -1188,7 +1264,6 @@ struct Classify {
     const int64_t du = G.offK[u + 1] - G.offK[u], dv = G.offC[v + 1] - G.offC[v];
     return min(G.S[u], du * dv * 16);
   }
-  __device__ __forceinline__ bool tip_huge(const Lists& G, uint32_t u) const { return G.wk[u] > huge_work; }
 };
 
 // Estimated work of peeling item x (plus one, so that items without work still count): the
@@ -1294,7 +1369,7 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
   unsigned pg = (unsigned)(*(volatile unsigned long long*)&ctl->fbig[(r0 & 1ull) ^ 1ull] >> 32);
   unsigned ph = (unsigned)(*(volatile unsigned long long*)&ctl->fhuge[(r0 & 1ull) ^ 1ull] >> 32);
   // Tip: flat items of the previous round whose counters are still to be cleared.
-  unsigned clear_n = 0, clear_nh = 0;
+  unsigned clear_n = 0, clear_nh = 0, clear_nb = 0;
   bool clear_lists = false;  // by tip_items_lists
 
   for (unsigned long long r = r0;; ++r) {
@@ -1305,10 +1380,9 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
     if (alive == 0 || pause) {
       if (!kWing && clear_n) {
         Acc none{kInf, 0};
-        if (clear_lists)
-          tip_items_lists(G, W, ctl, W.fhuge[npar], clear_nh, W.front[npar] + (W.N - 1), clear_n, true, S, kept, none);
-        else
-          tip_items_flat(G, W, ctl, W.fhuge[npar], clear_nh, W.front[npar] + (W.N - 1), clear_n, true, S, kept, none);
+        const TipWave V{W.fhuge[npar], W.front[npar], W.N - 1, clear_nh, clear_nb, clear_n};
+        if (clear_lists) tip_items_lists(G, W, ctl, V, true, S, kept, none);
+        else tip_items_flat(G, W, ctl, V, true, S, kept, none);
       }
       if (cta0 && threadIdx.x == 0) {
         ctl->round = r;
@@ -1541,9 +1615,11 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
             const unsigned long long pairs = c != 0 ? (unsigned long long)wk + d : 0ull;
             const uint4 it = make_uint4(x, b, d, (uint32_t)min(pairs, 0xFFFFFFFFull));
             const unsigned long long add = (1ull << 32) | 1ull;
-            if (cls.tip_small(G, x)) {
+            if (cls.tip_small(W, wk, d)) {
               W.front[par][atomicAdd(&ctl->fsmall[par], add) >> 32] = it;
-            } else if (cls.tip_huge(G, x) && W.gshared != nullptr) {
+            } else if (wk > cls.huge_work && W.gshared != nullptr) {
+              atomicAdd(&ctl->huge_sum[par], pairs);
+              atomicMax(&ctl->huge_max[par], pairs);
               W.fhuge[par][atomicAdd(&ctl->fhuge[par], add) >> 32] = it;
             } else {
               W.front[par][W.N - 1 - (int64_t)(atomicAdd(&ctl->fbig[par], add) >> 32)] = it;
@@ -1567,10 +1643,9 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
       }
       if (!kWing && clear_n) {
         Acc none{kInf, 0};
-        if (clear_lists)
-          tip_items_lists(G, W, ctl, W.fhuge[npar], clear_nh, W.front[npar] + (W.N - 1), clear_n, true, S, kept, none);
-        else
-          tip_items_flat(G, W, ctl, W.fhuge[npar], clear_nh, W.front[npar] + (W.N - 1), clear_n, true, S, kept, none);
+        const TipWave V{W.fhuge[npar], W.front[npar], W.N - 1, clear_nh, clear_nb, clear_n};
+        if (clear_lists) tip_items_lists(G, W, ctl, V, true, S, kept, none);
+        else tip_items_flat(G, W, ctl, V, true, S, kept, none);
         clear_n = 0;
       }
       if (cta0 && threadIdx.x == 0) s_st.scanned += nl - near_done;
@@ -1597,6 +1672,9 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
       ctl->round_est[npar] = 0;
       ctl->cur_small[npar] = 0;
       ctl->cur_big[npar] = 0;
+      ctl->cur_huge[npar] = 0;
+      ctl->huge_sum[npar] = 0;
+      ctl->huge_max[npar] = 0;
       s_st.rounds += 1;
       s_st.n_small += ns;
       s_st.n_big += nb;
@@ -1605,13 +1683,19 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
     }
     alive -= ns + nb + nh;
     {
+      // Tip items: the huge ones run over the whole grid, in waves of up to ngroups; when the round
+      // has so few items that one wave holds them all, they all run there (one warp or CTA per item
+      // leaves the rest of the grid idle).
+      const unsigned ng = kWing ? 0u : (W.gshared ? min(W.ngroups, kMaxGroups) : 0u);
+      const unsigned items = ns + nb + nh;
+      const bool flat_all = !kWing && vgrid() >= 8 && items > 0 && items <= min(ng, kFlatAll);
       // Warp-level items: warps claim runs of consecutive units and process an item's units of a
       // run as one first-level slice, independently of the other warps (tip: an item is one
       // unit).  The first run of a warp is its own number; the cursor hands out the later ones.
       const unsigned gwarps = vgrid() * kPW;
       const unsigned Kw = kWing ? max(1u, nwu / (4u * gwarps)) : 1u;
       const uint4* const fsm = W.front[par];
-      for (unsigned u = (vblock() * kPW + warp) * Kw; u < nwu;) {
+      for (unsigned u = (vblock() * kPW + warp) * Kw; u < nwu && !flat_all;) {
         const unsigned uend = min(u + Kw, nwu);
         if (kWing) {
           uint32_t lo = 0, hi = ns;  // the last item whose first unit <= u, 32-way search
@@ -1632,7 +1716,7 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
           }
         } else {
           const uint4 it = fsm[u];
-          if (it.w) tip_item_warp(G, W, ctl, it.x, wkeys, wkeys + kTipWarpSlots, Q, A);
+          if (it.w) tip_item_warp(G, W, ctl, it, wkeys, Q, A);
         }
         if (gwarps * Kw >= nwu) break;
         unsigned c = 0;
@@ -1640,12 +1724,6 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
         u = gwarps * Kw + __shfl_sync(0xffffffffu, c, 0);
       }
       if (ns) __syncthreads();  // warp tables and the CTA table share memory
-      // Tip items: the huge ones run over the whole grid, in waves of up to ngroups; when the
-      // round has so few CTA-level items that one wave holds them all, they run there too (one
-      // CTA per item leaves the rest of the grid idle: rounds of 2^12 wedges took 40 us in phase
-      // P on one CTA each, 24 us spread over the grid).
-      const unsigned ng = kWing ? 0u : (W.gshared ? min(W.ngroups, kMaxGroups) : 0u);
-      const bool flat_all = !kWing && vgrid() >= 8 && nb + nh > 0 && nb + nh <= min(ng, kFlatAll);
       if (nu && !flat_all) {
         const uint4* const fbg = W.front[par] + (W.N - 1);  // item q: fbg[-q]
         if (kWing && nb <= kOneSlice && 2 * nb <= vgrid()) {
@@ -1712,30 +1790,42 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
           }
         }
       }
-      if constexpr (!kWing) if (nh || flat_all) {
-        const unsigned total = flat_all ? nb + nh : nh;
-        for (unsigned w0 = 0; w0 < total; w0 += ng) {
-          const unsigned n = min(ng, total - w0);
-          const unsigned in_huge = nh > w0 ? min(n, nh - w0) : 0u;
-          const uint4* hl = W.fhuge[par] + w0;
-          clear_lists = total <= ng && tip_items_lists(G, W, ctl, hl, in_huge, W.front[par] + (W.N - 1), n, false, S, kept, A);
-          if (!clear_lists) tip_items_flat(G, W, ctl, hl, in_huge, W.front[par] + (W.N - 1), n, false, S, kept, A);
-          if (w0 + ng < total) {  // the slices are reused by the next wave
-            if (!grid_barrier(ctl)) return false;
-            tip_items_flat(G, W, ctl, hl, in_huge, W.front[par] + (W.N - 1), n, true, S, kept, A);
-            if (!grid_barrier(ctl)) return false;
-          } else {
-            clear_n = n;
-            clear_nh = in_huge;
+      if constexpr (!kWing) {
+        bool waves = nh || flat_all;
+        // More huge items than a wave holds: one CTA each, unless the longest would outlast the rest
+        // (every wave costs three barriers; 472 items in waves of one took 22 ms on 44 CTAs, one CTA each 5).
+        if (nh > ng && !flat_all) {
+          const unsigned long long sum = *(volatile unsigned long long*)&ctl->huge_sum[par];
+          const unsigned long long longest = *(volatile unsigned long long*)&ctl->huge_max[par];
+          if (longest <= 4 * (sum / vgrid()) + 4096ull * (nh / ng)) {
+            waves = false;
+            for (unsigned u0 = vblock(); u0 < nh;) {
+              if (threadIdx.x == 0) S.item = atomicAdd(&ctl->cur_huge[par], 1u);
+              const uint4 it = W.fhuge[par][u0];
+              if (it.w) tip_item_block(G, W, ctl, it.x, pool, S, Q, A);
+              __syncthreads();
+              u0 = vgrid() + S.item;
+              __syncthreads();
+            }
           }
         }
-        // The last wave's counters are cleared by the next round (its lists start at w0 = 0 when
-        // there was one wave; later waves are cleared here).
-        if (total > ng) {
-          const unsigned w0 = (total - 1) / ng * ng;
-          if (!grid_barrier(ctl)) return false;
-          tip_items_flat(G, W, ctl, W.fhuge[par] + w0, clear_nh, W.front[par] + (W.N - 1), clear_n, true, S, kept, A);
-          clear_n = 0;
+        if (waves) {
+          const unsigned total = flat_all ? items : nh;
+          for (unsigned w0 = 0; w0 < total; w0 += ng) {
+            const unsigned n = min(ng, total - w0);
+            const TipWave V{W.fhuge[par] + w0, W.front[par], W.N - 1, nh > w0 ? min(n, nh - w0) : 0u, nb, n};
+            clear_lists = total <= ng && tip_items_lists(G, W, ctl, V, false, S, kept, A);
+            if (!clear_lists) tip_items_flat(G, W, ctl, V, false, S, kept, A);
+            if (total > ng) {  // the slices are reused by the next wave or round
+              if (!grid_barrier(ctl)) return false;
+              tip_items_flat(G, W, ctl, V, true, S, kept, A);
+              if (w0 + ng < total && !grid_barrier(ctl)) return false;
+            } else {  // cleared by the next round
+              clear_n = n;
+              clear_nh = V.nh;
+              clear_nb = nb;
+            }
+          }
         }
       }
     }
@@ -1959,11 +2049,16 @@ __global__ void ctl_status_kernel(const Ctl* __restrict__ ctls, unsigned n, unsi
 // shares); with part null, the totals over all items (partition 0).
 template <bool kWing>
 __global__ void part_stats_kernel(Lists G, Classify cls, const uint32_t* __restrict__ part, int64_t N,
-                                  unsigned* cnt, unsigned long long* work) {
+                                  bool with_fixed, unsigned* cnt, unsigned long long* work) {
   for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < N; x += (int64_t)gridDim.x * blockDim.x) {
     const uint32_t p = part ? part[x] : 0u;
     atomicAdd(&cnt[p], 1u);
-    atomicAdd(&work[p], item_weight<kWing>(G, cls, (uint32_t)x));
+    const unsigned long long w = item_weight<kWing>(G, cls, (uint32_t)x);
+    // An item's fixed cost in its own units: a tip item takes a CTA about 5 us and 3.5 ns a wedge (a
+    // partition of 2967 items of 800 wedges ran 20 ms on its one CTA, one of 18 items with three
+    // quarters of the wedges 2.4 ms).
+    const unsigned long long fixed = kWing ? 256ull : (w <= kTipWarpSlots ? 128ull : 1400ull);
+    atomicAdd(&work[p], w + (with_fixed ? fixed : 0ull));
   }
 }
 
@@ -2293,6 +2388,8 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
   W.ngroups = ngroups;
   W.gscratch = gscratch.get();
   W.gscratch_len = scratch_len;
+  W.tip_cb = 31;
+  while (W.tip_cb > 1 && ((uint64_t)(G.nK - 1) >> (32 - W.tip_cb)) != 0) --W.tip_cb;
   W.N = N;
   W.item0 = 0;
   W.part_out = two_phase ? part.get() : nullptr;
@@ -2447,7 +2544,7 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
     DevBuf<unsigned long long> iwork(ninst, s);
     PB_CUDA_TRY(cudaMemsetAsync(icnt.get(), 0, sizeof(unsigned) * ninst, s));
     PB_CUDA_TRY(cudaMemsetAsync(iwork.get(), 0, sizeof(unsigned long long) * ninst, s));
-    PB_LAUNCH(part_stats_kernel<kWing>, grid_for(N), 256, 0, s, G, cls, (const uint32_t*)gid.get(), N, icnt.get(),
+    PB_LAUNCH(part_stats_kernel<kWing>, grid_for(N), 256, 0, s, G, cls, (const uint32_t*)gid.get(), N, false, icnt.get(),
               iwork.get());
     std::vector<unsigned long long> hiw(ninst);
     PB_CUDA_TRY(cudaMemcpyAsync(hiw.data(), iwork.get(), sizeof(unsigned long long) * ninst, cudaMemcpyDeviceToHost, s));
@@ -2487,7 +2584,7 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
     DevBuf<unsigned long long> pwork(ntot, s);
     PB_CUDA_TRY(cudaMemsetAsync(pcnt.get(), 0, sizeof(unsigned) * ntot, s));
     PB_CUDA_TRY(cudaMemsetAsync(pwork.get(), 0, sizeof(unsigned long long) * ntot, s));
-    PB_LAUNCH(part_stats_kernel<kWing>, grid_for(N), 256, 0, s, G, cls, (const uint32_t*)key2.get(), N, pcnt.get(),
+    PB_LAUNCH(part_stats_kernel<kWing>, grid_for(N), 256, 0, s, G, cls, (const uint32_t*)key2.get(), N, true, pcnt.get(),
               pwork.get());
     std::vector<unsigned> hcnt(ntot);
     std::vector<unsigned long long> hwork(ntot);
@@ -2562,7 +2659,7 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
     DevBuf<unsigned> ctot(1, s);
     PB_CUDA_TRY(cudaMemsetAsync(wtot.get(), 0, sizeof(unsigned long long), s));
     PB_CUDA_TRY(cudaMemsetAsync(ctot.get(), 0, sizeof(unsigned), s));
-    PB_LAUNCH(part_stats_kernel<kWing>, grid_for(N), 256, 0, s, G, cls, (const uint32_t*)nullptr, N, ctot.get(),
+    PB_LAUNCH(part_stats_kernel<kWing>, grid_for(N), 256, 0, s, G, cls, (const uint32_t*)nullptr, N, false, ctot.get(),
               wtot.get());
     unsigned long long total_w = 0;
     readback(&total_w, wtot.get(), sizeof(total_w), s);
@@ -2677,7 +2774,7 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
   DevBuf<unsigned long long> pwork(nparts, s);
   PB_CUDA_TRY(cudaMemsetAsync(pcnt.get(), 0, sizeof(unsigned) * nparts, s));
   PB_CUDA_TRY(cudaMemsetAsync(pwork.get(), 0, sizeof(unsigned long long) * nparts, s));
-  PB_LAUNCH(part_stats_kernel<kWing>, grid_for(N), 256, 0, s, G0, cls, (const uint32_t*)part.get(), N, pcnt.get(),
+  PB_LAUNCH(part_stats_kernel<kWing>, grid_for(N), 256, 0, s, G0, cls, (const uint32_t*)part.get(), N, true, pcnt.get(),
             pwork.get());
   std::vector<unsigned> hcnt(nparts);
   std::vector<unsigned long long> hwork(nparts);
