@@ -30,21 +30,6 @@ namespace {
 enum Per { VERT = 0, EDGE = 1, TOTAL = 2 };
 constexpr uint32_t kChunk = 512;  // wedges per materialising warp
 
-// Per slot: its row and its wedges as 64-bit numbers (scanned afterwards).
-__global__ void slot_rows_kernel(const uint32_t* __restrict__ off, const uint32_t* __restrict__ pref, int64_t n,
-                                 uint32_t* rowid, int64_t* wide) {
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const unsigned lane = threadIdx.x & 31u;
-  for (int64_t r = warp; r < n; r += nwarps) {
-    const uint32_t e = off[r + 1];
-    for (uint32_t j = off[r] + lane; j < e; j += 32) {
-      rowid[j] = (uint32_t)r;
-      wide[j] = pref[j];
-    }
-  }
-}
-
 // The last index s in [lo, hi) with a[s] <= t (a ascending, a[lo] <= t): 32-way search by a warp.
 __device__ __forceinline__ int64_t warp_last_le(const int64_t* __restrict__ a, int64_t lo, int64_t hi, int64_t t) {
   while (hi - lo > 1) {
@@ -60,9 +45,11 @@ __device__ __forceinline__ int64_t warp_last_le(const int64_t* __restrict__ a, i
 // Materialises wedges [t_begin, t_end) (global flattened indices) at positions t - t_begin.
 // Bound by its writes (20 bytes a wedge).  A warp takes kChunk wedges and walks their slots 32 at
 // a time: lanes load 32 slots at once, every wedge finds its slot by a search over the lanes'
-// prefixes, so neighbouring lanes write neighbouring positions.  Groups of 32 slots without wedges
-// are left by a search over the prefix (most slots of the low ranks hold none: walking them one by
-// one took 129 ms for the 1e7 wedges of a uniform graph with 1e6 edges, this walk 0.1 ms).
+// prefixes, so neighbouring lanes write neighbouring positions.  Where a group of 32 slots holds no
+// wedge, every lane searches the prefix for a wedge of its own: most slots of the low ranks hold
+// none, and a wedge may lie thousands of slots behind the one before it.  (1e7 wedges of a uniform
+// graph with 1e6 edges: empty slots walked one by one 129 ms, searched over for one wedge at a time
+// 1.9, for 32 0.23.)
 template <class K>
 __global__ void materialize_kernel(const uint32_t* __restrict__ off, const uint32_t* __restrict__ adj,
                                    const uint32_t* __restrict__ pref, const int64_t* __restrict__ spre,
@@ -106,7 +93,24 @@ __global__ void materialize_kernel(const uint32_t* __restrict__ off, const uint3
         t = gend;
         s += 32;
       } else {
-        s = warp_last_le(spre, s, m2, t);
+        const int64_t x = t + lane;
+        int64_t lo = s, hi = m2;  // the last slot with spre[slot] <= x
+        while (hi - lo > 1) {
+          const int64_t mid = (lo + hi) >> 1;
+          if (spre[mid] <= x) lo = mid;
+          else hi = mid;
+        }
+        if (x < c1) {
+          const uint32_t slot2 = off[adj[lo] >> 1] + (uint32_t)(x - spre[lo]);
+          const int64_t pos = x - t_begin;
+          keys[pos] = ((K)(rowid[lo] - i0) << ubits) | (K)(adj[slot2] >> 1);
+          vals[pos] = (uint32_t)pos;
+          jarr[pos] = (uint32_t)lo;
+          s2arr[pos] = slot2;
+        }
+        const int last = (int)min((int64_t)31, c1 - t - 1);
+        s = __shfl_sync(0xffffffffu, lo, last);
+        t += last + 1;
       }
     }
   }
@@ -167,20 +171,72 @@ __global__ void run_starts_kernel(const uint32_t* __restrict__ head, const uint3
   if (blockIdx.x == 0 && threadIdx.x == 0) start[rid[n]] = (uint32_t)n;
 }
 
+// Runs lie in endpoint order, so neighbouring lanes mostly credit one endpoint i: their credits are
+// added up in the warp first; those of the lowest ranks (which share wedges with most endpoints) in
+// shared memory (3.8e6 wedges of a Zipf graph: 178 us with every credit on its own, 145 so).
+constexpr uint32_t kHotRanks = 256;
+
 template <class K>
-__global__ void sort_credit_kernel(const K* __restrict__ keys, const uint32_t* __restrict__ vals,
+__global__ void __launch_bounds__(256) sort_credit_kernel(const K* __restrict__ keys, const uint32_t* __restrict__ vals,
                                    const uint32_t* __restrict__ jarr, const uint32_t* __restrict__ s2arr,
                                    const uint32_t* __restrict__ head, const uint32_t* __restrict__ rid,
                                    const uint32_t* __restrict__ start, int64_t n, Credit C) {
-  for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t r = rid[p] - (head[p] ? 0u : 1u);  // rid = heads strictly before p
-    const int64_t w = (int64_t)start[r + 1] - start[r];
-    const uint64_t key = keys[p];
-    const uint32_t i = C.endpoint(key), u2 = C.end2(key);
-    const uint32_t pos = vals[p];
-    const uint32_t j = jarr[pos];
-    C.wedge(i, j, s2arr[pos], w);
-    if (head[p]) C.pair(i, u2, w);
+  __shared__ uint32_t hot[2 * kHotRanks];  // low and high words
+  for (uint32_t s = threadIdx.x; s < 2 * kHotRanks; s += blockDim.x) hot[s] = 0;
+  __syncthreads();
+  const unsigned lane = threadIdx.x & 31u;
+  auto credit = [&](uint32_t x, unsigned long long v) {
+    if (x < kHotRanks) {
+      const uint32_t lo = (uint32_t)v, old = atomicAdd(&hot[x], lo);
+      const uint32_t hi = (uint32_t)(v >> 32) + (old + lo < old ? 1u : 0u);
+      if (hi) atomicAdd(&hot[kHotRanks + x], hi);
+    } else {
+      C.add(x, (int64_t)v);
+    }
+  };
+  unsigned long long total = 0;
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t p0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; p0 < n; p0 += step) {  // whole warps
+    const int64_t p = p0 + lane;
+    unsigned long long mine = 0;  // butterflies of the run that begins here
+    uint32_t i = 0xFFFFFFFFu;
+    if (p < n) {
+      const uint32_t h = head[p], r = rid[p] - (h ? 0u : 1u);  // rid = heads strictly before p
+      const int64_t w = (int64_t)start[r + 1] - start[r];
+      const uint64_t key = keys[p];
+      i = C.endpoint(key);
+      if (w >= 2) {
+        if (C.per == EDGE || (C.per == VERT && (C.adj[C.off[i]] & 1u))) {
+          const uint32_t pos = vals[p];
+          C.wedge(i, jarr[pos], s2arr[pos], w);
+        } else if (h) {
+          mine = (unsigned long long)(w * (w - 1) / 2);
+          if (C.per == VERT) credit(C.end2(key), mine);
+        }
+      }
+    }
+    if (C.per == VERT) {
+      if (!__any_sync(0xffffffffu, mine != 0)) continue;
+      const unsigned long long incl = warp_inclusive_scan(mine);
+      const uint32_t next = __shfl_down_sync(0xffffffffu, i, 1), prev = __shfl_up_sync(0xffffffffu, i, 1);
+      const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || i != prev);
+      const int first = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+      const unsigned long long before = __shfl_sync(0xffffffffu, incl, first > 0 ? first - 1 : 0);
+      const unsigned long long sum = incl - (first > 0 ? before : 0ull);
+      if (sum && (lane == 31 || next != i)) credit(i, sum);
+    } else {
+      total += mine;
+    }
+  }
+  if (C.per == TOTAL) {
+    total = warp_sum(total);
+    if (lane == 0 && total) atomicAdd(C.total, total);
+  } else if (C.per == VERT) {
+    __syncthreads();
+    for (uint32_t s = threadIdx.x; s < kHotRanks; s += blockDim.x) {
+      const unsigned long long v = ((unsigned long long)hot[kHotRanks + s] << 32) | hot[s];
+      if (v) C.add(s, (int64_t)v);
+    }
   }
 }
 
@@ -358,11 +414,10 @@ CountResult count_ranked_materialized(const Ranked& R, int per, int64_t* out, bo
   PB_CUDA_TRY(cudaEventCreate(&e0));
   PB_CUDA_TRY(cudaEventCreate(&e1));
   PB_CUDA_TRY(cudaEventRecord(e0, s));
-  // Per-slot rows and exclusive wedge prefix (the flattened wedge index of each slot's first wedge).
+  // Per-slot exclusive wedge prefix (the flattened wedge index of each slot's first wedge).
   DevBuf<int64_t> spre(m2 + 1, s);
-  DevBuf<uint32_t> rowid(m2, s);
-  PB_LAUNCH(slot_rows_kernel, grid_for(n * 32), 256, 0, s, R.off.get(), R.pref.get(), n, rowid.get(), spre.get());
-  exclusive_scan_i64(spre.get(), spre.get(), m2, s);
+  const uint32_t* rowid = R.rowid.get();
+  exclusive_scan_u32_i64(R.pref.get(), spre.get(), m2, s);
   // Batch budget: -m, capped so that one batch's arrays stay within a few GiB.
   const int64_t cap = std::min<int64_t>(max_wedges > 0 ? max_wedges : (int64_t)1 << 27, (int64_t)1 << 27);
   // Endpoint wedge prefix on the host, to cut batches at endpoint boundaries (one batch: its ends).
@@ -387,7 +442,7 @@ CountResult count_ranked_materialized(const Ranked& R, int per, int64_t* out, bo
     using K = std::remove_pointer_t<decltype(keys)>;
     DevBuf<uint32_t> vals(cnt, s), vals2(cnt, s), jarr(cnt, s), s2arr(cnt, s);
     PB_LAUNCH(materialize_kernel<K>, materialize_grid(cnt), 256, 0, s, R.off.get(), R.adj.get(), R.pref.get(),
-              spre.get(), rowid.get(), m2, tb, tb + cnt, C.i0, ubits, keys, vals.get(), jarr.get(), s2arr.get());
+              spre.get(), rowid, m2, tb, tb + cnt, C.i0, ubits, keys, vals.get(), jarr.get(), s2arr.get());
     bool alt;
     if constexpr (sizeof(K) == 4) alt = radix_sort_pairs_u32(keys, vals.get(), keys2, vals2.get(), cnt, 0, key_bits, s);
     else alt = radix_sort_pairs_u64(keys, vals.get(), keys2, vals2.get(), cnt, 0, key_bits, s);
@@ -423,7 +478,7 @@ CountResult count_ranked_materialized(const Ranked& R, int per, int64_t* out, bo
         DevBuf<uint64_t> keys(cnt, s), keys2(cnt, s);
         DevBuf<uint32_t> vals(cnt, s), jarr(cnt, s), s2arr(cnt, s);
         PB_LAUNCH(materialize_kernel<uint64_t>, materialize_grid(cnt), 256, 0, s, R.off.get(), R.adj.get(),
-                  R.pref.get(), spre.get(), rowid.get(), m2, tb, te, (uint32_t)i0, ubits, keys.get(), vals.get(),
+                  R.pref.get(), spre.get(), rowid, m2, tb, te, (uint32_t)i0, ubits, keys.get(), vals.get(),
                   jarr.get(), s2arr.get());
         // Semisort: bucket keys by hash (about 1024 wedges per bucket), one stable radix pass.
         int bits = bits_for((uint64_t)std::max<int64_t>(1, cnt / 1024));

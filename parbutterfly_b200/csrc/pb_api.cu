@@ -263,7 +263,9 @@ void run_count(pb_ctx* ctx, const pb_graph* g, const pb_opts& o, int per, int us
   build_ranked_csr(*g, R, per == PB_EDGE, s);
   T.mark();
   tr.stage("relabel");
-  wedge_scan(R, s);
+  const bool materialised = o.count_type == PB_SORT || o.count_type == PB_ASORT || o.count_type == PB_HIST ||
+                            o.count_type == PB_AHIST;
+  wedge_scan(R, s, materialised);
   T.mark();
   tr.stage("scan");
   CountConfig cfg;

@@ -33,6 +33,7 @@ struct Ranked {
   DevBuf<uint32_t> adj;    // 2m tagged ranks
   DevBuf<uint32_t> eout;   // 2m output edge index (per-edge counting only)
   DevBuf<uint32_t> pref;   // 2m: wedges of slot (i,j) = #{u2 in N(v): u2 < min(i,v)}
+  DevBuf<uint32_t> rowid;  // 2m: the row of each slot (SORT / HIST only)
   DevBuf<int64_t> wsum;    // n+1: exclusive prefix of per-endpoint wedge counts
   int64_t w_rank = 0;
   uint32_t max_deg = 0;
@@ -46,7 +47,7 @@ void side_wedge_sums(const pb_graph& g, unsigned long long* sums, cudaStream_t s
 void cmp_wedge_counts(const pb_graph& g, int* use_v, int64_t* w_min, int64_t* wv, int64_t* wu, cudaStream_t s);
 void vertex_order(const pb_graph& g, int rank_type, int use_v, Ranked& R, cudaStream_t s);
 void build_ranked_csr(const pb_graph& g, Ranked& R, bool with_eout, cudaStream_t s);
-void wedge_scan(Ranked& R, cudaStream_t s);
+void wedge_scan(Ranked& R, cudaStream_t s, bool with_rows = false);  // with_rows: fills rowid too
 void edge_to_idxs(const pb_graph& g, int use_v, uint32_t* eti, cudaStream_t s);
 
 // Counting stage (pb_count.cu).  per: 0 VERT (out: rank-space counts [n]), 1 EDGE (out: [m]

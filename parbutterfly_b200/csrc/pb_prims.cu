@@ -27,8 +27,8 @@ __device__ T block_exclusive_scan(T x, T* smem /*[32]*/, T& total) {
   return warp_prefix + incl - x;
 }
 
-template <class T>
-__global__ void scan_reduce_kernel(const T* __restrict__ in, int64_t n, T* __restrict__ partials) {
+template <class T, class I>
+__global__ void scan_reduce_kernel(const I* __restrict__ in, int64_t n, T* __restrict__ partials) {
   __shared__ T smem[32];
   const int64_t base = (int64_t)blockIdx.x * kScanTile;
   T sum = 0;
@@ -42,8 +42,8 @@ __global__ void scan_reduce_kernel(const T* __restrict__ in, int64_t n, T* __res
   if (threadIdx.x == 0) partials[blockIdx.x] = total;
 }
 
-template <class T>
-__global__ void scan_tile_kernel(const T* in, T* out, int64_t n, const T* __restrict__ tile_offsets) {
+template <class T, class I>
+__global__ void scan_tile_kernel(const I* in, T* out, int64_t n, const T* __restrict__ tile_offsets) {
   __shared__ T smem[32];
   const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
   T v[kScanItems];
@@ -51,7 +51,7 @@ __global__ void scan_tile_kernel(const T* in, T* out, int64_t n, const T* __rest
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
     int64_t idx = base + k;
-    v[k] = idx < n ? in[idx] : T(0);
+    v[k] = idx < n ? (T)in[idx] : T(0);
     sum += v[k];
   }
   T total;
@@ -64,8 +64,8 @@ __global__ void scan_tile_kernel(const T* in, T* out, int64_t n, const T* __rest
   }
 }
 
-template <class T>
-__global__ void scan_small_kernel(const T* in, T* out, int64_t n) {
+template <class T, class I>
+__global__ void scan_small_kernel(const I* in, T* out, int64_t n) {
   // one block, n <= kScanTile; writes out[n] = total
   __shared__ T smem[32];
   const int64_t base = (int64_t)threadIdx.x * kScanItems;
@@ -74,7 +74,7 @@ __global__ void scan_small_kernel(const T* in, T* out, int64_t n) {
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
     int64_t idx = base + k;
-    v[k] = idx < n ? in[idx] : T(0);
+    v[k] = idx < n ? (T)in[idx] : T(0);
     sum += v[k];
   }
   T total;
@@ -88,17 +88,17 @@ __global__ void scan_small_kernel(const T* in, T* out, int64_t n) {
   if (threadIdx.x == 0) out[n] = total;
 }
 
-template <class T>
-void exclusive_scan_impl(const T* in, T* out, int64_t n, cudaStream_t s) {
+template <class T, class I>
+void exclusive_scan_impl(const I* in, T* out, int64_t n, cudaStream_t s) {
   if (n <= kScanTile) {
-    PB_LAUNCH(scan_small_kernel<T>, 1, kScanBlock, 0, s, in, out, n);
+    PB_LAUNCH((scan_small_kernel<T, I>), 1, kScanBlock, 0, s, in, out, n);
     return;
   }
   const int64_t tiles = (n + kScanTile - 1) / kScanTile;
   DevBuf<T> partials(tiles + 1, s);
-  PB_LAUNCH(scan_reduce_kernel<T>, (unsigned)tiles, kScanBlock, 0, s, in, n, partials.get());
-  exclusive_scan_impl<T>(partials.get(), partials.get(), tiles, s);
-  PB_LAUNCH(scan_tile_kernel<T>, (unsigned)tiles, kScanBlock, 0, s, in, out, n, partials.get());
+  PB_LAUNCH((scan_reduce_kernel<T, I>), (unsigned)tiles, kScanBlock, 0, s, in, n, partials.get());
+  exclusive_scan_impl<T, T>(partials.get(), partials.get(), tiles, s);
+  PB_LAUNCH((scan_tile_kernel<T, I>), (unsigned)tiles, kScanBlock, 0, s, in, out, n, partials.get());
   PB_CUDA_TRY(cudaMemcpyAsync(out + n, partials.get() + tiles, sizeof(T), cudaMemcpyDeviceToDevice, s));
 }
 
@@ -367,10 +367,13 @@ int bits_for(uint64_t x) {  // bits needed to represent values < x+1
 }  // namespace
 
 void exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, cudaStream_t s) {
-  exclusive_scan_impl<int64_t>(in, out, n, s);
+  exclusive_scan_impl<int64_t, int64_t>(in, out, n, s);
+}
+void exclusive_scan_u32_i64(const uint32_t* in, int64_t* out, int64_t n, cudaStream_t s) {
+  exclusive_scan_impl<int64_t, uint32_t>(in, out, n, s);
 }
 void exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, cudaStream_t s) {
-  exclusive_scan_impl<uint32_t>(in, out, n, s);
+  exclusive_scan_impl<uint32_t, uint32_t>(in, out, n, s);
 }
 
 bool radix_sort_pairs_u64(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t* vals_alt, int64_t n,

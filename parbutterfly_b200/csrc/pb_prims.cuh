@@ -9,6 +9,7 @@ namespace pb {
 // out[0..n] = exclusive prefix sums of in[0..n); out[n] = total.  in and out may alias.
 void exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, cudaStream_t s);
 void exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, cudaStream_t s);
+void exclusive_scan_u32_i64(const uint32_t* in, int64_t* out, int64_t n, cudaStream_t s);  // 64-bit sums
 
 // Stable LSD radix sort of (key, value) pairs on key bits [begin_bit, end_bit).  Sorted data
 // ends in (keys, vals) or (keys_alt, vals_alt); the return value says which (true = alt).

@@ -297,7 +297,7 @@ __global__ void below_self_kernel(const uint32_t* __restrict__ off, const uint32
 // prefix length is a binary search for i in N(v) (when i < v) or the per-vertex below[v].
 __global__ void wedge_scan_kernel(const uint32_t* __restrict__ off, const uint32_t* __restrict__ adj,
                                   const uint32_t* __restrict__ below, int64_t n, int64_t m2, uint32_t chunk, uint32_t* pref,
-                                  int64_t* wcount) {
+                                  int64_t* wcount, uint32_t* rowid) {
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const unsigned lane = threadIdx.x & 31u;
@@ -314,6 +314,7 @@ __global__ void wedge_scan_kernel(const uint32_t* __restrict__ off, const uint32
           L = below ? below[v] : lower_bound_u32(adj, vb, off[v + 1], v << 1) - vb;
         }
         pref[j] = L;
+        if (rowid) rowid[j] = i;
       }
       // One add per row and group of 32 slots (a row's slots are neighbouring lanes).
       const int64_t incl = warp_inclusive_scan((int64_t)L);
@@ -498,10 +499,11 @@ void build_ranked_csr(const pb_graph& g, Ranked& R, bool with_eout, cudaStream_t
   }
 }
 
-void wedge_scan(Ranked& R, cudaStream_t s) {
+void wedge_scan(Ranked& R, cudaStream_t s, bool with_rows) {
   const int64_t n = R.n;
   R.wsum.alloc(n + 1, s);
   R.pref.alloc(R.m2 > 0 ? R.m2 : 1, s);
+  if (with_rows) R.rowid.alloc(R.m2 > 0 ? R.m2 : 1, s);
   if (n == 0) {
     PB_CUDA_TRY(cudaMemsetAsync(R.wsum.get(), 0, sizeof(int64_t), s));
     R.w_rank = 0;
@@ -519,7 +521,7 @@ void wedge_scan(Ranked& R, cudaStream_t s) {
   const uint32_t chunk = slot_chunk(R.m2);
   if (R.m2 > 0)
     PB_LAUNCH(wedge_scan_kernel, grid_for((R.m2 + chunk - 1) / chunk * 32), 256, 0, s, R.off.get(), R.adj.get(),
-              below.get(), n, R.m2, chunk, R.pref.get(), wc.get());
+              below.get(), n, R.m2, chunk, R.pref.get(), wc.get(), R.rowid.get());
   exclusive_scan_i64(wc.get(), R.wsum.get(), n, s);
   readback(&R.w_rank, R.wsum.get() + n, sizeof(int64_t), s);
   if (R.co.get()) {
