@@ -42,8 +42,12 @@ constexpr uint32_t kEmpty = 0xFFFFFFFFu;
 constexpr int kWarpTable = 1024;  // slots per warp
 constexpr int kWarpsPerBlockSmall = 8;
 constexpr uint32_t kHotRanks = 256;   // count_warp_kernel: vertex counts gathered per CTA
-constexpr uint32_t kWarpRow = 1024;   // longer rows take a CTA
-constexpr uint32_t kMidRow = 16384;   // longer rows take a large CTA
+// A row is walked by the threads that own its endpoint, however few wedges it has, so long rows move
+// up a class: beyond kWarpRow slots to a CTA of 128 threads, beyond kMidRow to one of 512.  Limits of
+// (1024, 16384) left the 128-thread class of 2^18 R-MAT edges waiting for its longest rows: aggregation
+// 0.43 ms, (512, 1024) 0.34, (128, 512) 0.32, (256, 1024) 0.30; 2^24 edges take 18.7 ms with each.
+constexpr uint32_t kWarpRow = 256;
+constexpr uint32_t kMidRow = 1024;
 
 enum Per { VERT = 0, EDGE = 1, TOTAL = 2 };
 

@@ -28,6 +28,10 @@ GRAPHS = {
     "rows": lambda: BipartiteGraph.from_edges(
         40_000, 6, np.r_[np.arange(1023), np.arange(1024), np.arange(1025), np.arange(16_385), 39_998, 39_999],
         np.r_[np.zeros(1023, int), np.ones(1024, int), np.full(1025, 2), np.full(16_385, 3), 4, 5]),
+    # Rows of 255 .. 257 slots, the first length of the small CTAs.
+    "rows_256": lambda: BipartiteGraph.from_edges(
+        3_000, 5, np.r_[np.arange(255), np.arange(256), np.arange(257), 2_998, 2_999],
+        np.r_[np.zeros(255, int), np.ones(256, int), np.full(257, 2), 3, 4]),
     # More vertices than leave ten count bits beside a key: two-array tables.
     "many_vertices": lambda: _biclique(30, 600, 60_000, 3, 2_200_000),
     # Prefixes on both sides of the length that all warps of a CTA walk together.
