@@ -11,8 +11,8 @@
 // the endpoint credits matter, never both.
 //
 // Aggregators (the multiplicity table w), by the wedges W_i of the endpoint:
-//   warp : W_i <= small_w; one warp, an open-addressing table in shared memory.
-//   mid  : W_i <= mid_w and the table fits a CTA of 128 threads; many such CTAs share an SM, since
+//   warp : W_i <= small_w and a short row; one warp, an open-addressing table in shared memory.
+//   mid  : W_i <= mid_w and a row and a table that suit a CTA of 128 threads; many such CTAs share an SM, since
 //          an endpoint of this size is a chain of a few round trips, not a throughput problem.
 //   block: larger endpoints, one CTA of 512 threads per endpoint taken from a global work counter.
 // The CTA kernels choose among dense counters over [0, i) (BATCHS-style; 16 bits wide when the

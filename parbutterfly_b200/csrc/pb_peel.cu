@@ -1854,9 +1854,10 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
 // instance tip peel runs faster on the latter (light rounds: fewer CTAs also shorten its grid
 // barriers), and so does the wing peel while its rounds are light; with more edges the rounds are
 // heavy and the intersections need the warps.  Wing peel of R-MAT graphs, one against two CTAs:
-// 2^18 edges 220 / 243 ms, 2^20 665 / 724, 2^21 1254 / 1303, 2^22 2491 / 2424, 2^24 11369 / 9881.
+// 2^18 edges 186 / 213 ms, 2^20 566 / 643, 2^21 1040 / 1147, 2^22 2032 / 2122, 2^23 4167 / 4128,
+// 2^24 9248 / 8514.
 // Batches keep two (more graphs at a time).
-constexpr int64_t kWingOneCta = int64_t(3) << 20;
+constexpr int64_t kWingOneCta = int64_t(6) << 20;
 template <bool kWing, int kMinBlocks>
 __global__ void __launch_bounds__(kPT, kMinBlocks) peel_kernel(Lists G, const Lists* levels, Instances I, Ctl* ctls,
                                                                Classify cls) {
