@@ -366,7 +366,8 @@ __device__ __forceinline__ int64_t block_sum_i64(int64_t x, int64_t* smem) {
 // prefixes N(v)[0, L) of up to kLong wedges go to the warps in turn, longer ones are walked by all
 // warps together.  Lane t of a walk takes entries t, t + 32, ... with four loads in flight, so loads
 // and atomics on the entries' slots are coalesced.  f(slot2, u2) per wedge; part_end(j, vt): all
-// lanes of a warp, after its part of neighbour slot j.
+// lanes of a warp, after its part of neighbour slot j.  Ends with a barrier, so a walk may follow
+// another at once and read what its f wrote.
 constexpr uint32_t kLong = 512;
 
 template <uint32_t kStride, class F>
@@ -420,8 +421,11 @@ __device__ __forceinline__ void block_wedges(uint32_t b, uint32_t e, const Param
       part_end(j0 + k, S.vt[k]);
     }
     __syncthreads();
-    if (tid == 0) S.n_short = S.n_long = 0;  // the next chunk's adds come after a barrier below
-    if (j0 + NT < e) __syncthreads();
+    if (tid == 0) S.n_short = S.n_long = 0;
+    // The next adds to the counters come from the next chunk or from the caller's next walk, so the
+    // reset is closed by a barrier in both cases: an add that came before it would be lost, and with
+    // it a neighbour list of the walk.
+    __syncthreads();
   }
 }
 
@@ -561,7 +565,6 @@ __global__ void __launch_bounds__(NT, kMinBlocks) count_block_kernel(Params P, c
         }
       }, nothing);
     }
-    __syncthreads();
     if (need_center) {
       // Phase 2: centre / edge credits.
       uint32_t mine = 0;
