@@ -33,6 +33,7 @@
 #include "pb_engine.cuh"
 #include "pb_mlp.cuh"
 #include "pb_prims.cuh"
+#include "pb_walk.cuh"
 
 namespace pb {
 
@@ -161,9 +162,9 @@ struct SlotRow {
   uint32_t L, vt, vs;
 };
 
-__device__ __forceinline__ SlotRow load_slot(uint32_t j, uint32_t e, const Params& P) {
+__device__ __forceinline__ SlotRow load_slot(uint32_t j, bool valid, const Params& P) {
   SlotRow r{0, kEmpty, 0};
-  if (j < e) {
+  if (valid) {
     r.L = P.pref[j];
     r.vt = P.adj[j];
     if ((r.vt >> 1) < P.n) r.vs = P.off[r.vt >> 1];
@@ -180,8 +181,8 @@ template <class Slots, class F, class End>
 __device__ __forceinline__ void warp_wedges(uint32_t b, uint32_t e, SlotRow row, const Params& P, Slots&& slots, F&& f,
                                             End&& group_end) {
   const unsigned lane = lane_id();
-  for (uint32_t j0 = b; j0 < e; j0 += 32) {
-    if (j0 != b) row = load_slot(j0 + lane, e, P);
+  walk_groups(b, e - b, 32, lane, [&](uint32_t j, bool valid) {
+    if (j != b + lane) row = load_slot(j, valid, P);
     slots();
     const uint32_t incl = warp_inclusive_scan(row.L);
     const uint32_t from = row.vs - (incl - row.L);  // slot2 = from + t
@@ -207,8 +208,8 @@ __device__ __forceinline__ void warp_wedges(uint32_t b, uint32_t e, SlotRow row,
         if (x[r] != kEmpty) f(at[r], s2[r], x[r] >> 1);
     }
     __syncwarp();
-    group_end(j0 + lane, row.vt);
-  }
+    group_end(j, row.vt);
+  });
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -240,7 +241,7 @@ __global__ void __launch_bounds__(256, kOneWord ? 6 : 3) count_warp_kernel(Param
   // Two list entries ahead, one row ahead.
   uint4 next = q < n_items ? items[q] : make_uint4(0, 0, 0, 0);
   uint4 after = q + nwarps < n_items ? items[q + nwarps] : make_uint4(0, 0, 0, 0);
-  SlotRow next_row = load_slot(next.y + lane, next.z, P);
+  SlotRow next_row = load_slot(next.y + lane, lane < next.z - next.y, P);
   for (; q < n_items; q += nwarps) {
     const uint4 it = next;
     const SlotRow row = next_row;
@@ -249,7 +250,7 @@ __global__ void __launch_bounds__(256, kOneWord ? 6 : 3) count_warp_kernel(Param
     after = q + 2 * nwarps < n_items ? items[q + 2 * nwarps] : make_uint4(0, 0, 0, 0);
     // The next endpoint's first slots: issued here, their row starts (a dependent load) below.
     next_row = SlotRow{0, kEmpty, 0};
-    if (next.y + lane < next.z) {
+    if (lane < next.z - next.y) {
       next_row.L = P.pref[next.y + lane];
       next_row.vt = P.adj[next.y + lane];
     }
@@ -370,26 +371,27 @@ __device__ __forceinline__ int64_t block_sum_i64(int64_t x, int64_t* smem) {
 // another at once and read what its f wrote.
 constexpr uint32_t kLong = 512;
 
-template <uint32_t kStride, class F>
-__device__ __forceinline__ void walk_prefix(const uint32_t* __restrict__ adj, uint32_t beg, uint32_t end, F&& f) {
-  for (uint32_t s0 = beg; s0 < end; s0 += 4 * kStride) {
+template <int kStride, class F>
+__device__ __forceinline__ void walk_prefix(const uint32_t* __restrict__ adj, uint32_t beg, uint32_t len, uint32_t first,
+                                            F&& f) {
+  walk_turns<kStride>(beg, len, first, [&](uint32_t s0, int32_t left) {
     uint32_t x[4];
 #pragma unroll
-    for (uint32_t r = 0; r < 4; ++r) x[r] = s0 + r * kStride < end ? __ldg(adj + s0 + r * kStride) : kEmpty;
+    for (int r = 0; r < 4; ++r) x[r] = left > r * kStride ? __ldg(adj + (s0 + r * kStride)) : kEmpty;
 #pragma unroll
-    for (uint32_t r = 0; r < 4; ++r)
+    for (int r = 0; r < 4; ++r)
       if (x[r] != kEmpty) f(s0 + r * kStride, x[r] >> 1);
-  }
+  });
 }
 
 template <int NT, class F, class End>
 __device__ __forceinline__ void block_wedges(uint32_t b, uint32_t e, const Params& P, BlockShared<NT>& S, F&& f,
                                              End&& part_end) {
   const uint32_t tid = threadIdx.x, lane = tid & 31u;
-  for (uint32_t j0 = b; j0 < e; j0 += NT) {
-    const uint32_t j = j0 + tid;
+  walk_groups(b, e - b, NT, tid, [&](uint32_t j, bool valid) {
+    const uint32_t j0 = j - tid;
     uint32_t L = 0, vt = 0, vs = 0;
-    if (j < e) {
+    if (valid) {
       L = P.pref[j];
       vt = P.adj[j];
       if ((vt >> 1) < P.n) vs = P.off[vt >> 1];
@@ -410,13 +412,13 @@ __device__ __forceinline__ void block_wedges(uint32_t b, uint32_t e, const Param
     const uint32_t ns = S.n_short, nl = S.n_long;
     for (uint32_t p = tid >> 5; p < ns; p += NT / 32) {
       const uint32_t k = S.list[p], beg = S.vs[k];
-      walk_prefix<32>(P.adj, beg + lane, beg + S.len[k], f);
+      walk_prefix<32>(P.adj, beg, S.len[k], lane, f);
       __syncwarp();
       part_end(j0 + k, S.vt[k]);
     }
     for (uint32_t p = 0; p < nl; ++p) {
       const uint32_t k = S.list[NT - 1 - p], beg = S.vs[k];
-      walk_prefix<NT>(P.adj, beg + tid, beg + S.len[k], f);
+      walk_prefix<NT>(P.adj, beg, S.len[k], tid, f);
       __syncwarp();
       part_end(j0 + k, S.vt[k]);
     }
@@ -426,7 +428,7 @@ __device__ __forceinline__ void block_wedges(uint32_t b, uint32_t e, const Param
     // reset is closed by a barrier in both cases: an add that came before it would be lost, and with
     // it a neighbour list of the walk.
     __syncthreads();
-  }
+  });
 }
 
 // The mid aggregator: CTAs of 128 threads with a table of about 18 KiB, ten to an SM.
@@ -467,8 +469,8 @@ struct Geom {
 // neighbour, the prefix length minus the entries below d (one binary search each).
 __device__ __forceinline__ uint64_t warp_high_wedges(const Params& P, const uint4& it, int64_t W, uint32_t d) {
   unsigned long long lo_w = 0;
-  for (uint32_t j = it.y + lane_id(); j < it.z; j += 32) {
-    const uint32_t v = P.adj[j] >> 1;
+  for (uint32_t t = lane_id(); t < it.z - it.y; t += 32) {
+    const uint32_t j = it.y + t, v = P.adj[j] >> 1;
     if (v >= P.n) continue;
     const uint32_t vb = P.off[v];
     lo_w += min(lower_bound_u32(P.adj, vb, P.off[v + 1], d << 1) - vb, P.pref[j]);
@@ -704,8 +706,8 @@ __global__ void item_features_kernel(Params P, const uint4* __restrict__ items, 
     const int64_t W = P.wsum[i + 1] - P.wsum[i];
     const uint32_t hy_dense = G.hy_dense();
     unsigned long long lo_w = 0, sumdeg = 0;
-    for (uint32_t j = b + lane; j < e; j += 32) {
-      const uint32_t v = P.adj[j] >> 1;
+    for (uint32_t t = lane; t < e - b; t += 32) {
+      const uint32_t j = b + t, v = P.adj[j] >> 1;
       if (v >= P.n) continue;
       const uint32_t vb = P.off[v], ve = P.off[v + 1];
       sumdeg += ve - vb;

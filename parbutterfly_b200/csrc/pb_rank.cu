@@ -5,6 +5,7 @@
 
 #include "pb_engine.cuh"
 #include "pb_prims.cuh"
+#include "pb_walk.cuh"
 
 namespace pb {
 
@@ -203,12 +204,12 @@ __global__ void invert_order_kernel(Lists L, const uint32_t* __restrict__ order,
   }
 }
 
-// Calls f(valid, slot, row) for every slot of [s0, s1) of a CSR (row: the slot's row), 32 slots of
+// Calls f(valid, slot, row) for every slot of [s0, s0 + len) of a CSR (row: the slot's row), 32 slots of
 // one warp at a time: work is cut by slots, not rows, since rows are as uneven as degrees (one
 // warp per row left the last hubs running alone: the wedge scan of the power-law graph with 1e7 edges
 // took 4.4 ms, in chunks of slots 0.29; its fill 1.2 and 0.14).
 template <class F>
-__device__ __forceinline__ void warp_slots(const uint32_t* __restrict__ off, int64_t n, uint32_t s0, uint32_t s1, F&& f) {
+__device__ __forceinline__ void warp_slots(const uint32_t* __restrict__ off, int64_t n, uint32_t s0, uint32_t len, F&& f) {
   const unsigned lane = threadIdx.x & 31u;
   int64_t lo = 0, hi = n;  // the last row with off[row] <= s0, 32-way search
   while (hi - lo > 1) {
@@ -218,8 +219,7 @@ __device__ __forceinline__ void warp_slots(const uint32_t* __restrict__ off, int
     hi = min(lo + step, hi);
   }
   uint32_t r = (uint32_t)lo;
-  for (uint32_t s = s0; s < s1; s += 32) {
-    const uint32_t slot = s + lane;
+  walk_groups(s0, len, 32, lane, [&](uint32_t slot, bool valid) {
     uint32_t row = r;
     for (uint32_t base = r;; base += 32) {
       // Starts of rows base + 1 .. base + 32 (off[n] lies above every slot).
@@ -229,12 +229,12 @@ __device__ __forceinline__ void warp_slots(const uint32_t* __restrict__ off, int
       for (uint32_t step = 16; step > 0; step >>= 1)
         if (__shfl_sync(0xffffffffu, bnd, c + step - 1) <= slot) c += step;
       if (__shfl_sync(0xffffffffu, bnd, c) <= slot) ++c;
-      if (slot < s1 && row == base) row = base + c;
-      if (!__any_sync(0xffffffffu, slot < s1 && row == base + 32)) break;
+      if (valid && row == base) row = base + c;
+      if (!__any_sync(0xffffffffu, valid && row == base + 32)) break;
     }
-    f(slot < s1, slot, row);
+    f(valid, slot, row);
     r = __shfl_sync(0xffffffffu, row, 31);
-  }
+  });
 }
 // Slots a warp takes at a time: 256 share the search for the first row, 32 while that many warps are
 // all resident (small graphs are bound by one warp's chain).
@@ -254,7 +254,7 @@ __global__ void ranked_fill_kernel(Lists L, const uint32_t* __restrict__ order, 
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t c = warp * chunk; c < m2; c += nwarps * chunk) {
-    warp_slots(roff, n, (uint32_t)c, (uint32_t)min(c + (int64_t)chunk, m2), [&](bool valid, uint32_t s, uint32_t r) {
+    warp_slots(roff, n, (uint32_t)c, (uint32_t)min((int64_t)chunk, m2 - c), [&](bool valid, uint32_t s, uint32_t r) {
       if (!valid) return;
       const int64_t x = order[r];
       uint32_t b, e; const uint32_t* a; int64_t sh;
@@ -302,7 +302,7 @@ __global__ void wedge_scan_kernel(const uint32_t* __restrict__ off, const uint32
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const unsigned lane = threadIdx.x & 31u;
   for (int64_t c = warp * chunk; c < m2; c += nwarps * chunk) {
-    warp_slots(off, n, (uint32_t)c, (uint32_t)min(c + (int64_t)chunk, m2), [&](bool valid, uint32_t j, uint32_t i) {
+    warp_slots(off, n, (uint32_t)c, (uint32_t)min((int64_t)chunk, m2 - c), [&](bool valid, uint32_t j, uint32_t i) {
       uint32_t L = 0;
       if (valid) {
         const uint32_t v = adj[j] >> 1;
