@@ -289,12 +289,17 @@ void run_count(pb_ctx* ctx, const pb_graph* g, const pb_opts& o, int per, int us
   if (hooks.model || hooks.trace_X) cfg.sched = &hooks;
   // Autotuner: the first call on a graph signature times the block aggregator under each
   // candidate geometry (shared-memory table bytes, CTAs per SM, warp/CTA boundary in wedges)
-  // with the plain rule and keeps the fastest for this and later calls on the context.
+  // with the plain rule and keeps the fastest for this and later calls on the context.  The first
+  // candidate is the plain path's geometry; no candidate asks for more CTAs per SM than the kernel's
+  // registers admit (three) or its tables leave room for.  Where a smaller table already holds the
+  // counters of every rank, the larger ones of the same CTA count would run the same and are left out.
   st.autotuned = 0;
   if (fused && o.autotune && R.w_rank > 0) {
-    static const int kGeom[10][3] = {{48 << 10, 4, 512}, {32 << 10, 4, 512}, {48 << 10, 2, 512}, {96 << 10, 2, 512},
-                                     {200 << 10, 1, 512}, {48 << 10, 4, 256}, {32 << 10, 4, 256},
-                                     {48 << 10, 2, 256}, {96 << 10, 2, 256}, {200 << 10, 1, 256}};
+    const CountConfig plain;
+    const int kGeom[10][3] = {{plain.smem_bytes, plain.blocks_per_sm, plain.small_w},
+                              {48 << 10, 3, 512}, {48 << 10, 2, 512}, {96 << 10, 2, 512}, {200 << 10, 1, 512},
+                              {72 << 10, 3, 256}, {48 << 10, 3, 256}, {48 << 10, 2, 256}, {96 << 10, 2, 256},
+                              {200 << 10, 1, 256}};
     const auto key = std::make_tuple(R.n, R.m2, R.w_rank, per);
     auto it = ctx->tuned.find(key);
     if (it == ctx->tuned.end()) {
@@ -306,13 +311,22 @@ void run_count(pb_ctx* ctx, const pb_graph* g, const pb_opts& o, int per, int us
       }
       double best = 1e300;
       std::array<int, 3> bg = {kGeom[0][0], kGeom[0][1], kGeom[0][2]};
+      auto same_as_smaller = [&](const int* gm) {
+        for (const auto& o : kGeom)
+          if (o[0] < gm[0] && o[1] == gm[1] && o[2] == gm[2] && R.max_deg <= 0xFFFFu && count_table_ranks(o[0]) >= R.n)
+            return true;
+        return false;
+      };
       for (const auto& gm : kGeom) {
+        if (same_as_smaller(gm)) continue;
         CountConfig t = cfg;
         t.sched = nullptr;
         t.smem_bytes = gm[0];
         t.blocks_per_sm = gm[1];
         t.small_w = gm[2];
         const CountResult r = count_ranked(R, per, tgt, t, s);
+        if (trace_on())
+          fprintf(stderr, "[pb] autotune %d bytes x %d CTAs, warp %d: %.3f ms\n", gm[0], gm[1], gm[2], r.agg_ms);
         if (r.agg_ms < best) {
           best = r.agg_ms;
           bg = {gm[0], gm[1], gm[2]};

@@ -838,7 +838,11 @@ __global__ void sched_explore_kernel(const uint8_t* __restrict__ valid, uint32_t
   }
 }
 
+uint32_t table_words(size_t smem_bytes, size_t fixed) { return (uint32_t)((smem_bytes - fixed) / 4) & ~31u; }
+
 }  // namespace
+
+int64_t count_table_ranks(int smem_bytes) { return 2 * (int64_t)table_words(smem_bytes, shared_fixed<kBlock>()); }
 
 CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConfig& cfg, cudaStream_t s) {
   CountResult res;
@@ -894,7 +898,7 @@ CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConf
   if (hook_smem) smem_bytes = std::max(16384, std::min(atoi(hook_smem), cfg.smem_bytes));
   if (const char* ev = getenv("PB_COUNT_SMALL_W")) small_w = std::max(0, std::min(atoi(ev), small_w));
   int blocks_per_sm = cfg.blocks_per_sm;
-  if (const char* ev = getenv("PB_COUNT_BPS")) blocks_per_sm = std::max(1, std::min(atoi(ev), 4));
+  if (const char* ev = getenv("PB_COUNT_BPS")) blocks_per_sm = std::max(1, std::min(atoi(ev), kBlockPerSm));
   int64_t sched_min_w = kSchedMinWedges;
   if (const char* ev = getenv("PB_SCHED_MIN_WEDGES")) sched_min_w = atoll(ev);  // test hook: score light items too
 
@@ -904,7 +908,7 @@ CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConf
   const int count_bits = 32 - std::max(1, key_bits);
   auto geom_of = [&](size_t bytes, size_t fixed) {
     Geom g;
-    g.tw = (uint32_t)((bytes - fixed) / 4) & ~31u;
+    g.tw = table_words(bytes, fixed);
     g.hy_words = (g.tw / 4 * 3) & ~31u;
     g.cb = count_bits;
     return g;

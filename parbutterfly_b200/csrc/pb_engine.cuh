@@ -107,6 +107,8 @@ struct CountResult {
 // Fills the result from the tail's host copy and the (completed) events; throws on a recorded
 // bounds violation.
 void finish_count(CountResult& res, const CountTail& tail, const cudaEvent_t* ev);
+// Ranks whose 16-bit counters the block aggregator holds in smem_bytes of shared memory.
+int64_t count_table_ranks(int smem_bytes);
 CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConfig& cfg, cudaStream_t s);
 // SORT (hist = false) and HIST (hist = true) aggregators over materialised wedge batches of at
 // most max_wedges wedges (pb_agg_sort.cu).
