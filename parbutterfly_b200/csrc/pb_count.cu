@@ -431,9 +431,16 @@ __device__ __forceinline__ void block_wedges(uint32_t b, uint32_t e, const Param
   });
 }
 
-// The mid aggregator: CTAs of 128 threads with a table of about 18 KiB, ten to an SM.
-constexpr int kMidSmem = 22 << 10;
+// The mid aggregator: CTAs of 128 threads with a table of about 19.5 KiB, ten to an SM.  An SM has
+// 228 KiB, of which every resident CTA takes one for the system: with 22 KiB each, nine fit and the
+// tenth of the grid starts when the others are through (aggregation of the R-MAT graph with 2^24 edges
+// per edge 18.46 ms; a grid of nine per SM 18.43, ten of 21.5 KiB 18.15).
+constexpr int kMidSmem = 43 << 9;
 constexpr int kMidPerSm = 10;
+constexpr int kSmBytes = 228 << 10, kCtaReserved = 1 << 10;
+static_assert(kMidPerSm * (kMidSmem + kCtaReserved) <= kSmBytes, "the mid CTAs of an SM must be resident together");
+static_assert(kBlockPerSm * (CountConfig{}.smem_bytes + kCtaReserved) <= kSmBytes,
+              "the block CTAs of an SM must be resident together");
 constexpr int64_t kMidWedges = 2047;
 
 enum Mode : uint32_t { MODE_DENSE = 0, MODE_HASH = 1, MODE_GLOBAL = 2, MODE_HYBRID = 3 };
