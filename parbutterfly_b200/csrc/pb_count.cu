@@ -42,6 +42,7 @@ namespace {
 constexpr uint32_t kEmpty = 0xFFFFFFFFu;
 constexpr int kWarpTable = 1024;  // slots per warp
 constexpr int kWarpsPerBlockSmall = 8;
+constexpr int64_t kListRange = int64_t(1) << 26;  // endpoints that the item lists hold at a time
 constexpr uint32_t kHotRanks = 256;   // count_warp_kernel: vertex counts gathered per CTA
 // A row is walked by the threads that own its endpoint, however few wedges it has, so long rows move
 // up a class: beyond kWarpRow slots to a CTA of 128 threads, beyond kMidRow to one of 512.  Limits of
@@ -670,15 +671,16 @@ __global__ void edge_gather_kernel(Params P, const uint32_t* __restrict__ eout) 
   }
 }
 
-// Splits the endpoints with wedges into the warp, mid and block lists.
+// Splits the endpoints [i0, n) with wedges into the warp, mid and block lists.
 // counts: [0] block, [1] global scratch, [2] block cursor, [3] warp, [4] mid, [5] mid cursor.
-__global__ void classify_endpoints_kernel(const int64_t* __restrict__ wsum, const uint32_t* __restrict__ off, int64_t n,
-                                          int small_w, int64_t mid_w, Geom mid, uint4* small_items, uint4* mid_items,
-                                          uint4* items, uint32_t* counts, uint32_t* err) {
+__global__ void classify_endpoints_kernel(const int64_t* __restrict__ wsum, const uint32_t* __restrict__ off,
+                                          int64_t i0, int64_t n, int small_w, int64_t mid_w, Geom mid,
+                                          uint4* small_items, uint4* mid_items, uint4* items, uint32_t* counts,
+                                          uint32_t* err) {
   const int64_t step = (int64_t)gridDim.x * blockDim.x;
-  const int64_t rounds = (n + step - 1) / step;
+  const int64_t rounds = (n - i0 + step - 1) / step;
   for (int64_t r = 0; r < rounds; ++r) {
-    const int64_t i = r * step + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t i = i0 + r * step + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int64_t W = 0;
     uint4 it = make_uint4(0, 0, 0, 0);
     if (i < n) {
@@ -845,6 +847,14 @@ __global__ void sched_explore_kernel(const uint8_t* __restrict__ valid, uint32_t
   }
 }
 
+// What the scheduled items of one list ran with, read back when the call's kernels are through.
+struct SchedRecord {
+  uint32_t items;
+  DevBuf<float> F, pred;
+  DevBuf<uint8_t> used;
+  DevBuf<unsigned long long> cycles;
+};
+
 uint32_t table_words(size_t smem_bytes, size_t fixed) { return (uint32_t)((smem_bytes - fixed) / 4) & ~31u; }
 
 }  // namespace
@@ -873,9 +883,6 @@ CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConf
     own_tail.alloc(1, s);
     tail = own_tail.get();
     PB_CUDA_TRY(cudaMemsetAsync(tail, 0, sizeof(CountTail), s));
-  } else {
-    // (the autotuner runs several counts on one tail)
-    PB_CUDA_TRY(cudaMemsetAsync(tail->counts, 0, sizeof(tail->counts), s));
   }
   P.err = cfg.err ? cfg.err : tail->err;
   P.mstats = tail->mstats;
@@ -928,148 +935,159 @@ CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConf
   int64_t mid_w = kMidWedges;
   if (hook_smem || (sh && sh->trace_X)) mid_w = 0;
   else if (sh && sh->model) mid_w = std::min(mid_w, sched_min_w - 1);
-  DevBuf<uint4> lists((size_t)n * 3, s);  // warp, mid and block lists
-  uint4 *small_items = lists.get(), *mid_items = small_items + n, *items = mid_items + n;
-  DevBuf<uint8_t> modes(n, s);
-  PB_LAUNCH(classify_endpoints_kernel, std::max(1, std::min(ceil_div(n, 256), sms * 8)), 256, 0, s, R.wsum.get(),
-            R.off.get(), n, small_w, mid_w, Gm, small_items, mid_items, items, counts, P.err);
-  uint32_t hc[5];
-  readback(hc, counts, sizeof(hc), s);
-  const uint32_t n_block = hc[0], n_small = hc[3], n_mid = hc[4];
-  if (n_block > 0) {
-    PB_LAUNCH(plain_modes_kernel, (int)std::min<int64_t>(ceil_div(n_block, 8), sms * 8), 256, 0, s, P, items,
-              counts, G, modes.get(), counts + 1);
-    readback(&hc[1], counts + 1, sizeof(uint32_t), s);
-  }
-  res.n_big = (int)(n_block + n_mid);
-
   // Under graph capture nothing is timed or read back here (the recording run checked).
   const bool cap = capturing();
   cudaEvent_t ev[2] = {nullptr, nullptr};
-  if (!cap) {
-    if (cfg.ev) std::copy(cfg.ev, cfg.ev + 2, ev);
-    else
-      for (auto& e : ev) PB_CUDA_TRY(cudaEventCreate(&e));
-    PB_CUDA_TRY(cudaEventRecord(ev[0], s));
-  }
-  // Scheduler: per-item modes (learned or exploring) and the record of what each item ran
-  // with and how long it took.
-  const bool sched_on = sh && n_block > 0 && (sh->model || sh->explore || sh->trace_X);
-  DevBuf<float> sF, sPred;
-  DevBuf<uint8_t> sValid, sUsed;
-  DevBuf<uint32_t> sNG;
-  DevBuf<unsigned long long> sCyc;
-  bool need_global = hc[1] > 0;
-  if (sched_on) {
-    const uint32_t ni = n_block;
-    cudaEvent_t a0, a1;
-    PB_CUDA_TRY(cudaEventCreate(&a0));
-    PB_CUDA_TRY(cudaEventCreate(&a1));
-    PB_CUDA_TRY(cudaEventRecord(a0, s));
-    sF.alloc((size_t)ni * kMlpIn, s);
-    sValid.alloc(ni, s);
-    sUsed.alloc(ni, s);
-    sCyc.alloc(ni, s);
-    sNG.alloc(1, s);
-    PB_CUDA_TRY(cudaMemsetAsync(sNG.get(), 0, sizeof(uint32_t), s));
-    const int g1 = std::max(1, std::min(ceil_div(ni, 256), sms * 8));
-    // Learned choices score only the items heavy enough for the mode to matter (the rest keep
-    // the plain rule, so the scheduler's own cost stays small); tracing covers every item.
-    if (sh->model && !sh->trace_X) {
-      DevBuf<uint32_t> sub(ni, s), nsub(1, s);
-      PB_CUDA_TRY(cudaMemsetAsync(nsub.get(), 0, sizeof(uint32_t), s));
-      PB_LAUNCH(heavy_items_kernel, g1, 256, 0, s, items, ni, R.wsum.get(), sched_min_w, sub.get(), nsub.get());
-      uint32_t nh = 0;
-      readback(&nh, nsub.get(), sizeof(nh), s);
-      sPred.alloc(ni, s);
-      PB_CUDA_TRY(cudaMemsetAsync(sPred.get(), 0xFF, sizeof(float) * ni, s));  // NaN: no prediction
-      PB_CUDA_TRY(cudaMemsetAsync(sF.get(), 0, sF.bytes(), s));
-      if (nh > 0) {
-        DevBuf<uint4> hitems(nh, s);
-        DevBuf<float> hF((size_t)nh * kMlpIn, s), hPr(nh, s);
-        DevBuf<uint8_t> hValid(nh, s), hModes(nh, s);
-        const int gh = std::max(1, std::min(ceil_div(nh, 256), sms * 8));
-        PB_LAUNCH(gather_items_kernel, gh, 256, 0, s, items, sub.get(), nh, hitems.get());
-        PB_LAUNCH(item_features_kernel, std::max(1, std::min(ceil_div((int64_t)nh * 32, 256), sms * 8)), 256, 0, s, P,
-                  hitems.get(), nh, G, hF.get(), hValid.get());
-        DevBuf<float> X((size_t)nh * 3 * kMlpIn, s), y((size_t)nh * 3, s);
-        PB_LAUNCH(sched_candidates_kernel, std::max(1, std::min(ceil_div((int64_t)nh * 3 * kMlpIn, 256), sms * 8)), 256,
-                  0, s, hF.get(), nh, X.get());
-        sh->model->predict_dev(X.get(), (int64_t)nh * 3, y.get(), s);
-        PB_LAUNCH(sched_choose_kernel, gh, 256, 0, s, y.get(), hValid.get(), nh, hModes.get(), hPr.get(), sNG.get());
-        PB_LAUNCH(scatter_scored_kernel, gh, 256, 0, s, sub.get(), nh, hModes.get(), hPr.get(), hF.get(), modes.get(),
-                  sPred.get(), sF.get());
-      }
-    } else {
-      PB_LAUNCH(item_features_kernel, std::max(1, std::min(ceil_div((int64_t)ni * 32, 256), sms * 8)), 256, 0, s, P,
-                items, ni, G, sF.get(), sValid.get());
-    }
-    if (sh->model && sh->trace_X) {
-      DevBuf<float> X((size_t)ni * 3 * kMlpIn, s), y((size_t)ni * 3, s);
-      PB_LAUNCH(sched_candidates_kernel, std::max(1, std::min(ceil_div((int64_t)ni * 3 * kMlpIn, 256), sms * 8)), 256,
-                0, s, sF.get(), ni, X.get());
-      sh->model->predict_dev(X.get(), (int64_t)ni * 3, y.get(), s);
-      sPred.alloc(ni, s);
-      PB_LAUNCH(sched_choose_kernel, g1, 256, 0, s, y.get(), sValid.get(), ni, modes.get(), sPred.get(), sNG.get());
-    } else if (sh->explore) {
-      PB_LAUNCH(sched_explore_kernel, g1, 256, 0, s, sValid.get(), ni, sh->seed, modes.get(), sNG.get());
-    }
-    P.mode_out = sUsed.get();
-    P.cycles = sCyc.get();
-    uint32_t ng = 0;
-    PB_CUDA_TRY(cudaMemcpyAsync(&ng, sNG.get(), sizeof(ng), cudaMemcpyDeviceToHost, s));
-    PB_CUDA_TRY(cudaEventRecord(a1, s));
-    PB_CUDA_TRY(cudaEventSynchronize(a1));
-    need_global = ng > 0 || hc[1] > 0;  // unscored items follow the plain rule
-    float ms = 0;
-    PB_CUDA_TRY(cudaEventElapsedTime(&ms, a0, a1));
-    sh->ms = ms;
-    cudaEventDestroy(a0);
-    cudaEventDestroy(a1);
-  }
+  if (!cap && !cfg.ev)
+    for (auto& e : ev) PB_CUDA_TRY(cudaEventCreate(&e));
+  else if (!cap)
+    std::copy(cfg.ev, cfg.ev + 2, ev);
+  // The lists hold kListRange endpoints at a time, so that they take 3.2 GB at most (48 bytes an endpoint,
+  // where the other arrays of a call take 40 to 48).
+  const int64_t nl = std::min(n, kListRange);
+  DevBuf<uint4> lists((size_t)nl * 3, s);  // warp, mid and block lists
+  uint4 *small_items = lists.get(), *mid_items = small_items + nl, *items = mid_items + nl;
+  DevBuf<uint8_t> modes(nl, s);
   DevBuf<uint32_t> gscratch;
-  if (n_block > 0) {
-    int grid = (int)std::min<int64_t>(n_block, (int64_t)sms * blocks_per_sm);
-    if (need_global) {
-      // One dense counter array of n entries per CTA: at very large n (the 1e9-edge R-MAT) the
-      // CTA count is capped so the arrays stay within half of the free device memory (64 GB at
-      // most).
-      size_t free_b = 0, total_b = 0;
-      PB_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-      const size_t budget = std::min<size_t>(free_b / 2, size_t(64) << 30);
-      const size_t per_cta = (size_t)n * sizeof(uint32_t);
-      grid = (int)std::max<int64_t>(1, std::min<int64_t>(grid, (int64_t)(budget / per_cta)));
-      gscratch.alloc((size_t)grid * (size_t)n, s);
-      PB_CUDA_TRY(cudaMemsetAsync(gscratch.get(), 0, gscratch.bytes(), s));
+  std::vector<SchedRecord> records;
+  for (int64_t i0 = 0; i0 < n; i0 += kListRange) {
+    const int64_t i1 = std::min(n, i0 + kListRange);
+    if (i0 > 0) PB_CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(tail->counts), s));
+    PB_LAUNCH(classify_endpoints_kernel, std::max(1, std::min(ceil_div(i1 - i0, 256), sms * 8)), 256, 0, s, R.wsum.get(),
+              R.off.get(), i0, i1, small_w, mid_w, Gm, small_items, mid_items, items, counts, P.err);
+    uint32_t hc[5];
+    readback(hc, counts, sizeof(hc), s);
+    const uint32_t n_block = hc[0], n_small = hc[3], n_mid = hc[4];
+    if (n_block > 0) {
+      PB_LAUNCH(plain_modes_kernel, (int)std::min<int64_t>(ceil_div(n_block, 8), sms * 8), 256, 0, s, P, items,
+                counts, G, modes.get(), counts + 1);
+      readback(&hc[1], counts + 1, sizeof(uint32_t), s);
     }
-    P.modes = modes.get();
-    auto kern = count_block_kernel<kBlock, kBlockPerSm>;
-    PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
-    PB_LAUNCH(kern, grid, kBlock, smem_bytes, s, P, items, counts, counts + 2, gscratch.get(), G);
-  }
-  P.modes = nullptr;
-  P.mode_out = nullptr;
-  P.cycles = nullptr;
-  if (n_mid > 0) {
-    auto kern = count_block_kernel<kMidBlock, kMidPerSm>;
-    PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMidSmem));
-    PB_LAUNCH(kern, (int)std::min<int64_t>(n_mid, (int64_t)sms * kMidPerSm), kMidBlock, kMidSmem, s, P, mid_items,
-              counts + 4, counts + 5, (uint32_t*)nullptr, Gm);
-  }
-  if (n_small > 0) {
-    const bool one_word = (uint32_t)small_w <= (1u << count_bits) - 2u;
-    auto kern = one_word ? count_warp_kernel<true> : count_warp_kernel<false>;
-    const int smem =
-        (2 * (int)kHotRanks + kWarpsPerBlockSmall * ((one_word ? 1 : 2) * kWarpTable + 32)) * (int)sizeof(uint32_t);
-    PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    PB_LAUNCH(kern, (int)std::min<int64_t>(ceil_div(n_small, kWarpsPerBlockSmall), (int64_t)sms * (one_word ? 6 : 3)),
-              kWarpsPerBlockSmall * 32, smem, s, P, small_items, counts + 3, count_bits);
+    res.n_big += (int)(n_block + n_mid);
+    if (!cap && i0 == 0) PB_CUDA_TRY(cudaEventRecord(ev[0], s));
+    // Scheduler: per-item modes (learned or exploring) and the record of what each item ran
+    // with and how long it took.
+    const bool sched_on = sh && n_block > 0 && (sh->model || sh->explore || sh->trace_X);
+    DevBuf<float> sF, sPred;
+    DevBuf<uint8_t> sValid, sUsed;
+    DevBuf<uint32_t> sNG;
+    DevBuf<unsigned long long> sCyc;
+    bool need_global = hc[1] > 0;
+    if (sched_on) {
+      const uint32_t ni = n_block;
+      cudaEvent_t a0, a1;
+      PB_CUDA_TRY(cudaEventCreate(&a0));
+      PB_CUDA_TRY(cudaEventCreate(&a1));
+      PB_CUDA_TRY(cudaEventRecord(a0, s));
+      sF.alloc((size_t)ni * kMlpIn, s);
+      sValid.alloc(ni, s);
+      sUsed.alloc(ni, s);
+      sCyc.alloc(ni, s);
+      sNG.alloc(1, s);
+      PB_CUDA_TRY(cudaMemsetAsync(sNG.get(), 0, sizeof(uint32_t), s));
+      const int g1 = std::max(1, std::min(ceil_div(ni, 256), sms * 8));
+      // Learned choices score only the items heavy enough for the mode to matter (the rest keep
+      // the plain rule, so the scheduler's own cost stays small); tracing covers every item.
+      if (sh->model && !sh->trace_X) {
+        DevBuf<uint32_t> sub(ni, s), nsub(1, s);
+        PB_CUDA_TRY(cudaMemsetAsync(nsub.get(), 0, sizeof(uint32_t), s));
+        PB_LAUNCH(heavy_items_kernel, g1, 256, 0, s, items, ni, R.wsum.get(), sched_min_w, sub.get(), nsub.get());
+        uint32_t nh = 0;
+        readback(&nh, nsub.get(), sizeof(nh), s);
+        sPred.alloc(ni, s);
+        PB_CUDA_TRY(cudaMemsetAsync(sPred.get(), 0xFF, sizeof(float) * ni, s));  // NaN: no prediction
+        PB_CUDA_TRY(cudaMemsetAsync(sF.get(), 0, sF.bytes(), s));
+        if (nh > 0) {
+          DevBuf<uint4> hitems(nh, s);
+          DevBuf<float> hF((size_t)nh * kMlpIn, s), hPr(nh, s);
+          DevBuf<uint8_t> hValid(nh, s), hModes(nh, s);
+          const int gh = std::max(1, std::min(ceil_div(nh, 256), sms * 8));
+          PB_LAUNCH(gather_items_kernel, gh, 256, 0, s, items, sub.get(), nh, hitems.get());
+          PB_LAUNCH(item_features_kernel, std::max(1, std::min(ceil_div((int64_t)nh * 32, 256), sms * 8)), 256, 0, s, P,
+                    hitems.get(), nh, G, hF.get(), hValid.get());
+          DevBuf<float> X((size_t)nh * 3 * kMlpIn, s), y((size_t)nh * 3, s);
+          PB_LAUNCH(sched_candidates_kernel, std::max(1, std::min(ceil_div((int64_t)nh * 3 * kMlpIn, 256), sms * 8)), 256,
+                    0, s, hF.get(), nh, X.get());
+          sh->model->predict_dev(X.get(), (int64_t)nh * 3, y.get(), s);
+          PB_LAUNCH(sched_choose_kernel, gh, 256, 0, s, y.get(), hValid.get(), nh, hModes.get(), hPr.get(), sNG.get());
+          PB_LAUNCH(scatter_scored_kernel, gh, 256, 0, s, sub.get(), nh, hModes.get(), hPr.get(), hF.get(), modes.get(),
+                    sPred.get(), sF.get());
+        }
+      } else {
+        PB_LAUNCH(item_features_kernel, std::max(1, std::min(ceil_div((int64_t)ni * 32, 256), sms * 8)), 256, 0, s, P,
+                  items, ni, G, sF.get(), sValid.get());
+      }
+      if (sh->model && sh->trace_X) {
+        DevBuf<float> X((size_t)ni * 3 * kMlpIn, s), y((size_t)ni * 3, s);
+        PB_LAUNCH(sched_candidates_kernel, std::max(1, std::min(ceil_div((int64_t)ni * 3 * kMlpIn, 256), sms * 8)), 256,
+                  0, s, sF.get(), ni, X.get());
+        sh->model->predict_dev(X.get(), (int64_t)ni * 3, y.get(), s);
+        sPred.alloc(ni, s);
+        PB_LAUNCH(sched_choose_kernel, g1, 256, 0, s, y.get(), sValid.get(), ni, modes.get(), sPred.get(), sNG.get());
+      } else if (sh->explore) {
+        PB_LAUNCH(sched_explore_kernel, g1, 256, 0, s, sValid.get(), ni, sh->seed, modes.get(), sNG.get());
+      }
+      P.mode_out = sUsed.get();
+      P.cycles = sCyc.get();
+      uint32_t ng = 0;
+      PB_CUDA_TRY(cudaMemcpyAsync(&ng, sNG.get(), sizeof(ng), cudaMemcpyDeviceToHost, s));
+      PB_CUDA_TRY(cudaEventRecord(a1, s));
+      PB_CUDA_TRY(cudaEventSynchronize(a1));
+      need_global = ng > 0 || hc[1] > 0;  // unscored items follow the plain rule
+      float ms = 0;
+      PB_CUDA_TRY(cudaEventElapsedTime(&ms, a0, a1));
+      sh->ms += ms;
+      cudaEventDestroy(a0);
+      cudaEventDestroy(a1);
+    }
+    if (n_block > 0) {
+      int grid = (int)std::min<int64_t>(n_block, (int64_t)sms * blocks_per_sm);
+      if (need_global) {
+        // One dense counter array of n entries per CTA: at very large n (the 1e9-edge R-MAT) the
+        // CTA count is capped so the arrays stay within half of the free device memory (64 GB at
+        // most).
+        if (!gscratch.get()) {
+          size_t free_b = 0, total_b = 0;
+          PB_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
+          const size_t budget = std::min<size_t>(free_b / 2, size_t(64) << 30);
+          const size_t per_cta = (size_t)n * sizeof(uint32_t);
+          const int want = i1 < n ? sms * blocks_per_sm : grid;  // later lists may be longer
+          const int ctas = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)(budget / per_cta)));
+          gscratch.alloc((size_t)ctas * (size_t)n, s);
+          PB_CUDA_TRY(cudaMemsetAsync(gscratch.get(), 0, gscratch.bytes(), s));
+        }
+        grid = (int)std::min<int64_t>(grid, (int64_t)(gscratch.n / (size_t)n));
+      }
+      P.modes = modes.get();
+      auto kern = count_block_kernel<kBlock, kBlockPerSm>;
+      PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
+      PB_LAUNCH(kern, grid, kBlock, smem_bytes, s, P, items, counts, counts + 2, gscratch.get(), G);
+    }
+    P.modes = nullptr;
+    P.mode_out = nullptr;
+    P.cycles = nullptr;
+    if (n_mid > 0) {
+      auto kern = count_block_kernel<kMidBlock, kMidPerSm>;
+      PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMidSmem));
+      PB_LAUNCH(kern, (int)std::min<int64_t>(n_mid, (int64_t)sms * kMidPerSm), kMidBlock, kMidSmem, s, P, mid_items,
+                counts + 4, counts + 5, (uint32_t*)nullptr, Gm);
+    }
+    if (n_small > 0) {
+      const bool one_word = (uint32_t)small_w <= (1u << count_bits) - 2u;
+      auto kern = one_word ? count_warp_kernel<true> : count_warp_kernel<false>;
+      const int smem =
+          (2 * (int)kHotRanks + kWarpsPerBlockSmall * ((one_word ? 1 : 2) * kWarpTable + 32)) * (int)sizeof(uint32_t);
+      PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      PB_LAUNCH(kern, (int)std::min<int64_t>(ceil_div(n_small, kWarpsPerBlockSmall), (int64_t)sms * (one_word ? 6 : 3)),
+                kWarpsPerBlockSmall * 32, smem, s, P, small_items, counts + 3, count_bits);
+    }
+    if (sched_on) records.push_back({n_block, std::move(sF), std::move(sPred), std::move(sUsed), std::move(sCyc)});
   }
   if (per == EDGE)
     PB_LAUNCH(edge_gather_kernel, std::max(1, std::min(ceil_div(R.m2, 256), sms * 8)), 256, 0, s, P, R.eout.get());
   if (cap) return res;
   PB_CUDA_TRY(cudaEventRecord(ev[1], s));
-  if (cfg.tail && cfg.ev && !sched_on) {
+  if (cfg.tail && cfg.ev && records.empty()) {
     res.pending = true;
     return res;
   }
@@ -1077,20 +1095,20 @@ CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConf
   PB_CUDA_TRY(cudaMemcpyAsync(&h, tail, sizeof(h), cudaMemcpyDeviceToHost, s));
   PB_CUDA_TRY(cudaStreamSynchronize(s));
   finish_count(res, h, ev);
-  if (sched_on) {
-    const uint32_t ni = n_block;
+  double mae_sum = 0;
+  int64_t npred = 0;
+  for (const SchedRecord& r : records) {
+    const uint32_t ni = r.items;
     std::vector<float> hF((size_t)ni * kMlpIn), hPred;
     std::vector<uint8_t> hUsed(ni);
     std::vector<unsigned long long> hCyc(ni);
-    PB_CUDA_TRY(cudaMemcpy(hF.data(), sF.get(), sF.bytes(), cudaMemcpyDeviceToHost));
-    PB_CUDA_TRY(cudaMemcpy(hUsed.data(), sUsed.get(), sUsed.bytes(), cudaMemcpyDeviceToHost));
-    PB_CUDA_TRY(cudaMemcpy(hCyc.data(), sCyc.get(), sCyc.bytes(), cudaMemcpyDeviceToHost));
+    PB_CUDA_TRY(cudaMemcpy(hF.data(), r.F.get(), r.F.bytes(), cudaMemcpyDeviceToHost));
+    PB_CUDA_TRY(cudaMemcpy(hUsed.data(), r.used.get(), r.used.bytes(), cudaMemcpyDeviceToHost));
+    PB_CUDA_TRY(cudaMemcpy(hCyc.data(), r.cycles.get(), r.cycles.bytes(), cudaMemcpyDeviceToHost));
     if (sh->model) {
       hPred.resize(ni);
-      PB_CUDA_TRY(cudaMemcpy(hPred.data(), sPred.get(), sPred.bytes(), cudaMemcpyDeviceToHost));
+      PB_CUDA_TRY(cudaMemcpy(hPred.data(), r.pred.get(), r.pred.bytes(), cudaMemcpyDeviceToHost));
     }
-    double pc = 0, mc = 0, mae = 0;
-    int64_t npred = 0;
     for (uint32_t q = 0; q < ni; ++q) {
       const double cyc = (double)std::max<unsigned long long>(hCyc[q], 1ull);
       const double lc = std::log2(cyc);
@@ -1101,17 +1119,15 @@ CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConf
         sh->trace_y->push_back((float)lc);
       }
       if (sh->model && hPred[q] >= 0.f) {  // items the model predicted (not the fallback)
-        mc += cyc;
-        pc += std::exp2((double)hPred[q]);
-        mae += std::fabs((double)hPred[q] - lc);
+        sh->meas_cycles += cyc;
+        sh->pred_cycles += std::exp2((double)hPred[q]);
+        mae_sum += std::fabs((double)hPred[q] - lc);
         ++npred;
       }
     }
-    sh->items = ni;
-    sh->meas_cycles = mc;
-    sh->pred_cycles = pc;
-    sh->mae_log2 = npred ? mae / npred : 0.0;
+    sh->items += ni;
   }
+  if (!records.empty()) sh->mae_log2 = npred ? mae_sum / npred : 0.0;
   if (!cfg.ev)
     for (auto& e : ev) cudaEventDestroy(e);
   return res;

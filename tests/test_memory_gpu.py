@@ -1,0 +1,80 @@
+"""Device memory that calls take beside their inputs and outputs: graphs of many vertices and few
+edges, where arrays per vertex decide, and calls that must get by with what is left of a device."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import oracle
+from parbutterfly_b200 import butterflies as pb
+from parbutterfly_b200.graph import BipartiteGraph
+
+pytestmark = pytest.mark.gpu
+
+USED_HIGH = 8  # CU_MEMPOOL_ATTR_USED_MEM_HIGH
+
+
+class _Pool:
+    """The device's default memory pool, from which the library allocates."""
+
+    def __init__(self):
+        import torch
+        torch.cuda.init()
+        self.cu = C.CDLL("libcuda.so.1")
+        self.pool = C.c_void_p()
+        assert self.cu.cuDeviceGetDefaultMemPool(C.byref(self.pool), 0) == 0
+
+    def reset(self):
+        assert self.cu.cuMemPoolSetAttribute(self.pool, USED_HIGH, C.byref(C.c_uint64(0))) == 0
+        return self.high()
+
+    def high(self):
+        x = C.c_uint64()
+        assert self.cu.cuMemPoolGetAttribute(self.pool, USED_HIGH, C.byref(x)) == 0
+        return x.value
+
+    def trim(self):
+        assert self.cu.cuMemPoolTrimTo(self.pool, C.c_size_t(0)) == 0
+
+
+@pytest.fixture(scope="module")
+def pool():
+    return _Pool()
+
+
+def _spread(nu, k, nv, deg, seed):
+    """k U-vertices spread over [0, nu), each with `deg` draws of nv V-vertices: the graph on the GPU, the
+    same graph without the isolated U-vertices, and the U-vertices' ids."""
+    import torch
+    rng = np.random.default_rng(seed)
+    ids = np.unique(np.r_[0, nu - 1, rng.integers(0, nu, k)])
+    small = BipartiteGraph.from_edges(nv, ids.size, rng.integers(0, nv, ids.size * deg), np.repeat(np.arange(ids.size), deg))
+    at = torch.from_numpy(ids).cuda()
+    deg_u = torch.zeros(nu + 1, dtype=torch.int64, device="cuda")
+    deg_u[at + 1] = torch.from_numpy(np.diff(small.offsetsU.astype(np.int64))).cuda()
+    off_u = torch.cumsum(deg_u, 0).to(torch.int32)
+    del deg_u
+    off_v, edg_u = (torch.from_numpy(a.astype(np.int32)).cuda() for a in (small.offsetsV, small.edgesU))
+    edg_v = at[torch.from_numpy(small.edgesV.astype(np.int64)).cuda()].to(torch.int32)
+    torch.cuda.synchronize()
+    return (nv, nu, off_v, edg_v, off_u, edg_u), small, at
+
+
+def test_count_lists_of_many_vertices(ctx, pool):
+    """Endpoints in three stretches of the ranks; item lists for all vertices at once would take 48 bytes
+    each."""
+    import torch
+    nu = (1 << 27) + 12_345
+    arrays, small, at = _spread(nu, 40_000, 1000, 5, 1)
+    dg = pb.DeviceGraph(ctx, device_arrays=arrays)
+    del arrays
+    base = pool.reset()
+    out = torch.zeros(nu, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    pb.count(dg, "BATCHS", "SIDE", use_v=True, out=out)
+    assert pool.high() - base < 56 * nu  # 28 for the ranking and the sums, 24 for lists of 2^26 endpoints
+    assert np.array_equal(out[at].cpu().numpy(), oracle.count(small, "VERT", "SIDE", use_v=True)[0])
+    assert int(torch.count_nonzero(out)) == int(torch.count_nonzero(out[at]))
+    assert np.array_equal(pb.count_e(dg, "HASH", "SIDE", use_v=True), oracle.count(small, "EDGE", "SIDE", use_v=True)[0])
+    assert pb.count_total(dg, "SERIAL", "SIDE", use_v=True) == oracle.count(small, "TOTAL", "SIDE", use_v=True)[0]
+    dg.close()
