@@ -1932,13 +1932,20 @@ __global__ void center_of_kernel(const uint32_t* __restrict__ offC, int64_t nC, 
     for (uint32_t j = offC[v] + lane; j < offC[v + 1]; j += 32) center_of[j] = (uint32_t)v;
 }
 
-__global__ void max_i64_kernel(const int64_t* __restrict__ a, int64_t n, unsigned long long* out) {
-  unsigned long long m = 0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+// out[0] = the maximum of a, out[1] = how many entries lie above `above`.
+__global__ void max_i64_kernel(const int64_t* __restrict__ a, int64_t n, int64_t above, unsigned long long* out) {
+  unsigned long long m = 0, c = 0;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     m = max(m, (unsigned long long)a[i]);
+    c += a[i] > above;
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, m);
+  c = warp_sum(c);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(out, m);
+    if (c) atomicAdd(out + 1, c);
+  }
 }
 
 // Live-entry count per vertex.  kByEdge: an entry is live when its edge is not peeled
@@ -2235,10 +2242,6 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
   DevBuf<int64_t> cnt(N, s);
   DevBuf<uint32_t> eti, iota, center_of, alist0(N, s), alist1(N, s), nearl(N, s);
   DevBuf<uint4> fr0(N, s), fr1(N, s), fh0, fh1;
-  if (!kWing) {
-    fh0.alloc(N, s);
-    fh1.alloc(N, s);
-  }
   // Independent instances (the graphs of a batch) or the whole input as one.
   std::vector<int64_t> pbase{0}, psize{N};
   std::vector<double> pweight{1.0};
@@ -2255,7 +2258,7 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
     if (pbase.empty()) return res;
   }
   // Grid-shared dense counters: tip peeling keeps one slice per heavy item of a wave (they run
-  // concurrently), up to 32 slices within kGsharedBudget.
+  // concurrently), up to kMaxGroups slices within kGsharedBudget.
   const int64_t gstride = std::max(G.nK, G.nC) + 1;
   const unsigned ngroups =
       (unsigned)std::max<int64_t>(1, std::min<int64_t>(kMaxGroups, kGsharedBudget / (4 * gstride)));
@@ -2290,6 +2293,10 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
   std::vector<std::unique_ptr<DevBuf<int64_t>>> work_bufs;
   std::vector<std::unique_ptr<DevBuf<uint32_t>>> info_bufs;
   auto refresh_work = [&](Lists& L) {
+    if (!two_phase) {  // stream-ordered: whoever reads the old ones has been launched
+      work_bufs.clear();
+      info_bufs.clear();
+    }
     auto buf = std::make_unique<DevBuf<int64_t>>(kWing ? L.nK + L.nC : L.nK, s);
     if (kWing) {
       if (L.nK) PB_LAUNCH(nbr_degree_sum_kernel, grid_for(L.nK * 32), 256, 0, s, L.offK, L.edgK, L.offC, L.nK, buf->get());
@@ -2302,17 +2309,16 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
       PB_LAUNCH(total_weight_kernel<kWing>, grid_for(N), 256, 0, s, L, cls, N, total.get());
       PB_LAUNCH(wing_info_kernel, grid_for(N), 256, 0, s, L, cls, N, total.get(), info->get());
       L.info = info->get();
-      if (!two_phase) info_bufs.clear();
       info_bufs.push_back(std::move(info));
     } else {
       PB_LAUNCH(tip_work_kernel, grid_for(L.nK * 32), 256, 0, s, L.offK, L.edgK, L.offC, L.nK, buf->get());
       L.wk = buf->get();
     }
-    if (!two_phase) work_bufs.clear();
     work_bufs.push_back(std::move(buf));
   };
   bool need_scratch = false;
   int64_t scratch_len = 0;
+  int64_t n_huge = 0;  // tip items that may run over the whole grid (the lists only shrink)
   if (kWing) {
     eti.alloc(g.m, s);
     iota.alloc(g.m, s);
@@ -2329,13 +2335,17 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
     scratch_len = std::max(G.nK, G.nC);
   } else {
     refresh_work(G);
-    DevBuf<unsigned long long> mx(1, s);
-    PB_CUDA_TRY(cudaMemsetAsync(mx.get(), 0, sizeof(unsigned long long), s));
-    PB_LAUNCH(max_i64_kernel, grid_for(G.nK), 256, 0, s, G.wk, G.nK, mx.get());
-    unsigned long long hmx = 0;
-    readback(&hmx, mx.get(), sizeof(hmx), s);
-    need_scratch = 2ull * hmx > (uint64_t)kTipSlots;
+    DevBuf<unsigned long long> mx(2, s);
+    PB_CUDA_TRY(cudaMemsetAsync(mx.get(), 0, 2 * sizeof(unsigned long long), s));
+    PB_LAUNCH(max_i64_kernel, grid_for(G.nK), 256, 0, s, G.wk, G.nK, cls.huge_work, mx.get());
+    unsigned long long hmx[2];
+    readback(hmx, mx.get(), sizeof(hmx), s);
+    need_scratch = 2ull * hmx[0] > (uint64_t)kTipSlots;
     scratch_len = G.nK;
+    // One list for all heavy items of a round; the graphs of a batch have a stretch of N each.
+    n_huge = (int64_t)hmx[1];
+    fh0.alloc(batch ? N : n_huge + 1, s);
+    fh1.alloc(batch ? N : n_huge + 1, s);
   }
   const Lists G0 = G;  // the full lists (version 0)
 
@@ -2503,6 +2513,34 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
     }
   };
 
+  // Fine passes: grid-shared counters, and the lists of the items that run on them, must be per instance,
+  // since partitions share item ids.  Instances with a CTA range of their own get one slice each
+  // while kGsharedBudget lasts; the others never take the grid-level path.
+  const int64_t slices = std::max<int64_t>(1, kGsharedBudget / (4 * gstride));
+  std::vector<DevBuf<uint32_t>> slice_bufs;
+  std::vector<DevBuf<uint4>> heavy_bufs;
+  auto heavy_lists = [&](Work& x, uint32_t ncta) {
+    x.gshared = nullptr;
+    x.fhuge[0] = x.fhuge[1] = nullptr;
+    x.ngroups = 1;
+    if (!kWing && ncta >= 2 && (int64_t)slice_bufs.size() < slices) {
+      slice_bufs.emplace_back((size_t)gstride, s);
+      PB_CUDA_TRY(cudaMemsetAsync(slice_bufs.back().get(), 0, slice_bufs.back().bytes(), s));
+      x.gshared = slice_bufs.back().get();
+      for (auto& f : x.fhuge) {
+        heavy_bufs.emplace_back((size_t)std::min(x.N, n_huge), s);
+        f = heavy_bufs.back().get();
+      }
+    }
+  };
+
+  auto release_coarse = [&] {  // what the coarse pass alone used
+    gshared.release();
+    fh0.release();
+    fh1.release();
+    wgt.release();
+  };
+
   if (batch) {
     const int ninst = (int)pbase.size();
     std::vector<Work> ws(ninst, W);
@@ -2564,6 +2602,7 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
     res.coarse_rounds = res.fine_rounds_max;
     res.rounds = 0;
     res.fine_rounds_max = 0;
+    release_coarse();
     // Global partition keys (graph-major) and the fine instances in that order.
     std::vector<uint32_t> pb0(ninst + 1, 0);
     for (int i = 0; i < ninst; ++i) pb0[i + 1] = pb0[i] + std::max(1u, coarse[i].npart);
@@ -2613,8 +2652,6 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
         x.near = nearl.get() + b;
         x.front[0] = fr0.get() + b;
         x.front[1] = fr1.get() + b;
-        x.fhuge[0] = kWing ? nullptr : fh0.get() + b;
-        x.fhuge[1] = kWing ? nullptr : fh1.get() + b;
         x.N = n;
         x.item0 = (uint32_t)b;
         fws.push_back(x);
@@ -2629,22 +2666,10 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
       }
     }
     PB_REQUIRE(b == N, PB_ECUDA, "two-phase peel: partition sizes do not add up");
-    const int64_t gstride_b = gstride;
-    const int64_t slices = std::max<int64_t>(1, kGsharedBudget / (4 * gstride_b));
-    std::vector<std::unique_ptr<DevBuf<uint32_t>>> gsl;
-    auto per_slot = [&](Work& x, uint32_t ncta) {
-      x.gshared = nullptr;
-      x.ngroups = 1;
-      if (!kWing && ncta >= 2 && (int64_t)gsl.size() < slices) {
-        gsl.push_back(std::make_unique<DevBuf<uint32_t>>((size_t)gstride_b, s));
-        PB_CUDA_TRY(cudaMemsetAsync(gsl.back()->get(), 0, gsl.back()->bytes(), s));
-        x.gshared = gsl.back()->get();
-      }
-    };
     std::vector<Ctl> fine;
     const int64_t coarse_work = res.work;
     res.work = 0;
-    launch_instances(fws, fcs, fw, nullptr, per_slot, &fine);
+    launch_instances(fws, fcs, fw, nullptr, heavy_lists, &fine);
     std::vector<int64_t> per_graph(ninst, 0);
     for (size_t q = 0; q < fine.size(); ++q) per_graph[graph_of[q]] += (int64_t)fine[q].rounds;
     res.rounds = *std::max_element(per_graph.begin(), per_graph.end());  // the longest graph, as above
@@ -2760,6 +2785,7 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
   if (!two_phase) return res;
 
   // ---- fine pass: one instance per partition, all in one launch ----------------------------
+  release_coarse();
   res.coarse_rounds = res.rounds;
   const unsigned nparts = hctl.npart;
   PB_REQUIRE(nparts >= 1, PB_ECUDA, "two-phase peel: the coarse pass opened no partition");
@@ -2816,8 +2842,6 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
     x.near = nearl.get() + b;
     x.front[0] = fr0.get() + b;
     x.front[1] = fr1.get() + b;
-    x.fhuge[0] = kWing ? nullptr : fh0.get() + b;
-    x.fhuge[1] = kWing ? nullptr : fh1.get() + b;
     x.N = n;
     x.item0 = (uint32_t)b;
     ws.push_back(x);
@@ -2833,21 +2857,7 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
   const int64_t coarse_work = res.work;
   res.rounds = 0;
   res.work = 0;
-  // Grid-shared counters (grid-level items) must be per instance here, since partitions share
-  // item ids: instances with a CTA range of their own get one slice each while the 256 MB
-  // budget lasts; the others never take the grid-level path.
-  const int64_t slices = std::max<int64_t>(1, kGsharedBudget / (4 * gstride));
-  std::vector<std::unique_ptr<DevBuf<uint32_t>>> gsl;
-  auto per_slot = [&](Work& x, uint32_t ncta) {
-    x.gshared = nullptr;
-    x.ngroups = 1;
-    if (!kWing && ncta >= 2 && (int64_t)gsl.size() < slices) {
-      gsl.push_back(std::make_unique<DevBuf<uint32_t>>((size_t)gstride, s));
-      PB_CUDA_TRY(cudaMemsetAsync(gsl.back()->get(), 0, gsl.back()->bytes(), s));
-      x.gshared = gsl.back()->get();
-    }
-  };
-  launch_instances(ws, cs, weights, dlevels.get(), per_slot, nullptr, true);
+  launch_instances(ws, cs, weights, dlevels.get(), heavy_lists, nullptr, true);
   res.work += coarse_work;
   res.parts = (int64_t)ws.size();
   if (trace)

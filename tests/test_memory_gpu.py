@@ -78,3 +78,26 @@ def test_count_lists_of_many_vertices(ctx, pool):
     assert np.array_equal(pb.count_e(dg, "HASH", "SIDE", use_v=True), oracle.count(small, "EDGE", "SIDE", use_v=True)[0])
     assert pb.count_total(dg, "SERIAL", "SIDE", use_v=True) == oracle.count(small, "TOTAL", "SIDE", use_v=True)[0]
     dg.close()
+
+
+@pytest.mark.parametrize("parts", [0, 4])
+def test_tip_lists_of_many_vertices(ctx, pool, parts):
+    """Descriptors of heavy items are kept for the vertices that can be heavy, not for all."""
+    import torch
+    nu = (1 << 27) + 12_345
+    arrays, small, at = _spread(nu, 4_000, 300, 5, 2)
+    dg = pb.DeviceGraph(ctx, device_arrays=arrays)
+    del arrays
+    out = torch.zeros(nu, dtype=torch.int64, device="cuda")
+    counts = torch.zeros_like(out)
+    torch.cuda.synchronize()
+    pb.count(dg, "BATCHS", "ADEG", use_v=True, out=counts)
+    base = pool.reset()
+    pb.peel(dg, counts, use_v=True, out=out, peel_parts=parts)
+    # Lists, frontiers, counts, work and states: 61 bytes; batched rounds 16 (opening counts,
+    # partitions, weights) and 16 (sorted items) more; grid-shared counters 2 GiB.
+    assert pool.high() - base < (64 if parts == 0 else 96) * nu + (2 << 30) + (64 << 20)
+    want = oracle.peel_vert(small, oracle.count(small, "VERT", "ADEG", use_v=True)[0], use_v=True)[0]
+    assert np.array_equal(out[at].cpu().numpy(), want)
+    assert int(torch.count_nonzero(out)) == int(np.count_nonzero(want))
+    dg.close()
