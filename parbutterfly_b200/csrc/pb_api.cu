@@ -108,6 +108,19 @@ int sm_count() {
   return cached[dev];
 }
 
+size_t device_bytes_left() {
+  size_t free_b = 0, total_b = 0;
+  PB_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
+  int dev = 0;
+  cudaMemPool_t pool;
+  uint64_t reserved = 0, used = 0;
+  PB_CUDA_TRY(cudaGetDevice(&dev));
+  PB_CUDA_TRY(cudaDeviceGetDefaultMemPool(&pool, dev));
+  PB_CUDA_TRY(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved));
+  PB_CUDA_TRY(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
+  return free_b + (size_t)(reserved > used ? reserved - used : 0);
+}
+
 namespace {
 
 // Sets the device and the launch counter of a context for the duration of one API call.

@@ -112,6 +112,8 @@ inline bool capturing() { return g_recorder && g_recorder->capturing; }
 
 // Number of SMs of the current device (cached per process; one device per context).
 int sm_count();
+// Device memory an allocation can still get: the device's free memory and what the pool keeps unused.
+size_t device_bytes_left();
 
 // ---- device helpers -----------------------------------------------------------------------
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }

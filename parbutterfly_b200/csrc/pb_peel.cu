@@ -2376,6 +2376,13 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
     PB_CUDA_TRY(cudaFuncSetAttribute(fine_kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     PB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fine_kern, kPT, smem));
     fine_grid = sm_count() * std::max(1, per_sm);
+    // ... unless their dense counters would take more than half of what is left of the device (the
+    // fine pass's lists are still to come).  Below 4 GiB there is nothing to ask.
+    const size_t scratch = need_scratch ? (size_t)fine_grid * (size_t)scratch_len * sizeof(uint32_t) : 0;
+    if (fine_grid > grid && scratch > size_t(4) << 30 && scratch > device_bytes_left() / 2) {
+      fine_kern = kern;
+      fine_grid = grid;
+    }
   }
 
   DevBuf<uint32_t> gscratch;

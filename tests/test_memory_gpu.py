@@ -101,3 +101,41 @@ def test_tip_lists_of_many_vertices(ctx, pool, parts):
     assert np.array_equal(out[at].cpu().numpy(), want)
     assert int(torch.count_nonzero(out)) == int(np.count_nonzero(want))
     dg.close()
+
+
+@pytest.fixture
+def short_of_memory(pool):
+    """leave(n): takes the device's memory until n bytes are left."""
+    import torch
+    held = []
+
+    def leave(n):
+        torch.cuda.synchronize()
+        pool.trim()
+        torch.cuda.empty_cache()
+        free = torch.cuda.mem_get_info()[0]
+        if free < n:
+            pytest.skip("less memory free than the call needs")
+        held.append(torch.empty(free - n, dtype=torch.uint8, device="cuda"))
+
+    yield leave
+    held.clear()
+    torch.cuda.empty_cache()
+
+
+def test_batched_tip_rounds_short_of_memory(ctx, pool, short_of_memory):
+    """Dense counters of one CTA per SM fit what is left (9.9 GB), those of two do not."""
+    import torch
+    arrays, small, _ = _spread(1 << 24, 40_000, 30, 3, 3)
+    dg = pb.DeviceGraph(ctx, device_arrays=arrays)
+    del arrays
+    out = torch.zeros(1 << 24, dtype=torch.int64, device="cuda")
+    counts = torch.zeros_like(out)
+    torch.cuda.synchronize()
+    pb.count(dg, "BATCHS", "ADEG", use_v=True, out=counts)
+    short_of_memory(17 << 30)
+    pb.peel(dg, counts, use_v=True, out=out, peel_parts=4)
+    want = oracle.peel_vert(small, oracle.count(small, "VERT", "ADEG", use_v=True)[0], use_v=True)[0]
+    got = out.cpu().numpy()
+    assert np.array_equal(got[got > 0], want[want > 0])
+    dg.close()
