@@ -379,7 +379,14 @@ __global__ void validate_uses_kernel(const uint32_t* __restrict__ uses, int64_t 
 // Slots from which the ranked rows are built by one radix sort of (row, neighbour) pairs over the
 // whole CSR instead of a sort within each row.  Relabel of R-MAT graphs, per vertex, radix against row
 // sort: 2^18 slots 0.115 / 0.098 ms, 2^19 0.119 / 0.121, 2^20 0.125 / 0.190, 2^23 0.449 / 1.033.
+// The radix sort holds every array twice (12 bytes a slot more, 16 with output edges, and its counters); where
+// that does not fit what is left of the device, rows are sorted in place whatever the size.
 constexpr int64_t kRankSort = int64_t(1) << 19;
+bool radix_fits(int64_t m2, bool with_eout) {
+  const size_t bytes = (size_t)m2 * (with_eout ? 16 : 12) + (size_t)m2 / 4;
+  // A recorded pipeline must take the same way when it is captured, so it does not ask.
+  return bytes <= size_t(1) << 30 || g_recorder != nullptr || bytes <= device_bytes_left();
+}
 
 int bits_for(uint64_t x) {
   int b = 0;
@@ -481,7 +488,7 @@ void build_ranked_csr(const pb_graph& g, Ranked& R, bool with_eout, cudaStream_t
   if (R.m2 == 0) return;
   const uint32_t chunk = slot_chunk(R.m2);
   const int grid = grid_for((R.m2 + chunk - 1) / chunk * 32);
-  if (R.m2 < kRankSort) {
+  if (R.m2 < kRankSort || !radix_fits(R.m2, with_eout)) {
     PB_LAUNCH(ranked_fill_kernel, grid, 256, 0, s, lists_of(g), R.order.get(), R.rank.get(), R.off.get(), n, R.m2, chunk, R.use_v,
               (uint32_t*)nullptr, R.adj.get(), with_eout ? R.eout.get() : nullptr);
     segmented_sort_rows(R.off.get(), n, R.adj.get(), with_eout ? R.eout.get() : nullptr, bits_for((uint64_t)(2 * n)),

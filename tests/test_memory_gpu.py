@@ -139,3 +139,24 @@ def test_batched_tip_rounds_short_of_memory(ctx, pool, short_of_memory):
     got = out.cpu().numpy()
     assert np.array_equal(got[got > 0], want[want > 0])
     dg.close()
+
+
+def test_relabel_short_of_memory(ctx, pool, short_of_memory):
+    """A per-edge count of 2^26 edges needs 3.0 GB beside the graph when rows are sorted in place, 3.9 GB
+    when the slots are sorted as a whole; with 3.45 GB left it takes the first way."""
+    import torch
+    n, d = 1 << 21, 32  # v's neighbours are v + 127 j, so u's are u - 127 j
+    v = torch.arange(n, device="cuda").unsqueeze(1)
+    j = 127 * torch.arange(d, device="cuda").unsqueeze(0)
+    edg_v = torch.sort((v + j) % n, 1)[0].to(torch.int32).reshape(-1)
+    edg_u = torch.sort((v - j) % n, 1)[0].to(torch.int32).reshape(-1)
+    off = (d * torch.arange(n + 1, device="cuda")).to(torch.int32)
+    torch.cuda.synchronize()
+    dg = pb.DeviceGraph(ctx, device_arrays=(n, n, off, edg_v, off, edg_u))
+    del edg_v, edg_u, off, v, j
+    short_of_memory(3450 << 20)
+    got = pb.count_e(dg, "HASH", "SIDE").reshape(n, d)
+    # v and v + 127 t share d - |t| neighbours.
+    want = np.array([sum(d - 1 - abs(j - k) for k in range(d) if k != j) for j in range(d)])
+    assert (got[:n - 127 * d] == want).all() and int(got.sum()) == n * int(want.sum())
+    dg.close()
