@@ -162,10 +162,12 @@ def graph_from_text(ctx: Context, data) -> DeviceGraph:
     torch uint8 CUDA tensor; tokenised, parsed and validated by GPU kernels."""
     h = C.c_void_p()
     if isinstance(data, (bytes, bytearray)):
-        # The library only reads the text during the call: no copy is made of it here.
-        buf = C.c_char_p(data) if isinstance(data, bytes) else (C.c_char * len(data)).from_buffer(data)
-        ctx.check(ctx._lib.pb_graph_parse_text(ctx.handle, C.cast(buf, C.c_void_p), len(data), C.byref(h)),
-                  "pb_graph_parse_text")
+        # The library only reads the text during the call, so bytes are passed as they are.  A bytearray is
+        # copied: exported, it could not be resized while the traceback of a failed call lives, and
+        # other threads may change it during the call.
+        text = bytes(data)
+        buf = C.cast(C.c_char_p(text), C.c_void_p)
+        ctx.check(ctx._lib.pb_graph_parse_text(ctx.handle, buf, len(text), C.byref(h)), "pb_graph_parse_text")
     else:
         import torch
         torch.cuda.synchronize()

@@ -136,3 +136,30 @@ def test_binary_format_roundtrip(tmp_path):
         np.testing.assert_array_equal(getattr(h, name), getattr(g, name))
     with pytest.raises(_ffi.PBError):
         BipartiteGraph.read_binary(str(tmp_path / "missing"))
+
+
+def test_text_in_a_bytearray_stays_the_callers():
+    """graph_from_text reads a copy of a bytearray: the caller may resize it after a failed call,
+    whose traceback is still held, and change it while the call runs."""
+    from parbutterfly_b200 import butterflies as pb
+
+    text = bytearray(b"AdjacencyHypergraph\n1\n1\n1\n1\n0\n0\n0\n0\n")
+    want = bytes(text)
+
+    class Lib:
+        def pb_graph_parse_text(self, handle, data, n, out):
+            text[:] = b"x" * len(text)
+            text.extend(b"more")
+            assert C.string_at(data, n) == want
+            return _ffi.PB_EINVAL
+
+    class Ctx:
+        handle, _lib = None, Lib()
+
+        def check(self, status, what):
+            raise _ffi.PBError(status, what)
+
+    with pytest.raises(_ffi.PBError) as failed:
+        pb.graph_from_text(Ctx(), text)
+    text.clear()
+    assert failed.value.status == _ffi.PB_EINVAL
