@@ -43,6 +43,7 @@ constexpr uint32_t kEmpty = 0xFFFFFFFFu;
 constexpr int kWarpTable = 1024;  // slots per warp
 constexpr int kWarpsPerBlockSmall = 8;
 constexpr int64_t kListRange = int64_t(1) << 26;  // endpoints that the item lists hold at a time
+constexpr size_t kAskBytes = size_t(256) << 20;  // per-slot counts above this ask what is left of the device
 constexpr uint32_t kHotRanks = 256;   // count_warp_kernel: vertex counts gathered per CTA
 // A row is walked by the threads that own its endpoint, however few wedges it has, so long rows move
 // up a class: beyond kWarpRow slots to a CTA of 128 threads, beyond kMidRow to one of 512.  Limits of
@@ -65,7 +66,8 @@ struct Params {
   int64_t m2;       // slots of the ranked CSR
   uint32_t* err;    // record of the first bounds violation {code, index lo, index hi, aux}
   uint32_t* sacc32;             // per-edge counts per slot: 32 bits wide when every count fits,
-  unsigned long long* sacc64;   // else 64 (the other is null)
+  unsigned long long* sacc64;   // else 64; both null: credits go to out at once, through eout
+  const uint32_t* __restrict__ eout;
   unsigned long long* mstats;  // per mode (dense, hash, hybrid, global): endpoints, wedges
   // Block aggregator (null for the mid kernel):
   const uint8_t* modes;        // modes[q]: aggregation mode of item q
@@ -97,7 +99,8 @@ __device__ __forceinline__ bool slot_ok(const Params& P, uint64_t slot, uint32_t
 // Per-edge credit of a slot (checked by the caller).
 __device__ __forceinline__ void credit_slot(const Params& P, uint32_t slot, uint32_t v) {
   if (P.sacc32) atomicAdd(&P.sacc32[slot], v);
-  else atomicAdd(&P.sacc64[slot], (unsigned long long)v);
+  else if (P.sacc64) atomicAdd(&P.sacc64[slot], (unsigned long long)v);
+  else credit(P, P.eout[slot], v, 12);
 }
 
 // Fibonacci hashing: the high bits of key * 2^32/phi, folded into the table size (any size).
@@ -664,10 +667,10 @@ __global__ void __launch_bounds__(NT, kMinBlocks) count_block_kernel(Params P, c
 }
 
 // Per-edge results: the credits of an edge's two slots, added at its output index.
-__global__ void edge_gather_kernel(Params P, const uint32_t* __restrict__ eout) {
+__global__ void edge_gather_kernel(Params P) {
   for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < P.m2; s += (int64_t)gridDim.x * blockDim.x) {
     const unsigned long long v = P.sacc32 ? (unsigned long long)P.sacc32[s] : P.sacc64[s];
-    if (v) credit(P, eout[s], (int64_t)v, 12);
+    if (v) credit(P, P.eout[s], (int64_t)v, 12);
   }
 }
 
@@ -887,23 +890,6 @@ CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConf
   P.err = cfg.err ? cfg.err : tail->err;
   P.mstats = tail->mstats;
   uint32_t* const counts = tail->counts;
-  // Per-edge counts are gathered per slot, in 32 bits when they fit: (max degree - 1)^2 < 2^32.
-  DevBuf<uint32_t> sacc32;
-  DevBuf<unsigned long long> sacc64;
-  const uint64_t md = R.max_deg > 0 ? R.max_deg - 1 : 0;
-  const char* acc64 = getenv("PB_EDGE_ACC64");  // test hook: force 64-bit per-edge accumulation
-  const bool force64 = acc64 && *acc64 == '1';
-  if (per == EDGE) {
-    if (md * md < (1ull << 32) && !force64) {
-      sacc32.alloc(R.m2, s);
-      PB_CUDA_TRY(cudaMemsetAsync(sacc32.get(), 0, sacc32.bytes(), s));
-      P.sacc32 = sacc32.get();
-    } else {
-      sacc64.alloc(R.m2, s);
-      PB_CUDA_TRY(cudaMemsetAsync(sacc64.get(), 0, sacc64.bytes(), s));
-      P.sacc64 = sacc64.get();
-    }
-  }
   const int sms = sm_count();
   int small_w = std::min(cfg.small_w, kWarpTable / 2);
   int smem_bytes = cfg.smem_bytes;
@@ -948,6 +934,29 @@ CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConf
   DevBuf<uint4> lists((size_t)nl * 3, s);  // warp, mid and block lists
   uint4 *small_items = lists.get(), *mid_items = small_items + nl, *items = mid_items + nl;
   DevBuf<uint8_t> modes(nl, s);
+  // Per-edge counts are gathered per slot, in 32 bits when they fit: (max degree - 1)^2 < 2^32.  The
+  // slots' counts take 8 or 16 bytes an edge, so above kAskBytes they must find room: where they would
+  // take more than half of what is left of the device (global scratch is still to come), every
+  // credit goes to its edge at once, which takes no memory.
+  DevBuf<uint32_t> sacc32;
+  DevBuf<unsigned long long> sacc64;
+  const uint64_t md = R.max_deg > 0 ? R.max_deg - 1 : 0;
+  const char* acc64 = getenv("PB_EDGE_ACC64");  // test hook: force 64-bit per-edge accumulation
+  const bool wide_acc = md * md >= (1ull << 32) || (acc64 && *acc64 == '1');
+  if (per == EDGE) {
+    P.eout = R.eout.get();
+    const size_t bytes = (size_t)R.m2 * (wide_acc ? 8 : 4);
+    const bool direct = bytes > kAskBytes && bytes > device_bytes_left() / 2;
+    if (!direct && !wide_acc) {
+      sacc32.alloc(R.m2, s);
+      PB_CUDA_TRY(cudaMemsetAsync(sacc32.get(), 0, sacc32.bytes(), s));
+      P.sacc32 = sacc32.get();
+    } else if (!direct) {
+      sacc64.alloc(R.m2, s);
+      PB_CUDA_TRY(cudaMemsetAsync(sacc64.get(), 0, sacc64.bytes(), s));
+      P.sacc64 = sacc64.get();
+    }
+  }
   DevBuf<uint32_t> gscratch;
   std::vector<SchedRecord> records;
   for (int64_t i0 = 0; i0 < n; i0 += kListRange) {
@@ -1083,8 +1092,8 @@ CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConf
     }
     if (sched_on) records.push_back({n_block, std::move(sF), std::move(sPred), std::move(sUsed), std::move(sCyc)});
   }
-  if (per == EDGE)
-    PB_LAUNCH(edge_gather_kernel, std::max(1, std::min(ceil_div(R.m2, 256), sms * 8)), 256, 0, s, P, R.eout.get());
+  if (P.sacc32 || P.sacc64)
+    PB_LAUNCH(edge_gather_kernel, std::max(1, std::min(ceil_div(R.m2, 256), sms * 8)), 256, 0, s, P);
   if (cap) return res;
   PB_CUDA_TRY(cudaEventRecord(ev[1], s));
   if (cfg.tail && cfg.ev && records.empty()) {

@@ -144,6 +144,18 @@ def test_batched_tip_rounds_short_of_memory(ctx, pool, short_of_memory):
 def test_relabel_short_of_memory(ctx, pool, short_of_memory):
     """A per-edge count of 2^26 edges needs 3.0 GB beside the graph when rows are sorted in place, 3.9 GB
     when the slots are sorted as a whole; with 3.45 GB left it takes the first way."""
+    _check_shifts(ctx, short_of_memory, 3450 << 20)
+
+
+@pytest.mark.parametrize("acc64", [False, True])
+def test_edge_credits_short_of_memory(ctx, pool, short_of_memory, monkeypatch, acc64):
+    """The same count with 2.7 GB left: 2.4 GB are needed without counts per slot, 3.0 or 3.5 with them."""
+    if acc64:
+        monkeypatch.setenv("PB_EDGE_ACC64", "1")
+    _check_shifts(ctx, short_of_memory, 2600 << 20)
+
+
+def _check_shifts(ctx, short_of_memory, left):
     import torch
     n, d = 1 << 21, 32  # v's neighbours are v + 127 j, so u's are u - 127 j
     v = torch.arange(n, device="cuda").unsqueeze(1)
@@ -154,7 +166,7 @@ def test_relabel_short_of_memory(ctx, pool, short_of_memory):
     torch.cuda.synchronize()
     dg = pb.DeviceGraph(ctx, device_arrays=(n, n, off, edg_v, off, edg_u))
     del edg_v, edg_u, off, v, j
-    short_of_memory(3450 << 20)
+    short_of_memory(left)
     got = pb.count_e(dg, "HASH", "SIDE").reshape(n, d)
     # v and v + 127 t share d - |t| neighbours.
     want = np.array([sum(d - 1 - abs(j - k) for k in range(d) if k != j) for j in range(d)])
