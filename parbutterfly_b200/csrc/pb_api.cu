@@ -971,7 +971,7 @@ pb_status pb_batch_create(pb_ctx* ctx, const pb_graph* const* gs, int32_t k, con
       b->geom = {ctx->stats.count_smem_bytes, ctx->stats.count_blocks_per_sm, ctx->stats.count_small_w};
       b->tuned = true;
     }
-    b->rec.status = (unsigned*)b->rec.pinned_alloc(2 * sizeof(unsigned));
+    b->rec.status = (unsigned*)b->rec.pinned_alloc(3 * sizeof(unsigned));
     // 1. Recording run (eager): every host readback is logged.
     g_recorder = &b->rec;
     try {
@@ -1025,6 +1025,7 @@ pb_status pb_batch_run(pb_ctx* ctx, pb_batch* b, int64_t* const* counts, int64_t
         PB_CUDA_TRY(cudaMemcpyAsync(tips[g], b->tips.get() + b->kbase[g], bytes, cudaMemcpyDefault, s));
     }
     PB_CUDA_TRY(cudaStreamSynchronize(s));
+    PB_REQUIRE(b->rec.status[2] == 0, PB_ETIMEOUT, "batch graph: a grid barrier wait of the ranking ran out of time");
     if (b->U.nu > 0) {
       const unsigned err = b->rec.status[0], alive = b->rec.status[1];
       PB_REQUIRE(err != 0xFFFFFFFFu, PB_ECUDA, "batch graph: the peel reported no status");

@@ -102,7 +102,7 @@ struct Recorder {
   std::vector<std::vector<uint8_t>> log;
   size_t pos = 0;
   std::vector<void*> pinned;  // host memory the captured graph reads or writes (kept alive)
-  unsigned* status = nullptr; // pinned {peel error bits, unpeeled items} written by the graph
+  unsigned* status = nullptr; // pinned {peel error bits, unpeeled items, ranking error} written by the graph
   ~Recorder();
   void* pinned_alloc(size_t bytes);
 };

@@ -80,6 +80,12 @@ struct CoCtl {
   unsigned long long bar;
   uint32_t err, kmax[2], len[2];
 };
+// Bound of every barrier wait, and the arrivals that complete a barrier: the CTAs (test hook: one more, so
+// that every wait runs out).
+struct CoWait {
+  unsigned long long timeout_ns;
+  unsigned arrivals;
+};
 constexpr uint32_t kCoDone = 0x80000000u;  // finished (keys are degrees or their logarithms, below 2^23)
 constexpr uint32_t kCoUnit = 256;
 constexpr int kCoThreads = 1024;
@@ -87,7 +93,7 @@ constexpr unsigned long long kCoTimeoutNs = 60ull * 1000000000ull;
 
 // Grid barrier of a cooperative launch: arrivals are counted in a word that is never reset.
 // Bounded: on expiry sets err and returns false in every CTA.
-__device__ bool co_barrier(CoCtl* c, unsigned long long target) {
+__device__ bool co_barrier(CoCtl* c, unsigned long long target, unsigned long long timeout_ns) {
   __syncthreads();
   int bad = 0;
   if (threadIdx.x == 0) {
@@ -100,7 +106,7 @@ __device__ bool co_barrier(CoCtl* c, unsigned long long target) {
         unsigned long long now;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
         if (!t0) t0 = now;
-        else if (now - t0 > kCoTimeoutNs) {
+        else if (now - t0 > timeout_ns) {
           atomicExch(&c->err, 1u);
           atomicOr(&c->bar, 1ull << 63);
         }
@@ -112,7 +118,7 @@ __device__ bool co_barrier(CoCtl* c, unsigned long long target) {
 }
 
 __global__ void __launch_bounds__(kCoThreads, 1) cocore_kernel(Lists L, int64_t n, int approx, uint32_t* key, uint32_t* dact,
-                                                              uint2* units, CoCtl* ctl) {
+                                                              uint2* units, CoCtl* ctl, CoWait wait) {
   __shared__ uint32_t s_k, s_len;
   const unsigned lane = threadIdx.x & 31u;
   const int64_t gtid = (int64_t)blockIdx.x * kCoThreads + threadIdx.x, gthreads = (int64_t)gridDim.x * kCoThreads;
@@ -133,7 +139,7 @@ __global__ void __launch_bounds__(kCoThreads, 1) cocore_kernel(Lists L, int64_t 
     }
     post_max(m, &ctl->kmax[0]);
   }
-  if (!co_barrier(ctl, target += gridDim.x)) return;
+  if (!co_barrier(ctl, target += wait.arrivals, wait.timeout_ns)) return;
   for (unsigned par = 0;; par ^= 1u) {
     if (threadIdx.x == 0) s_k = *(volatile uint32_t*)&ctl->kmax[par];
     __syncthreads();
@@ -160,7 +166,7 @@ __global__ void __launch_bounds__(kCoThreads, 1) cocore_kernel(Lists L, int64_t 
       for (uint32_t c = 0; c < nu; ++c) units[at + c] = make_uint2((uint32_t)x, c);
     }
     post_max(m, &ctl->kmax[par ^ 1u]);
-    if (!co_barrier(ctl, target += gridDim.x)) return;
+    if (!co_barrier(ctl, target += wait.arrivals, wait.timeout_ns)) return;
     if (threadIdx.x == 0) s_len = *(volatile uint32_t*)&ctl->len[par];
     __syncthreads();
     if (blockIdx.x == 0 && threadIdx.x == 0) {  // every CTA has read kmax[par]; len[par ^ 1] is the last round's
@@ -182,7 +188,7 @@ __global__ void __launch_bounds__(kCoThreads, 1) cocore_kernel(Lists L, int64_t 
         }
       }
     }
-    if (!co_barrier(ctl, target += gridDim.x)) return;
+    if (!co_barrier(ctl, target += wait.arrivals, wait.timeout_ns)) return;
   }
 }
 
@@ -450,8 +456,13 @@ void vertex_order(const pb_graph& g, int rank_type, int use_v, Ranked& R, cudaSt
     int ap = approx;
     uint32_t *kp = key.get(), *dp = dact.get();
     uint2* up = units.get();
-    void* args[] = {&lists, &nn, &ap, &kp, &dp, &up, &ctl};
+    CoWait wait{kCoTimeoutNs, 0};
+    if (const char* e = getenv("PB_RANK_BARRIER_TIMEOUT_MS")) wait.timeout_ns = 1000000ull * strtoull(e, nullptr, 10);
+    void* args[] = {&lists, &nn, &ap, &kp, &dp, &up, &ctl, &wait};
     const int grid = std::max(1, std::min(sm_count(), ceil_div(n, kCoThreads)));
+    wait.arrivals = (unsigned)grid;
+    // Test hook: no barrier completes, with 1 in any ranking, with 2 in captured graphs.
+    if (const char* e = getenv("PB_RANK_TEST_STUCK_BARRIER")) wait.arrivals += *e == '1' || (*e == '2' && capturing());
     PB_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)cocore_kernel, dim3(grid), dim3(kCoThreads), args, 0, s));
     if (g_launch_counter) ++*g_launch_counter;
     PB_LAUNCH(cocore_keys_kernel, grid_for(n), 256, 0, s, key.get(), n, kmax, keys.get(), ids);
@@ -533,7 +544,11 @@ void wedge_scan(Ranked& R, cudaStream_t s, bool with_rows) {
   readback(&R.w_rank, R.wsum.get() + n, sizeof(int64_t), s);
   if (R.co.get()) {
     uint32_t err = 0;
-    readback(&err, &reinterpret_cast<CoCtl*>(R.co.get())->err, sizeof(err), s);
+    const uint32_t* word = &reinterpret_cast<CoCtl*>(R.co.get())->err;
+    // A captured graph hands the word of every replay to the recorder's status.
+    if (capturing())
+      PB_CUDA_TRY(cudaMemcpyAsync(g_recorder->status + 2, word, sizeof(err), cudaMemcpyDeviceToHost, s));
+    readback(&err, word, sizeof(err), s);
     PB_REQUIRE(err == 0, PB_ETIMEOUT, "ranking: a grid barrier wait ran out of time");
   }
 }

@@ -44,3 +44,33 @@ def test_ranked_csr(ctx, name, rank):
     assert ctx.stats()["w_rank"] == w_rank
     assert np.array_equal(pb.count_e(dg, "BATCHS", rank), oracle.count(g, "EDGE", rank)[0])
     dg.close()
+
+
+def test_barrier_timeout_reports_status_and_context_survives(ctx, monkeypatch):
+    """A barrier wait of the co-core ranking that cannot complete (test hook) runs out after the
+    configured bound: single calls and replays of a captured batch return PB_ETIMEOUT."""
+    from parbutterfly_b200._ffi import PB_ETIMEOUT, PBError
+    g = BipartiteGraph.zipf(3_000, 4_000, 30_000, 1.3, 38)
+    dg = ctx.upload(g)
+    want = oracle.count(g, "VERT", "ACOCORE")[0]
+    tips = oracle.peel_vert(g, want)[0]
+    monkeypatch.setenv("PB_RANK_BARRIER_TIMEOUT_MS", "300")
+    monkeypatch.setenv("PB_RANK_TEST_STUCK_BARRIER", "1")
+    with pytest.raises(PBError) as ex:
+        pb.count(dg, "HASH", "ACOCORE")
+    assert ex.value.status == PB_ETIMEOUT
+    monkeypatch.setenv("PB_RANK_TEST_STUCK_BARRIER", "2")
+    batch = pb.BatchGraph([dg, dg], rank_type="ACOCORE")
+    for _ in range(2):
+        with pytest.raises(PBError) as ex:
+            batch.run()
+        assert ex.value.status == PB_ETIMEOUT
+    batch.close()
+    monkeypatch.delenv("PB_RANK_TEST_STUCK_BARRIER")
+    assert np.array_equal(pb.count(dg, "HASH", "ACOCORE"), want)
+    batch = pb.BatchGraph([dg, dg], rank_type="ACOCORE")
+    for _ in range(2):
+        c, t = batch.run()
+        assert all(np.array_equal(x, want) for x in c) and all(np.array_equal(x, tips) for x in t)
+    batch.close()
+    dg.close()
