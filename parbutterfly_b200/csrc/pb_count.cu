@@ -68,14 +68,14 @@ struct Params {
   uint32_t* sacc32;             // per-edge counts per slot: 32 bits wide when every count fits,
   unsigned long long* sacc64;   // else 64; both null: credits go to out at once, through eout
   const uint32_t* __restrict__ eout;
-  unsigned long long* mstats;  // per mode (dense, hash, hybrid, global): endpoints, wedges
+  unsigned long long* mstats;  // per mode (dense, hash, global, hybrid): endpoints, wedges
   // Block aggregator (null for the mid kernel):
   const uint8_t* modes;        // modes[q]: aggregation mode of item q
   uint8_t* mode_out;           // mode_out[q]: mode item q ran with (scheduler hooks)
   unsigned long long* cycles;  // cycles[q]: SM cycles item q took (clock64, thread 0)
 };
 
-// Records the first bounds violation (checked mode only).
+// Records the first bounds violation.
 __device__ __noinline__ void record_violation(uint32_t* err, uint32_t code, uint64_t idx, uint32_t aux) {
   if (atomicCAS(&err[0], 0u, code) == 0u) {
     err[1] = (uint32_t)idx;
@@ -579,7 +579,8 @@ __global__ void __launch_bounds__(NT, kMinBlocks) count_block_kernel(Params P, c
       }, nothing);
     }
     if (need_center) {
-      // Phase 2: centre / edge credits.
+      // Phase 2: centre / edge credits.  A part's sum fits 32 bits: the w(i, u2) of distinct u2 add
+      // up to at most the edges of the graph, fewer than 2^31 (lists are strictly ascending).
       uint32_t mine = 0;
       auto charge = [&](uint32_t slot2, uint32_t w) {
         if (w > 1) {

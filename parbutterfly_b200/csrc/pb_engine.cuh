@@ -77,12 +77,10 @@ struct CountTail {
 };
 struct CountConfig {
   int strategy = STRAT_AUTO;
-  int small_w = 512;          // endpoints with W_i <= small_w go to the warp aggregator
-  int block_threads = 512;    // threads of the block aggregator
+  int small_w = 512;            // endpoints with W_i <= small_w go to the warp aggregator
   int smem_bytes = 72 * 1024;   // dynamic shared memory of the block aggregator
   int blocks_per_sm = 3;
-  int split_w = 0;            // endpoints above this many wedges are split across CTAs (0: auto)
-  uint32_t* err = nullptr;    // checked mode: device record of the first bounds violation
+  uint32_t* err = nullptr;      // checked mode: device record of the first bounds violation
   SchedHooks* sched = nullptr;
   // The caller's zeroed tail and two events for the aggregation's time: count_ranked then leaves
   // reading them (finish_count) to the caller, who has a wait of its own to come, unless the

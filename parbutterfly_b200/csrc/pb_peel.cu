@@ -1850,7 +1850,7 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
 }
 
 // kMinBlocks: CTAs per SM the register allocation must allow.  2 caps a thread at 64 registers
-// (some spill); 1 leaves about 108 and no spills, at half the resident warps.  The single-
+// (some spill); 1 leaves 128 and no spills, at half the resident warps.  The single-
 // instance tip peel runs faster on the latter (light rounds: fewer CTAs also shorten its grid
 // barriers), and so does the wing peel while its rounds are light; with more edges the rounds are
 // heavy and the intersections need the warps.  Wing peel of R-MAT graphs, one against two CTAs:

@@ -343,15 +343,6 @@ __global__ void big_row_scatter_kernel(const uint32_t* __restrict__ off, const u
   }
 }
 
-__global__ void reduce_max_u32_kernel(const uint32_t* __restrict__ in, int64_t n, uint32_t* out) {
-  uint32_t m = 0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    m = max(m, in[i]);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, m);
-}
-
 __global__ void compact_flags_kernel(const uint8_t* __restrict__ flags, int64_t n, uint32_t* ids,
                                      uint32_t* count) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -416,12 +407,6 @@ void segmented_sort_rows(const uint32_t* off, int64_t nrows, uint32_t* keys, uin
   bool alt = radix_sort_pairs_u64(tk.get(), tv.get(), tk2.get(), tv2.get(), tot, 0, total_bits, s);
   PB_LAUNCH(big_row_scatter_kernel, std::min<uint32_t>(nbig, sms * 4), 256, 0, s, off, big_rows, nbig,
             tstart.get(), alt ? tk2.get() : tk.get(), alt ? tv2.get() : tv.get(), key_bits, keys, vals);
-}
-
-void reduce_max_u32(const uint32_t* in, int64_t n, uint32_t* out_dev, cudaStream_t s) {
-  PB_CUDA_TRY(cudaMemsetAsync(out_dev, 0, sizeof(uint32_t), s));
-  if (n <= 0) return;
-  PB_LAUNCH(reduce_max_u32_kernel, std::min(ceil_div(n, 256), sm_count() * 8), 256, 0, s, in, n, out_dev);
 }
 
 void compact_flags(const uint8_t* flags, int64_t n, uint32_t* ids_out, uint32_t* count_dev, cudaStream_t s) {

@@ -25,10 +25,6 @@ bool radix_sort_pairs_u32(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, ui
 void segmented_sort_rows(const uint32_t* off, int64_t nrows, uint32_t* keys, uint32_t* vals, int key_bits,
                          uint32_t max_row, cudaStream_t s);
 
-// Sum / max reductions into a single device value (result written to *out, host-visible
-// after stream sync).
-void reduce_max_u32(const uint32_t* in, int64_t n, uint32_t* out_dev, cudaStream_t s);
-
 // ids[0..count) of i in [0,n) with pred(flags[i]) — flags are uint8; returns via device count.
 void compact_flags(const uint8_t* flags, int64_t n, uint32_t* ids_out, uint32_t* count_dev, cudaStream_t s);
 

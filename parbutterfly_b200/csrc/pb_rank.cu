@@ -485,9 +485,7 @@ void build_ranked_csr(const pb_graph& g, Ranked& R, bool with_eout, cudaStream_t
   const int64_t n = R.n;
   R.m2 = 2 * g.m;
   R.off.alloc(n + 1, s);
-  // Padded to whole 16-byte groups: the aggregators walk rows with 16-byte loads of aligned
-  // groups of four entries (entries outside the row are masked, never used).
-  R.adj.alloc((size_t)((R.m2 + 3) & ~int64_t(3)) + 4, s);
+  R.adj.alloc(R.m2 > 0 ? R.m2 : 1, s);
   if (with_eout) R.eout.alloc(R.m2 > 0 ? R.m2 : 1, s);
   R.max_deg = g.max_deg;
   if (n == 0) {
@@ -506,7 +504,7 @@ void build_ranked_csr(const pb_graph& g, Ranked& R, bool with_eout, cudaStream_t
                         g.max_deg, s);
     return;
   }
-  DevBuf<uint32_t> dest(R.m2, s), dest2(R.m2, s), adj2(R.adj.n, s), eout2;
+  DevBuf<uint32_t> dest(R.m2, s), dest2(R.m2, s), adj2(R.m2, s), eout2;
   if (with_eout) eout2.alloc(R.m2, s);
   PB_LAUNCH(ranked_fill_kernel, grid, 256, 0, s, lists_of(g), R.order.get(), R.rank.get(), R.off.get(), n, R.m2, chunk, R.use_v,
             dest.get(), R.adj.get(), with_eout ? R.eout.get() : nullptr);
