@@ -1070,7 +1070,8 @@ CountResult count_ranked(const Ranked& R, int per, int64_t* out, const CountConf
       }
       P.modes = modes.get();
       auto kern = count_block_kernel<kBlock, kBlockPerSm>;
-      PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
+      // The limit belongs to the kernel, not to the call: other threads launch it with other geometries.
+      PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmBytes - kCtaReserved));
       PB_LAUNCH(kern, grid, kBlock, smem_bytes, s, P, items, counts, counts + 2, gscratch.get(), G);
     }
     P.modes = nullptr;

@@ -5,13 +5,20 @@ import os
 import re
 import subprocess
 import sys
+import threading
 
 import pytest
+
+import oracle
+from parbutterfly_b200 import butterflies as pb
+from parbutterfly_b200._ffi import PBError
+from parbutterfly_b200.graph import BipartiteGraph
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 SCRIPT = """
 from parbutterfly_b200 import butterflies as pb
+from parbutterfly_b200._ffi import PBError
 from parbutterfly_b200.graph import BipartiteGraph
 with pb.Context(0) as ctx:
     dg = ctx.upload(BipartiteGraph.rmat(SCALE, SCALE - 2, 60000, 0.55, 0.15, 0.15, 0.15, 73))
@@ -39,3 +46,37 @@ def test_plain_geometry_is_a_candidate(scale):
         assert tried[0][0] < said["plain"][0] and tried[0][1:] == said["plain"][1:]
     for smem, ctas, _ in tried:
         assert ctas * (smem + 1024) <= 228 * 1024 and ctas * 512 * 40 <= 65536  # 40 registers a thread
+
+
+@pytest.mark.gpu
+def test_threads_with_different_geometries():
+    """Two threads tune (tables of up to 200 KiB a CTA, tuned anew on every context), two count with the
+    plain geometry."""
+    gs = [BipartiteGraph.rmat(12, 10, 60000 + 10 * k, 0.55, 0.15, 0.15, 0.15, 80 + k) for k in range(100)]
+    want = [oracle.count(g, "TOTAL", "ADEG")[0] for g in gs]
+    failures, tuning = [], [2]
+
+    def work(tune):
+        try:
+            for _ in range(8 if tune else 1000):
+                with pb.Context(0) as ctx:
+                    for g, w in zip(gs, want):
+                        dg = ctx.upload(g)
+                        try:
+                            if pb.count_total(dg, "HASH", "ADEG", autotune=tune) != w:
+                                failures.append("totals differ")
+                        except PBError as e:
+                            failures.append(str(e))
+                        dg.close()
+                if tuning[0] == 0:
+                    break
+        finally:
+            if tune:
+                tuning[0] -= 1
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in (True, True, False, False)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert failures == []
