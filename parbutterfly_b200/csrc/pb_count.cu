@@ -337,8 +337,9 @@ __global__ void __launch_bounds__(256, kOneWord ? 6 : 3) count_warp_kernel(Param
 // ---------------------------------------------------------------------------------------------
 constexpr int kBlock = 512;    // threads of the block aggregator
 constexpr int kBlockPerSm = 3; // with 72 KiB of shared memory each (pb_engine.cuh): aggregation of
-                               // the R-MAT graph of 2^24 edges, per edge: 18.6 ms; 512 threads x 2
-                               // per SM 22.0, 256 x 4 21.5, 256 x 6 21.7, 1024 x 1 27.2
+                               // the R-MAT graph of 2^24 edges, per edge: 18.6 ms (18.0 with today's
+                               // mid class); 512 threads x 2 per SM 22.0, 256 x 4 21.5, 256 x 6 21.7,
+                               // 1024 x 1 27.2
 constexpr int kMidBlock = 128; // threads of the mid aggregator
 
 template <int NT>
@@ -509,8 +510,10 @@ __global__ void plain_modes_kernel(Params P, const uint4* __restrict__ items, co
   }
 }
 
-// One CTA of NT threads per endpoint.  Bound by shared-memory atomics and latency; the two table
-// walks read 4 bytes a wedge each, mostly from L2.
+// One CTA of NT threads per endpoint.  Bound by its instructions and barriers: on the R-MAT graph with 2^24
+// edges (12.4 ms with 512 threads, 3.6 with 128) the schedulers issue in 69% (62%) of the cycles while
+// the shared-memory pipe is busy for 45%, L2 for 12% and DRAM for 4%; the largest stalls are the
+// barriers between chunks.  The two table walks read 4 bytes a wedge each, mostly from L2.
 template <int NT, int kMinBlocks>
 __global__ void __launch_bounds__(NT, kMinBlocks) count_block_kernel(Params P, const uint4* __restrict__ items,
                                                                      const uint32_t* __restrict__ n_items_dev,
