@@ -213,7 +213,11 @@ __global__ void invert_order_kernel(Lists L, const uint32_t* __restrict__ order,
 // Calls f(valid, slot, row) for every slot of [s0, s0 + len) of a CSR (row: the slot's row), 32 slots of
 // one warp at a time: work is cut by slots, not rows, since rows are as uneven as degrees (one
 // warp per row left the last hubs running alone: the wedge scan of the power-law graph with 1e7 edges
-// took 4.4 ms, in chunks of slots 0.29; its fill 1.2 and 0.14).
+// took 4.4 ms, in chunks of slots 0.29; its fill 1.2 and 0.14).  The rows of a group's slots are found in the
+// next kRowWindows windows of 32 rows, beyond them by a search: vertices without edges may lie millions
+// of rows deep between two slots (2^24 vertices, 20,000 edges, SIDE order: walked through, a count took
+// 286 ms, searched over 1.8).
+constexpr int kRowWindows = 4;
 template <class F>
 __device__ __forceinline__ void warp_slots(const uint32_t* __restrict__ off, int64_t n, uint32_t s0, uint32_t len, F&& f) {
   const unsigned lane = threadIdx.x & 31u;
@@ -227,6 +231,7 @@ __device__ __forceinline__ void warp_slots(const uint32_t* __restrict__ off, int
   uint32_t r = (uint32_t)lo;
   walk_groups(s0, len, 32, lane, [&](uint32_t slot, bool valid) {
     uint32_t row = r;
+    int windows = 0;
     for (uint32_t base = r;; base += 32) {
       // Starts of rows base + 1 .. base + 32 (off[n] lies above every slot).
       const uint32_t bnd = off[min((int64_t)base + 1 + lane, n)];
@@ -237,6 +242,24 @@ __device__ __forceinline__ void warp_slots(const uint32_t* __restrict__ off, int
       if (__shfl_sync(0xffffffffu, bnd, c) <= slot) ++c;
       if (valid && row == base) row = base + c;
       if (!__any_sync(0xffffffffu, valid && row == base + 32)) break;
+      if (++windows < kRowWindows) continue;
+      // Many empty rows: the lanes that are left search, in steps that double.
+      if (valid && row == base + 32) {
+        int64_t first = row, step = 32;
+        while (first + step < n && off[first + step] <= slot) {
+          first += step;
+          step *= 2;
+        }
+        int64_t end = min(first + step, n);  // off[first] <= slot < off[end]
+        while (end - first > 1) {
+          const int64_t mid = (first + end) >> 1;
+          if (off[mid] <= slot) first = mid;
+          else end = mid;
+        }
+        row = (uint32_t)first;
+      }
+      __syncwarp();
+      break;
     }
     f(valid, slot, row);
     r = __shfl_sync(0xffffffffu, row, 31);

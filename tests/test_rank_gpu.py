@@ -46,6 +46,27 @@ def test_ranked_csr(ctx, name, rank):
     dg.close()
 
 
+@pytest.mark.parametrize("rank", ["SIDE", "COCORE", "ACOCORE"])
+def test_long_runs_of_empty_rows(ctx, rank):
+    """Millions of vertices without edges between two slots: the rows are found by a search, not by
+    walking through the run (which took the two stages 70 ms each on this graph)."""
+    n, rng = 1 << 22, np.random.default_rng(39)
+
+    def ids():
+        x = rng.integers(0, 3_000, 20_000)
+        return np.where(x < 1_500, x, np.where(x < 1_700, 100_000 + 37 * x, n - 1 - x))
+
+    g = BipartiteGraph.from_edges(n, n, ids(), ids())
+    dg = ctx.upload(g)
+    want = oracle.count(g, "VERT", rank)[0]
+    for _ in range(2):
+        assert np.array_equal(pb.count(dg, "HASH", rank), want)
+    st = ctx.stats()
+    assert st["ms_relabel"] + st["ms_scan"] < 14.0
+    assert np.array_equal(pb.count_e(dg, "SORT", rank), oracle.count(g, "EDGE", rank)[0])
+    dg.close()
+
+
 def test_barrier_timeout_reports_status_and_context_survives(ctx, monkeypatch):
     """A barrier wait of the co-core ranking that cannot complete (test hook) runs out after the
     configured bound: single calls and replays of a captured batch return PB_ETIMEOUT."""
