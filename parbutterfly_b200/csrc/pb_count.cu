@@ -349,7 +349,8 @@ struct BlockShared {
   uint32_t len[NT];
   uint16_t list[NT];
   int64_t red[32];
-  uint32_t item, n_short, n_long;
+  uint32_t item, long_above;
+  uint32_t n_short[2], n_long[2], turn;  // block_wedges: list counters of the chunks in turn
 };
 template <int NT>
 constexpr size_t shared_fixed() { return (sizeof(BlockShared<NT>) + 15) & ~size_t(15); }
@@ -369,12 +370,20 @@ __device__ __forceinline__ int64_t block_sum_i64(int64_t x, int64_t* smem) {
 }
 
 // Iterates every wedge of an endpoint with the whole CTA, NT neighbours at a time.  Neighbours with
-// prefixes N(v)[0, L) of up to kLong wedges go to the warps in turn, longer ones are walked by all
+// prefixes N(v)[0, L) of up to S.long_above wedges go to the warps in turn, longer ones are walked by all
 // warps together.  Lane t of a walk takes entries t, t + 32, ... with four loads in flight, so loads
 // and atomics on the entries' slots are coalesced.  f(slot2, u2) per wedge; part_end(j, vt): all
 // lanes of a warp, after its part of neighbour slot j.  Ends with a barrier, so a walk may follow
 // another at once and read what its f wrote.
+// A list that all warps walk costs each of them a turn however short its part is, so it must be long
+// beside a warp's share of the chunk: above a quarter of it, and above kLong.
 constexpr uint32_t kLong = 512;
+template <int NT>
+__device__ __forceinline__ uint32_t long_above(int64_t W, uint32_t deg) {
+  if (NT == kMidBlock) return kLong;  // at most kMidWedges wedges
+  const float chunk = (float)W * fminf(1.f, (float)NT / (float)deg);
+  return max(kLong, (uint32_t)fminf(chunk / (float)(4 * (NT / 32)), 1e9f));
+}
 
 template <int kStride, class F>
 __device__ __forceinline__ void walk_prefix(const uint32_t* __restrict__ adj, uint32_t beg, uint32_t len, uint32_t first,
@@ -407,14 +416,21 @@ __device__ __forceinline__ void block_wedges(uint32_t b, uint32_t e, const Param
     S.vt[tid] = vt;
     S.len[tid] = L;
     // Neighbours without wedges are left out: slots k of the chunk, in any order.
-    const unsigned some = __ballot_sync(0xffffffffu, L > 0 && L <= kLong);
+    const uint32_t limit = S.long_above, turn = S.turn;
+    const unsigned some = __ballot_sync(0xffffffffu, L > 0 && L <= limit);
     unsigned at = 0;
-    if (lane == 0 && some) at = atomicAdd(&S.n_short, (uint32_t)__popc(some));
+    if (lane == 0 && some) at = atomicAdd(&S.n_short[turn], (uint32_t)__popc(some));
     at = __shfl_sync(0xffffffffu, at, 0) + __popc(some & ((1u << lane) - 1u));
-    if (L > 0 && L <= kLong) S.list[at] = (uint16_t)tid;
-    if (L > kLong) S.list[NT - 1 - atomicAdd(&S.n_long, 1u)] = (uint16_t)tid;
+    if (L > 0 && L <= limit) S.list[at] = (uint16_t)tid;
+    if (L > limit) S.list[NT - 1 - atomicAdd(&S.n_long[turn], 1u)] = (uint16_t)tid;
     __syncthreads();
-    const uint32_t ns = S.n_short, nl = S.n_long;
+    const uint32_t ns = S.n_short[turn], nl = S.n_long[turn];
+    // Every thread has taken its turn by now, and the next chunk (of this walk or of the caller's next
+    // one) adds to the other counters only behind the barrier below, so they are cleared in between.
+    if (tid == 0) {
+      S.turn = turn ^ 1u;
+      S.n_short[turn ^ 1u] = S.n_long[turn ^ 1u] = 0;
+    }
     for (uint32_t p = tid >> 5; p < ns; p += NT / 32) {
       const uint32_t k = S.list[p], beg = S.vs[k];
       walk_prefix<32>(P.adj, beg, S.len[k], lane, f);
@@ -427,11 +443,6 @@ __device__ __forceinline__ void block_wedges(uint32_t b, uint32_t e, const Param
       __syncwarp();
       part_end(j0 + k, S.vt[k]);
     }
-    __syncthreads();
-    if (tid == 0) S.n_short = S.n_long = 0;
-    // The next adds to the counters come from the next chunk or from the caller's next walk, so the
-    // reset is closed by a barrier in both cases: an add that came before it would be lost, and with
-    // it a neighbour list of the walk.
     __syncthreads();
   });
 }
@@ -525,7 +536,7 @@ __global__ void __launch_bounds__(NT, kMinBlocks) count_block_kernel(Params P, c
   const uint32_t n_items = *n_items_dev;
   const unsigned lane = lane_id();
   int64_t total = 0;
-  if (threadIdx.x == 0) S.n_short = S.n_long = 0;
+  if (threadIdx.x == 0) S.turn = S.n_short[0] = S.n_long[0] = 0;
   // The first item of a CTA is its own number; the cursor hands out the later ones.
   for (uint32_t q = blockIdx.x; q < n_items;) {
     if (threadIdx.x == 0) S.item = gridDim.x + atomicAdd(cursor, 1u);
@@ -538,6 +549,7 @@ __global__ void __launch_bounds__(NT, kMinBlocks) count_block_kernel(Params P, c
     Mode mode;
     if (NT == kMidBlock) mode = G.rule(i, W, deg, 0);
     else mode = (Mode)(P.modes[q] & 3u);
+    if (threadIdx.x == 0) S.long_above = long_above<NT>(W, deg);
     if (threadIdx.x == 0 && P.mstats) {
       atomicAdd(&P.mstats[mode], 1ull);
       atomicAdd(&P.mstats[4 + mode], (unsigned long long)W);

@@ -64,3 +64,19 @@ def test_degrees_beyond_16_bits(ctx):
         assert np.array_equal(pb.count(dg, "BATCHS", "SIDE", use_v=use_v), oracle.count(g, "VERT", "SIDE", use_v=use_v)[0])
         assert np.array_equal(pb.count_e(dg, "HASH", "SIDE", use_v=use_v), oracle.count(g, "EDGE", "SIDE", use_v=use_v)[0])
     dg.close()
+
+
+@pytest.mark.parametrize("rows", [300, 512, 513, 1100])
+def test_lists_beside_a_warps_share(ctx, rows):
+    """Dense rows of lists that a warp each walks, lists of all warps among them: the limit between the
+    two lies at a quarter of a warp's share of the row's chunk."""
+    hub = 20_000
+    g = BipartiteGraph.from_edges(rows + 2, hub, np.r_[np.repeat(np.arange(rows), 700), np.full(hub, rows),
+                                                       np.full(hub // 2, rows + 1)],
+                                  np.r_[np.tile(np.arange(700), rows), np.arange(hub), np.arange(0, hub, 2)])
+    dg = ctx.upload(g)
+    for rank in ["SIDE", "DEG"]:
+        for use_v in (False, True):
+            assert np.array_equal(pb.count(dg, "BATCHS", rank, use_v=use_v), oracle.count(g, "VERT", rank, use_v=use_v)[0])
+        assert np.array_equal(pb.count_e(dg, "HASH", rank), oracle.count(g, "EDGE", rank)[0])
+    dg.close()
