@@ -89,6 +89,12 @@ struct CoWait {
 constexpr uint32_t kCoDone = 0x80000000u;  // finished (keys are degrees or their logarithms, below 2^23)
 constexpr uint32_t kCoUnit = 256;
 constexpr int kCoThreads = 1024;
+// The grid has a thread per vertex, and where rows are long a warp per four units of all lists: the two
+// CTAs of K_{1000,1000}'s vertices took 480 us over its 8,000 units.  ACOCORE ranking with one / two / four / eight
+// units a warp: K_{1000,1000} 66 / 68 / 76 / 89 us, 3000 x 3000 with 1.4e6 edges 90 / 89 / 95 / 102 (203 by
+// vertices); the 46 COCORE rounds of a uniform graph with 1e6 edges 519 / 509 / 460 / 461, since a round's
+// barriers grow with the CTAs.
+constexpr int64_t kCoUnitsPerWarp = 4;
 constexpr unsigned long long kCoTimeoutNs = 60ull * 1000000000ull;
 
 // Grid barrier of a cooperative launch: arrivals are counted in a word that is never reset.
@@ -482,7 +488,8 @@ void vertex_order(const pb_graph& g, int rank_type, int use_v, Ranked& R, cudaSt
     CoWait wait{kCoTimeoutNs, 0};
     if (const char* e = getenv("PB_RANK_BARRIER_TIMEOUT_MS")) wait.timeout_ns = 1000000ull * strtoull(e, nullptr, 10);
     void* args[] = {&lists, &nn, &ap, &kp, &dp, &up, &ctl, &wait};
-    const int grid = std::max(1, std::min(sm_count(), ceil_div(n, kCoThreads)));
+    const int64_t unit_ctas = 2 * g.m / (kCoUnitsPerWarp * kCoUnit * (kCoThreads / 32));
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(sm_count(), std::max<int64_t>(ceil_div(n, kCoThreads), unit_ctas)));
     wait.arrivals = (unsigned)grid;
     // Test hook: no barrier completes, with 1 in any ranking, with 2 in captured graphs.
     if (const char* e = getenv("PB_RANK_TEST_STUCK_BARRIER")) wait.arrivals += *e == '1' || (*e == '2' && capturing());

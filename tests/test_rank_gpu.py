@@ -67,6 +67,20 @@ def test_long_runs_of_empty_rows(ctx, rank):
     dg.close()
 
 
+@pytest.mark.parametrize("a,b", [(1000, 1000), (257, 8000)])
+def test_few_vertices_with_long_lists(ctx, a, b):
+    """The lists of a few vertices are spread over the device, not over the CTAs that hold a thread per
+    vertex (the 8,000 units of K_{1000,1000} took two CTAs 0.48 ms; spread, 0.08)."""
+    g = BipartiteGraph.from_edges(a, b, np.repeat(np.arange(a), b), np.tile(np.arange(b), a))
+    dg = ctx.upload(g)
+    ms = []
+    for rank in ["ACOCORE", "COCORE"] * 4:
+        assert pb.count_total(dg, "HASH", rank) == (a * (a - 1) // 2) * (b * (b - 1) // 2)
+        ms.append(ctx.stats()["ms_rank"])
+    assert min(ms) < 0.25
+    dg.close()
+
+
 def test_barrier_timeout_reports_status_and_context_survives(ctx, monkeypatch):
     """A barrier wait of the co-core ranking that cannot complete (test hook) runs out after the
     configured bound: single calls and replays of a captured batch return PB_ETIMEOUT."""
