@@ -172,3 +172,19 @@ def _check_shifts(ctx, short_of_memory, left):
     want = np.array([sum(d - 1 - abs(j - k) for k in range(d) if k != j) for j in range(d)])
     assert (got[:n - 127 * d] == want).all() and int(got.sum()) == n * int(want.sum())
     dg.close()
+
+
+def test_tip_counters_follow_the_peeled_side(ctx, pool):
+    """Few vertices peeled against many: the heavy items' counters are slices of the peeled side (slices of
+    the longer one took 512 bytes a centre)."""
+    nv, nu = 400_000, 40
+    rng = np.random.default_rng(8)
+    g = BipartiteGraph.from_edges(nv, nu, rng.integers(0, nv, 1_000_000), rng.integers(0, nu, 1_000_000))
+    dg = ctx.upload(g)
+    counts = pb.count(dg, "BATCHS", "ADEG", use_v=True)
+    want = oracle.peel_vert(g, counts)[0]
+    for parts in (0, 8):
+        base = pool.reset()
+        assert np.array_equal(pb.peel(dg, counts, peel_parts=parts), want)
+        assert pool.high() - base < 128 * nv
+    dg.close()
