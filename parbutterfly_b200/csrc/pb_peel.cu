@@ -1856,8 +1856,19 @@ __device__ bool peel_instance(const Lists& G, const Work& W, Ctl* ctl, const Cla
 // heavy and the intersections need the warps.  Wing peel of R-MAT graphs, one against two CTAs:
 // 2^18 edges 186 / 213 ms, 2^20 566 / 643, 2^21 1040 / 1147, 2^22 2032 / 2122, 2^23 4167 / 4128,
 // 2^24 9248 / 8514.
+// Fewer edges take two as well where rounds are heavy, since edges alike are peeled together: the dearest edge
+// is within four times the mean of the estimated work, and the mean is not small; and where most work lies with
+// probe sets too long for shared memory, since probes wait for device memory.  One against two CTAs (in brackets
+// dearest / mean, mean, share of long sets):
+//   K_{60,3000} 118 / 81 ms (1, 180,000, 0), uniform 2000 x 2000 with 4e5 edges 61 / 47 (1.3, 35,000, 0),
+//   1500 x 1500 with 1e5 9.4 / 8.8 (1.4, 4,086, 0), 3000 x 3000 with 6e4 1.01 / 1.13 (2, 386, 0);
+//   four hubs of 20,000 39.7 / 26.4 (2.2, 35,600, 1.0), two 17.8 / 14.1 (10, 4,115, 0.9);
+//   Zipf with 3e5 edges 139 / 168 (20, 7,800, 0.05), R-MAT as above (12 to 24, 10,800 to 30,000, at most 0.01).
+// Asking takes a wait of the host, which is left out where edges are few or, by their degrees, cheap.
 // Batches keep two (more graphs at a time).
 constexpr int64_t kWingOneCta = int64_t(6) << 20;
+constexpr int64_t kWingAskSpread = int64_t(1) << 15;
+constexpr int64_t kWingHeavyMean = 2048;
 template <bool kWing, int kMinBlocks>
 __global__ void __launch_bounds__(kPT, kMinBlocks) peel_kernel(Lists G, const Lists* levels, Instances I, Ctl* ctls,
                                                                Classify cls) {
@@ -2111,6 +2122,29 @@ __global__ void total_weight_kernel(Lists G, Classify cls, int64_t N, unsigned l
   if ((threadIdx.x & 31) == 0 && s) atomicAdd(total, s);
 }
 
+// out: summed estimated work of all edges, of those with a probe set above kWingSet, and the largest.
+__global__ void wing_spread_kernel(Lists G, Classify cls, int64_t N, unsigned long long* out) {
+  unsigned long long all = 0, wide = 0, most = 0;
+  for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < N; x += (int64_t)gridDim.x * blockDim.x) {
+    const uint32_t v = G.center_of[x], u = G.u_of[x];
+    const int64_t cv = cls.cost_v(G, v, u), cu = cls.cost_u(G, v, u);
+    const int64_t psize = cv <= cu ? G.offK[u + 1] - G.offK[u] : G.offC[v + 1] - G.offC[v];
+    const unsigned long long w = item_weight<true>(G, cls, (uint32_t)x);
+    all += w;
+    if (psize > (int64_t)kWingSet) wide += w;
+    most = max(most, w);
+  }
+  all = warp_sum(all);
+  wide = warp_sum(wide);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+  if ((threadIdx.x & 31) == 0 && all) {
+    atomicAdd(out, all);
+    if (wide) atomicAdd(out + 1, wide);
+    atomicMax(out + 2, most);
+  }
+}
+
 // gid[x] = i for the items x in [base[i], base[i + 1]) (one CTA per range).
 __global__ void range_ids_kernel(const uint32_t* __restrict__ base, uint32_t n, const uint32_t* unused, uint32_t* gid) {
   const uint32_t i = blockIdx.x;
@@ -2356,7 +2390,19 @@ PeelResult run_peel(const pb_graph& g, int use_v, const int64_t* counts, int64_t
   if constexpr (!kWing) {
     if (!batch) kern = peel_kernel<false, 1>;
   } else {
-    if (!two_phase && g.m <= kWingOneCta) kern = peel_kernel<true, 1>;
+    bool one = !two_phase && g.m <= kWingOneCta;
+    // Two CTAs per SM double the markers of long probe sets; above 4 GiB that is not worth it.
+    const bool room = !need_scratch || 2 * (int64_t)sm_count() * scratch_len * 4 <= int64_t(4) << 30;
+    if (one && room && g.m > kWingAskSpread && (int64_t)g.max_deg * g.max_deg >= kWingHeavyMean) {
+      DevBuf<unsigned long long> spread(3, s);
+      PB_CUDA_TRY(cudaMemsetAsync(spread.get(), 0, spread.bytes(), s));
+      PB_LAUNCH(wing_spread_kernel, std::min(grid_for(N), 2 * sm_count()), 256, 0, s, G, cls, N, spread.get());
+      unsigned long long h[3];
+      readback(h, spread.get(), sizeof(h), s);
+      const double mean = (double)h[0] / (double)N;
+      one = h[1] <= h[0] / 2 && (mean < (double)kWingHeavyMean || (double)h[2] > 4.0 * mean);
+    }
+    if (one) kern = peel_kernel<true, 1>;
   }
   PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per_sm = 0;

@@ -59,3 +59,42 @@ def test_wing_rounds(ctx, monkeypatch, sizes, extra, small_work):
         c = pb.count_e(dg, "HASH", "ADEG", use_v=use_v)
         assert np.array_equal(pb.peel_e(dg, c, use_v=use_v), oracle.peel_edge(g, c, use_v=use_v)[0])
     dg.close()
+
+
+def _hubs(n, h, m, seed):
+    rng = np.random.default_rng(seed)
+    return BipartiteGraph.from_edges(n, n, np.r_[np.repeat(np.arange(h), n), rng.integers(0, n, m)],
+                                     np.r_[np.tile(np.arange(n), h), rng.integers(0, n, m)])
+
+
+@pytest.mark.parametrize("graph", [
+    lambda: _hubs(6000, 4, 40_000, 3),                      # most work with probe sets above 4,096 entries
+    lambda: _hubs(4096, 5, 30_000, 4),                      # probe sets of 4,096
+    lambda: BipartiteGraph.uniform(700, 500, 32_768, 5),    # even work, at and above the size from which it is looked at
+    lambda: BipartiteGraph.uniform(700, 500, 32_769, 5),
+])
+def test_wing_kernels_of_one_and_two_ctas(ctx, graph):
+    g = graph()
+    dg = ctx.upload(g)
+    c = pb.count_e(dg, "HASH", "ADEG")
+    assert np.array_equal(pb.peel_e(dg, c), oracle.peel_edge(g, c)[0])
+    dg.close()
+
+
+def test_wing_hubs_run_two_ctas_per_sm(ctx, monkeypatch):
+    """Hubs whose lists exceed shared memory: probes wait for device memory, so a CTA per SM (forced below) is
+    too few (39.7 ms against 26.4)."""
+    import torch
+    dg = ctx.upload(_hubs(20_000, 4, 100_000, 5))
+    c = pb.count_e(dg, "HASH", "ADEG")
+
+    def best():
+        runs = [(pb.peel_e(dg, c), ctx.stats()["ms_peel"]) for _ in range(4)]
+        return runs[0][0], min(t for _, t in runs)
+
+    out, ms = best()
+    monkeypatch.setenv("PB_PEEL_CTAS", str(torch.cuda.get_device_properties(0).multi_processor_count))
+    out_one, ms_one = best()
+    assert np.array_equal(out, out_one)
+    assert ms < 0.85 * ms_one
+    dg.close()
