@@ -98,3 +98,17 @@ def test_wing_hubs_run_two_ctas_per_sm(ctx, monkeypatch):
     assert np.array_equal(out, out_one)
     assert ms < 0.85 * ms_one
     dg.close()
+
+
+@pytest.mark.parametrize("few", [1, 8, 31, 32, 33, 63, 64])
+def test_tip_of_few_vertices(ctx, few):
+    """A handful of heavy vertices against many: slices of counters around multiples of a memory line, and
+    waves of all vertices."""
+    g = BipartiteGraph.uniform(few, 3000, 1500 * few, 12)
+    dg = ctx.upload(g)
+    for use_v in (False, True):
+        c = pb.count(dg, "BATCHS", "ADEG", use_v=use_v)
+        want = oracle.peel_vert(g, c, use_v=use_v)[0]
+        for parts in (0, 3):
+            assert np.array_equal(pb.peel(dg, c, use_v=use_v, peel_parts=parts), want)
+    dg.close()
